@@ -153,7 +153,7 @@ __device__ __forceinline__ void row_key_interval(int i, int seq_k, int window, i
   const bool lower = MK == FLEXATTN_MASK_SLIDING_WINDOW || MK == FLEXATTN_MASK_SLIDING_WINDOW_CAUSAL ||
                      MK == FLEXATTN_MASK_S2;  // j > i - window
   const bool upper = MK == FLEXATTN_MASK_CAUSAL || MK == FLEXATTN_MASK_SLIDING_WINDOW_CAUSAL || MK == FLEXATTN_MASK_S2;  // j <= i
-  klo = lower ? i - window + 1 : 0;
+  klo = lower && window <= i ? i - window + 1 : 0;  // (never near INT_MIN, where klo - j would wrap around)
   khi = upper ? (i + 1 < seq_k ? i + 1 : seq_k) : seq_k;
 }
 // S2: the stride grid's bits inside 32 columns when the first of them is on the grid (bit 0, stride, 2 stride ...).

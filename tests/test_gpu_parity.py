@@ -110,6 +110,19 @@ def test_s2_strides(window, stride, backend, dtype):
     assert_close(got, want, dtype, what=f"s2 {window}/{stride}/{backend}")
 
 
+@pytest.mark.parametrize("mask_kind", ["sliding_window", "sliding_window_causal"])
+@pytest.mark.parametrize("window", [515, 2**31 - 1])
+@pytest.mark.parametrize("backend,dtype", [("simt", torch.float32), ("tcgen05", torch.bfloat16)])
+def test_window_as_wide_as_the_row_or_an_int(mask_kind, window, backend, dtype):
+    """A window no row reaches the end of, up to the largest there is: the ragged last tile, which is always partial, keeps
+    the same pairs in the query rows' bitmaps (forward, dQ) as in the key rows' (dK/dV)."""
+    fa = _fa()
+    (q, k, v, do), host = make_qkvdo((1, 2, 515, 64), (1, 2, 515, 64), 78, dtype)
+    got = run_hot_path(fa, q, k, v, do, sm_scale=0.125, mask_kind=mask_kind, backend=backend, window=window)
+    want = oracle_hot_path(*host, sm_scale=0.125, mask_kind=mask_kind, window=window)
+    assert_close(got, want, dtype, what=f"{mask_kind} {window}/{backend}")
+
+
 @pytest.mark.parametrize("score_kind", ["none", "alibi", "softcap"])
 @pytest.mark.parametrize("mask_kind", sorted(MASKS))
 def test_simt_bfloat16(mask_kind, score_kind):
