@@ -191,7 +191,7 @@ POISON_OUTPUTS = os.environ.get("FLEXATTN_POISON_OUTPUTS", "0") not in ("", "0")
 
 class Problem:
     """One attention problem: shapes, score/mask spec and the tensors bound so far.  Owns the mask-map
-    workspace (a torch buffer) and rebuilds the map only when the mask inputs change."""
+    workspace (a torch buffer) and rebuilds the map only when the mask inputs or the stream change."""
 
     _map_cache: "OrderedDict[tuple, torch.Tensor]" = OrderedDict()
     _MAP_CACHE_ENTRIES = 16
@@ -307,23 +307,23 @@ class Problem:
         doc_key = None
         if self.doc_ids is not None:
             doc_key = (self.doc_ids.data_ptr(), self.doc_ids._version)
-        key = (self.device.index, p.mask_kind, p.window, p.stride, p.batch, p.seq_q, p.seq_k, doc_key)
+        # A map belongs to the stream it was built on: there it is complete before any kernel reads it, and an evicted buffer
+        # goes back to the pool of that stream, behind the kernels that still read it.  Another stream builds its own.
+        stream = _stream_ptr(self.device)
+        key = (self.device.index, stream, p.mask_kind, p.window, p.stride, p.batch, p.seq_q, p.seq_k, doc_key)
         cache = Problem._map_cache
-        hit = cache.get(key)
-        ws = None if hit is None else hit[0]
-        fresh = ws is None
+        entry = cache.pop(key, None)
+        fresh = entry is None
         if fresh:
-            ws = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
-        else:
-            cache.move_to_end(key)
-        p.workspace, p.workspace_bytes = ws.data_ptr(), nbytes
-        self.workspace = ws
-        if fresh:
-            check(lib.flexattn_build_mask_map(_stream_ptr(self.device), ctypes.byref(p)), "flexattn_build_mask_map")
             # the entry keeps the doc-id tensor alive, so its (pointer, version) key cannot be recycled
-            cache[key] = (ws, self.doc_ids)
-            while len(cache) > Problem._MAP_CACHE_ENTRIES:
-                cache.popitem(last=False)
+            entry = (torch.empty(nbytes, dtype=torch.uint8, device=self.device), self.doc_ids)
+        self.workspace = entry[0]
+        p.workspace, p.workspace_bytes = self.workspace.data_ptr(), nbytes
+        if fresh:
+            check(lib.flexattn_build_mask_map(stream, ctypes.byref(p)), "flexattn_build_mask_map")
+        cache[key] = entry   # at the end: the first entry is the one that was not used for longest
+        while len(cache) > Problem._MAP_CACHE_ENTRIES:
+            cache.popitem(last=False)
 
     def read_map(self, which: int, b: int, index: int):
         out = (ctypes.c_int32 * 4)()
