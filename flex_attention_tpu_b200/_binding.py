@@ -268,10 +268,12 @@ class Problem:
         self._bind_workspace()
 
     _slope_cache: "OrderedDict[tuple, torch.Tensor]" = OrderedDict()
+    _SLOPE_CACHE_ENTRIES = 64
 
     def _device_slopes(self, alibi_slopes, H):
         """[H] float32 slopes on the device.  Host values are uploaded once and cached: a pageable
-        host-to-device copy waits for the stream, which would serialise every call behind the last."""
+        host-to-device copy waits for the stream, which would serialise every call behind the last.
+        A copy belongs to its stream like a mask map does (`_bind_workspace`)."""
         if isinstance(alibi_slopes, torch.Tensor) and alibi_slopes.is_cuda:
             slopes = alibi_slopes.to(torch.float32).flatten()
             if slopes.numel() == 1:
@@ -279,8 +281,9 @@ class Problem:
             if slopes.numel() != H:
                 raise ValueError(f"need one ALiBi slope per head ({H}), got {slopes.numel()}")
             return slopes.contiguous()
+        cache, stream = Problem._slope_cache, _stream_ptr(self.device)
         if type(alibi_slopes) is tuple:   # the host values of a score spec: known after its first call
-            t = Problem._slope_cache.get((self.device.index, alibi_slopes))
+            t = cache.get((stream, self.device.index, alibi_slopes))
             if t is not None and t.numel() == H:
                 return t
         vals = tuple(float(x) for x in torch.as_tensor(alibi_slopes, dtype=torch.float32).flatten().tolist())
@@ -288,13 +291,13 @@ class Problem:
             vals = vals * H
         if len(vals) != H:
             raise ValueError(f"need one ALiBi slope per head ({H}), got {len(vals)}")
-        cache = Problem._slope_cache
-        t = cache.get((self.device.index, vals))
+        key = (stream, self.device.index, vals)
+        t = cache.get(key)
         if t is None:
-            t = cache[(self.device.index, vals)] = torch.tensor(vals, dtype=torch.float32).to(self.device)
+            t = cache[key] = torch.tensor(vals, dtype=torch.float32).to(self.device)
         if type(alibi_slopes) is tuple:
-            cache[(self.device.index, alibi_slopes)] = t
-        while len(cache) > 32:
+            cache[(stream, self.device.index, alibi_slopes)] = t
+        while len(cache) > Problem._SLOPE_CACHE_ENTRIES:
             cache.popitem(last=False)
         return t
 

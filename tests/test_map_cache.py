@@ -1,5 +1,5 @@
-"""The mask maps the binding keeps between calls, without a GPU: a fake library that only notes on which stream a map was
-built and into which buffer."""
+"""The mask maps and ALiBi slopes the binding keeps between calls, without a GPU: a fake library that only notes on which
+stream a map was built and into which buffer."""
 import ctypes
 from collections import OrderedDict
 
@@ -27,6 +27,7 @@ def host(monkeypatch):
     monkeypatch.setattr(B, "lib", h.lib)
     monkeypatch.setattr(B, "_stream_ptr", lambda device: h.stream)
     monkeypatch.setattr(B.Problem, "_map_cache", OrderedDict())
+    monkeypatch.setattr(B.Problem, "_slope_cache", OrderedDict())
     return h
 
 
@@ -70,3 +71,13 @@ def test_document_ids_changed_in_place_give_a_new_map(host):
     assert _bound(doc_ids=ids).p.workspace == first.p.workspace
     ids[0, 128:] = 1
     assert _bound(doc_ids=ids).p.workspace != first.p.workspace and len(host.lib.built) == 2
+
+
+def test_slopes_belong_to_the_stream_they_were_uploaded_on(host):
+    """An evicted copy goes back to the pool of its own stream, where nothing waits for the kernels of another."""
+    prob, slopes = _bound(), (0.5, 0.25)
+    a = prob._device_slopes(slopes, 2)
+    assert prob._device_slopes(slopes, 2) is a and a.tolist() == [0.5, 0.25]
+    host.stream = 8
+    b = prob._device_slopes(slopes, 2)
+    assert b is not a and b.tolist() == a.tolist() and prob._device_slopes([0.5, 0.25], 2) is b
