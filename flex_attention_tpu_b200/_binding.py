@@ -232,7 +232,9 @@ class Problem:
                 Problem._images[key] = bytes(p)
         else:
             p = FlexAttnParams.from_buffer_copy(image)
-        self._keep = {}  # tensors whose pointers sit in `p`, by field name
+        # Tensors of the problem itself whose pointers sit in `p`, by field name.  The tensors of a call are not among them:
+        # autograd keeps the problem with the graph of the output, so a problem that held its output would hold itself.
+        self._keep = {}
         if mask_kind == MASK_DOCUMENT:
             if doc_ids is None:
                 raise ValueError("document mask needs segment/doc ids")
@@ -336,7 +338,7 @@ class Problem:
 
     # ------------------------------------------------------------------ tensors
     def _bind(self, **tensors):
-        p, keep, device, dtype = self.p, self._keep, self.device, self.dtype
+        p, device, dtype = self.p, self.device, self.dtype
         for name, t in tensors.items():
             if t is None:
                 continue
@@ -348,7 +350,6 @@ class Problem:
             if t.dtype != want:
                 raise ValueError(f"{name} must be {want}, got {t.dtype}")
             setattr(p, name, t.data_ptr())
-            keep[name] = t
 
     def _new(self, shape, dtype=None):
         if POISON_OUTPUTS:
@@ -359,7 +360,6 @@ class Problem:
         B, H, Sq, D = self.shape_q
         o, l, m = self._new(self.shape_q), self._new((B, H, Sq), torch.float32), self._new((B, H, Sq), torch.float32)
         self._bind(q=q, k=k, v=v)
-        self._keep.update(o=o, l=l, m=m)
         self.p.o, self.p.l, self.p.m = o.data_ptr(), l.data_ptr(), m.data_ptr()
         check_user(lib.flexattn_fwd(_stream_ptr(self.device), ctypes.byref(self.p)), "flexattn_fwd", self.p.user_score)
         return o, l, m
@@ -415,7 +415,6 @@ class Problem:
         dq, dk, dv = self._new(self.shape_q), self._new(self.shape_k), self._new(self.shape_k)
         dab = self._new(self.ab.shape, torch.float32) if want_dab else None
         self._bind(q=q, k=k, v=v, o=o, d_o=do, l=l, m=m)
-        self._keep.update(delta=delta, dq=dq, dk=dk, dv=dv)
         p = self.p
         p.delta, p.dq, p.dk, p.dv = delta.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr()
         p.dab = dab.data_ptr() if want_dab else None
