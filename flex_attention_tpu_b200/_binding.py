@@ -138,8 +138,13 @@ def _device_index(device):
     return device.index if device.index is not None else torch.cuda.current_device()
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_capturing = torch.cuda.is_current_stream_capturing
+
+
 def _stream_ptr(device):
-    return torch._C._cuda_getCurrentRawStream(_device_index(device))
+    index = device.index
+    return _raw_stream(torch.cuda.current_device() if index is None else index)
 
 
 def _ptr(t):
@@ -195,6 +200,10 @@ class Problem:
 
     _map_cache: "OrderedDict[tuple, torch.Tensor]" = OrderedDict()
     _MAP_CACHE_ENTRIES = 16
+    # maps and slopes that captured graphs read: one of each, a few KB, kept for good (nobody tells when a graph has gone).
+    # Beyond this many a graph builds the map it reads.
+    _graph_held = {}
+    _GRAPH_HELD_ENTRIES = 256
     _images = {}   # sizes and options -> the parameter struct they give (no pointers in it): filling the fields one by one
                    # and asking for the workspace size costs a short call more than its launches
 
@@ -205,21 +214,21 @@ class Problem:
             raise ValueError("flex attention tensors must live on a CUDA device (no CPU path exists)")
         if q.dim() != 4 or k.dim() != 4:
             raise ValueError("expected [batch, heads, seq, head_dim] tensors")
-        if q.dtype not in (torch.bfloat16, torch.float32):
-            raise NotImplementedError(f"dtype {q.dtype} is not supported (bfloat16 or float32)")
-        self.device = q.device
-        self.dtype = q.dtype
-        B, H, Sq, D = q.shape
-        self.shape_q = (B, H, Sq, D)
-        self.shape_k = tuple(k.shape)
+        self.device, self.dtype, shape_q, shape_k = q.device, q.dtype, q.shape, k.shape
+        device, dtype = self.device, self.dtype
+        if dtype not in (torch.bfloat16, torch.float32):
+            raise NotImplementedError(f"dtype {dtype} is not supported (bfloat16 or float32)")
+        stream, capturing = _stream_ptr(device), _capturing()
+        B, H, Sq, D = self.shape_q = tuple(shape_q)
+        self.shape_k = tuple(shape_k)
+        Sk = shape_k[2]
         sm_scale, softcap, window, stride = float(sm_scale), float(softcap), int(window), int(stride)
-        key = (q.device, q.dtype, q.shape, k.shape[2], sm_scale, score_kind, softcap, mask_kind, window, stride, backend,
-               user_score)
+        key = (device, dtype, shape_q, Sk, sm_scale, score_kind, softcap, mask_kind, window, stride, backend, user_score)
         image = Problem._images.get(key)
         if image is None:
             p = FlexAttnParams()
-            p.batch, p.heads, p.seq_q, p.seq_k, p.head_dim = B, H, Sq, k.shape[2], D
-            p.dtype = DTYPE_BF16 if q.dtype == torch.bfloat16 else DTYPE_F32
+            p.batch, p.heads, p.seq_q, p.seq_k, p.head_dim = B, H, Sq, Sk, D
+            p.dtype = DTYPE_BF16 if dtype == torch.bfloat16 else DTYPE_F32
             p.sm_scale = sm_scale
             p.score_kind, p.softcap = int(score_kind), softcap
             p.mask_kind, p.window, p.stride = int(mask_kind), window, stride
@@ -241,38 +250,40 @@ class Problem:
             doc_ids = torch.as_tensor(doc_ids)
             if doc_ids.dim() == 1:
                 doc_ids = doc_ids[None].expand(B, -1)
-            doc_ids = doc_ids.to(device=self.device, dtype=torch.int32).contiguous()
-            if doc_ids.shape != (B, max(Sq, k.shape[2])):
-                raise ValueError(f"doc ids must be [batch, {max(Sq, k.shape[2])}], got {tuple(doc_ids.shape)}")
+            doc_ids = doc_ids.to(device=device, dtype=torch.int32).contiguous()
+            if doc_ids.shape != (B, max(Sq, Sk)):
+                raise ValueError(f"doc ids must be [batch, {max(Sq, Sk)}], got {tuple(doc_ids.shape)}")
             p.doc_ids = doc_ids.data_ptr()
             self._keep["doc_ids"] = doc_ids
         self.doc_ids = doc_ids if mask_kind == MASK_DOCUMENT else None
         if score_kind == SCORE_ALIBI:
-            slopes = self._device_slopes(alibi_slopes, H)
+            slopes = self._device_slopes(alibi_slopes, H, stream, capturing)
             p.alibi_slopes = slopes.data_ptr()
             self._keep["alibi_slopes"] = slopes
-        if status is None:
-            raise_if_failed(self.device)
-            status = _mailbox(self.device)
-        p.status = status.data_ptr()
+        own_status = status is None
+        if own_status:
+            status = _mailbox(device)
+        p.status = at = status.data_ptr()
+        if own_status and ctypes.c_int32.from_address(at).value != 0:
+            raise_if_failed(device)
         self._keep["status"] = status
         self.ab = None
         if ab is not None:
             # dense additive bias [B,H,Sq,Sk], float32
             if not (isinstance(ab, torch.Tensor) and ab.is_cuda):
                 raise ValueError("ab must be a CUDA tensor")
-            if tuple(ab.shape) != (B, H, Sq, k.shape[2]):
-                raise ValueError(f"Attention bias shape mismatch: expected {(B, H, Sq, k.shape[2])}, got {tuple(ab.shape)}")
+            if tuple(ab.shape) != (B, H, Sq, Sk):
+                raise ValueError(f"Attention bias shape mismatch: expected {(B, H, Sq, Sk)}, got {tuple(ab.shape)}")
             self.ab = ab.to(torch.float32).contiguous()
             p.ab = self.ab.data_ptr()
             self._keep["ab"] = self.ab
         self.p = p
-        self._bind_workspace()
+        self._bind_workspace(stream, capturing, (device.index, mask_kind, window, stride, B, Sq, Sk))
 
     _slope_cache: "OrderedDict[tuple, torch.Tensor]" = OrderedDict()
     _SLOPE_CACHE_ENTRIES = 64
 
-    def _device_slopes(self, alibi_slopes, H):
+    def _device_slopes(self, alibi_slopes, H, stream, capturing):
         """[H] float32 slopes on the device.  Host values are uploaded once and cached: a pageable
         host-to-device copy waits for the stream, which would serialise every call behind the last.
         A copy belongs to its stream like a mask map does (`_bind_workspace`)."""
@@ -283,9 +294,10 @@ class Problem:
             if slopes.numel() != H:
                 raise ValueError(f"need one ALiBi slope per head ({H}), got {slopes.numel()}")
             return slopes.contiguous()
-        cache, stream = Problem._slope_cache, _stream_ptr(self.device)
+        cache = Problem._slope_cache
+        find = Problem._hold_for_graph if capturing else OrderedDict.get
         if type(alibi_slopes) is tuple:   # the host values of a score spec: known after its first call
-            t = cache.get((stream, self.device.index, alibi_slopes))
+            t = find(cache, (stream, self.device.index, alibi_slopes))
             if t is not None and t.numel() == H:
                 return t
         vals = tuple(float(x) for x in torch.as_tensor(alibi_slopes, dtype=torch.float32).flatten().tolist())
@@ -294,7 +306,7 @@ class Problem:
         if len(vals) != H:
             raise ValueError(f"need one ALiBi slope per head ({H}), got {len(vals)}")
         key = (stream, self.device.index, vals)
-        t = cache.get(key)
+        t = find(cache, key)
         if t is None:
             t = cache[key] = torch.tensor(vals, dtype=torch.float32).to(self.device)
         if type(alibi_slopes) is tuple:
@@ -304,7 +316,8 @@ class Problem:
         return t
 
     # ------------------------------------------------------------------ mask map
-    def _bind_workspace(self):
+    def _bind_workspace(self, stream, capturing, sizes):
+        """The workspace with the mask map, which depends on `sizes` and, for documents, on the ids."""
         p = self.p
         nbytes = p.workspace_bytes
         if nbytes == 0:
@@ -314,21 +327,43 @@ class Problem:
             doc_key = (self.doc_ids.data_ptr(), self.doc_ids._version)
         # A map belongs to the stream it was built on: there it is complete before any kernel reads it, and an evicted buffer
         # goes back to the pool of that stream, behind the kernels that still read it.  Another stream builds its own.
-        stream = _stream_ptr(self.device)
-        key = (self.device.index, stream, p.mask_kind, p.window, p.stride, p.batch, p.seq_q, p.seq_k, doc_key)
+        key = (stream, *sizes, doc_key)
         cache = Problem._map_cache
-        entry = cache.pop(key, None)
+        # Under capture a map of document ids is part of the graph: a replay reads the ids it finds.  So is a map that has not
+        # been built before, and no later call may take it for a finished one.
+        if capturing:
+            entry = None if doc_key is not None else self._hold_for_graph(cache, key)
+        else:
+            entry = cache.get(key)
+            if entry is not None:
+                try:
+                    cache.move_to_end(key)
+                except KeyError:   # another thread has just evicted it
+                    pass
         fresh = entry is None
         if fresh:
             # the entry keeps the doc-id tensor alive, so its (pointer, version) key cannot be recycled
             entry = (torch.empty(nbytes, dtype=torch.uint8, device=self.device), self.doc_ids)
         self.workspace = entry[0]
-        p.workspace, p.workspace_bytes = self.workspace.data_ptr(), nbytes
+        p.workspace = self.workspace.data_ptr()
         if fresh:
             check(lib.flexattn_build_mask_map(stream, ctypes.byref(p)), "flexattn_build_mask_map")
-        cache[key] = entry   # at the end: the first entry is the one that was not used for longest
-        while len(cache) > Problem._MAP_CACHE_ENTRIES:
-            cache.popitem(last=False)
+            if not capturing:
+                cache[key] = entry
+                while len(cache) > Problem._MAP_CACHE_ENTRIES:
+                    cache.popitem(last=False)
+
+    @staticmethod
+    def _hold_for_graph(cache, key):
+        """The entry under `key` that a call outside the capture has made, on whatever stream (work enqueued before the
+        capture comes before the replays), or None.  It outlives the cache from here on."""
+        held, what = Problem._graph_held, (cache is Problem._map_cache, *key[1:])
+        entry = held.get(what)
+        if entry is None and (not what[0] or len(held) < Problem._GRAPH_HELD_ENTRIES):
+            entry = next((e for k, e in list(cache.items()) if k[1:] == key[1:]), None)
+            if entry is not None:
+                held[what] = entry
+        return entry
 
     def read_map(self, which: int, b: int, index: int):
         out = (ctypes.c_int32 * 4)()
@@ -338,12 +373,12 @@ class Problem:
 
     # ------------------------------------------------------------------ tensors
     def _bind(self, **tensors):
-        p, device, dtype = self.p, self.device, self.dtype
+        p, dtype, index = self.p, self.dtype, self.device.index
         for name, t in tensors.items():
             if t is None:
                 continue
-            if t.device != device:
-                raise ValueError(f"{name} must be on {device}")
+            if t.get_device() != index:
+                raise ValueError(f"{name} must be on {self.device}")
             if not t.is_contiguous():
                 raise ValueError(f"{name} must be contiguous")
             want = torch.float32 if name in ("l", "m", "delta") else dtype

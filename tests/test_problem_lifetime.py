@@ -23,6 +23,7 @@ def prob(monkeypatch):
     monkeypatch.setattr(B, "_stream_ptr", lambda device: 7)
     monkeypatch.setattr(B, "TWO_STREAM_BACKWARD", False)
     p = object.__new__(B.Problem)
+    monkeypatch.setattr(torch.Tensor, "get_device", lambda t: None)   # what a CPU device's index is
     p.device, p.dtype, p.shape_q, p.shape_k = torch.device("cpu"), torch.bfloat16, (1, 2, 8, 64), (1, 2, 8, 64)
     p.p, p._keep, p.ab = B.FlexAttnParams(), {}, None
     return p
