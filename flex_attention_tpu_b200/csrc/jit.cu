@@ -287,6 +287,8 @@ extern "C" int flexattn_user_score_compile(int32_t handle, int which, int32_t he
   std::lock_guard<std::mutex> lock(g_mu);
   UserScore* u = find(handle);
   if (u == nullptr) return FLEXATTN_ERR_UNSUPPORTED_MOD;
+  // both forms a launch may ask for (the forward for long rows takes no dense bias)
   const Compiled* c = nullptr;
-  return compile_locked(u, which, false, head_dim, mask_kind, &c);
+  const int e = compile_locked(u, which, false, head_dim, mask_kind, &c);
+  return e != FLEXATTN_OK || which == 3 ? e : compile_locked(u, which, true, head_dim, mask_kind, &c);
 }

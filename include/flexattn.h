@@ -231,8 +231,8 @@ int flexattn_user_score_destroy(int32_t handle);
  * that uses the handle.  Never NULL. */
 const char* flexattn_user_score_log(int32_t handle);
 /* Compiles (without loading or launching: needs no GPU) the kernel `which` (0 forward, 1 dQ, 2 dK/dV, 3 forward for long rows) for the
- * handle, head_dim and mask_kind, exactly as the first launch would.  Returns FLEXATTN_OK, or
- * FLEXATTN_ERR_JIT_COMPILE / FLEXATTN_ERR_JIT_UNAVAILABLE.  A test and warm-up hook. */
+ * handle, head_dim and mask_kind, exactly as the first launch would: the form without and, but for 3, the form with a dense
+ * bias.  Returns FLEXATTN_OK, or FLEXATTN_ERR_JIT_COMPILE / FLEXATTN_ERR_JIT_UNAVAILABLE.  A test and warm-up hook. */
 int flexattn_user_score_compile(int32_t handle, int which, int32_t head_dim, int32_t mask_kind);
 
 /* Clears the calling device's abort word (stream-ordered memset on `stream`), re-enabling the tensor-core

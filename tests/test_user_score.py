@@ -81,3 +81,18 @@ def test_kernels_compile_around_a_user_function_without_a_gpu():
     p = B.FlexAttnParams()
     p.batch, p.heads, p.seq_q, p.seq_k, p.head_dim, p.score_kind = 1, 1, 128, 128, 128, B.SCORE_USER
     assert B.lib.flexattn_fwd(None, ctypes.byref(p)) == 7          # no handle
+
+
+def test_the_warm_up_hook_compiles_the_dense_bias_form_as_well():
+    """A launch with a dense bias uses a form compiled for it: a program that warmed its handle up must not find the compiler
+    in that launch.  The score function here is one that only this form cannot compile."""
+    from flex_attention_tpu_b200 import _binding as B
+    h = ctypes.c_int32(0)
+    expr = b"s + 0.0f * (float)sizeof(char[FLEXATTN_DENSE_BIAS ? -1 : 1])"
+    assert B.lib.flexattn_user_score_create(expr, b"1.0f", ctypes.byref(h)) == 0
+    codes = [B.lib.flexattn_user_score_compile(h.value, which, 64, B.MASK_NONE) for which in (0, 1, 2, 3)]
+    log = B.lib.flexattn_user_score_log(h.value)
+    B.lib.flexattn_user_score_destroy(h.value)
+    if 12 in codes:
+        pytest.skip("libnvrtc is not installed here")
+    assert codes == [13, 13, 13, 0], log.decode()      # (the forward for long rows has no such form)
