@@ -249,7 +249,9 @@ int flexattn_fwd(void* stream, const FlexAttnParams* p) {
     const int forced = forced_fwd_kernel();
     if (forced == 0 || forced == 3) {
       d.kv_splits = kv_splits(p);
-      if (forced == 3 && d.kv_splits == 0 && pair_can && p->score_kind != FLEXATTN_SCORE_USER) d.kv_splits = 1;
+      if (forced == 3 && d.kv_splits == 0 && pair_can && p->score_kind != FLEXATTN_SCORE_USER &&
+          p->mask_kind != FLEXATTN_MASK_DOCUMENT)
+        d.kv_splits = 1;
       if (d.kv_splits > 0) return launch_sm100_fwd_split(st, d, p->score_kind, p->mask_kind);
     }
     if (pair_can && (forced == 1 || (forced == 0 && mean_kv_tiles(p) >= kPairMinTiles && pair_pays(p))))

@@ -8,6 +8,7 @@
 //   * inside a CTA over two online-softmax streams, even and odd tiles of the chunk, each with a warpgroup, a score buffer
 //     and an accumulator of its own (thread t owns query row t, as in fwd_pair_sm100.cu): while one stream computes
 //     exponentials the tensor core works for the other.
+// Every mask but documents, whose tile counts are only known on the device: the launch is sized before.
 // The partial results (running maximum, sum, unnormalised O in f32) of all streams meet at the end through distributed
 // shared memory: CTA r of the cluster merges every C-th row, so no workspace and no second launch are needed.
 //
@@ -29,7 +30,6 @@ struct SplitSmem {
   uint64_t bar_q, bar_k[kMaxStages], bar_v[kMaxStages], bar_kfree[kMaxStages], bar_vfree[kMaxStages], bar_s[2], bar_p[2], bar_pv[2];
   uint32_t tmem_base;
   int32_t dead;            // the abort word was set on entry
-  int32_t doc[2][kTile];   // per stream: document ids of the kv tile being processed
 };
 
 __device__ __forceinline__ void cluster_sync() {
@@ -215,27 +215,14 @@ __global__ void __launch_bounds__(kThreads, 1)
     const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     const uint32_t colS = kColS + (uint32_t)s * 128u, colO = kColO + (uint32_t)s * 128u;
     const float c2 = P.sm_scale * kLog2e;
-    const long long n_rows = (long long)slices * P.seq_q, n_doc = (long long)P.batch * P.doc_stride;
     const float slope2 = (SK == FLEXATTN_SCORE_ALIBI && FLEXATTN_DBG_OK(h, P.heads, 6, 601)) ? P.alibi_slopes[h] * kLog2e : 0.f;
     const float capl2 = P.cap * kLog2e;
     const float csc = (SK == FLEXATTN_SCORE_SOFTCAP) ? P.sm_scale / P.cap : 0.f;
-    const int32_t* doc = (MK == FLEXATTN_MASK_DOCUMENT) ? P.doc_ids + (size_t)b * P.doc_stride : nullptr;
-    const int di = (MK == FLEXATTN_MASK_DOCUMENT && i < P.seq_q && FLEXATTN_DBG_OK((long long)b * P.doc_stride + i, n_doc, 6, 602))
-                       ? doc[i] : 0;
     float m_ref = kMasked, m_true = kMasked, l = 0.f;
     const ScoreCtx ctx{P.sm_scale, b, h};
-    constexpr bool kDoc = MK == FLEXATTN_MASK_DOCUMENT;
-    bool doc_runs = false;
-    int klo = 0, khi = P.seq_k;  // the row's interval of kept keys, where the mask has one
+    int klo = 0, khi = P.seq_k;  // the row's interval of kept keys
     const uint32_t pattern = MK == FLEXATTN_MASK_S2 ? stride_pattern32(P.stride) : 0u;
-    if constexpr (kMaskIsBits<MK>) row_key_interval<MK>(i, P.seq_k, P.window, klo, khi);
-    if constexpr (kDoc) {
-      doc_runs = FLEXATTN_DBG_OK(b, P.batch, 6, 606) && P.doc_sorted[b] != 0;
-      if (doc_runs && i < P.seq_q && FLEXATTN_DBG_OK((long long)b * P.doc_stride + i, n_doc, 6, 607)) {
-        klo = P.run_lo[(size_t)b * P.doc_stride + i];
-        khi = i + 1 < P.seq_k ? i + 1 : P.seq_k;
-      }
-    }
+    row_key_interval<MK>(i, P.seq_k, P.window, klo, khi);
     bool ok = !dead;
     int fail_at = 0;
     const int N = (NT - s + 1) / 2;  // tiles s, s + 2, ... of the chunk
@@ -243,13 +230,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       const uint32_t par = n & 1;
       const int kt = kv_tile_at<SK>(lo, hi, 2 * n + s), j0 = kt * kTile;
       const bool partial = !(kt >= rm.z && kt < rm.w);
-      if (MK == FLEXATTN_MASK_DOCUMENT && partial && !doc_runs) {
-        ptx::named_bar_sync(1 + s, 128);  // readers of the previous partial tile are done
-        const int j = j0 + row;
-        sh->doc[s][row] = (j < P.seq_k && FLEXATTN_DBG_OK((long long)b * P.doc_stride + j, n_doc, 6, 603)) ? doc[j] : -1;
-        ptx::named_bar_sync(1 + s, 128);
-      }
-      // a failed wait never leaves the loop early: every thread keeps executing the same named barriers
+      // a failed wait never leaves the loop early: every thread gets to the barrier behind it
       if (ok) {
         ok = __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_s[s], par));
         if (!ok) fail_at = 10;
@@ -277,19 +258,10 @@ __global__ void __launch_bounds__(kThreads, 1)
       // scores and folds sm_scale*log2e into the FMA that also subtracts the running max)
       float tmax, xs = 1.0f;
       if (partial) {
-        if constexpr (kDoc) {
-          if (doc_runs)
-            tmax = score_row<SK, MK, true, true>(x, i, j0, P.seq_k, P.window, P.stride, c2, slope2, capl2, csc, di, sh->doc[s],
-                                                 ctx, klo, khi, pattern);
-          else
-            tmax = score_row<SK, MK, true, false>(x, i, j0, P.seq_k, P.window, P.stride, c2, slope2, capl2, csc, di,
-                                                  sh->doc[s], ctx);
-        } else {
-          tmax = score_row<SK, MK, true>(x, i, j0, P.seq_k, P.window, P.stride, c2, slope2, capl2, csc, di, sh->doc[s], ctx,
-                                         klo, khi, pattern);
-        }
+        tmax = score_row<SK, MK, true>(x, i, j0, P.seq_k, P.window, P.stride, c2, slope2, capl2, csc, 0, nullptr, ctx, klo, khi,
+                                       pattern);
       } else if constexpr (SK != FLEXATTN_SCORE_NONE) {
-        tmax = score_row<SK, MK, false>(x, i, j0, P.seq_k, P.window, P.stride, c2, slope2, capl2, csc, di, sh->doc[s], ctx);
+        tmax = score_row<SK, MK, false>(x, i, j0, P.seq_k, P.window, P.stride, c2, slope2, capl2, csc, 0, nullptr, ctx);
       } else {
         float mx[4] = {x[0], x[1], x[2], x[3]};
 #pragma unroll
@@ -479,7 +451,6 @@ int launch_mask(cudaStream_t st, const DevParams& d, int mask, const CUtensorMap
     case FLEXATTN_MASK_SLIDING_WINDOW: return launch_one<D, SK, FLEXATTN_MASK_SLIDING_WINDOW>(st, d, tq, tk, tv, af);
     case FLEXATTN_MASK_SLIDING_WINDOW_CAUSAL:
       return launch_one<D, SK, FLEXATTN_MASK_SLIDING_WINDOW_CAUSAL>(st, d, tq, tk, tv, af);
-    case FLEXATTN_MASK_DOCUMENT: return launch_one<D, SK, FLEXATTN_MASK_DOCUMENT>(st, d, tq, tk, tv, af);
     case FLEXATTN_MASK_S2: return launch_one<D, SK, FLEXATTN_MASK_S2>(st, d, tq, tk, tv, af);
     default: return FLEXATTN_ERR_UNSUPPORTED_MOD;
   }

@@ -58,10 +58,10 @@ CHILD = textwrap.dedent("""
 """)
 
 
-@pytest.mark.parametrize("fwd_kernel", ["", "pair"])
+@pytest.mark.parametrize("fwd_kernel", ["", "pair", "split"])
 def test_bounds_checked_build_reports_nothing_and_matches_the_oracle(fwd_kernel):
     env = dict(os.environ, FLEXATTN_DEBUG="1")
-    if fwd_kernel:  # the forward kernel for long rows, forced onto these short ones (where it can run)
+    if fwd_kernel:  # a forward kernel for long rows, forced onto these short ones (where it can run)
         env["FLEXATTN_FWD_KERNEL"] = fwd_kernel
     r = subprocess.run([sys.executable, "-c", CHILD % (ROOT, os.path.join(ROOT, "tests"))], capture_output=True, text=True,
                        timeout=900, env=env)
