@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 import torch
 
-from helpers import assert_close, make_qkvdo, oracle_hot_path, run_hot_path
+from helpers import assert_close, build_mods, errors, make_qkvdo, oracle_hot_path, run_hot_path
 from oracle import mha_reference_cpu as oracle
 
 pytestmark = pytest.mark.gpu
@@ -25,7 +25,8 @@ def _reference_form(q_tile, k_tile):
     return se.where(x >= 0.0, x, 0.5 * x) + 0.1 * se.sigmoid(x)
 
 
-# (the 1700-key unmasked and the 3300-key causal case are long enough for the two-query-tile forward kernel)
+# (all on the persistent forward kernel: the two-query-tile one takes long rows of many slices, and is forced around a user
+# function in test_gpu_fwd_kernels.py)
 CASES = [("softcap", _softcap, "causal", 128, 777), ("distance", _distance_and_head, "none", 128, 500),
          ("distance", _distance_and_head, "document", 64, 700), ("leaky", _reference_form, "sliding_window_causal", 128, 640),
          ("distance", _distance_and_head, "none", 128, 1700), ("softcap", _softcap, "causal", 64, 3300)]
@@ -67,3 +68,31 @@ def test_user_score_needs_the_tensor_core_kernels():
     sf = fa.util.make_jax_score_fn(_softcap)
     with pytest.raises(FlexAttnError):      # float32 inputs run on the CUDA-core kernels, which have no compiled user path
         fa._flex_attention_impl(q, q, q, None, None, True, True, 1.0, 1, 128, 128, 128, False, None, None, sf)
+
+
+@pytest.mark.parametrize("mask_kind,Sq,Sk,D", [("causal", 500, 500, 64), ("none", 300, 433, 128)])
+def test_user_score_with_a_dense_bias(mask_kind, Sq, Sk, D):
+    """The forms of the three kernels that are compiled at run time with a dense bias, which joins the user's score."""
+    import flex_attention_tpu_b200 as fa
+    B, H, sm = 1, 2, 1.0 / np.sqrt(D)
+    (q, k, v, do), host = make_qkvdo((B, H, Sq, D), (B, H, Sk, D), 1400 + Sq, torch.bfloat16)
+    ab_h = (0.7 * np.random.default_rng(9).standard_normal((B, H, Sq, Sk))).astype(np.float32)
+    ab = torch.from_numpy(ab_h).cuda()
+    mf, bf, sf, _ = build_mods(fa, mask_kind, "user", user_fn=_distance_and_head)
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    o, l, m = fa._flex_attention_impl(q, k, v, ab, None, True, False, sm, 1, 128, 128, 128, False, bf, mf, sf, status=status)
+    delta = fa.bwd_preprocess(o, do)
+    dq, dab = fa.flex_attention_bwd_dq(q, k, v, ab, None, l, m, o, do, delta, sm_scale=sm, score_fn=sf, mask_fn=mf,
+                                       block_mask_fn=bf, return_dab=True, status=status)
+    dk, dv = fa.flash_attention_bwd_dkv(k, v, q, ab, None, l, m, delta, do, sm_scale=sm, score_fn=sf, mask_fn=mf,
+                                        block_mask_fn=bf, status=status)
+    torch.cuda.synchronize()
+    assert status.tolist() == [0, 0, 0, 0], status.tolist()
+    kw = dict(sm_scale=sm, mask_kind=mask_kind, score_kind="user", user=(sf, sf.dscore))
+    qh, kh, vh, doh = host
+    ro, rl, rm = oracle.mha_reference(qh, kh, vh, ab_h, save_residuals=True, **kw)
+    rdq, rdk, rdv, rdab = oracle.mha_bwd_reference(qh, kh, vh, ro, doh, rl, rm, ab_h, return_dab=True, **kw)
+    assert_close(dict(o=o, l=l, m=m, dq=dq, dk=dk, dv=dv), dict(o=ro, l=rl, m=rm, dq=rdq, dk=rdk, dv=rdv), torch.bfloat16,
+                 what=f"user score with bias {mask_kind}/D{D}")
+    e = errors(dab, rdab)   # float32, but delta comes from the bf16-rounded o: the relative bound of the bias tests
+    assert e["max_rel"] <= 1e-2, e
