@@ -27,7 +27,7 @@
 
 
 // The dense-bias form of this kernel is compiled from the same text in a file of its own (bwd_dq_bias_sm100.cu): with the bias decided at run
-// time, its registers and branches cost the ordinary form 2-4 %.
+// time, its registers and branches cost the ordinary kernels 2-7 %.
 #ifndef FLEXATTN_DENSE_BIAS
 #define FLEXATTN_DENSE_BIAS 0
 #endif

@@ -8,9 +8,9 @@
 // per-tile barrier between warpgroups; K and V are loaded once for both tiles.
 //
 //   warps 0..3 / 4..7 : softmax of stream A / B (registers raised to 208 per thread).
-//   warp 8, lane 0    : MMA issuer of both streams: O_s += P_s V, then S_s = Q_s K_next^T over the columns P_s
+//   warp 8, one thread: MMA issuer of both streams: O_s += P_s V, then S_s = Q_s K_next^T over the columns P_s
 //                       occupied (MMAs of one thread execute in issue order).
-//   warp 9, lane 0    : TMA producer: Q_A, Q_B once, K and V through two-stage rings.
+//   warp 9, one thread: TMA producer: Q_A, Q_B once, K and V through two-stage rings.
 //   warps 10, 11      : idle (they complete the warpgroup whose registers are lowered to 88).
 //
 // Tensor memory: S_A, S_B, O_A, O_B = 4 x 128 columns.  Shared memory: Q_A, Q_B (reused to stage the outputs),

@@ -8,11 +8,12 @@
 // of the next item start while the softmax and the epilogue of the current one are still running, and the
 // per-item prologue (loads in flight, first scores) and epilogue (normalise, store) cost no tensor-core time.
 //
-//   warp 8, lane 0 : MMA issuer.  S[T % 3] = Q K[T]^T runs up to three kv tiles ahead of the softmax;
+//   warps 8, 9, 10 : one elected thread each.
+//   warp 8         : MMA issuer.  S[T % 3] = Q K[T]^T runs up to three kv tiles ahead of the softmax;
 //                    O += P[T] V[T] is issued as soon as the softmax has written P[T] over S[T % 3].
-//   warp 9, lane 0 : TMA producer for Q (one buffer: the next item's Q is loaded as soon as the last Q K^T of the
+//   warp 9         : TMA producer for Q (one buffer: the next item's Q is loaded as soon as the last Q K^T of the
 //                    current item has run, three tiles before its softmax ends) and K (two-stage ring).
-//   warp 10, lane 0: TMA producer for V (two-stage ring).  Each ring stage is refilled as soon as the MMA that
+//   warp 10        : TMA producer for V (two-stage ring).  Each ring stage is refilled as soon as the MMA that
 //                    read it has completed (tcgen05.commit -> mbarrier).
 //   warps 0..7     : softmax, two warpgroups.  Threads t and t + 128 share query row t (= TMEM lane t)
 //                    and take one 64-column half of every score tile each; partial row maxima are
@@ -25,10 +26,10 @@
 // Tensor memory: S0, S1, S2 (3 x 128 columns) + O (D columns) = 512 for D = 128.  Shared memory: Q, an output
 // staging tile, 2 K and 2 V tiles (192 KB for D = 128).
 #include "sched.cuh"
-#include "sm100.cuh"
+#include "score_row.cuh"
 
 // The dense-bias form of this kernel is compiled from the same text in a file of its own (fwd_pipe_bias_sm100.cu): with the bias decided at run
-// time, its registers and branches cost the ordinary form 2-4 %.
+// time, its registers and branches cost the ordinary kernels 2-7 %.
 #ifndef FLEXATTN_DENSE_BIAS
 #define FLEXATTN_DENSE_BIAS 0
 #endif
@@ -42,16 +43,6 @@ constexpr int kThreads = 352;
 constexpr int kMmaWarp = 8, kTmaWarp = 9, kTmaWarpV = 10;
 constexpr int kHalf = kTile / 2;
 constexpr int kSBufs = 3;
-
-// Order in which an item's kv tiles are visited.  The ALiBi bias slope * (k_idx - q_idx) grows with the key
-// position, so in ascending order the running row maximum of a steep head rises by more than the lazy-rescale
-// threshold at EVERY tile, and each rescale waits for the previous P V and rewrites O.  Visiting the tiles from the
-// last one down meets the largest bias first and rescales (almost) never; other score kinds keep ascending order.
-template <int SK>
-__device__ __forceinline__ int kv_tile_at(int first, int end, int n) {
-  return SK == FLEXATTN_SCORE_ALIBI ? end - 1 - n : first + n;
-}
-constexpr float kLazyRescale = 8.0f;  // log2 units
 
 constexpr int kBiasScratch = 8 * 4 * ptx::kBiasScratchWords;  // bytes: a block of the dense bias per softmax warp
 
@@ -67,12 +58,6 @@ struct PipeSmem {
 // x: this thread's 64 raw scores (columns c_base .. c_base+63 of the tile) -> log2-domain logits in place;
 // returns their maximum.  kBias: the dense bias, read 16 columns at a time through the warp's scratch, is added after the score
 // function and before the mask.
-// what a user score function sees besides the score and the positions
-struct ScoreCtx {
-  float sm_scale;
-  int b, h;
-};
-
 // kInterval: the row's kept keys are the interval [klo, khi) (interval mask kinds; documents over sorted ids): a
 // partial tile then tests one bit per element of a bitmap built once per 32 columns.
 template <int SK, int MK, bool kPartial, bool kBias = false, bool kInterval = kMaskIsBits<MK>>

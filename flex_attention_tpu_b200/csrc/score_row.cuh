@@ -1,4 +1,5 @@
-// One thread = one query row: the scores of a 128-column tile, shared by the forward kernels that work that way.
+// What the forward kernels share: the order of an item's kv tiles, and the scores of a 128-column tile where one thread is
+// one query row.
 #pragma once
 #include "sm100.cuh"
 
@@ -7,8 +8,10 @@ namespace FLEXATTN_TU_NAMESPACE {
 
 constexpr float kLazyRescale = 8.0f;  // log2 units
 
-// kv tile visited at step n of the range [first, end): from the last one down under ALiBi (the bias grows with the
-// key position, so the running maximum is met first and the lazy rescale almost never fires), ascending otherwise.
+// kv tile visited at step n of the range [first, end).  The ALiBi bias slope * (k_idx - q_idx) grows with the key
+// position, so in ascending order the running row maximum of a steep head rises by more than the lazy-rescale
+// threshold at EVERY tile, and each rescale waits for the previous P V and rewrites O.  Visiting the tiles from the
+// last one down meets the largest bias first and rescales (almost) never; other score kinds keep ascending order.
 template <int SK>
 __device__ __forceinline__ int kv_tile_at(int first, int end, int n) {
   return SK == FLEXATTN_SCORE_ALIBI ? end - 1 - n : first + n;
