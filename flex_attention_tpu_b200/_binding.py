@@ -73,6 +73,10 @@ def _load():
         fn.argtypes = [ctypes.c_void_p, P]
     lib.flexattn_bwd.restype = ctypes.c_int
     lib.flexattn_bwd.argtypes = [ctypes.c_void_p, ctypes.c_void_p, P]
+    lib.flexattn_bwd_scratch_bytes.restype = ctypes.c_size_t
+    lib.flexattn_bwd_scratch_bytes.argtypes = [P]
+    lib.flexattn_bwd_fused.restype = ctypes.c_int
+    lib.flexattn_bwd_fused.argtypes = [ctypes.c_void_p, P, ctypes.c_void_p, ctypes.c_size_t]
     lib.flexattn_fwd_noalloc.restype = ctypes.c_int
     lib.flexattn_fwd_noalloc.argtypes = [ctypes.c_void_p, P]
     lib.flexattn_noalloc_scratch_bytes.restype = ctypes.c_size_t
@@ -235,12 +239,13 @@ class Problem:
             p.backend = int(backend)
             p.user_score = int(user_score)
             p.workspace_bytes = lib.flexattn_workspace_bytes(ctypes.byref(p))
+            self._bwd_scratch = lib.flexattn_bwd_scratch_bytes(ctypes.byref(p))
             if p.workspace_bytes:
                 if len(Problem._images) >= 256:
                     Problem._images.clear()
-                Problem._images[key] = bytes(p)
+                Problem._images[key] = bytes(p), self._bwd_scratch
         else:
-            p = FlexAttnParams.from_buffer_copy(image)
+            p, self._bwd_scratch = FlexAttnParams.from_buffer_copy(image[0]), image[1]
         # Tensors of the problem itself whose pointers sit in `p`, by field name.  The tensors of a call are not among them:
         # autograd keeps the problem with the graph of the output, so a problem that held its output would hold itself.
         self._keep = {}
@@ -454,6 +459,11 @@ class Problem:
         p.delta, p.dq, p.dk, p.dv = delta.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr()
         p.dab = dab.data_ptr() if want_dab else None
         stream = _stream_ptr(self.device)
+        if self._bwd_scratch and self.ab is None:
+            scratch = torch.empty(self._bwd_scratch, dtype=torch.uint8, device=self.device)
+            check_user(lib.flexattn_bwd_fused(stream, ctypes.byref(p), scratch.data_ptr(), self._bwd_scratch),
+                       "flexattn_bwd_fused", p.user_score)
+            return delta, dq, dk, dv
         side = _side_stream(self.device).cuda_stream if two_streams else stream
         try:
             check_user(lib.flexattn_bwd(stream, side, ctypes.byref(p)), "flexattn_bwd", p.user_score)

@@ -44,7 +44,7 @@ def _stamp(src):
 
 
 # sources the library carries as text: a user score function is compiled into these kernels at run time (csrc/jit.cu)
-EMBEDDED = ["fwd_pipe_sm100.cu", "bwd_dq_sm100.cu", "bwd_dkv_sm100.cu", "fwd_pair_sm100.cu", "sched.cuh", "score_row.cuh", "sm100.cuh",
+EMBEDDED = ["fwd_pipe_sm100.cu", "bwd_dq_sm100.cu", "bwd_dkv_sm100.cu", "bwd_fused_sm100.cu", "fwd_pair_sm100.cu", "sched.cuh", "score_row.cuh", "sm100.cuh",
             "common.cuh",
             os.path.join("..", "..", "include", "flexattn.h")]
 

@@ -341,6 +341,45 @@ int flexattn_bwd(void* stream, void* side_stream, const FlexAttnParams* p) {
   return e;
 }
 
+namespace {
+int forced_bwd_kernel() {  // 0: choose by shape, 1: fused, 2: separate kernels
+  static const int choice = [] {
+    const char* e = getenv("FLEXATTN_BWD_KERNEL");
+    if (e == nullptr) return 0;
+    return strcmp(e, "fused") == 0 ? 1 : strcmp(e, "split") == 0 ? 2 : 0;
+  }();
+  return choice;
+}
+bool fused_can(const FlexAttnParams* p) {
+  int e = FLEXATTN_OK;
+  return use_tcgen05(p, &e) && e == FLEXATTN_OK && p->ab == nullptr && p->dab == nullptr;
+}
+bool fused_pays(const FlexAttnParams* p) {
+  const int forced = forced_bwd_kernel();
+  if (forced) return forced == 1;
+  const long long items = (long long)((p->seq_k + FLEXATTN_TILE - 1) / FLEXATTN_TILE) * p->batch * p->heads;
+  return items >= sm_count();
+}
+}  // namespace
+
+size_t flexattn_bwd_scratch_bytes(const FlexAttnParams* p) {
+  if (validate_common(p) != FLEXATTN_OK || !fused_can(p) || !fused_pays(p)) return 0;
+  return bwd_fused_scratch_bytes(p->batch * p->heads, (p->seq_q + FLEXATTN_TILE - 1) / FLEXATTN_TILE, p->head_dim);
+}
+
+int flexattn_bwd_fused(void* stream, const FlexAttnParams* p, void* scratch, size_t scratch_bytes) {
+  NvtxRange nvtx("flexattn_bwd_fused");
+  int e = prologue(p);
+  if (e) return e;
+  FLEXATTN_REQUIRE(p->q); FLEXATTN_REQUIRE(p->k); FLEXATTN_REQUIRE(p->v); FLEXATTN_REQUIRE(p->o); FLEXATTN_REQUIRE(p->d_o);
+  FLEXATTN_REQUIRE(p->l); FLEXATTN_REQUIRE(p->m); FLEXATTN_REQUIRE(p->delta);
+  FLEXATTN_REQUIRE(p->dq); FLEXATTN_REQUIRE(p->dk); FLEXATTN_REQUIRE(p->dv); FLEXATTN_REQUIRE(scratch);
+  if (!fused_can(p)) return FLEXATTN_ERR_UNSUPPORTED_BACKEND;
+  const DevParams d = make_dev(p);
+  if (scratch_bytes < bwd_fused_scratch_bytes(d.batch * d.heads, d.n_qt, d.head_dim)) return FLEXATTN_ERR_WORKSPACE_TOO_SMALL;
+  return launch_sm100_bwd_fused(static_cast<cudaStream_t>(stream), d, p->score_kind, p->mask_kind, scratch);
+}
+
 int flexattn_read_mask_map(void* stream, const FlexAttnParams* p, int which, int b, int index, int32_t out[4]) {
   int e = prologue(p);
   if (e) return e;

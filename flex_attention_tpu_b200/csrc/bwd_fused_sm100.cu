@@ -1,0 +1,971 @@
+// The whole backward in one pass over the tile pairs on the 5th-generation tensor cores (sm_100a): five contractions
+// per pair where the separate dQ and dK/dV kernels (bwd_dq_sm100.cu, bwd_dkv_sm100.cu; the reference's two Pallas
+// kernels, flex_attention_dq_bwd.py:282-385 and flex_attention_dkv_kernel.py:177-280) take seven, and the exponentials
+// of a pair once instead of twice.
+//
+//   S^T  = K Q^T, dP^T = V dO^T      thread = key row, columns = query positions
+//   P^T, dS^T                        bf16 over S^T / dP^T in tensor memory; dS^T also as a shared-memory tile
+//   dV += P^T dO ; dK += dS^T Q      A from tensor memory
+//   dQ_part = dS K                   A = the dS^T tile read M-major, B = K read MN-major
+//
+// A work item is a 128-row kv tile of one slice; dK and dV stay in tensor memory over its query tiles, dQ_part is added
+// to an f32 scratch in L2 with bulk reductions and becomes bf16 in a last small kernel.  Tensor memory is full at D = 128
+// (S, dP, dK, dV = 512 columns): dQ_part takes the dP columns, whose dS^T the dK MMA has read by then (MMAs of one thread
+// execute in issue order), and dP of the next tile follows once the drain warps hold dQ_part in registers.  Issue order:
+//
+//   ... dV(n) S(n+1) dK(n) dQ(n) dP(n+1) dV(n+1) S(n+2) ...      (D = 64: dP(n+1) before dQ(n), which has its own columns)
+//
+// Results repeat bit for bit: the parts of a query tile are added in ONE order, kv tiles from the last one down.  A flag
+// per query tile says which kv tile has been added last; the turn warp waits for the predecessor's.  Items are taken in
+// list order from a ticket counter and wait only for items earlier in the list, which are running or done, so somebody
+// always gets on; under a causal mask the kv tiles of a slice walk along the diagonal one step apart, and the waits are
+// over before they begin.  Slices are taken in groups whose Q, dO and scratch fit L2.
+//
+// Persistent: one CTA of 16 warps per SM.  0-7 element-wise (two warpgroups, 64 query columns each), 8-11 drain,
+// 12 MMA issue, 13 loads, 14 turn, 15 publishes flags.
+#include "sched.cuh"
+#include "sm100.cuh"
+
+namespace flexattn {
+namespace FLEXATTN_TU_NAMESPACE {
+
+constexpr int kThreads = 512;
+constexpr int kDrainWarp = 8, kMmaWarp = 12, kTmaWarp = 13, kTurnWarp = 14, kFlagWarp = 15;
+constexpr int kRegsEw = 152, kRegsDrain = 152, kRegsRest = 56;  // 2 * 152 + 152 + 56 = 4 * 128: what the launch holds
+constexpr int kItemRing = 4;
+constexpr int kFusedId = 7;  // kernel id in the status words
+constexpr uint32_t kSlotBytes = 4096;  // 32 columns of a drain warp's 32 rows; two slots per warp
+
+struct FusedArgs {
+  float* dq_acc;       // [slices][n_qt][128 * D]: element (32 w + lane, 4 c + k) of a tile at ((w * D / 4 + c) * 32 + lane) * 4 + k
+  const float* stats;  // [slices][n_qt][2][128]: -(m log2e + log2 l) pre-scaled for pack_bf16_trunc, delta
+  int32_t* flags;      // [slices][n_qt]: n_kt - (kv tile added last), 0: none
+  int32_t* ticket;
+  int slice0, slices, group;  // slices of this launch (of batch * heads), and how many form a group
+};
+
+struct FusedSmem {
+  uint64_t bar_k[2], bar_v[2], bar_kfree[2], bar_vfree[2], bar_q[2], bar_do[2], bar_qfree[2], bar_dofree[2];
+  uint64_t bar_s, bar_dp, bar_p, bar_ds, bar_dq, bar_drained, bar_accfree, bar_stage[2], bar_stagefree[2];
+  uint64_t bar_turn[2], bar_turnfree[2], bar_red[2], bar_item[kItemRing], bar_itemfree[kItemRing];
+  uint32_t tmem_base;
+  alignas(16) int4 item_a[kItemRing];  // {slice of this launch (-1: no more), kv tile, first q tile, end q tile}
+  alignas(16) int2 item_b[kItemRing];  // {first fully kept q tile, end of the fully kept run}
+  alignas(16) int4 turn[2];            // {query tile of this launch (-1: no more), first to be added?, flag value, -}
+  alignas(16) float stats[2][2][kTile];
+};
+
+// what the score functions see besides the score
+struct FusedScoreCtx {
+  float sm_scale, c2, slope2, capl2, csc;
+  int b, h, j;
+};
+
+__device__ __forceinline__ void load_cols32(float (&dst)[32], const float* __restrict__ src) {
+#pragma unroll
+  for (int c = 0; c < 32; c += 4) {
+    const float4 t = *reinterpret_cast<const float4*>(src + c);
+    dst[c] = t.x;
+    dst[c + 1] = t.y;
+    dst[c + 2] = t.z;
+    dst[c + 3] = t.w;
+  }
+}
+
+// 32 query columns from i_first on: raw S^T in s, out p * dsigma (what dS^T needs) in s and packed bf16 P^T.
+// nl: the columns' statistics; keep: kept columns of this key row (partial tiles).
+template <int SK, bool kPartial>
+__device__ __forceinline__ void fused_p32(uint32_t (&s)[32], uint32_t (&pk)[16], const float (&nl)[32], uint32_t keep,
+                                          int i_first, const FusedScoreCtx& x) {
+  if constexpr (SK == FLEXATTN_SCORE_SOFTCAP || SK == FLEXATTN_SCORE_USER) {
+#pragma unroll
+    for (int c = 0; c < 32; c += 2) {
+      float pv[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int cc = c + u;
+        float arg, dsig;
+        if constexpr (SK == FLEXATTN_SCORE_USER) {
+          const float sc = __uint_as_float(s[cc]) * x.sm_scale;
+          arg = fmaf(user_score(sc, x.b, x.h, i_first + cc, x.j), kLog2e, nl[cc]);
+          dsig = user_dscore(sc, x.b, x.h, i_first + cc, x.j);
+        } else {
+          const float th = ptx::tanh_approx(__uint_as_float(s[cc]) * x.csc);
+          arg = fmaf(x.capl2, th, nl[cc]);
+          dsig = fmaf(-th, th, 1.f);
+        }
+        float p = ptx::ex2(arg);
+        if constexpr (kPartial) p = (keep >> cc) & 1u ? p : 0.f;
+        pv[u] = p;
+        s[cc] = __float_as_uint(p * dsig);
+      }
+      pk[c >> 1] = ptx::pack_bf16_trunc(pv[0], pv[1]);
+    }
+  } else {
+    const uint64_t c22 = ptx::pack2(x.c2, x.c2);
+    const float abase = x.slope2 * (float)(x.j - i_first);  // ALiBi: slope * (j - i), one packed add per pair of columns
+    uint64_t b2 = ptx::pack2(abase, abase - x.slope2);
+    const uint64_t bstep2 = ptx::pack2(-2.f * x.slope2, -2.f * x.slope2);
+#pragma unroll
+    for (int c = 0; c < 32; c += 2) {
+      const uint64_t sv2 = ptx::pack2(__uint_as_float(s[c]), __uint_as_float(s[c + 1]));
+      const uint64_t nl2 = ptx::pack2(nl[c], nl[c + 1]);
+      uint64_t arg2;
+      if constexpr (SK == FLEXATTN_SCORE_ALIBI) {
+        arg2 = ptx::fma2(sv2, c22, ptx::add2(b2, nl2));
+        b2 = ptx::add2(b2, bstep2);
+      } else {
+        arg2 = ptx::fma2(sv2, c22, nl2);
+      }
+      float a0, a1;
+      ptx::unpack2(arg2, a0, a1);
+      float p0 = ptx::ex2(a0), p1 = ptx::ex2(a1);
+      if constexpr (kPartial) {
+        p0 = (keep >> c) & 1u ? p0 : 0.f;
+        p1 = (keep >> (c + 1)) & 1u ? p1 : 0.f;
+      }
+      pk[c >> 1] = ptx::pack_bf16_trunc(p0, p1);
+      s[c] = __float_as_uint(p0);
+      s[c + 1] = __float_as_uint(p1);
+    }
+  }
+}
+
+// dS^T = (p dsigma) * (dP^T - delta), packed bf16
+__device__ __forceinline__ void fused_ds32(const uint32_t (&pd)[32], const uint32_t (&pr)[32], uint32_t (&pk)[16],
+                                           const float (&dl)[32]) {
+#pragma unroll
+  for (int c = 0; c < 32; c += 2) {
+    float d0, d1;
+    const uint64_t pd2 = ptx::pack2(__uint_as_float(pd[c]), __uint_as_float(pd[c + 1]));
+    const uint64_t pr2 = ptx::pack2(__uint_as_float(pr[c]), __uint_as_float(pr[c + 1]));
+    ptx::unpack2(ptx::mul2(pd2, ptx::sub2(pr2, ptx::pack2(dl[c], dl[c + 1]))), d0, d1);
+    pk[c >> 1] = ptx::pack_bf16_trunc(d0, d1);
+  }
+}
+
+__device__ __forceinline__ int ld_acquire(const int32_t* p) {
+  int v;
+  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_release(int32_t* p, int v) {
+  asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ void bulk_load(void* smem_dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                   ptx::smem_u32(smem_dst)),
+               "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(ptx::smem_u32(bar))
+               : "memory");
+}
+__device__ __forceinline__ void bulk_store(float* dst, const void* smem_src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(reinterpret_cast<uint64_t>(dst)),
+               "r"(ptx::smem_u32(smem_src)), "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_add_f32(float* dst, const void* smem_src, uint32_t bytes) {
+  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(
+                   reinterpret_cast<uint64_t>(dst)),
+               "r"(ptx::smem_u32(smem_src)), "r"(bytes)
+               : "memory");
+}
+
+template <int D, int SK, int MK>
+__global__ void __launch_bounds__(kThreads, 1)
+    fused_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
+                       const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
+                       const __grid_constant__ CUtensorMap tm_dk, const __grid_constant__ CUtensorMap tm_dv,
+                       const DevParams P, const FusedArgs F, int* abort_flag) {
+  constexpr int kPanels = D / 64;
+  constexpr uint32_t kTileBytes = kPanels * ptx::kPanelBytes;
+  // At D = 128 shared memory holds one K, V (those of the next item wait for this one's last MMAs) and one dO, whose two
+  // readers dP(n), dV(n) are neighbours on the tensor core: the next one has the time of S, dK, dQ to arrive.
+  constexpr int kKvStages = D == 64 ? 2 : 1, kDoStages = D == 64 ? 2 : 1;
+  constexpr uint32_t kStatBytes = 2 * kTile * sizeof(float);
+  constexpr uint32_t kTmemCols = 512;
+  constexpr uint32_t kColS = 0, kColDP = 128, kColDK = 256, kColDV = 256 + D;
+  constexpr bool kOwnDq = D == 64;  // dQ_part has columns of its own
+  constexpr uint32_t kColDQ = kOwnDq ? 384 : kColDP;
+  constexpr bool kDoc = MK == FLEXATTN_MASK_DOCUMENT;
+
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint8_t* sK = smem;
+  uint8_t* sV = sK + kKvStages * kTileBytes;
+  uint8_t* sQ = sV + kKvStages * kTileBytes;   // two stages
+  uint8_t* sDO = sQ + 2 * kTileBytes;
+  uint8_t* sDS = sDO + kDoStages * kTileBytes;  // dS^T: 128 keys x 128 queries; panel h belongs to warpgroup h
+  uint8_t* sOut = sDS + 2 * ptx::kPanelBytes;   // dQ_part on its way out: two slots per drain warp
+  FusedSmem* sh = reinterpret_cast<FusedSmem*>(sOut + 8 * kSlotBytes);
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (aborted_on_entry(abort_flag, P.status, kFusedId)) return;
+  if (ptx::smem_u32(smem) & 1023u) {  // the swizzled tiles need it (no room is left to round up)
+    if (tid == 0) give_up(abort_flag, P.status, kFusedId, 98);
+    return;
+  }
+  if (tid == 0) {
+    for (int s = 0; s < 2; ++s) {
+      ptx::mbar_init(&sh->bar_k[s], 1);
+      ptx::mbar_init(&sh->bar_v[s], 1);
+      ptx::mbar_init(&sh->bar_kfree[s], 1);
+      ptx::mbar_init(&sh->bar_vfree[s], 1);
+      ptx::mbar_init(&sh->bar_q[s], 1);
+      ptx::mbar_init(&sh->bar_do[s], 1);
+      ptx::mbar_init(&sh->bar_qfree[s], 1);
+      ptx::mbar_init(&sh->bar_dofree[s], 1);
+      ptx::mbar_init(&sh->bar_stage[s], 4);  // the four warps of a warpgroup
+      ptx::mbar_init(&sh->bar_stagefree[s], 1);
+      ptx::mbar_init(&sh->bar_turn[s], 1);
+      ptx::mbar_init(&sh->bar_turnfree[s], 5);  // four drain warps and the flag warp
+      ptx::mbar_init(&sh->bar_red[s], 4);
+    }
+    ptx::mbar_init(&sh->bar_s, 1);
+    ptx::mbar_init(&sh->bar_dp, 1);
+    ptx::mbar_init(&sh->bar_p, 8);
+    ptx::mbar_init(&sh->bar_ds, 8);
+    ptx::mbar_init(&sh->bar_dq, 1);
+    ptx::mbar_init(&sh->bar_drained, 4);
+    ptx::mbar_init(&sh->bar_accfree, 8);
+    for (int s = 0; s < kItemRing; ++s) {
+      ptx::mbar_init(&sh->bar_item[s], 1);
+      ptx::mbar_init(&sh->bar_itemfree[s], 14);  // eight element-wise warps, four drain warps, MMA, turn
+    }
+    ptx::fence_barrier_init();
+  }
+  if (warp == kMmaWarp) {
+    ptx::tmem_alloc(&sh->tmem_base, kTmemCols);
+    ptx::tmem_relinquish();
+  }
+  ptx::tc_fence_before();
+  __syncthreads();
+  ptx::tc_fence_after();
+  const uint32_t tmem = sh->tmem_base;
+
+  // In every role: r = index of an item of this CTA, u = index among its items with work (phases of what happens once
+  // per item), T = index of a tile in the stream of all of them (stage T % 2, phase (T / 2) & 1, or phase T & 1).
+  if (warp < kDrainWarp) {
+    ptx::setmaxnreg_inc<kRegsEw>();
+    // ------------------------------------------------------------------ element-wise warpgroups
+    const int row = tid & 127, half = warp >> 2;
+    const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    const uint32_t colS = kColS + 64 * half, colDP = kColDP + 64 * half;
+    uint8_t* panel = sDS + half * ptx::kPanelBytes;
+    uint8_t* panel_row = panel + row * 128;
+    FusedScoreCtx x;
+    x.sm_scale = P.sm_scale;
+    x.c2 = P.sm_scale * kLog2e;
+    x.slope2 = 0.f;
+    x.capl2 = P.cap * kLog2e;
+    x.csc = (SK == FLEXATTN_SCORE_SOFTCAP) ? P.sm_scale / P.cap : 0.f;
+    const long long n_doc = (long long)P.batch * P.doc_stride;
+    int T = 0, stores = 0, fail_at = 0;
+    bool ok = true;
+    // one 64-column panel of this warpgroup, already written, leaves through a bulk store; the panel is free on return
+    auto store_panel = [&](const CUtensorMap* tm, int col, int kt, int bh) {
+      ptx::fence_proxy_async_smem();
+      ptx::mbar_arrive_warp(&sh->bar_stage[half]);
+      if ((warp & 3) == 0) {
+        ok = __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_stage[half], stores & 1));
+        if (ok && lane == 0) {
+          ptx::tma_store_3d(tm, panel, col, kt * kTile, bh);
+          ptx::tma_store_commit();
+          ptx::tma_store_wait_read();
+          ptx::mbar_arrive(&sh->bar_stagefree[half]);
+        }
+        __syncwarp();
+      }
+      ok = ok && __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_stagefree[half], stores & 1));
+      if (!ok) fail_at = 13;
+      ++stores;
+    };
+    for (int r = 0; ok; ++r) {
+      ok = __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_item[r % kItemRing], (r / kItemRing) & 1));
+      if (!ok) { fail_at = 9; break; }
+      const int4 ia = sh->item_a[r % kItemRing];
+      const int2 ib = sh->item_b[r % kItemRing];
+      ptx::mbar_arrive_warp(&sh->bar_itemfree[r % kItemRing]);
+      if (ia.x < 0) break;
+      const int bh = F.slice0 + ia.x, kt = ia.y, N = ia.w - ia.z;
+      const int j = kt * kTile + row;  // this thread's key position
+      const bool row_ok = j < P.seq_k;
+      x.b = bh / P.heads;
+      x.h = bh - x.b * P.heads;
+      x.j = j;
+      if constexpr (SK == FLEXATTN_SCORE_ALIBI)
+        x.slope2 = FLEXATTN_DBG_OK(x.h, P.heads, kFusedId, 701) ? __ldg(&P.alibi_slopes[x.h]) * kLog2e : 0.f;
+      // the queries [qlo, qhi) this key row keeps, where the mask is an interval of them (all kinds but documents whose
+      // ids come back); a key past the end keeps nothing
+      bool doc_runs = false;
+      int qlo = 0, qhi = 0, dj = -2;
+      const int32_t* doc = nullptr;
+      if constexpr (!kDoc) row_query_interval<MK>(j, P.seq_q, P.window, P.stride, qlo, qhi);
+      if constexpr (kDoc) {
+        const long long at = (long long)x.b * P.doc_stride + j;
+        doc = P.doc_ids + (size_t)x.b * P.doc_stride;
+        doc_runs = FLEXATTN_DBG_OK(x.b, P.batch, kFusedId, 702) && P.doc_sorted[x.b] != 0;
+        if (row_ok && FLEXATTN_DBG_OK(at, n_doc, kFusedId, 703)) {
+          dj = doc[j];
+          if (doc_runs) {
+            qlo = j;
+            qhi = min(P.run_hi[at], P.seq_q);
+          }
+        }
+      }
+      for (int n = 0; n < N && ok; ++n, ++T) {
+        const int st = T & 1, qt = ia.z + n, i0 = qt * kTile + 64 * half;
+        const bool partial = !(qt >= ib.x && qt < ib.y);
+        const float* nlse = sh->stats[st][0] + 64 * half;
+        const float* delta = sh->stats[st][1] + 64 * half;
+        ok = __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_q[st], (T >> 1) & 1));  // the statistics came with Q
+        if (!ok) { fail_at = 10; break; }
+        float stat[32];
+        load_cols32(stat, nlse);
+        ok = __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_s, T & 1));
+        if (!ok) { fail_at = 11; break; }
+        ptx::tc_fence_after();
+        uint32_t p[2][32];
+        ptx::tmem_ld32(lane_base + colS, p[0]);
+        ptx::tmem_ld32(lane_base + colS + 32, p[1]);
+        ptx::tmem_wait_ld();
+        ptx::tmem_ld_acquire(p[0]);
+        ptx::tmem_ld_acquire(p[1]);
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+          uint32_t pk[16];
+          const int i1 = i0 + 32 * g;
+          if (g == 1) load_cols32(stat, nlse + 32);
+          if (partial) {
+            uint32_t keep = range_bits32(qlo - i1, qhi - i1);
+            if constexpr (kDoc) {
+              if (!doc_runs) {
+                keep = 0u;
+                for (int c = 0; c < 32; ++c) {
+                  const int i = i1 + c;
+                  if (i < P.seq_q && i >= j && FLEXATTN_DBG_OK((long long)x.b * P.doc_stride + i, n_doc, kFusedId, 704) &&
+                      __ldg(doc + i) == dj)
+                    keep |= 1u << c;
+                }
+              }
+            }
+            fused_p32<SK, true>(p[g], pk, stat, keep, i1, x);
+          } else {
+            fused_p32<SK, false>(p[g], pk, stat, 0u, i1, x);
+          }
+          // P^T over the first half of this warpgroup's S^T columns (read by now)
+          ptx::tmem_st16(lane_base + colS + 16 * g, pk);
+        }
+        ptx::tmem_wait_st();
+        ptx::tc_fence_before();
+        ptx::mbar_arrive_warp(&sh->bar_p);
+
+        load_cols32(stat, delta);
+        if (T > 0) {  // dQ(T - 1) has read the dS^T tile
+          ok = __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_dq, (T - 1) & 1));
+          if (!ok) { fail_at = 14; break; }
+        }
+        ok = __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_dp, T & 1));
+        if (!ok) { fail_at = 12; break; }
+        ptx::tc_fence_after();
+        uint32_t pr[2][32];
+        ptx::tmem_ld32(lane_base + colDP, pr[0]);
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+          uint32_t pk[16];
+          if (g == 1) load_cols32(stat, delta + 32);
+          ptx::tmem_wait_ld();
+          ptx::tmem_ld_acquire(pr[g]);
+          if (g == 0) ptx::tmem_ld32(lane_base + colDP + 32, pr[1]);
+          fused_ds32(p[g], pr[g], pk, stat);
+          // columns 32.. of this warpgroup are read after the first store, which lands on 0..15
+          ptx::tmem_st16(lane_base + colDP + 16 * g, pk);
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            *reinterpret_cast<uint4*>(panel_row + (((4 * g + c) ^ (row & 7)) << 4)) =
+                make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
+        }
+        ptx::tmem_wait_st();
+        ptx::tc_fence_before();
+        ptx::fence_proxy_async_smem();  // the tile is an MMA operand
+        ptx::mbar_arrive_warp(&sh->bar_ds);
+      }
+      if (!ok) break;
+      // dK * sm_scale (warpgroup 0) and dV (warpgroup 1) as bf16; the accumulators are free once they are in registers
+      if (N > 0) {
+        ok = __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_dq, (T - 1) & 1));  // ... and every MMA before it
+        if (!ok) { fail_at = 15; break; }
+        ptx::tc_fence_after();
+      }
+      uint32_t out[D / 2];
+      const float sc = half ? 1.f : P.sm_scale;
+#pragma unroll
+      for (int c0 = 0; c0 < D; c0 += 32) {
+        uint32_t v[32];
+        if (N > 0) {
+          ptx::tmem_ld32(lane_base + (half ? kColDV : kColDK) + c0, v);
+          ptx::tmem_wait_ld();
+          ptx::tmem_ld_acquire(v);
+        } else {
+#pragma unroll
+          for (int c = 0; c < 32; ++c) v[c] = 0u;
+        }
+#pragma unroll
+        for (int c = 0; c < 32; c += 2)
+          out[(c0 + c) >> 1] = ptx::pack_bf16(__uint_as_float(v[c]) * sc, __uint_as_float(v[c + 1]) * sc);
+      }
+      if (N > 0) {
+        ptx::tc_fence_before();
+        ptx::mbar_arrive_warp(&sh->bar_accfree);
+      }
+#pragma unroll
+      for (int p0 = 0; p0 < kPanels; ++p0) {
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+          *reinterpret_cast<uint4*>(panel_row + ((c ^ (row & 7)) << 4)) =
+              make_uint4(out[32 * p0 + 4 * c], out[32 * p0 + 4 * c + 1], out[32 * p0 + 4 * c + 2], out[32 * p0 + 4 * c + 3]);
+        if (ok) store_panel(half ? &tm_dv : &tm_dk, p0 * 64, kt, bh);
+      }
+    }
+    if (!ok && lane == 0) give_up(abort_flag, P.status, kFusedId, fail_at);
+  } else if (warp < kMmaWarp) {
+    ptx::setmaxnreg_inc<kRegsDrain>();
+    // ------------------------------------------------------------------ drain: dQ_part -> scratch
+    // Through shared memory and the bulk engine: vector reductions straight from the registers (25 bytes per cycle and SM,
+    // as fast) fill the load/store queue, behind which every shared-memory access and barrier of the other warps waits
+    // (4000 cycles per tile instead of 2900).
+    const int w = warp - kDrainWarp;
+    const uint32_t lane_base = tmem + ((uint32_t)(w * 32) << 16);
+    uint8_t* slots = sOut + 2 * w * kSlotBytes;
+    int T = 0, fail_at = 0;
+    bool ok = true, pending = false;
+    // the bulk operations of tile t have completed: the flag warp may say so
+    auto finish = [&](int t) {
+      if (lane == 0) {
+        ptx::tma_store_wait_all();
+        asm volatile("fence.proxy.async.global;" ::: "memory");
+        ptx::mbar_arrive(&sh->bar_red[t & 1]);
+      }
+      __syncwarp();
+      pending = false;
+    };
+    for (int r = 0; ok; ++r) {
+      ok = __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_item[r % kItemRing], (r / kItemRing) & 1));
+      if (!ok) { fail_at = 30; break; }
+      const int4 ia = sh->item_a[r % kItemRing];
+      ptx::mbar_arrive_warp(&sh->bar_itemfree[r % kItemRing]);
+      if (ia.x < 0) break;
+      for (int qt = ia.z; qt < ia.w && ok; ++qt, ++T) {
+        ok = __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_dq, T & 1));
+        if (!ok) { fail_at = 31; break; }
+        ptx::tc_fence_after();
+        uint32_t v[D / 32][32];
+#pragma unroll
+        for (int c = 0; c < D / 32; ++c) ptx::tmem_ld32(lane_base + kColDQ + 32 * c, v[c]);
+        ptx::tmem_wait_ld();
+#pragma unroll
+        for (int c = 0; c < D / 32; ++c) ptx::tmem_ld_acquire(v[c]);
+        ptx::tc_fence_before();
+        ptx::mbar_arrive_warp(&sh->bar_drained);  // the columns are free
+        if (pending) finish(T - 1);
+        ok = __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_turn[T & 1], (T >> 1) & 1));
+        if (!ok) { fail_at = 32; break; }
+        const int4 turn = sh->turn[T & 1];
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(&sh->bar_turnfree[T & 1]);
+        if (FLEXATTN_DBG_OK(turn.x, (long long)F.slices * P.n_qt, kFusedId, 705)) {
+          float* dst = F.dq_acc + ((size_t)turn.x * kTile + 32 * w) * D;
+#pragma unroll
+          for (int c = 0; c < D / 32; ++c) {
+            uint8_t* slot = slots + (c & 1) * kSlotBytes;
+            if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");  // the slot's last one has been read
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < 32; k += 4)
+              *reinterpret_cast<uint4*>(slot + k * 128 + lane * 16) = make_uint4(v[c][k], v[c][k + 1], v[c][k + 2], v[c][k + 3]);
+            ptx::fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              if (turn.y) bulk_store(dst + c * 1024, slot, kSlotBytes);  // the first part of a query tile: nothing to add to
+              else bulk_add_f32(dst + c * 1024, slot, kSlotBytes);
+              ptx::tma_store_commit();
+            }
+          }
+        }
+        pending = true;
+        if (qt + 1 == ia.w) finish(T);
+      }
+    }
+    if (pending) finish(T - 1);
+    if (!ok && lane == 0) give_up(abort_flag, P.status, kFusedId, fail_at);
+  } else {
+    ptx::setmaxnreg_dec<kRegsRest>();
+    if (warp == kTmaWarp) {
+      // ---------------------------------------------------------------- loads; takes the items
+      if (ptx::elect_one()) {
+        bool ok = true;
+        ptx::prefetch_tensormap(&tm_q);
+        ptx::prefetch_tensormap(&tm_do);
+        ptx::prefetch_tensormap(&tm_k);
+        ptx::prefetch_tensormap(&tm_v);
+        auto load_tile = [&](uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, int row0, int bh, uint32_t extra) {
+          ptx::mbar_arrive_expect_tx(bar, kTileBytes + extra);
+#pragma unroll
+          for (int p = 0; p < kPanels; ++p) ptx::tma_load_3d(dst + p * ptx::kPanelBytes, tm, bar, p * 64, row0, bh);
+        };
+        const int total = F.slices * P.n_kt;
+        int T = 0, u = 0;
+        int w = atomicAdd(F.ticket, 1);
+        for (int r = 0;; ++r) {
+          if (r >= kItemRing) {
+            ok = ptx::mbar_wait_relaxed(&sh->bar_itemfree[r % kItemRing], (r / kItemRing - 1) & 1);
+            if (!ok) break;
+          }
+          if (w >= total) {
+            sh->item_a[r % kItemRing] = make_int4(-1, 0, 0, 0);
+            ptx::mbar_arrive(&sh->bar_item[r % kItemRing]);
+            break;
+          }
+          const int g = w / (F.group * P.n_kt), in_group = w - g * F.group * P.n_kt;
+          const int width = min(F.group, F.slices - g * F.group);
+          const int rank = in_group / width;
+          const int slice = g * F.group + in_group - rank * width, kt = P.n_kt - 1 - rank;
+          const int bh = F.slice0 + slice, b = bh / P.heads;
+          const int4 cm = __ldg(&P.col_map[(size_t)(P.map_rows > 1 ? b : 0) * P.n_kt + kt]);
+          sh->item_a[r % kItemRing] = make_int4(slice, kt, cm.x, cm.y);
+          sh->item_b[r % kItemRing] = make_int2(cm.z, cm.w);
+          ptx::mbar_arrive(&sh->bar_item[r % kItemRing]);
+          const int N = cm.y - cm.x;
+          auto load_q = [&](int n) {
+            const int st = (T + n) & 1;
+            if (T + n >= 2) ok = ok && ptx::mbar_wait_relaxed(&sh->bar_qfree[st], (((T + n) >> 1) - 1) & 1, 20);
+            if (!ok) return;
+            load_tile(sQ + st * kTileBytes, &tm_q, &sh->bar_q[st], (cm.x + n) * kTile, bh, kStatBytes);
+            bulk_load(sh->stats[st], F.stats + ((size_t)slice * P.n_qt + cm.x + n) * 2 * kTile, kStatBytes, &sh->bar_q[st]);
+          };
+          auto load_do = [&](int n) {
+            const int st = (T + n) % kDoStages;
+            if (T + n >= kDoStages)
+              ok = ok && ptx::mbar_wait_relaxed(&sh->bar_dofree[st], ((T + n) / kDoStages - 1) & 1, 20);
+            if (!ok) return;
+            load_tile(sDO + st * kTileBytes, &tm_do, &sh->bar_do[st], (cm.x + n) * kTile, bh, 0);
+          };
+          if (N > 0) {
+            const int ks = u % kKvStages, kph = (u / kKvStages - 1) & 1;
+            load_q(0);
+            // V and K of the previous item (D = 64: of the last but one) have been read
+            if (u >= kKvStages) ok = ok && ptx::mbar_wait_relaxed(&sh->bar_vfree[ks], kph, 20);
+            if (!ok) break;
+            load_tile(sV + ks * kTileBytes, &tm_v, &sh->bar_v[ks], kt * kTile, bh, 0);
+            load_do(0);
+            if (u >= kKvStages) ok = ok && ptx::mbar_wait_relaxed(&sh->bar_kfree[ks], kph, 20);
+            if (!ok) break;
+            load_tile(sK + ks * kTileBytes, &tm_k, &sh->bar_k[ks], kt * kTile, bh, 0);
+            for (int n = 1; n < N && ok; ++n) {
+              if (kDoStages == 1) {  // dO(n) waits for dV(n-1), later than Q(n) for dK(n-2)
+                load_q(n);
+                load_do(n);
+              } else {
+                load_do(n);
+                load_q(n);
+              }
+            }
+            if (!ok) break;
+            T += N;
+            ++u;
+          }
+          w = atomicAdd(F.ticket, 1);
+        }
+        if (!ok) give_up(abort_flag, P.status, kFusedId, 20);
+      }
+    } else if (warp == kMmaWarp) {
+      // ---------------------------------------------------------------- MMA issue
+      if (ptx::elect_one()) {
+        bool ok = true;
+        int fail_at = 1;
+        constexpr uint32_t idesc_s = ptx::make_idesc(128, 128, false);
+        constexpr uint32_t idesc_acc = ptx::make_idesc(128, D, true);
+        constexpr uint32_t idesc_dq = ptx::make_idesc(128, D, true, true);
+        const uint32_t aK = ptx::smem_u32(sK), aV = ptx::smem_u32(sV), aQ = ptx::smem_u32(sQ), aDO = ptx::smem_u32(sDO);
+        const uint32_t aDS = ptx::smem_u32(sDS);
+        int T = 0, u = 0;
+        // descriptors are rebuilt for each group of MMAs: kept across the loop they need a hundred registers
+        auto kmajor = [](uint32_t a) {
+          asm volatile("" : "+r"(a));
+          return ptx::base_kmajor(a);
+        };
+        auto mnmajor = [](uint32_t a) {
+          asm volatile("" : "+r"(a));
+          return ptx::base_mnmajor(a);
+        };
+        auto wait = [&](uint64_t* bar, uint32_t par, int site) {
+          if (ok && !ptx::mbar_wait(bar, par)) {
+            ok = false;
+            fail_at = site;
+          }
+        };
+        auto do_off = [&](int t) { return (uint32_t)(t % kDoStages) * kTileBytes; };
+        auto issue_s = [&](int t, uint32_t k_off) {  // S^T = K Q^T
+          const ptx::DescBase bK = kmajor(aK + k_off), bQ = kmajor(aQ + (uint32_t)(t & 1) * kTileBytes);
+          ptx::tc_fence_after();
+#pragma unroll
+          for (int kk = 0; kk < D / 16; ++kk)
+            ptx::mma_ss(tmem + kColS, ptx::desc_at(bK, ptx::koff_kmajor(kk)), ptx::desc_at(bQ, ptx::koff_kmajor(kk)), idesc_s, kk > 0);
+          ptx::mma_commit(&sh->bar_s);
+        };
+        // dP^T = V dO^T of tile t; the dP columns are free of dS^T(t - 1) (issue order) and of dQ_part(t - 1) (drained)
+        auto issue_dp = [&](int t, uint32_t k_off) {
+          wait(&sh->bar_do[t % kDoStages], (t / kDoStages) & 1, 7);
+          if (!kOwnDq && t > 0) wait(&sh->bar_drained, (t - 1) & 1, 17);
+          if (!ok) return;
+          const ptx::DescBase bV = kmajor(aV + k_off), bDO = kmajor(aDO + do_off(t));
+          ptx::tc_fence_after();
+#pragma unroll
+          for (int kk = 0; kk < D / 16; ++kk)
+            ptx::mma_ss(tmem + kColDP, ptx::desc_at(bV, ptx::koff_kmajor(kk)), ptx::desc_at(bDO, ptx::koff_kmajor(kk)), idesc_s, kk > 0);
+          ptx::mma_commit(&sh->bar_dp);
+        };
+        for (int r = 0; ok; ++r) {
+          wait(&sh->bar_item[r % kItemRing], (r / kItemRing) & 1, 1);
+          if (!ok) break;
+          const int4 ia = sh->item_a[r % kItemRing];
+          ptx::mbar_arrive(&sh->bar_itemfree[r % kItemRing]);
+          if (ia.x < 0) break;
+          const int N = ia.w - ia.z;
+          if (N <= 0) continue;
+          const int ks = u % kKvStages;
+          const uint32_t kph = (u / kKvStages) & 1, k_off = (uint32_t)ks * kTileBytes;
+          wait(&sh->bar_q[T & 1], (T >> 1) & 1, 2);
+          wait(&sh->bar_k[ks], kph, 3);
+          if (!ok) break;
+          issue_s(T, k_off);
+          wait(&sh->bar_v[ks], kph, 4);
+          issue_dp(T, k_off);
+          for (int n = 0; n < N && ok; ++n, ++T) {
+            const bool more = n + 1 < N;
+            wait(&sh->bar_p, T & 1, 8);
+            if (n == 0 && u > 0) wait(&sh->bar_accfree, (u - 1) & 1, 16);  // dK, dV of the previous item have been read
+            if (!ok) break;
+            ptx::tc_fence_after();
+            {  // dV += P^T dO; warpgroup w wrote query columns [64 w, 64 w + 64) at column 64 w of the S^T block
+              const ptx::DescBase bDOt = mnmajor(aDO + do_off(T));
+#pragma unroll
+              for (int kk = 0; kk < kTile / 16; ++kk)
+                ptx::mma_ts(tmem + kColDV, tmem + kColS + 64 * (kk >> 2) + (kk & 3) * 8, ptx::desc_at(bDOt, ptx::koff_mnmajor(kk)),
+                            idesc_acc, n > 0 || kk > 0);
+              ptx::mma_commit(&sh->bar_dofree[T % kDoStages]);
+              if (!more) ptx::mma_commit(&sh->bar_vfree[ks]);
+            }
+            if (more) {
+              wait(&sh->bar_q[(T + 1) & 1], ((T + 1) >> 1) & 1, 18);
+              if (!ok) break;
+              issue_s(T + 1, k_off);
+            }
+            wait(&sh->bar_ds, T & 1, 19);
+            if (!ok) break;
+            ptx::tc_fence_after();
+            {  // dK += dS^T Q
+              const ptx::DescBase bQt = mnmajor(aQ + (uint32_t)(T & 1) * kTileBytes);
+#pragma unroll
+              for (int kk = 0; kk < kTile / 16; ++kk)
+                ptx::mma_ts(tmem + kColDK, tmem + kColDP + 64 * (kk >> 2) + (kk & 3) * 8, ptx::desc_at(bQt, ptx::koff_mnmajor(kk)),
+                            idesc_acc, n > 0 || kk > 0);
+              ptx::mma_commit(&sh->bar_qfree[T & 1]);
+            }
+            if (kOwnDq) {
+              if (more) issue_dp(T + 1, k_off);
+              if (T > 0) wait(&sh->bar_drained, (T - 1) & 1, 21);
+              if (!ok) break;
+              ptx::tc_fence_after();
+            }
+            {  // dQ_part = dS K
+              const ptx::DescBase bDS = mnmajor(aDS), bKt = mnmajor(aK + k_off);
+#pragma unroll
+              for (int kk = 0; kk < kTile / 16; ++kk)
+                ptx::mma_ss(tmem + kColDQ, ptx::desc_at(bDS, ptx::koff_mnmajor(kk)), ptx::desc_at(bKt, ptx::koff_mnmajor(kk)),
+                            idesc_dq, kk > 0);
+              ptx::mma_commit(&sh->bar_dq);
+              if (!more) ptx::mma_commit(&sh->bar_kfree[ks]);
+            }
+            if (!kOwnDq && more) issue_dp(T + 1, k_off);
+          }
+          ++u;
+        }
+        if (!ok) give_up(abort_flag, P.status, kFusedId, fail_at);
+      }
+    } else if (warp == kTurnWarp) {
+      // ---------------------------------------------------------------- whose turn it is at a query tile
+      int T = 0, fail_at = 40;
+      bool ok = true;
+      auto publish = [&](int tile, int first, int value) {
+        if (T >= 2) ok = ok && __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_turnfree[T & 1], ((T >> 1) - 1) & 1));
+        if (!ok) { fail_at = 41; return; }
+        if (lane == 0) {
+          sh->turn[T & 1] = make_int4(tile, first, value, 0);
+          ptx::mbar_arrive(&sh->bar_turn[T & 1]);
+        }
+        __syncwarp();
+        ++T;
+      };
+      for (int r = 0; ok; ++r) {
+        ok = __all_sync(0xffffffffu, ptx::mbar_wait_relaxed(&sh->bar_item[r % kItemRing], (r / kItemRing) & 1));
+        if (!ok) break;
+        const int4 ia = sh->item_a[r % kItemRing];
+        ptx::mbar_arrive_warp(&sh->bar_itemfree[r % kItemRing]);
+        if (ia.x < 0) {
+          publish(-1, 0, 0);
+          break;
+        }
+        const int b = (F.slice0 + ia.x) / P.heads;
+        const int4* cmap = P.col_map + (size_t)(P.map_rows > 1 ? b : 0) * P.n_kt;
+        for (int qt = ia.z; qt < ia.w && ok; ++qt) {
+          // the kv tile added before this one: the next higher one that sees the query tile
+          int pred = -1;
+          for (int j0 = ia.y + 1; j0 < P.n_kt && pred < 0; j0 += 32) {
+            bool sees = false;
+            if (j0 + lane < P.n_kt) {
+              const int2 range = __ldg(reinterpret_cast<const int2*>(cmap + j0 + lane));
+              sees = qt >= range.x && qt < range.y;
+            }
+            const unsigned any = __ballot_sync(0xffffffffu, sees);
+            if (any) pred = j0 + __ffs(any) - 1;
+          }
+          const int tile = ia.x * P.n_qt + qt;
+          if (pred >= 0) {
+            const int32_t* flag = F.flags + tile;
+            const int want = P.n_kt - pred;
+            if (FLEXATTN_DBG_OK(tile, (long long)F.slices * P.n_qt, kFusedId, 706) && ld_acquire(flag) < want) {
+              const unsigned long long t0 = ptx::globaltimer_ns();
+              int polls = 0;
+              while (ok && ld_acquire(flag) < want) {
+                if ((++polls & 63) == 0 && ptx::globaltimer_ns() - t0 > ptx::kWaitLimitNs) ok = false;
+              }
+            }
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) { fail_at = 42; break; }
+            asm volatile("fence.proxy.async.global;" ::: "memory");  // the parts are added through the async proxy
+          }
+          publish(tile, pred < 0, P.n_kt - ia.y);
+        }
+      }
+      if (!ok && lane == 0) give_up(abort_flag, P.status, kFusedId, fail_at);
+    } else {
+      // ---------------------------------------------------------------- flags: a part has been added
+      bool ok = true;
+      for (int T = 0; ok; ++T) {
+        ok = __all_sync(0xffffffffu, ptx::mbar_wait_relaxed(&sh->bar_turn[T & 1], (T >> 1) & 1, 40));
+        if (!ok) break;
+        const int4 turn = sh->turn[T & 1];
+        if (turn.x < 0) break;
+        ok = __all_sync(0xffffffffu, ptx::mbar_wait_relaxed(&sh->bar_red[T & 1], (T >> 1) & 1, 20));
+        if (!ok) break;
+        if (lane == 0) {
+          __threadfence();  // what the drain warps have added comes before the flag
+          if (FLEXATTN_DBG_OK(turn.x, (long long)F.slices * P.n_qt, kFusedId, 707)) st_release(F.flags + turn.x, turn.z);
+          ptx::mbar_arrive(&sh->bar_turnfree[T & 1]);
+        }
+        __syncwarp();
+      }
+      if (!ok && lane == 0) give_up(abort_flag, P.status, kFusedId, 50);
+    }
+  }
+
+  ptx::tc_fence_before();
+  __syncthreads();
+  if (warp == kMmaWarp) {
+    ptx::tc_fence_after();
+    ptx::tmem_dealloc(tmem, kTmemCols);
+  }
+}
+
+#ifndef FLEXATTN_JIT
+// Before it: delta = rowsum(o * do) to the caller, both row statistics to the padded tiles the loads take, flags and ticket
+// to zero.  One 16-byte chunk of o and do per thread, as in delta.cu.
+template <int D>
+__global__ void __launch_bounds__(256) prep_kernel(const DevParams P, const FusedArgs F, float* stats) {
+  constexpr int kTpr = D / 8;
+  const long long rows = (long long)F.slices * P.n_qt * kTile;
+  const long long idx = (long long)blockIdx.x * 256 + threadIdx.x, row = idx / kTpr;
+  if (idx <= (long long)F.slices * P.n_qt) F.flags[idx] = 0;  // the ticket is the one behind them
+  float acc = 0.f;
+  const long long slice = row / (P.n_qt * kTile);
+  const int i = (int)(row - slice * (P.n_qt * kTile));
+  const bool live = row < rows && i < P.seq_q;
+  const long long at = (F.slice0 + slice) * P.seq_q + i;
+  if (live) {
+    const uint4 a = __ldg(static_cast<const uint4*>(P.o) + at * kTpr + (threadIdx.x & (kTpr - 1)));
+    const uint4 b = __ldg(static_cast<const uint4*>(P.d_o) + at * kTpr + (threadIdx.x & (kTpr - 1)));
+    const __nv_bfloat162* pa = reinterpret_cast<const __nv_bfloat162*>(&a);
+    const __nv_bfloat162* pb = reinterpret_cast<const __nv_bfloat162*>(&b);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const float2 fa = __bfloat1622float2(pa[c]), fb = __bfloat1622float2(pb[c]);
+      acc = fmaf(fa.x, fb.x, acc);
+      acc = fmaf(fa.y, fb.y, acc);
+    }
+  }
+#pragma unroll
+  for (int s = kTpr / 2; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
+  if (row < rows && (threadIdx.x & (kTpr - 1)) == 0) {
+    float nl = -1.0e30f;  // rows past the end and fully masked ones: p = 0
+    if (live) {
+      P.delta[at] = acc;
+      const float l = P.l[at];
+      if (l > 0.f) nl = ptx::kRoundLog2 - fmaf(P.m[at], kLog2e, __log2f(l));
+    }
+    float* t = stats + (row / kTile) * 2 * kTile + (row % kTile);
+    t[0] = nl;
+    t[kTile] = acc;
+  }
+}
+
+// After it: the f32 tiles become dq, times sm_scale.  A thread takes 16 columns of a row: the loads of a warp are 512
+// consecutive bytes, its stores whole 32-byte sectors.  A query tile no kv tile sees was never written: zero.
+template <int D>
+__global__ void __launch_bounds__(256) finish_kernel(const DevParams P, const FusedArgs F) {
+  const int tile = blockIdx.x, slice = tile / P.n_qt, qt = tile - slice * P.n_qt, bh = F.slice0 + slice;
+  const int4* cmap = P.col_map + (size_t)(P.map_rows > 1 ? bh / P.heads : 0) * P.n_kt;
+  bool seen = false;
+  for (int j = threadIdx.x; j < P.n_kt; j += 256) {
+    const int2 range = __ldg(reinterpret_cast<const int2*>(cmap + j));
+    seen = seen || (qt >= range.x && qt < range.y);
+  }
+  seen = __syncthreads_or(seen);
+  const float* src = F.dq_acc + (size_t)tile * kTile * D;
+#pragma unroll
+  for (int e = threadIdx.x; e < kTile * D / 16; e += 256) {
+    const int lane = e & 31, c16 = (e >> 5) % (D / 16), w = (e >> 5) / (D / 16);
+    const int i = qt * kTile + 32 * w + lane;
+    uint32_t out[8];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (seen) v = __ldcs(reinterpret_cast<const float4*>(src + ((size_t)(w * (D / 4) + 4 * c16 + c) * 32 + lane) * 4));
+      out[2 * c] = ptx::pack_bf16(v.x * P.sm_scale, v.y * P.sm_scale);
+      out[2 * c + 1] = ptx::pack_bf16(v.z * P.sm_scale, v.w * P.sm_scale);
+    }
+    if (i < P.seq_q) {
+      uint4* dst = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(P.dq) + ((size_t)bh * P.seq_q + i) * D + 16 * c16);
+      dst[0] = make_uint4(out[0], out[1], out[2], out[3]);
+      dst[1] = make_uint4(out[4], out[5], out[6], out[7]);
+    }
+  }
+}
+
+constexpr size_t smem_bytes(int D) {
+  return (size_t)(D == 64 ? 8 : 5) * (D / 64) * ptx::kPanelBytes + 2 * ptx::kPanelBytes + 8 * kSlotBytes + sizeof(FusedSmem);
+}
+static_assert(smem_bytes(128) <= 232448 && smem_bytes(64) <= 232448, "more shared memory than a CTA can have");
+
+struct Maps {
+  CUtensorMap q, d_o, k, v, dk, dv;
+};
+
+template <int D, int SK, int MK>
+int launch_one(cudaStream_t st, const DevParams& d, const FusedArgs& f, const Maps& t, unsigned grid, int* af) {
+  constexpr size_t smem = smem_bytes(D);
+  auto kern = fused_sm100_kernel<D, SK, MK>;
+  static SmemAttrOnce attr_once{};  // per kernel instantiation, per device
+  if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), (int)smem, &attr_once) != FLEXATTN_OK) return FLEXATTN_ERR_CUDA;
+  kern<<<grid, kThreads, smem, st>>>(t.q, t.d_o, t.k, t.v, t.dk, t.dv, d, f, af);
+  return cudaGetLastError() == cudaSuccess ? FLEXATTN_OK : FLEXATTN_ERR_CUDA;
+}
+
+template <int D, int SK>
+int launch_mask(cudaStream_t st, const DevParams& d, int mask, const FusedArgs& f, const Maps& t, unsigned grid, int* af) {
+  switch (mask) {
+    case FLEXATTN_MASK_NONE: return launch_one<D, SK, FLEXATTN_MASK_NONE>(st, d, f, t, grid, af);
+    case FLEXATTN_MASK_CAUSAL: return launch_one<D, SK, FLEXATTN_MASK_CAUSAL>(st, d, f, t, grid, af);
+    case FLEXATTN_MASK_SLIDING_WINDOW: return launch_one<D, SK, FLEXATTN_MASK_SLIDING_WINDOW>(st, d, f, t, grid, af);
+    case FLEXATTN_MASK_SLIDING_WINDOW_CAUSAL:
+      return launch_one<D, SK, FLEXATTN_MASK_SLIDING_WINDOW_CAUSAL>(st, d, f, t, grid, af);
+    case FLEXATTN_MASK_DOCUMENT: return launch_one<D, SK, FLEXATTN_MASK_DOCUMENT>(st, d, f, t, grid, af);
+    case FLEXATTN_MASK_S2: return launch_one<D, SK, FLEXATTN_MASK_S2>(st, d, f, t, grid, af);
+    default: return FLEXATTN_ERR_UNSUPPORTED_MOD;
+  }
+}
+
+template <int D>
+int launch_score(cudaStream_t st, const DevParams& d, int score, int mask, const FusedArgs& f, const Maps& t, unsigned grid,
+                 int* af) {
+  switch (score) {
+    case FLEXATTN_SCORE_NONE: return launch_mask<D, FLEXATTN_SCORE_NONE>(st, d, mask, f, t, grid, af);
+    case FLEXATTN_SCORE_ALIBI: return launch_mask<D, FLEXATTN_SCORE_ALIBI>(st, d, mask, f, t, grid, af);
+    case FLEXATTN_SCORE_SOFTCAP: return launch_mask<D, FLEXATTN_SCORE_SOFTCAP>(st, d, mask, f, t, grid, af);
+    default: return FLEXATTN_ERR_UNSUPPORTED_MOD;
+  }
+}
+
+// The scratch of a launch, which serves as many slices as keep its f32 tiles within kAccLimit (one, if need be): a larger
+// problem runs in several launches that reuse it, so the scratch does not grow with it.
+constexpr long long kAccLimit = 1ll << 30;
+struct ScratchLayout {
+  int slices;  // of a launch
+  size_t off_stats, off_flags, bytes;
+};
+ScratchLayout scratch_layout(int slices, int n_qt, int head_dim) {
+  ScratchLayout L;
+  const long long acc = (long long)n_qt * kTile * head_dim * 4;
+  const long long most = kAccLimit / acc > 0 ? kAccLimit / acc : 1;
+  const long long launches = (slices + most - 1) / most;
+  L.slices = (int)((slices + launches - 1) / launches);
+  auto up = [](size_t n) { return (n + 255) & ~(size_t)255; };
+  L.off_stats = up((size_t)L.slices * acc);
+  L.off_flags = L.off_stats + up((size_t)L.slices * n_qt * 2 * kTile * sizeof(float));
+  L.bytes = L.off_flags + up(((size_t)L.slices * n_qt + 1) * sizeof(int32_t));
+  return L;
+}
+constexpr long long kL2Budget = 48ll << 20;  // Q, dO and scratch of a group of slices
+#endif  // !FLEXATTN_JIT
+
+}  // namespace FLEXATTN_TU_NAMESPACE
+
+#ifndef FLEXATTN_JIT
+size_t bwd_fused_scratch_bytes(int slices, int n_qt, int head_dim) { return scratch_layout(slices, n_qt, head_dim).bytes; }
+
+int launch_sm100_bwd_fused(cudaStream_t st, const DevParams& d, int score, int mask, void* scratch) {
+  int* af = abort_flag_ptr();
+  const int sms = sm_count();
+  if (af == nullptr || sms <= 0) return FLEXATTN_ERR_CUDA;
+  const int slices = d.batch * d.heads, D = d.head_dim;
+  if (D != 64 && D != 128) return FLEXATTN_ERR_UNSUPPORTED_HEAD_DIM;
+  const ScratchLayout L = scratch_layout(slices, d.n_qt, D);
+  Maps t;
+  int e = make_tile_map(&t.q, d.q, slices, d.seq_q, D);
+  if (!e) e = make_tile_map(&t.d_o, d.d_o, slices, d.seq_q, D);
+  if (!e) e = make_tile_map(&t.k, d.k, slices, d.seq_k, D);
+  if (!e) e = make_tile_map(&t.v, d.v, slices, d.seq_k, D);
+  if (!e) e = make_tile_map(&t.dk, d.dk, slices, d.seq_k, D);
+  if (!e) e = make_tile_map(&t.dv, d.dv, slices, d.seq_k, D);
+  char* base = static_cast<char*>(scratch);
+  float* stats = reinterpret_cast<float*>(base + L.off_stats);
+  for (int s0 = 0; s0 < slices && !e; s0 += L.slices) {
+    FusedArgs f;
+    f.dq_acc = reinterpret_cast<float*>(base);
+    f.stats = stats;
+    f.flags = reinterpret_cast<int32_t*>(base + L.off_flags);
+    f.slice0 = s0;
+    f.slices = slices - s0 < L.slices ? slices - s0 : L.slices;
+    f.ticket = f.flags + (size_t)f.slices * d.n_qt;
+    const long long live = 8ll * d.seq_q * D;  // bytes of Q, dO and scratch of a slice
+    f.group = (int)(kL2Budget / live < 1 ? 1 : kL2Budget / live < f.slices ? kL2Budget / live : f.slices);
+    const long long tiles = (long long)f.slices * d.n_qt, items = (long long)f.slices * d.n_kt;
+    const unsigned prep_blocks = (unsigned)((tiles * kTile * (D / 8) + 255) / 256);
+    if (D == 128) prep_kernel<128><<<prep_blocks, 256, 0, st>>>(d, f, stats);
+    else prep_kernel<64><<<prep_blocks, 256, 0, st>>>(d, f, stats);
+    if (cudaGetLastError() != cudaSuccess) return FLEXATTN_ERR_CUDA;
+    const unsigned grid = (unsigned)(items < sms ? items : sms);
+    if (score == FLEXATTN_SCORE_USER) {
+      void* args[] = {&t.q, &t.d_o, &t.k, &t.v, &t.dk, &t.dv, const_cast<DevParams*>(&d), &f, &af};
+      e = jit_launch(4, false, d.user_score, D, mask, grid, 1, kThreads, smem_bytes(D), st, args);
+    } else {
+      e = D == 128 ? launch_score<128>(st, d, score, mask, f, t, grid, af) : launch_score<64>(st, d, score, mask, f, t, grid, af);
+    }
+    if (e) return e;
+    if (D == 128) finish_kernel<128><<<(unsigned)tiles, 256, 0, st>>>(d, f);
+    else finish_kernel<64><<<(unsigned)tiles, 256, 0, st>>>(d, f);
+    if (cudaGetLastError() != cudaSuccess) return FLEXATTN_ERR_CUDA;
+  }
+  return e;
+}
+#endif  // !FLEXATTN_JIT
+
+}  // namespace flexattn

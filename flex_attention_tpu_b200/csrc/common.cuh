@@ -264,13 +264,16 @@ int launch_sm100_fwd_split(cudaStream_t st, const DevParams& d, int score, int m
 int split_clusters_at_once(int c);  // clusters of c CTAs of that kernel the device holds at a time; 0: unknown
 int launch_sm100_dq(cudaStream_t st, const DevParams& d, int score, int mask);
 int launch_sm100_dkv(cudaStream_t st, const DevParams& d, int score, int mask);
+// delta, dQ, dK and dV in one pass over the tile pairs; no dense bias.  scratch: bwd_fused_scratch_bytes
+int launch_sm100_bwd_fused(cudaStream_t st, const DevParams& d, int score, int mask, void* scratch);
+size_t bwd_fused_scratch_bytes(int slices, int n_qt, int head_dim);
 // ... with a dense bias (d.ab) and / or its gradient (d.dab, dQ only)
 int launch_sm100_fwd_pipe_bias(cudaStream_t st, const DevParams& d, int score, int mask);
 int launch_sm100_dq_bias(cudaStream_t st, const DevParams& d, int score, int mask);
 int launch_sm100_dkv_bias(cudaStream_t st, const DevParams& d, int score, int mask);
 
 // Launch of a kernel compiled at run time around a user score function (jit.cu).  which: 0 forward, 1 dQ, 2 dK/dV, each
-// also in a form for a dense bias, 3 forward for long rows;
+// also in a form for a dense bias, 3 forward for long rows, 4 fused backward;
 // args: the kernel's parameters as for cuLaunchKernel.  Returns a FlexAttnStatus.
 int jit_launch(int which, bool bias, int handle, int head_dim, int mask, unsigned grid_x, unsigned grid_y, unsigned threads,
                size_t smem_bytes, cudaStream_t st, void** args);

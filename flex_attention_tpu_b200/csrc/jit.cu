@@ -81,6 +81,7 @@ struct Driver {
   CUresult (*ModuleUnload)(CUmodule) = nullptr;
   CUresult (*ModuleGetFunction)(CUfunction*, CUmodule, const char*) = nullptr;
   CUresult (*FuncSetAttribute)(CUfunction, CUfunction_attribute, int) = nullptr;
+  CUresult (*FuncGetAttribute)(int*, CUfunction_attribute, CUfunction) = nullptr;
   CUresult (*LaunchKernel)(CUfunction, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, CUstream,
                            void**, void**) = nullptr;
   bool ok = false;
@@ -102,6 +103,7 @@ const Driver& driver() {
     sym(r.ModuleUnload, "cuModuleUnload");
     sym(r.ModuleGetFunction, "cuModuleGetFunction");
     sym(r.FuncSetAttribute, "cuFuncSetAttribute");
+    sym(r.FuncGetAttribute, "cuFuncGetAttribute");
     sym(r.LaunchKernel, "cuLaunchKernel");
     r.ok = all;
     return r;
@@ -135,9 +137,11 @@ UserScore* find(int handle) {
   return u->alive ? u : nullptr;
 }
 
-constexpr int kKernels = 4;  // forward (persistent), dQ, dK/dV, forward for long rows
-const char* const kKernelFile[kKernels] = {"fwd_pipe_sm100.cu", "bwd_dq_sm100.cu", "bwd_dkv_sm100.cu", "fwd_pair_sm100.cu"};
-const char* const kKernelName[kKernels] = {"fwd_pipe_sm100_kernel", "dq_sm100_kernel", "dkv_sm100_kernel", "fwd_pair_sm100_kernel"};
+constexpr int kKernels = 5;  // forward (persistent), dQ, dK/dV, forward for long rows, fused backward
+const char* const kKernelFile[kKernels] = {"fwd_pipe_sm100.cu", "bwd_dq_sm100.cu", "bwd_dkv_sm100.cu", "fwd_pair_sm100.cu",
+                                             "bwd_fused_sm100.cu"};
+const char* const kKernelName[kKernels] = {"fwd_pipe_sm100_kernel", "dq_sm100_kernel", "dkv_sm100_kernel", "fwd_pair_sm100_kernel",
+                                             "fused_sm100_kernel"};
 
 const char* embedded(const char* name) {
   for (int i = 0; i < kEmbeddedCount; ++i)
@@ -232,6 +236,14 @@ int jit_launch(int which, bool bias, int handle, int head_dim, int mask, unsigne
         L = Loaded{};
         return FLEXATTN_ERR_CUDA;
       }
+      // The fused backward hands the registers it was launched with round among its warpgroups; compiled for fewer it would
+      // wait for them without end.
+      int regs = 0;
+      if (which == 4 && (d.FuncGetAttribute(&regs, CU_FUNC_ATTRIBUTE_NUM_REGS, L.fn) != CUDA_SUCCESS || regs < 128)) {
+        d.ModuleUnload(L.module);
+        L = Loaded{};
+        return FLEXATTN_ERR_JIT_COMPILE;
+      }
     }
     if (L.smem_set < smem_bytes) {
       if (d.FuncSetAttribute(L.fn, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, (int)smem_bytes) != CUDA_SUCCESS)
@@ -287,8 +299,8 @@ extern "C" int flexattn_user_score_compile(int32_t handle, int which, int32_t he
   std::lock_guard<std::mutex> lock(g_mu);
   UserScore* u = find(handle);
   if (u == nullptr) return FLEXATTN_ERR_UNSUPPORTED_MOD;
-  // both forms a launch may ask for (the forward for long rows takes no dense bias)
+  // both forms a launch may ask for (the forward for long rows and the fused backward take no dense bias)
   const Compiled* c = nullptr;
   const int e = compile_locked(u, which, false, head_dim, mask_kind, &c);
-  return e != FLEXATTN_OK || which == 3 ? e : compile_locked(u, which, true, head_dim, mask_kind, &c);
+  return e != FLEXATTN_OK || which >= 3 ? e : compile_locked(u, which, true, head_dim, mask_kind, &c);
 }

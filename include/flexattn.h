@@ -177,6 +177,14 @@ int flexattn_bwd_dkv(void* stream, const FlexAttnParams* p);
  * side_stream == stream: everything on that stream.  Needs every pointer the three separate calls need. */
 int flexattn_bwd(void* stream, void* side_stream, const FlexAttnParams* p);
 
+/* The same results as flexattn_bwd (to rounding; they repeat bit for bit) in one pass over the tile pairs: five contractions
+ * per pair instead of seven, everything on `stream`.  For bf16 without a dense bias; needs `scratch` (device memory, 16-byte
+ * aligned, no contents kept between calls) of flexattn_bwd_scratch_bytes(p) bytes, at most about 1 GiB unless one slice needs
+ * more.  That function returns 0 where flexattn_bwd is the call to make: other types, a dense bias, or so few kv tiles that
+ * dQ and dK/dV are better off side by side (FLEXATTN_BWD_KERNEL=fused or =split in the environment decides instead). */
+size_t flexattn_bwd_scratch_bytes(const FlexAttnParams* p);
+int flexattn_bwd_fused(void* stream, const FlexAttnParams* p, void* scratch, size_t scratch_bytes);
+
 /* Forward without any caller-provided scratch memory.  It has no counterpart in the reference.
  *
  * For hosts that cannot allocate device memory and were handed only operands and results: code running
