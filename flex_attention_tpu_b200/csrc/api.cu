@@ -364,7 +364,7 @@ bool fused_pays(const FlexAttnParams* p) {
 
 size_t flexattn_bwd_scratch_bytes(const FlexAttnParams* p) {
   if (validate_common(p) != FLEXATTN_OK || !fused_can(p) || !fused_pays(p)) return 0;
-  return bwd_fused_scratch_bytes(p->batch * p->heads, (p->seq_q + FLEXATTN_TILE - 1) / FLEXATTN_TILE, p->head_dim);
+  return bwd_fused_scratch_bytes(*p);
 }
 
 int flexattn_bwd_fused(void* stream, const FlexAttnParams* p, void* scratch, size_t scratch_bytes) {
@@ -376,7 +376,7 @@ int flexattn_bwd_fused(void* stream, const FlexAttnParams* p, void* scratch, siz
   FLEXATTN_REQUIRE(p->dq); FLEXATTN_REQUIRE(p->dk); FLEXATTN_REQUIRE(p->dv); FLEXATTN_REQUIRE(scratch);
   if (!fused_can(p)) return FLEXATTN_ERR_UNSUPPORTED_BACKEND;
   const DevParams d = make_dev(p);
-  if (scratch_bytes < bwd_fused_scratch_bytes(d.batch * d.heads, d.n_qt, d.head_dim)) return FLEXATTN_ERR_WORKSPACE_TOO_SMALL;
+  if (scratch_bytes < bwd_fused_scratch_bytes(*p)) return FLEXATTN_ERR_WORKSPACE_TOO_SMALL;
   return launch_sm100_bwd_fused(static_cast<cudaStream_t>(stream), d, p->score_kind, p->mask_kind, scratch);
 }
 

@@ -9,7 +9,8 @@
 //   dQ_part = dS K                   A = the dS^T tile read M-major, B = K read MN-major
 //
 // A work item is a 128-row kv tile of one slice; dK and dV stay in tensor memory over its query tiles, dQ_part is added
-// to an f32 scratch in L2 with bulk reductions and becomes bf16 in a last small kernel.  Tensor memory is full at D = 128
+// to an f32 scratch in L2 with bulk reductions.  dq is stored by the CTA with the last part of a query tile,
+// which takes the sum back, or by a small kernel at the end (fused_plan says which).  Tensor memory is full at D = 128
 // (S, dP, dK, dV = 512 columns): dQ_part takes the dP columns, whose dS^T the dK MMA has read by then (MMAs of one thread
 // execute in issue order), and dP of the next tile follows once the drain warps hold dQ_part in registers.  Issue order:
 //
@@ -19,7 +20,8 @@
 // per query tile says which kv tile has been added last; the turn warp waits for the predecessor's.  Items are taken in
 // list order from a ticket counter and wait only for items earlier in the list, which are running or done, so somebody
 // always gets on; under a causal mask the kv tiles of a slice walk along the diagonal one step apart, and the waits are
-// over before they begin.  Slices are taken in groups whose Q, dO and scratch fit L2.
+// over before they begin.  Slices are taken in groups whose Q, dO and scratch fit L2, and the scratch is a ring of a few
+// groups' slices: the first part of a query tile waits until the tile's last user in the ring is done.
 //
 // Persistent: one CTA of 16 warps per SM.  0-7 element-wise (two warpgroups, 64 query columns each), 8-11 drain,
 // 12 MMA issue, 13 loads, 14 turn, 15 publishes flags.
@@ -34,24 +36,27 @@ constexpr int kDrainWarp = 8, kMmaWarp = 12, kTmaWarp = 13, kTurnWarp = 14, kFla
 constexpr int kRegsEw = 152, kRegsDrain = 152, kRegsRest = 56;  // 2 * 152 + 152 + 56 = 4 * 128: what the launch holds
 constexpr int kItemRing = 4;
 constexpr int kFusedId = 7;  // kernel id in the status words
+constexpr int kAllAdded = 0x40000000;
 constexpr uint32_t kSlotBytes = 4096;  // 32 columns of a drain warp's 32 rows; two slots per warp
 
 struct FusedArgs {
-  float* dq_acc;       // [slices][n_qt][128 * D]: element (32 w + lane, 4 c + k) of a tile at ((w * D / 4 + c) * 32 + lane) * 4 + k
-  const float* stats;  // [slices][n_qt][2][128]: -(m log2e + log2 l) pre-scaled for pack_bf16_trunc, delta
-  int32_t* flags;      // [slices][n_qt]: n_kt - (kv tile added last), 0: none
+  float* dq_acc;   // [ring][n_qt][128 * D]: element (32 w + lane, 4 c + k) of a tile at ((w * D / 4 + c) * 32 + lane) * 4 + k
+  float* stats;    // [slices][n_qt][2][128]: -(m log2e + log2 l) pre-scaled for pack_bf16_trunc, delta
+  int32_t* flags;  // [slices][n_qt]: n_kt - (kv tile added last), 0: none, kAllAdded
   int32_t* ticket;
-  int slice0, slices, group;  // slices of this launch (of batch * heads), and how many form a group
+  int slice0, slices;  // slices of this launch (of batch * heads)
+  int group, ring;     // how many of them form a group, and how many the scratch holds
+  int store_dq;        // the last part of a query tile stores dq; otherwise it is added like the others
 };
 
 struct FusedSmem {
   uint64_t bar_k[2], bar_v[2], bar_kfree[2], bar_vfree[2], bar_q[2], bar_do[2], bar_qfree[2], bar_dofree[2];
   uint64_t bar_s, bar_dp, bar_p, bar_ds, bar_dq, bar_drained, bar_accfree, bar_stage[2], bar_stagefree[2];
-  uint64_t bar_turn[2], bar_turnfree[2], bar_red[2], bar_item[kItemRing], bar_itemfree[kItemRing];
+  uint64_t bar_turn[2], bar_turnfree[2], bar_red[2], bar_back[4][2], bar_item[kItemRing], bar_itemfree[kItemRing];
   uint32_t tmem_base;
   alignas(16) int4 item_a[kItemRing];  // {slice of this launch (-1: no more), kv tile, first q tile, end q tile}
   alignas(16) int2 item_b[kItemRing];  // {first fully kept q tile, end of the fully kept run}
-  alignas(16) int4 turn[2];            // {query tile of this launch (-1: no more), first to be added?, flag value, -}
+  alignas(16) int4 turn[2];            // {slice (-1: no more), query tile, 1: first part, 2: last part (or both), flag value}
   alignas(16) float stats[2][2][kTile];
 };
 
@@ -152,6 +157,15 @@ __device__ __forceinline__ int ld_acquire(const int32_t* p) {
 __device__ __forceinline__ void st_release(int32_t* p, int v) {
   asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
+__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {  // does not wait
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred P;\n\tmbarrier.test_wait.parity.shared::cta.b64 P, [%1], %2;\n\tselp.u32 %0, 1, 0, P;\n\t}\n"
+      : "=r"(ok)
+      : "r"(ptx::smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 __device__ __forceinline__ void bulk_load(void* smem_dst, const void* src, uint32_t bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                    ptx::smem_u32(smem_dst)),
@@ -175,12 +189,15 @@ __global__ void __launch_bounds__(kThreads, 1)
     fused_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                        const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                        const __grid_constant__ CUtensorMap tm_dk, const __grid_constant__ CUtensorMap tm_dv,
-                       const DevParams P, const FusedArgs F, int* abort_flag) {
+                       const __grid_constant__ CUtensorMap tm_dq, const DevParams P, const FusedArgs F, int* abort_flag) {
   constexpr int kPanels = D / 64;
   constexpr uint32_t kTileBytes = kPanels * ptx::kPanelBytes;
   // At D = 128 shared memory holds one K, V (those of the next item wait for this one's last MMAs) and one dO, whose two
   // readers dP(n), dV(n) are neighbours on the tensor core: the next one has the time of S, dK, dQ to arrive.
   constexpr int kKvStages = D == 64 ? 2 : 1, kDoStages = D == 64 ? 2 : 1;
+  // dS^T(n) may be written once dQ(n-1) (one tile) or dQ(n-2) (two) has run: dP(n) was issued later, so its completion says so
+  constexpr int kDsStages = D == 64 ? 2 : 1;
+  constexpr uint32_t kDsBytes = 2 * ptx::kPanelBytes;
   constexpr uint32_t kStatBytes = 2 * kTile * sizeof(float);
   constexpr uint32_t kTmemCols = 512;
   constexpr uint32_t kColS = 0, kColDP = 128, kColDK = 256, kColDV = 256 + D;
@@ -194,7 +211,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint8_t* sQ = sV + kKvStages * kTileBytes;   // two stages
   uint8_t* sDO = sQ + 2 * kTileBytes;
   uint8_t* sDS = sDO + kDoStages * kTileBytes;  // dS^T: 128 keys x 128 queries; panel h belongs to warpgroup h
-  uint8_t* sOut = sDS + 2 * ptx::kPanelBytes;   // dQ_part on its way out: two slots per drain warp
+  uint8_t* sOut = sDS + kDsStages * kDsBytes;   // dQ_part on its way out: two slots per drain warp
   FusedSmem* sh = reinterpret_cast<FusedSmem*>(sOut + 8 * kSlotBytes);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -218,6 +235,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       ptx::mbar_init(&sh->bar_turn[s], 1);
       ptx::mbar_init(&sh->bar_turnfree[s], 5);  // four drain warps and the flag warp
       ptx::mbar_init(&sh->bar_red[s], 4);
+      for (int w = 0; w < 4; ++w) ptx::mbar_init(&sh->bar_back[w][s], 1);
     }
     ptx::mbar_init(&sh->bar_s, 1);
     ptx::mbar_init(&sh->bar_dp, 1);
@@ -359,13 +377,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         ptx::mbar_arrive_warp(&sh->bar_p);
 
         load_cols32(stat, delta);
-        if (T > 0) {  // dQ(T - 1) has read the dS^T tile
-          ok = __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_dq, (T - 1) & 1));
-          if (!ok) { fail_at = 14; break; }
-        }
         ok = __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_dp, T & 1));
         if (!ok) { fail_at = 12; break; }
         ptx::tc_fence_after();
+        uint8_t* ds_row = panel_row + (uint32_t)(T % kDsStages) * kDsBytes;
         uint32_t pr[2][32];
         ptx::tmem_ld32(lane_base + colDP, pr[0]);
 #pragma unroll
@@ -380,7 +395,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           ptx::tmem_st16(lane_base + colDP + 16 * g, pk);
 #pragma unroll
           for (int c = 0; c < 4; ++c)
-            *reinterpret_cast<uint4*>(panel_row + (((4 * g + c) ^ (row & 7)) << 4)) =
+            *reinterpret_cast<uint4*>(ds_row + (((4 * g + c) ^ (row & 7)) << 4)) =
                 make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
         }
         ptx::tmem_wait_st();
@@ -391,7 +406,10 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (!ok) break;
       // dK * sm_scale (warpgroup 0) and dV (warpgroup 1) as bf16; the accumulators are free once they are in registers
       if (N > 0) {
-        ok = __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_dq, (T - 1) & 1));  // ... and every MMA before it
+        // dQ of the last tile and every MMA before it.  At D = 64 the dQ before may still be running: a wait by parity has
+        // to take the phases one by one
+        if (kOwnDq && T > 1) ok = __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_dq, T & 1));
+        ok = ok && __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_dq, (T - 1) & 1));
         if (!ok) { fail_at = 15; break; }
         ptx::tc_fence_after();
       }
@@ -437,7 +455,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     uint8_t* slots = sOut + 2 * w * kSlotBytes;
     int T = 0, fail_at = 0;
     bool ok = true, pending = false;
-    // the bulk operations of tile t have completed: the flag warp may say so
+    uint32_t back_phase = 0;
+    // the bulk operations of tile t have completed, the flag warp may say so: one tile later, or at the end of the item
     auto finish = [&](int t) {
       if (lane == 0) {
         ptx::tma_store_wait_all();
@@ -453,7 +472,26 @@ __global__ void __launch_bounds__(kThreads, 1)
       const int4 ia = sh->item_a[r % kItemRing];
       ptx::mbar_arrive_warp(&sh->bar_itemfree[r % kItemRing]);
       if (ia.x < 0) break;
-      for (int qt = ia.z; qt < ia.w && ok; ++qt, ++T) {
+      for (int n = ia.z; n < ia.w && ok; ++n, ++T) {
+        // Last parts: the sum comes back through the slots, 32 columns at a time and two on their way; the first two are asked
+        // for before dQ_part is there, where the turn has come by then.
+        const float* back = nullptr;
+        auto fetch = [&](int c) {
+          if (lane != 0) return;
+          uint64_t* bar = &sh->bar_back[w][c & 1];
+          ptx::mbar_arrive_expect_tx(bar, kSlotBytes);
+          bulk_load(slots + (c & 1) * kSlotBytes, back + c * 1024, kSlotBytes, bar);
+        };
+        auto fetch_first = [&](const int4& turn) {
+          if ((turn.z & 3) == 2 && back == nullptr &&
+              FLEXATTN_DBG_OK((long long)turn.x * P.n_qt + turn.y, (long long)F.slices * P.n_qt, kFusedId, 708)) {
+            back = F.dq_acc + ((size_t)(turn.x % F.ring) * P.n_qt + turn.y) * kTile * D + w * 32 * D;
+            if (lane == 0) ptx::tma_store_wait_read();  // what the slots held has left
+            fetch(0);
+            fetch(1);
+          }
+        };
+        if (__all_sync(0xffffffffu, mbar_test_wait(&sh->bar_turn[T & 1], (T >> 1) & 1))) fetch_first(sh->turn[T & 1]);
         ok = __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_dq, T & 1));
         if (!ok) { fail_at = 31; break; }
         ptx::tc_fence_after();
@@ -469,10 +507,47 @@ __global__ void __launch_bounds__(kThreads, 1)
         ok = __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_turn[T & 1], (T >> 1) & 1));
         if (!ok) { fail_at = 32; break; }
         const int4 turn = sh->turn[T & 1];
+        fetch_first(turn);
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive(&sh->bar_turnfree[T & 1]);
-        if (FLEXATTN_DBG_OK(turn.x, (long long)F.slices * P.n_qt, kFusedId, 705)) {
-          float* dst = F.dq_acc + ((size_t)turn.x * kTile + 32 * w) * D;
+        const bool first = turn.z & 1, last = turn.z & 2;
+        float* tile = F.dq_acc + ((size_t)(turn.x % F.ring) * P.n_qt + turn.y) * kTile * D + w * 32 * D;
+        if (!FLEXATTN_DBG_OK((long long)turn.x * P.n_qt + turn.y, (long long)F.slices * P.n_qt, kFusedId, 705)) {
+        } else if (last) {
+          uint32_t out[D / 2];
+#pragma unroll
+          for (int c = 0; c < D / 32; ++c) {
+            const float4* sum = reinterpret_cast<const float4*>(slots + (c & 1) * kSlotBytes) + lane;
+            if (back != nullptr) ok = ok && __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_back[w][c & 1], back_phase));
+            if (!ok) fail_at = 33;
+#pragma unroll
+            for (int k = 0; k < 32; k += 4) {
+              const float4 a = back == nullptr ? make_float4(0.f, 0.f, 0.f, 0.f) : sum[(k >> 2) * 32];
+              out[16 * c + (k >> 1)] =
+                  ptx::pack_bf16((a.x + __uint_as_float(v[c][k])) * P.sm_scale, (a.y + __uint_as_float(v[c][k + 1])) * P.sm_scale);
+              out[16 * c + (k >> 1) + 1] =
+                  ptx::pack_bf16((a.z + __uint_as_float(v[c][k + 2])) * P.sm_scale, (a.w + __uint_as_float(v[c][k + 3])) * P.sm_scale);
+            }
+            __syncwarp();
+            if (c + 2 < D / 32 && ok && back != nullptr) fetch(c + 2);
+            if ((c & 1) && back != nullptr) back_phase ^= 1;
+          }
+          // dq leaves through the slots too, 64 columns in each; row by row from the registers it would fill the queue
+#pragma unroll
+          for (int p0 = 0; p0 < kPanels; ++p0)
+#pragma unroll
+            for (int c = 0; c < 8; ++c)
+              *reinterpret_cast<uint4*>(slots + p0 * kSlotBytes + lane * 128 + ((c ^ (lane & 7)) << 4)) =
+                  make_uint4(out[32 * p0 + 4 * c], out[32 * p0 + 4 * c + 1], out[32 * p0 + 4 * c + 2], out[32 * p0 + 4 * c + 3]);
+          ptx::fence_proxy_async_smem();
+          __syncwarp();
+          if (ok && lane == 0 && turn.y * kTile + 32 * w < P.seq_q) {
+#pragma unroll
+            for (int p0 = 0; p0 < kPanels; ++p0)
+              ptx::tma_store_3d(&tm_dq, slots + p0 * kSlotBytes, p0 * 64, turn.y * kTile + 32 * w, F.slice0 + turn.x);
+            ptx::tma_store_commit();
+          }
+        } else {
 #pragma unroll
           for (int c = 0; c < D / 32; ++c) {
             uint8_t* slot = slots + (c & 1) * kSlotBytes;
@@ -484,17 +559,16 @@ __global__ void __launch_bounds__(kThreads, 1)
             ptx::fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) {
-              if (turn.y) bulk_store(dst + c * 1024, slot, kSlotBytes);  // the first part of a query tile: nothing to add to
-              else bulk_add_f32(dst + c * 1024, slot, kSlotBytes);
+              if (first) bulk_store(tile + c * 1024, slot, kSlotBytes);  // nothing to add to
+              else bulk_add_f32(tile + c * 1024, slot, kSlotBytes);
               ptx::tma_store_commit();
             }
           }
         }
         pending = true;
-        if (qt + 1 == ia.w) finish(T);
+        if (n + 1 == ia.w) finish(T);
       }
     }
-    if (pending) finish(T - 1);
     if (!ok && lane == 0) give_up(abort_flag, P.status, kFusedId, fail_at);
   } else {
     ptx::setmaxnreg_dec<kRegsRest>();
@@ -677,7 +751,7 @@ __global__ void __launch_bounds__(kThreads, 1)
               ptx::tc_fence_after();
             }
             {  // dQ_part = dS K
-              const ptx::DescBase bDS = mnmajor(aDS), bKt = mnmajor(aK + k_off);
+              const ptx::DescBase bDS = mnmajor(aDS + (uint32_t)(T % kDsStages) * kDsBytes), bKt = mnmajor(aK + k_off);
 #pragma unroll
               for (int kk = 0; kk < kTile / 16; ++kk)
                 ptx::mma_ss(tmem + kColDQ, ptx::desc_at(bDS, ptx::koff_mnmajor(kk)), ptx::desc_at(bKt, ptx::koff_mnmajor(kk)),
@@ -695,11 +769,11 @@ __global__ void __launch_bounds__(kThreads, 1)
       // ---------------------------------------------------------------- whose turn it is at a query tile
       int T = 0, fail_at = 40;
       bool ok = true;
-      auto publish = [&](int tile, int first, int value) {
+      auto publish = [&](int slice, int qt, int which, int value) {
         if (T >= 2) ok = ok && __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_turnfree[T & 1], ((T >> 1) - 1) & 1));
         if (!ok) { fail_at = 41; return; }
         if (lane == 0) {
-          sh->turn[T & 1] = make_int4(tile, first, value, 0);
+          sh->turn[T & 1] = make_int4(slice, qt, which, value);
           ptx::mbar_arrive(&sh->bar_turn[T & 1]);
         }
         __syncwarp();
@@ -711,31 +785,37 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int4 ia = sh->item_a[r % kItemRing];
         ptx::mbar_arrive_warp(&sh->bar_itemfree[r % kItemRing]);
         if (ia.x < 0) {
-          publish(-1, 0, 0);
+          publish(-1, 0, 0, 0);
           break;
         }
-        const int b = (F.slice0 + ia.x) / P.heads;
+        const int b = (F.slice0 + ia.x) / P.heads, kt = ia.y;
         const int4* cmap = P.col_map + (size_t)(P.map_rows > 1 ? b : 0) * P.n_kt;
-        for (int qt = ia.z; qt < ia.w && ok; ++qt) {
-          // the kv tile added before this one: the next higher one that sees the query tile
-          int pred = -1;
-          for (int j0 = ia.y + 1; j0 < P.n_kt && pred < 0; j0 += 32) {
+        // nearest kv tile beyond this one, upwards or downwards, that sees query tile qt; -1: none
+        auto nearest = [&](int qt, int step) {
+          for (int j0 = kt + step; j0 >= 0 && j0 < P.n_kt; j0 += 32 * step) {
+            const int j = j0 + step * lane;
             bool sees = false;
-            if (j0 + lane < P.n_kt) {
-              const int2 range = __ldg(reinterpret_cast<const int2*>(cmap + j0 + lane));
+            if (j >= 0 && j < P.n_kt) {
+              const int2 range = __ldg(reinterpret_cast<const int2*>(cmap + j));
               sees = qt >= range.x && qt < range.y;
             }
             const unsigned any = __ballot_sync(0xffffffffu, sees);
-            if (any) pred = j0 + __ffs(any) - 1;
+            if (any) return j0 + step * (__ffs(any) - 1);
           }
-          const int tile = ia.x * P.n_qt + qt;
-          if (pred >= 0) {
-            const int32_t* flag = F.flags + tile;
-            const int want = P.n_kt - pred;
-            if (FLEXATTN_DBG_OK(tile, (long long)F.slices * P.n_qt, kFusedId, 706) && ld_acquire(flag) < want) {
+          return -1;
+        };
+        for (int qt = ia.z; qt < ia.w && ok; ++qt) {
+          const int pred = nearest(qt, 1);  // its part is added before this one
+          const bool last = F.store_dq && nearest(qt, -1) < 0;
+          // the first part of a tile waits for the slice that had its place in the ring before
+          const int prior = pred >= 0 ? ia.x : ia.x - F.ring;
+          const int want = pred >= 0 ? P.n_kt - pred : kAllAdded;
+          if (prior >= 0) {
+            const long long at = (long long)prior * P.n_qt + qt;
+            if (FLEXATTN_DBG_OK(at, (long long)F.slices * P.n_qt, kFusedId, 706) && ld_acquire(F.flags + at) < want) {
               const unsigned long long t0 = ptx::globaltimer_ns();
               int polls = 0;
-              while (ok && ld_acquire(flag) < want) {
+              while (ok && ld_acquire(F.flags + at) < want) {
                 if ((++polls & 63) == 0 && ptx::globaltimer_ns() - t0 > ptx::kWaitLimitNs) ok = false;
               }
             }
@@ -743,7 +823,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (!ok) { fail_at = 42; break; }
             asm volatile("fence.proxy.async.global;" ::: "memory");  // the parts are added through the async proxy
           }
-          publish(tile, pred < 0, P.n_kt - ia.y);
+          publish(ia.x, qt, (pred < 0 ? 1 : 0) | (last ? 2 : 0), last ? kAllAdded : P.n_kt - kt);
         }
       }
       if (!ok && lane == 0) give_up(abort_flag, P.status, kFusedId, fail_at);
@@ -759,7 +839,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (!ok) break;
         if (lane == 0) {
           __threadfence();  // what the drain warps have added comes before the flag
-          if (FLEXATTN_DBG_OK(turn.x, (long long)F.slices * P.n_qt, kFusedId, 707)) st_release(F.flags + turn.x, turn.z);
+          const long long at = (long long)turn.x * P.n_qt + turn.y;
+          if (FLEXATTN_DBG_OK(at, (long long)F.slices * P.n_qt, kFusedId, 707)) st_release(F.flags + at, turn.w);
           ptx::mbar_arrive(&sh->bar_turnfree[T & 1]);
         }
         __syncwarp();
@@ -778,18 +859,16 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 #ifndef FLEXATTN_JIT
 // Before it: delta = rowsum(o * do) to the caller, both row statistics to the padded tiles the loads take, flags and ticket
-// to zero.  One 16-byte chunk of o and do per thread, as in delta.cu.
+// to zero.  One 16-byte chunk of o and do per thread, as in delta.cu.  A query tile that no kv tile sees gets its zeros here.
 template <int D>
-__global__ void __launch_bounds__(256) prep_kernel(const DevParams P, const FusedArgs F, float* stats) {
-  constexpr int kTpr = D / 8;
-  const long long rows = (long long)F.slices * P.n_qt * kTile;
-  const long long idx = (long long)blockIdx.x * 256 + threadIdx.x, row = idx / kTpr;
-  if (idx <= (long long)F.slices * P.n_qt) F.flags[idx] = 0;  // the ticket is the one behind them
-  float acc = 0.f;
-  const long long slice = row / (P.n_qt * kTile);
-  const int i = (int)(row - slice * (P.n_qt * kTile));
-  const bool live = row < rows && i < P.seq_q;
+__global__ void __launch_bounds__(256) prep_kernel(const DevParams P, const FusedArgs F) {
+  constexpr int kTpr = D / 8, kRows = 256 / kTpr;  // rows of a block: all of one tile
+  const long long row = (long long)blockIdx.x * kRows + threadIdx.x / kTpr;
+  const long long tile = row / kTile, slice = tile / P.n_qt;
+  const int qt = (int)(tile - slice * P.n_qt), i = qt * kTile + (int)(row % kTile);
+  const bool live = i < P.seq_q;
   const long long at = (F.slice0 + slice) * P.seq_q + i;
+  float acc = 0.f;
   if (live) {
     const uint4 a = __ldg(static_cast<const uint4*>(P.o) + at * kTpr + (threadIdx.x & (kTpr - 1)));
     const uint4 b = __ldg(static_cast<const uint4*>(P.d_o) + at * kTpr + (threadIdx.x & (kTpr - 1)));
@@ -804,31 +883,43 @@ __global__ void __launch_bounds__(256) prep_kernel(const DevParams P, const Fuse
   }
 #pragma unroll
   for (int s = kTpr / 2; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
-  if (row < rows && (threadIdx.x & (kTpr - 1)) == 0) {
+  if ((threadIdx.x & (kTpr - 1)) == 0) {
     float nl = -1.0e30f;  // rows past the end and fully masked ones: p = 0
     if (live) {
       P.delta[at] = acc;
       const float l = P.l[at];
       if (l > 0.f) nl = ptx::kRoundLog2 - fmaf(P.m[at], kLog2e, __log2f(l));
     }
-    float* t = stats + (row / kTile) * 2 * kTile + (row % kTile);
+    float* t = F.stats + tile * 2 * kTile + (row % kTile);
     t[0] = nl;
     t[kTile] = acc;
   }
+  if (blockIdx.x % (kTile / kRows) == 0) {  // the first block of a tile
+    const int4* cmap = P.col_map + (size_t)(P.map_rows > 1 ? (F.slice0 + slice) / P.heads : 0) * P.n_kt;
+    bool seen = false;
+    for (int j = threadIdx.x; j < P.n_kt; j += 256) {
+      const int2 range = __ldg(reinterpret_cast<const int2*>(cmap + j));
+      seen = seen || (qt >= range.x && qt < range.y);
+    }
+    seen = __syncthreads_or(seen);
+    if (threadIdx.x == 0) {
+      F.flags[tile] = seen ? 0 : kAllAdded;
+      if (blockIdx.x == 0) *F.ticket = 0;
+    }
+    if (!seen) {
+      const long long first = ((F.slice0 + slice) * P.seq_q + qt * kTile) * kTpr;
+      const int n = min(kTile, P.seq_q - qt * kTile) * kTpr;
+      for (int c = threadIdx.x; c < n; c += 256) static_cast<uint4*>(P.dq)[first + c] = make_uint4(0u, 0u, 0u, 0u);
+    }
+  }
 }
 
-// After it: the f32 tiles become dq, times sm_scale.  A thread takes 16 columns of a row: the loads of a warp are 512
-// consecutive bytes, its stores whole 32-byte sectors.  A query tile no kv tile sees was never written: zero.
+// After it, where the last part of a query tile has been added like the others: the f32 tiles become dq, times sm_scale.  A
+// thread takes 16 columns of a row: the loads of a warp are 512 consecutive bytes, its stores whole 32-byte sectors.
 template <int D>
 __global__ void __launch_bounds__(256) finish_kernel(const DevParams P, const FusedArgs F) {
-  const int tile = blockIdx.x, slice = tile / P.n_qt, qt = tile - slice * P.n_qt, bh = F.slice0 + slice;
-  const int4* cmap = P.col_map + (size_t)(P.map_rows > 1 ? bh / P.heads : 0) * P.n_kt;
-  bool seen = false;
-  for (int j = threadIdx.x; j < P.n_kt; j += 256) {
-    const int2 range = __ldg(reinterpret_cast<const int2*>(cmap + j));
-    seen = seen || (qt >= range.x && qt < range.y);
-  }
-  seen = __syncthreads_or(seen);
+  const int tile = blockIdx.x, slice = tile / P.n_qt, qt = tile - slice * P.n_qt;
+  if (F.flags[tile] == kAllAdded) return;  // no kv tile sees it: zeroed before
   const float* src = F.dq_acc + (size_t)tile * kTile * D;
 #pragma unroll
   for (int e = threadIdx.x; e < kTile * D / 16; e += 256) {
@@ -837,13 +928,12 @@ __global__ void __launch_bounds__(256) finish_kernel(const DevParams P, const Fu
     uint32_t out[8];
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (seen) v = __ldcs(reinterpret_cast<const float4*>(src + ((size_t)(w * (D / 4) + 4 * c16 + c) * 32 + lane) * 4));
+      const float4 v = __ldcs(reinterpret_cast<const float4*>(src + ((size_t)(w * (D / 4) + 4 * c16 + c) * 32 + lane) * 4));
       out[2 * c] = ptx::pack_bf16(v.x * P.sm_scale, v.y * P.sm_scale);
       out[2 * c + 1] = ptx::pack_bf16(v.z * P.sm_scale, v.w * P.sm_scale);
     }
     if (i < P.seq_q) {
-      uint4* dst = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(P.dq) + ((size_t)bh * P.seq_q + i) * D + 16 * c16);
+      uint4* dst = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(P.dq) + ((size_t)(F.slice0 + slice) * P.seq_q + i) * D + 16 * c16);
       dst[0] = make_uint4(out[0], out[1], out[2], out[3]);
       dst[1] = make_uint4(out[4], out[5], out[6], out[7]);
     }
@@ -851,12 +941,12 @@ __global__ void __launch_bounds__(256) finish_kernel(const DevParams P, const Fu
 }
 
 constexpr size_t smem_bytes(int D) {
-  return (size_t)(D == 64 ? 8 : 5) * (D / 64) * ptx::kPanelBytes + 2 * ptx::kPanelBytes + 8 * kSlotBytes + sizeof(FusedSmem);
+  return (size_t)(D == 64 ? 8 : 5) * (D / 64) * ptx::kPanelBytes + (D == 64 ? 4 : 2) * ptx::kPanelBytes + 8 * kSlotBytes + sizeof(FusedSmem);
 }
 static_assert(smem_bytes(128) <= 232448 && smem_bytes(64) <= 232448, "more shared memory than a CTA can have");
 
 struct Maps {
-  CUtensorMap q, d_o, k, v, dk, dv;
+  CUtensorMap q, d_o, k, v, dk, dv, dq;
 };
 
 template <int D, int SK, int MK>
@@ -865,7 +955,7 @@ int launch_one(cudaStream_t st, const DevParams& d, const FusedArgs& f, const Ma
   auto kern = fused_sm100_kernel<D, SK, MK>;
   static SmemAttrOnce attr_once{};  // per kernel instantiation, per device
   if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), (int)smem, &attr_once) != FLEXATTN_OK) return FLEXATTN_ERR_CUDA;
-  kern<<<grid, kThreads, smem, st>>>(t.q, t.d_o, t.k, t.v, t.dk, t.dv, d, f, af);
+  kern<<<grid, kThreads, smem, st>>>(t.q, t.d_o, t.k, t.v, t.dk, t.dv, t.dq, d, f, af);
   return cudaGetLastError() == cudaSuccess ? FLEXATTN_OK : FLEXATTN_ERR_CUDA;
 }
 
@@ -894,32 +984,52 @@ int launch_score(cudaStream_t st, const DevParams& d, int score, int mask, const
   }
 }
 
-// The scratch of a launch, which serves as many slices as keep its f32 tiles within kAccLimit (one, if need be): a larger
-// problem runs in several launches that reuse it, so the scratch does not grow with it.
-constexpr long long kAccLimit = 1ll << 30;
-struct ScratchLayout {
-  int slices;  // of a launch
+// How a call is cut up.
+// Group: what a slice keeps live, 8 bytes per element of a query row (Q, dO, f32 sum), times the group has 48 MB of the 126 MB
+// of L2.  Under a causal window the live rows are the few around the diagonal.
+// store_dq: storing dq with the last part saves the finishing kernel and its pass over the sums, but costs the CTA that
+// does it half a tile's time.  That is a gain where many kv tiles share the work (windows: [4,32,8192,128] with 256 keys 1066
+// -> 970 us; documents: [2,16,16384,128] 1547 -> 1475) and where rows are short ([16,12,512,64] 84 -> 70); under a causal mask
+// or none the one kv tile that every query tile meets last does it all, and long rows wait for it ([2,8,1920,128] 89 -> 107).
+// Then the scratch is a ring of three groups: the one being finished, the one being started, and one between.  Without it the
+// scratch holds every slice of a launch, and there are as many launches as keep it within 1 GiB (one slice, if need be).
+struct FusedPlan {
+  int launch, group, ring, store_dq;  // slices of a launch, ...
   size_t off_stats, off_flags, bytes;
 };
-ScratchLayout scratch_layout(int slices, int n_qt, int head_dim) {
-  ScratchLayout L;
-  const long long acc = (long long)n_qt * kTile * head_dim * 4;
-  const long long most = kAccLimit / acc > 0 ? kAccLimit / acc : 1;
-  const long long launches = (slices + most - 1) / most;
-  L.slices = (int)((slices + launches - 1) / launches);
+FusedPlan fused_plan(int slices, int seq_q, int n_qt, int n_kt, int head_dim, int mask, int window) {
+  constexpr long long kL2Budget = 48ll << 20, kLimit = 1ll << 30;
+  const long long acc = (long long)n_qt * kTile * head_dim * 4, most = kLimit / acc > 0 ? kLimit / acc : 1;
+  const bool windowed = mask == FLEXATTN_MASK_SLIDING_WINDOW_CAUSAL && window < seq_q - 2 * kTile;
+  FusedPlan L;
+  L.store_dq = windowed || mask == FLEXATTN_MASK_DOCUMENT || n_kt <= 8;
+  L.launch = slices;
+  if (!L.store_dq) {
+    const long long launches = (slices + most - 1) / most;
+    L.launch = (int)((slices + launches - 1) / launches);
+  }
+  long long group = kL2Budget / (8ll * (windowed ? window + 2 * kTile : seq_q) * head_dim);
+  if (L.store_dq && 3 * group > most) group = most / 3;
+  if (group < 1) group = 1;
+  if (group > L.launch) group = L.launch;
+  L.group = (int)group;
+  L.ring = L.store_dq && 3 * group < slices ? (int)(3 * group) : L.launch;
   auto up = [](size_t n) { return (n + 255) & ~(size_t)255; };
-  L.off_stats = up((size_t)L.slices * acc);
-  L.off_flags = L.off_stats + up((size_t)L.slices * n_qt * 2 * kTile * sizeof(float));
-  L.bytes = L.off_flags + up(((size_t)L.slices * n_qt + 1) * sizeof(int32_t));
+  L.off_stats = up((size_t)L.ring * acc);
+  L.off_flags = L.off_stats + up((size_t)L.launch * n_qt * 2 * kTile * sizeof(float));
+  L.bytes = L.off_flags + up(((size_t)L.launch * n_qt + 1) * sizeof(int32_t));
   return L;
 }
-constexpr long long kL2Budget = 48ll << 20;  // Q, dO and scratch of a group of slices
 #endif  // !FLEXATTN_JIT
 
 }  // namespace FLEXATTN_TU_NAMESPACE
 
 #ifndef FLEXATTN_JIT
-size_t bwd_fused_scratch_bytes(int slices, int n_qt, int head_dim) { return scratch_layout(slices, n_qt, head_dim).bytes; }
+size_t bwd_fused_scratch_bytes(const FlexAttnParams& p) {
+  return fused_plan(p.batch * p.heads, p.seq_q, (p.seq_q + kTile - 1) / kTile, (p.seq_k + kTile - 1) / kTile, p.head_dim,
+                    p.mask_kind, p.window)
+      .bytes;
+}
 
 int launch_sm100_bwd_fused(cudaStream_t st, const DevParams& d, int score, int mask, void* scratch) {
   int* af = abort_flag_ptr();
@@ -927,7 +1037,8 @@ int launch_sm100_bwd_fused(cudaStream_t st, const DevParams& d, int score, int m
   if (af == nullptr || sms <= 0) return FLEXATTN_ERR_CUDA;
   const int slices = d.batch * d.heads, D = d.head_dim;
   if (D != 64 && D != 128) return FLEXATTN_ERR_UNSUPPORTED_HEAD_DIM;
-  const ScratchLayout L = scratch_layout(slices, d.n_qt, D);
+  const FusedPlan L = fused_plan(slices, d.seq_q, d.n_qt, d.n_kt, D, mask, d.window);
+  if ((long long)L.launch * d.n_kt > 0x7fffffff - 1024 || (long long)L.launch * d.n_qt > 0x7fffffff / 16) return FLEXATTN_ERR_BAD_SHAPE;
   Maps t;
   int e = make_tile_map(&t.q, d.q, slices, d.seq_q, D);
   if (!e) e = make_tile_map(&t.d_o, d.d_o, slices, d.seq_q, D);
@@ -935,31 +1046,31 @@ int launch_sm100_bwd_fused(cudaStream_t st, const DevParams& d, int score, int m
   if (!e) e = make_tile_map(&t.v, d.v, slices, d.seq_k, D);
   if (!e) e = make_tile_map(&t.dk, d.dk, slices, d.seq_k, D);
   if (!e) e = make_tile_map(&t.dv, d.dv, slices, d.seq_k, D);
+  if (!e) e = make_tile_map(&t.dq, d.dq, slices, d.seq_q, D, 32);  // a drain warp's rows
   char* base = static_cast<char*>(scratch);
-  float* stats = reinterpret_cast<float*>(base + L.off_stats);
-  for (int s0 = 0; s0 < slices && !e; s0 += L.slices) {
+  for (int s0 = 0; s0 < slices && !e; s0 += L.launch) {
     FusedArgs f;
     f.dq_acc = reinterpret_cast<float*>(base);
-    f.stats = stats;
+    f.stats = reinterpret_cast<float*>(base + L.off_stats);
     f.flags = reinterpret_cast<int32_t*>(base + L.off_flags);
     f.slice0 = s0;
-    f.slices = slices - s0 < L.slices ? slices - s0 : L.slices;
-    f.ticket = f.flags + (size_t)f.slices * d.n_qt;
-    const long long live = 8ll * d.seq_q * D;  // bytes of Q, dO and scratch of a slice
-    f.group = (int)(kL2Budget / live < 1 ? 1 : kL2Budget / live < f.slices ? kL2Budget / live : f.slices);
-    const long long tiles = (long long)f.slices * d.n_qt, items = (long long)f.slices * d.n_kt;
-    const unsigned prep_blocks = (unsigned)((tiles * kTile * (D / 8) + 255) / 256);
-    if (D == 128) prep_kernel<128><<<prep_blocks, 256, 0, st>>>(d, f, stats);
-    else prep_kernel<64><<<prep_blocks, 256, 0, st>>>(d, f, stats);
+    f.slices = slices - s0 < L.launch ? slices - s0 : L.launch;
+    f.group = L.group;
+    f.ring = L.ring;
+    f.store_dq = L.store_dq;
+    const int tiles = f.slices * d.n_qt, items = f.slices * d.n_kt;
+    f.ticket = f.flags + tiles;
+    if (D == 128) prep_kernel<128><<<tiles * 8u, 256, 0, st>>>(d, f);
+    else prep_kernel<64><<<tiles * 4u, 256, 0, st>>>(d, f);
     if (cudaGetLastError() != cudaSuccess) return FLEXATTN_ERR_CUDA;
     const unsigned grid = (unsigned)(items < sms ? items : sms);
     if (score == FLEXATTN_SCORE_USER) {
-      void* args[] = {&t.q, &t.d_o, &t.k, &t.v, &t.dk, &t.dv, const_cast<DevParams*>(&d), &f, &af};
+      void* args[] = {&t.q, &t.d_o, &t.k, &t.v, &t.dk, &t.dv, &t.dq, const_cast<DevParams*>(&d), &f, &af};
       e = jit_launch(4, false, d.user_score, D, mask, grid, 1, kThreads, smem_bytes(D), st, args);
     } else {
       e = D == 128 ? launch_score<128>(st, d, score, mask, f, t, grid, af) : launch_score<64>(st, d, score, mask, f, t, grid, af);
     }
-    if (e) return e;
+    if (e || f.store_dq) continue;
     if (D == 128) finish_kernel<128><<<(unsigned)tiles, 256, 0, st>>>(d, f);
     else finish_kernel<64><<<(unsigned)tiles, 256, 0, st>>>(d, f);
     if (cudaGetLastError() != cudaSuccess) return FLEXATTN_ERR_CUDA;

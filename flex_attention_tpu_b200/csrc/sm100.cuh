@@ -475,9 +475,9 @@ struct SmemAttrOnce {
 };
 int ensure_dynamic_smem(const void* kernel, int bytes, SmemAttrOnce* once);
 
-// Host side: 3-D tensor map over a [slices, rows, cols] bf16 array, box = {64 cols, 128 rows, 1 slice},
+// Host side: 3-D tensor map over a [slices, rows, cols] bf16 array, box = {64 cols, box_rows rows, 1 slice},
 // 128-byte swizzle, out-of-range rows read as zero.
-int make_tile_map(CUtensorMap* out, const void* base, int slices, int rows, int cols);
+int make_tile_map(CUtensorMap* out, const void* base, int slices, int rows, int cols, int box_rows = kTile);
 #endif  // !FLEXATTN_JIT
 
 // Kernels live in an unnamed namespace in ahead-of-time builds and in a named one when compiled at run time

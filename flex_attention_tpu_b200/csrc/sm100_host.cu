@@ -52,12 +52,12 @@ static EncodeFn encode_fn() {
   return fn;
 }
 
-int make_tile_map(CUtensorMap* out, const void* base, int slices, int rows, int cols) {
+int make_tile_map(CUtensorMap* out, const void* base, int slices, int rows, int cols, int box_rows) {
   EncodeFn fn = encode_fn();
   if (fn == nullptr) return FLEXATTN_ERR_CUDA;
   const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)slices};
   const cuuint64_t strides[2] = {(cuuint64_t)cols * 2, (cuuint64_t)cols * 2 * (cuuint64_t)rows};  // bytes, dims 1..2
-  const cuuint32_t box[3] = {64, (cuuint32_t)kTile, 1};
+  const cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 1};
   const cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,

@@ -1,0 +1,109 @@
+"""The fused backward (dQ, dK and dV in one pass over the tile pairs, dQ added up in an f32 scratch): every mask, both ways
+dq is stored, ragged and rectangular sizes, groups and rings smaller than the problem, query tiles that no key sees, repeats."""
+import ctypes
+import os
+
+import numpy as np
+import pytest
+import torch
+
+import workloads
+
+from helpers import assert_close, build_mods, make_qkvdo, oracle_hot_path, run_hot_path
+from oracle import mha_reference_cpu as oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _fused(fa, q, k, v, do, l, m, o, *, sm, mods, status=None):
+    """The C entry point itself, whatever the sizes: flexattn_bwd_fused with a scratch that starts as NaN."""
+    from flex_attention_tpu_b200 import _binding as B
+    from flex_attention_tpu_b200._resolve import make_problem
+    mf, bf, sf, seg = mods
+    prob = make_problem(q, k, ab=None, segment_ids=seg, causal=False, sm_scale=sm, mask_fn=mf, block_mask_fn=bf, score_fn=sf,
+                        status=status)
+    delta = torch.full(l.shape, float("nan"), device="cuda")
+    dq, dk, dv = (torch.full_like(t, float("nan")) for t in (q, k, v))
+    prob._bind(q=q, k=k, v=v, o=o, d_o=do, l=l, m=m, delta=delta, dq=dq, dk=dk, dv=dv)
+    nbytes = B.lib.flexattn_bwd_scratch_bytes(ctypes.byref(prob.p)) or 64 << 20
+    scratch = torch.full((nbytes // 4,), float("nan"), device="cuda")
+    B.check(B.lib.flexattn_bwd_fused(B._stream_ptr(prob.device), ctypes.byref(prob.p), scratch.data_ptr(), nbytes), "flexattn_bwd_fused")
+    torch.cuda.synchronize()
+    return dict(dq=dq, dk=dk, dv=dv, delta=delta)
+
+
+@pytest.mark.parametrize("B,H,Sq,Sk,D,mask_kind,score_kind", [
+    (1, 1, 1, 1, 128, "none", "none"),                # one row, one key
+    (1, 2, 128, 128, 64, "causal", "none"),           # one tile: its part is the first and the last
+    (1, 3, 129, 257, 128, "none", "softcap"),         # remainders of one row and one key
+    (2, 3, 777, 777, 64, "causal", "alibi"),          # short rows: dq stored with the last part
+    (2, 3, 777, 777, 128, "causal", "softcap"),
+    (1, 2, 1500, 1500, 128, "causal", "none"),        # longer rows: the finishing kernel
+    (1, 2, 1500, 1500, 64, "none", "none"),
+    (1, 3, 100, 1300, 128, "causal", "none"),         # kv tiles without any query: dK = dV = 0
+    (1, 2, 1300, 300, 64, "sliding_window_causal", "none"),   # query tiles without any key: dq = 0
+    (2, 3, 1411, 1411, 128, "sliding_window_causal", "alibi"),
+    (1, 2, 900, 900, 128, "sliding_window", "none"),
+    (2, 2, 1500, 1500, 128, "document", "softcap"),
+    (2, 2, 1500, 1500, 64, "document", "none"),
+    (1, 2, 1300, 1300, 64, "s2", "none"),
+    (1, 2, 1300, 1300, 128, "s2", "alibi"),
+])
+def test_fused_backward(B, H, Sq, Sk, D, mask_kind, score_kind):
+    import flex_attention_tpu_b200 as fa
+    (q, k, v, do), host = make_qkvdo((B, H, Sq, D), (B, H, Sk, D), 700 + Sq, torch.bfloat16)
+    kw = dict(sliding_window=dict(window=300), sliding_window_causal=dict(window=200), s2=dict(window=100, stride=48)).get(mask_kind, {})
+    if mask_kind == "document":
+        kw["doc_ids"] = workloads.draw_documents(np.random.default_rng(Sq), B, Sq, lo=60, hi=500)[0]
+    slopes = oracle.alibi_slopes(H) if score_kind == "alibi" else None
+    cap = 4.0 if score_kind == "softcap" else None
+    sm = 1.0 / np.sqrt(D)
+    fw = run_hot_path(fa, q, k, v, do, sm_scale=sm, mask_kind=mask_kind, score_kind=score_kind, cap=cap or 0.0, slopes=slopes, **kw)
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    mods = build_mods(fa, mask_kind, score_kind, slopes=slopes, cap=cap or 0.0, **kw)
+    got = _fused(fa, q, k, v, do, fw["l"], fw["m"], fw["o"], sm=sm, mods=mods, status=status)
+    assert status.tolist() == [0, 0, 0, 0]
+    rows = slice(0, Sk + 199) if mask_kind == "sliding_window_causal" and Sq > Sk else slice(None)   # fully masked rows: undefined
+    assert all(torch.isfinite(got[n]).all() for n in got)
+    if rows.stop is not None:
+        assert not got["dq"][:, :, (rows.stop + 127) // 128 * 128:].any()
+        fw = {n: (t[:, :, rows] if n in ("o", "l", "m", "dq") else t) for n, t in fw.items()}
+        got["dq"] = got["dq"][:, :, rows]
+        # against the separate kernels: both are within one operand rounding of each other
+        for n in ("dq", "dk", "dv"):
+            assert float((got[n].float() - fw[n].float()).norm() / fw[n].float().norm()) < 1e-2, n
+        return
+    want = oracle_hot_path(*host, sm_scale=sm, mask_kind=mask_kind, score_kind=score_kind, cap=cap, slopes=slopes, **kw)
+    got.update(o=fw["o"], l=fw["l"], m=fw["m"])
+    assert_close(got, want, torch.bfloat16, what=f"fused {Sq}x{Sk}")
+    assert torch.equal(got["delta"], fw["delta"])
+
+
+@pytest.mark.parametrize("B,H,S,D,mask_kind", [
+    (16, 16, 640, 64, "none"),                        # hundreds of items a CTA walks through, dq with the last part
+    (1, 30, 4096, 128, "sliding_window_causal"),      # more slices than the ring of sums holds
+    (3, 2, 16384, 128, "document"),                   # ... with groups of two slices
+    (4, 8, 2048, 128, "causal"),
+])
+def test_fused_backward_repeats_and_agrees(B, H, S, D, mask_kind):
+    """Larger problems, chosen by the library itself: the same bits every time, and the separate kernels' results."""
+    import flex_attention_tpu_b200 as fa
+    from flex_attention_tpu_b200 import _binding
+    (q, k, v, do), _ = make_qkvdo((B, H, S, D), (B, H, S, D), 31, torch.bfloat16)
+    kw = dict(window=300) if mask_kind == "sliding_window_causal" else {}
+    if mask_kind == "document":
+        ids = workloads.draw_documents(np.random.default_rng(5), B, S, lo=100, hi=3000)[0]
+        ids[1] = np.roll(ids[1], S // 3)              # one batch row whose ids come back: compared one by one
+        kw["doc_ids"] = ids
+    sm = 1.0 / np.sqrt(D)
+    fw = run_hot_path(fa, q, k, v, do, sm_scale=sm, mask_kind=mask_kind, **kw)
+    mf, bf, _, seg = build_mods(fa, mask_kind, "none", **kw)
+    args = (q, k, v, fw["o"], fw["l"], fw["m"], do)
+    outs = [fa.flex_attention_bwd(*args, segment_ids=seg, sm_scale=sm, mask_fns=None if mf is None else (mf, bf)) for _ in range(4)]
+    torch.cuda.synchronize()
+    _binding.raise_if_failed(q.device)
+    for r in outs[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(outs[0], r))
+    # dK, dV: the same operations in another order of q tiles at most; dQ: f32 sums of the same bf16 operands
+    for n, t in zip(("dq", "dk", "dv"), outs[0]):
+        assert float((t.float() - fw[n].float()).norm() / fw[n].float().norm()) < 2e-3, n
