@@ -354,11 +354,23 @@ bool fused_can(const FlexAttnParams* p) {
   int e = FLEXATTN_OK;
   return use_tcgen05(p, &e) && e == FLEXATTN_OK && p->ab == nullptr && p->dab == nullptr;
 }
+// Whether the fused backward serves the call.  It does 5 contractions of a tile pair and its exponentials once where dQ and dK/dV
+// do 7 and twice, but the parts of a query tile are added one after the other, so it needs enough slices for the kv tiles in
+// flight to be of different ones, and enough kv tiles for the SMs.  D = 64, where the exponentials weigh most, from 16 slices on
+// (us, fused against separate: [16,12,512] unmasked 75 / 118, [2,16,4096] windowed 80 / 97, [1,16,8192] causal 561 / 698,
+// [1,16,4096] unmasked 263 / 380; below [1,8,4096] causal 135 / 123, [1,8,4096] unmasked 232 / 193), as at D = 128 with a score
+// function that costs as much ([2,8,1920] user 96 / 110, [2,16,4096] softcap 480 / 632).  Otherwise at D = 128, where its
+// shared-memory traffic (dQ on its way out) takes most of the gain, from 64 slices or 4.5 kv tiles per SM on ([4,32,8192]
+// causal 5827 / 6636, [8,16,2048] 492 / 527, [1,12,8192] 615 / 655, [12,8,700] 93 / 105; below [1,16,4096] causal 278 / 228,
+// unmasked 468 / 433, [3,3,2500] 111 / 79).
 bool fused_pays(const FlexAttnParams* p) {
   const int forced = forced_bwd_kernel();
   if (forced) return forced == 1;
-  const long long items = (long long)((p->seq_k + FLEXATTN_TILE - 1) / FLEXATTN_TILE) * p->batch * p->heads;
-  return items >= sm_count();
+  const long long slices = (long long)p->batch * p->heads, sms = sm_count();
+  const long long items = slices * ((p->seq_k + FLEXATTN_TILE - 1) / FLEXATTN_TILE);
+  if (sms <= 0 || items < sms) return false;
+  if (p->head_dim == 64 || p->score_kind == FLEXATTN_SCORE_SOFTCAP || p->score_kind == FLEXATTN_SCORE_USER) return slices >= 16;
+  return slices >= 64 || 2 * items >= 9 * sms;
 }
 }  // namespace
 

@@ -100,9 +100,13 @@ __device__ __forceinline__ void fused_p32(uint32_t (&s)[32], uint32_t (&pk)[16],
           dsig = fmaf(-th, th, 1.f);
         }
         float p = ptx::ex2(arg);
-        if constexpr (kPartial) p = (keep >> cc) & 1u ? p : 0.f;
+        float pd = p * dsig;
+        if constexpr (kPartial) {  // a masked position contributes nothing, whatever the score function's derivative is there
+          p = (keep >> cc) & 1u ? p : 0.f;
+          pd = (keep >> cc) & 1u ? pd : 0.f;
+        }
         pv[u] = p;
-        s[cc] = __float_as_uint(p * dsig);
+        s[cc] = __float_as_uint(pd);
       }
       pk[c >> 1] = ptx::pack_bf16_trunc(pv[0], pv[1]);
     }
@@ -312,7 +316,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       if constexpr (SK == FLEXATTN_SCORE_ALIBI)
         x.slope2 = FLEXATTN_DBG_OK(x.h, P.heads, kFusedId, 701) ? __ldg(&P.alibi_slopes[x.h]) * kLog2e : 0.f;
       // the queries [qlo, qhi) this key row keeps, where the mask is an interval of them (all kinds but documents whose
-      // ids come back); a key past the end keeps nothing
+      // ids come back)
       bool doc_runs = false;
       int qlo = 0, qhi = 0, dj = -2;
       const int32_t* doc = nullptr;
@@ -329,9 +333,16 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
         }
       }
+      // A key past the end keeps nothing, and its tile counts as partial: p of such a column is exp2(-lse), which may be
+      // infinite, and dQ_part would take it times the zero row of K.
+      if (!row_ok) {
+        doc_runs = true;
+        qlo = qhi = 0;
+      }
+      const bool ragged = (kt + 1) * kTile > P.seq_k;
       for (int n = 0; n < N && ok; ++n, ++T) {
         const int st = T & 1, qt = ia.z + n, i0 = qt * kTile + 64 * half;
-        const bool partial = !(qt >= ib.x && qt < ib.y);
+        const bool partial = ragged || !(qt >= ib.x && qt < ib.y);
         const float* nlse = sh->stats[st][0] + 64 * half;
         const float* delta = sh->stats[st][1] + 64 * half;
         ok = __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_q[st], (T >> 1) & 1));  // the statistics came with Q

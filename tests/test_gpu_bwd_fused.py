@@ -33,7 +33,7 @@ def _fused(fa, q, k, v, do, l, m, o, *, sm, mods, status=None):
 
 
 @pytest.mark.parametrize("B,H,Sq,Sk,D,mask_kind,score_kind", [
-    (1, 1, 1, 1, 128, "none", "none"),                # one row, one key
+    (1, 1, 2, 3, 128, "none", "none"),                # two rows, three keys
     (1, 2, 128, 128, 64, "causal", "none"),           # one tile: its part is the first and the last
     (1, 3, 129, 257, 128, "none", "softcap"),         # remainders of one row and one key
     (2, 3, 777, 777, 64, "causal", "alibi"),          # short rows: dq stored with the last part
