@@ -208,8 +208,9 @@ class Problem:
     # Beyond this many a graph builds the map it reads.
     _graph_held = {}
     _GRAPH_HELD_ENTRIES = 256
+    _bwd_scratch = 0   # bytes of scratch the fused backward takes; 0: the separate kernels serve the problem
     _images = {}   # sizes and options -> the parameter struct they give (no pointers in it): filling the fields one by one
-                   # and asking for the workspace size costs a short call more than its launches
+                   # and asking for the sizes of workspace and scratch costs a short call more than its launches
 
     def __init__(self, q, k, *, sm_scale, mask_kind=MASK_NONE, window=0, stride=0, doc_ids=None,
                  score_kind=SCORE_NONE, softcap=0.0, alibi_slopes=None, backend=BACKEND_AUTO, status=None, ab=None,
@@ -459,7 +460,7 @@ class Problem:
         p.delta, p.dq, p.dk, p.dv = delta.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr()
         p.dab = dab.data_ptr() if want_dab else None
         stream = _stream_ptr(self.device)
-        if self._bwd_scratch and self.ab is None:
+        if self._bwd_scratch and self.ab is None:   # one kernel for all three gradients, on one stream
             scratch = torch.empty(self._bwd_scratch, dtype=torch.uint8, device=self.device)
             check_user(lib.flexattn_bwd_fused(stream, ctypes.byref(p), scratch.data_ptr(), self._bwd_scratch),
                        "flexattn_bwd_fused", p.user_score)
