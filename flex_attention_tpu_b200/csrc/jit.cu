@@ -293,14 +293,16 @@ extern "C" const char* flexattn_user_score_log(int32_t handle) {
 }
 
 extern "C" int flexattn_user_score_compile(int32_t handle, int which, int32_t head_dim, int32_t mask_kind) {
-  if (which < 0 || which >= kKernels) return FLEXATTN_ERR_UNSUPPORTED_MOD;
+  if (which < 0 || which > 3) return FLEXATTN_ERR_UNSUPPORTED_MOD;
   if (head_dim != 64 && head_dim != 128) return FLEXATTN_ERR_UNSUPPORTED_HEAD_DIM;
   if (mask_kind < FLEXATTN_MASK_NONE || mask_kind > FLEXATTN_MASK_S2) return FLEXATTN_ERR_UNSUPPORTED_MOD;
   std::lock_guard<std::mutex> lock(g_mu);
   UserScore* u = find(handle);
   if (u == nullptr) return FLEXATTN_ERR_UNSUPPORTED_MOD;
-  // both forms a launch may ask for (the forward for long rows and the fused backward take no dense bias)
+  // every form a launch may ask for: with a dense bias too (the forward for long rows takes none), and with dK/dV the fused
+  // backward, which serves in its place
   const Compiled* c = nullptr;
-  const int e = compile_locked(u, which, false, head_dim, mask_kind, &c);
-  return e != FLEXATTN_OK || which >= 3 ? e : compile_locked(u, which, true, head_dim, mask_kind, &c);
+  int e = compile_locked(u, which, false, head_dim, mask_kind, &c);
+  if (e == FLEXATTN_OK && which == 2) e = compile_locked(u, 4, false, head_dim, mask_kind, &c);
+  return e != FLEXATTN_OK || which == 3 ? e : compile_locked(u, which, true, head_dim, mask_kind, &c);
 }
