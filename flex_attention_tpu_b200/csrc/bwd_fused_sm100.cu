@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     x.capl2 = P.cap * kLog2e;
     x.csc = (SK == FLEXATTN_SCORE_SOFTCAP) ? P.sm_scale / P.cap : 0.f;
     const long long n_doc = (long long)P.batch * P.doc_stride;
-    int T = 0, stores = 0, fail_at = 0;
+    int T = 0, u = 0, stores = 0, fail_at = 0;
     bool ok = true;
     // one 64-column panel of this warpgroup, already written, leaves through a bulk store; the panel is free on return
     auto store_panel = [&](const CUtensorMap* tm, int col, int kt, int bh) {
@@ -417,11 +417,13 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (!ok) break;
       // dK * sm_scale (warpgroup 0) and dV (warpgroup 1) as bf16; the accumulators are free once they are in registers
       if (N > 0) {
-        // dQ of the last tile and every MMA before it.  At D = 64 the dQ before may still be running: a wait by parity has
-        // to take the phases one by one
-        if (kOwnDq && T > 1) ok = __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_dq, T & 1));
-        ok = ok && __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_dq, (T - 1) & 1));
+        // The last dQ of the item, and with it every MMA before: K has been read.  A wait by parity must not come a phase late, and
+        // how late these warps get here is not bounded; this barrier has one phase per item that uses the stage, and its next one
+        // needs their P.  (bar_dq, with a phase per tile, may be one or two further on.)
+        if constexpr (kDebugChecks) __nanosleep(20000);  // the bounds-checked build always gets here late
+        ok = __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_kfree[u % kKvStages], (u / kKvStages) & 1));
         if (!ok) { fail_at = 15; break; }
+        ++u;
         ptx::tc_fence_after();
       }
       uint32_t out[D / 2];
