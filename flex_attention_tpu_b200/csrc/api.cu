@@ -37,12 +37,18 @@ int validate_common(const FlexAttnParams* p) {
   return FLEXATTN_OK;
 }
 
-int validate_mods(const FlexAttnParams* p) {
+int validate_window(const FlexAttnParams* p) {
   const int mk = p->mask_kind;
   if ((mk == FLEXATTN_MASK_SLIDING_WINDOW || mk == FLEXATTN_MASK_SLIDING_WINDOW_CAUSAL || mk == FLEXATTN_MASK_S2) &&
       p->window <= 0)
     return FLEXATTN_ERR_UNSUPPORTED_MOD;
   if (mk == FLEXATTN_MASK_S2 && p->stride <= 0) return FLEXATTN_ERR_UNSUPPORTED_MOD;
+  return FLEXATTN_OK;
+}
+
+int validate_mods(const FlexAttnParams* p) {
+  const int mk = p->mask_kind, e = validate_window(p);
+  if (e) return e;
   if (mk == FLEXATTN_MASK_DOCUMENT && p->doc_ids == nullptr) return FLEXATTN_ERR_NULL_POINTER;
   if (p->score_kind == FLEXATTN_SCORE_ALIBI && p->alibi_slopes == nullptr) return FLEXATTN_ERR_NULL_POINTER;
   if (p->score_kind == FLEXATTN_SCORE_SOFTCAP && !(p->softcap > 0.f)) return FLEXATTN_ERR_UNSUPPORTED_MOD;
@@ -375,7 +381,8 @@ bool fused_pays(const FlexAttnParams* p) {
 }  // namespace
 
 size_t flexattn_bwd_scratch_bytes(const FlexAttnParams* p) {
-  if (validate_common(p) != FLEXATTN_OK || !fused_can(p) || !fused_pays(p)) return 0;
+  // (asked before the pointers are bound, so not all of `prologue`; the numbers below divide by the window)
+  if (validate_common(p) != FLEXATTN_OK || validate_window(p) != FLEXATTN_OK || !fused_can(p) || !fused_pays(p)) return 0;
   return bwd_fused_scratch_bytes(*p);
 }
 

@@ -2,6 +2,9 @@
 import ctypes
 import os
 import re
+import subprocess
+import sys
+import textwrap
 
 import pytest
 
@@ -82,6 +85,29 @@ def test_argument_validation_needs_no_gpu(B):
     assert B.lib.flexattn_fwd(None, ref) == 10                            # tcgen05 cannot serve f32
     assert B.lib.flexattn_bwd_preprocess(None, ref) == 1                  # do missing
     assert B.lib.flexattn_bwd(None, None, ref) == 1                       # ... refused before anything is launched
+
+
+def test_bwd_scratch_bytes_of_a_window_that_no_call_accepts():
+    """Every problem asks for this size before its mask is checked.  In a process of its own, with the fused backward for all
+    sizes: where a size is computed from such a window, the process may not survive it."""
+    code = textwrap.dedent("""
+        import ctypes
+        from flex_attention_tpu_b200 import _binding as B
+        p = B.FlexAttnParams()
+        p.batch, p.heads, p.seq_q, p.seq_k, p.head_dim = 8, 16, 2048, 2048, 128
+        sizes = []
+        for kind in (B.MASK_SLIDING_WINDOW, B.MASK_SLIDING_WINDOW_CAUSAL, B.MASK_S2):
+            p.mask_kind, p.stride = kind, 64
+            for p.window in (-(1 << 31), -257, -256, -255, -1, 0, 256):
+                sizes.append(B.lib.flexattn_bwd_scratch_bytes(ctypes.byref(p)) > 0)
+                assert B.lib.flexattn_fwd(None, ctypes.byref(p)) == (7 if p.window <= 0 else 1)   # bad window / no workspace
+        p.stride = 0
+        sizes.append(B.lib.flexattn_bwd_scratch_bytes(ctypes.byref(p)) > 0)
+        print(sizes == 3 * (6 * [False] + [True]) + [False])
+    """)
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, cwd=ROOT, timeout=300,
+                       env=dict(os.environ, FLEXATTN_BWD_KERNEL="fused"))
+    assert r.returncode == 0 and r.stdout.strip() == "True", (r.returncode, r.stdout, r.stderr[-2000:])
 
 
 def test_python_layer_rejects_what_the_kernels_cannot_run():
