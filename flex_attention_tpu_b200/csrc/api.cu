@@ -361,22 +361,64 @@ bool fused_can(const FlexAttnParams* p) {
   return use_tcgen05(p, &e) && e == FLEXATTN_OK && p->ab == nullptr && p->dab == nullptr;
 }
 // Whether the fused backward serves the call.  It does 5 contractions of a tile pair and its exponentials once where dQ and dK/dV
-// do 7 and twice, but the parts of a query tile are added one after the other, so it needs enough slices for the kv tiles in
-// flight to be of different ones, and enough kv tiles for the SMs.  D = 64, where the exponentials weigh most, from 16 slices on
-// (us, fused against separate: [16,12,512] unmasked 75 / 118, [2,16,4096] windowed 80 / 97, [1,16,8192] causal 561 / 698,
-// [1,16,4096] unmasked 263 / 380; below [1,8,4096] causal 135 / 123, [1,8,4096] unmasked 232 / 193), as at D = 128 with a score
-// function that costs as much ([2,8,1920] user 96 / 110, [2,16,4096] softcap 480 / 632).  Otherwise at D = 128, where its
-// shared-memory traffic (dQ on its way out) takes most of the gain, from 64 slices or 4.5 kv tiles per SM on ([4,32,8192]
-// causal 5827 / 6636, [8,16,2048] 492 / 527, [1,12,8192] 615 / 655, [12,8,700] 93 / 105; below [1,16,4096] causal 278 / 228,
-// unmasked 468 / 433, [3,3,2500] 111 / 79).
+// do 7 and twice, but the parts of a query tile are added one after the other: a kv tile has to stay some 2.4 tiles behind the
+// one before it in its slice.  `slack`, the query tiles a CTA walks per kv tile of the slice that is in flight, says whether
+// there is room for that.  Times in us, fused / separate, on 148 SMs; slices x queries x keys.
+// D = 64, where the exponentials weigh most:
+//   no mask     slack 2.6: 24 x 2048 127 / 159, 192 x 256 31 / 44; 1.7: 16 x 2048 128 / 111, 32 x 1024 x 8192 398 / 383;
+//               0.1: 16 x 128 x 8192 211 / 87.  Chains of few parts need less: 64 x 512 40 / 45, 48 x 512 37 / 37
+//   causal, S2  24 x 1024 43 / 43, 28 x 1000 43 / 48, 16 x 2048 78 / 79; 16 x 1536 65 / 54, 18 x 1152 52 / 41
+//   windows and documents, 16 slices on: 16 x 1280 25 / 30 and 33 / 36
+//   softcap and user functions (more per pair, the same chain): 16 x 2048 unmasked 131 / 148, 32 x 720 53 / 56;
+//               32 x 237 x 8081 303 / 185
+// D = 128, where its shared-memory traffic (dQ on its way out) takes most of the gain:
+//   no mask     128 x 1024 240 / 269, 12 x 8192 1159 / 1260, 160 x 512 x 64 53 / 61; 64 x 1024 147 / 130, 6 x 15360 1983 / 1897,
+//               32 x 2048 x 8192 976 / 870, 8 x 32768 15154 / 11871, 96 x 1024 x 384 107 / 95
+//   causal, S2  128 x 8192 6340 / 6970, 24 x 8192 1290 / 1357, 96 x 256 34 / 38; 16 x 16384 3453 / 3259, 9 x 16384 2100 / 1927,
+//               64 x 873 90 / 87, 64 x 1024 x 512 81 / 74
+//   windows and documents: 128 x 2048 documents 349 / 406, 32 x 4096 with 256 keys 143 / 148
+//   softcap     16 x 2048 causal 103 / 113, 40 x 512 38 / 39, 64 x 512 unmasked 57 / 63; 16 x 1536 causal 82 / 74,
+//               24 x 1024 unmasked 86 / 74, 64 x 14683 x 492 causal 1307 / 1205
+//   a window open ahead: 256 x 528 207 / 240; 128 x 4096 2154 / 2013
+//   user functions: none (16 x 2048 causal 113 / 108, unmasked 170 / 155; 64 x 4096 1099 / 1072, 1833 / 1910)
+// Either: 72 x 445 x 18173 causal 192 / 304, 64 x 256 x 8960 with 267 keys 66 / 113 (most kv tiles see no query);
+//         16 x 496 x 1206 causal 33 / 29, 24 x 264 x 4885 45 / 41
 bool fused_pays(const FlexAttnParams* p) {
   const int forced = forced_bwd_kernel();
   if (forced) return forced == 1;
   const long long slices = (long long)p->batch * p->heads, sms = sm_count();
-  const long long items = slices * ((p->seq_k + FLEXATTN_TILE - 1) / FLEXATTN_TILE);
-  if (sms <= 0 || items < sms) return false;
-  if (p->head_dim == 64 || p->score_kind == FLEXATTN_SCORE_SOFTCAP || p->score_kind == FLEXATTN_SCORE_USER) return slices >= 16;
-  return slices >= 64 || 2 * items >= 9 * sms;
+  if (sms <= 0 || slices < 1) return false;
+  const long long n_qt = (p->seq_q + FLEXATTN_TILE - 1) / FLEXATTN_TILE, n_kt = (p->seq_k + FLEXATTN_TILE - 1) / FLEXATTN_TILE;
+  const int mask = p->mask_kind;
+  const bool common_start = mask == FLEXATTN_MASK_NONE || mask == FLEXATTN_MASK_SLIDING_WINDOW;  // every kv tile begins at query 0
+  const bool long_rows = mask == FLEXATTN_MASK_CAUSAL || mask == FLEXATTN_MASK_S2;  // ... along the diagonal, all to the last query
+  const bool scored = p->score_kind == FLEXATTN_SCORE_SOFTCAP || p->score_kind == FLEXATTN_SCORE_USER;
+  const long long items = slices * (common_start || n_kt < n_qt ? n_kt : n_qt);  // kv tiles that see a query
+  // many kv tiles that see no query: the fused kernel only stores their zeros
+  if (!common_start && n_kt >= 3 * n_qt && slices >= 16 && slices * n_kt >= 7 * sms)
+    return p->head_dim == 64 || p->score_kind != FLEXATTN_SCORE_USER;
+  if (items < sms) return false;
+  const double slack = bwd_fused_slack(*p, (int)sms);
+  if (p->head_dim == 64) {
+    if (common_start) {
+      if (scored) return slices >= 16 && slack >= 1.1;
+      return slices >= 16 && (slack >= 2 || slices >= sms || (slack >= 1.25 && slices >= 8 * n_kt));
+    }
+    if (long_rows && !scored) return slices >= 24 || (slices >= 16 && slack >= 1.7);
+    return slices >= 16;
+  }
+  const bool few = slices < sms && items < 5 * sms;
+  if (p->score_kind == FLEXATTN_SCORE_USER) return false;
+  if (scored) {
+    if (slices < 16 || (n_qt > 2 * n_kt && few)) return false;
+    return common_start ? slack >= 1.7 || slices >= sms : slices >= 40 || 5 * items >= 8 * sms;
+  }
+  if (mask == FLEXATTN_MASK_SLIDING_WINDOW) return slices >= sms && n_qt <= 8;
+  if (slices >= sms && (slack >= 2.1 || n_qt <= 32)) return true;
+  if (n_qt > n_kt && few && (common_start || long_rows)) return false;
+  if (common_start) return slices >= 12 && slack >= 2.2 && 2 * items >= 5 * sms;
+  if (slices >= (long_rows ? 96 : 64)) return true;
+  return 2 * items >= 9 * sms && (long_rows ? slices >= 24 && slack >= 2.2 : slices >= 16);
 }
 }  // namespace
 

@@ -1038,10 +1038,20 @@ FusedPlan fused_plan(int slices, int seq_q, int n_qt, int n_kt, int head_dim, in
 }  // namespace FLEXATTN_TU_NAMESPACE
 
 #ifndef FLEXATTN_JIT
-size_t bwd_fused_scratch_bytes(const FlexAttnParams& p) {
+namespace {
+FusedPlan plan_of(const FlexAttnParams& p) {
   return fused_plan(p.batch * p.heads, p.seq_q, (p.seq_q + kTile - 1) / kTile, (p.seq_k + kTile - 1) / kTile, p.head_dim,
-                    p.mask_kind, p.window)
-      .bytes;
+                    p.mask_kind, p.window);
+}
+}  // namespace
+
+size_t bwd_fused_scratch_bytes(const FlexAttnParams& p) { return plan_of(p).bytes; }
+
+// A group of `width` slices on `sms` CTAs has sms / width kv tiles of each slice in flight (the groups of a launch taken as equal)
+double bwd_fused_slack(const FlexAttnParams& p, int sms) {
+  const FusedPlan L = plan_of(p);
+  const double width = (double)L.launch / ((L.launch + L.group - 1) / L.group);
+  return (p.seq_q + kTile - 1) / kTile * width / sms;
 }
 
 int launch_sm100_bwd_fused(cudaStream_t st, const DevParams& d, int score, int mask, void* scratch) {

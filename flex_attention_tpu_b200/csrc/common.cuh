@@ -267,6 +267,7 @@ int launch_sm100_dkv(cudaStream_t st, const DevParams& d, int score, int mask);
 // delta, dQ, dK and dV in one pass over the tile pairs; no dense bias.  scratch: bwd_fused_scratch_bytes
 int launch_sm100_bwd_fused(cudaStream_t st, const DevParams& d, int score, int mask, void* scratch);
 size_t bwd_fused_scratch_bytes(const FlexAttnParams& p);
+double bwd_fused_slack(const FlexAttnParams& p, int sms);  // query tiles a CTA walks per kv tile of its slice in flight
 // ... with a dense bias (d.ab) and / or its gradient (d.dab, dQ only)
 int launch_sm100_fwd_pipe_bias(cudaStream_t st, const DevParams& d, int score, int mask);
 int launch_sm100_dq_bias(cudaStream_t st, const DevParams& d, int score, int mask);
