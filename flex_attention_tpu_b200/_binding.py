@@ -460,8 +460,13 @@ class Problem:
         p.delta, p.dq, p.dk, p.dv = delta.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr()
         p.dab = dab.data_ptr() if want_dab else None
         stream = _stream_ptr(self.device)
-        if self._bwd_scratch and self.ab is None:   # one kernel for all three gradients, on one stream
-            scratch = torch.empty(self._bwd_scratch, dtype=torch.uint8, device=self.device)
+        scratch = None
+        if self._bwd_scratch and self.ab is None:
+            try:
+                scratch = torch.empty(self._bwd_scratch, dtype=torch.uint8, device=self.device)
+            except torch.OutOfMemoryError:   # the separate kernels need none
+                pass
+        if scratch is not None:   # one kernel for all three gradients, on one stream
             check_user(lib.flexattn_bwd_fused(stream, ctypes.byref(p), scratch.data_ptr(), self._bwd_scratch),
                        "flexattn_bwd_fused", p.user_score)
             return delta, dq, dk, dv

@@ -179,9 +179,11 @@ int flexattn_bwd(void* stream, void* side_stream, const FlexAttnParams* p);
 
 /* The same results as flexattn_bwd (to rounding; they repeat bit for bit) in one pass over the tile pairs: five contractions
  * per pair instead of seven, everything on `stream`.  For bf16 without a dense bias; needs `scratch` (device memory, 16-byte
- * aligned, no contents kept between calls) of flexattn_bwd_scratch_bytes(p) bytes, at most about 1 GiB unless one slice needs
- * more.  That function returns 0 where flexattn_bwd is the call to make: other types, a dense bias, or so few kv tiles that
- * dQ and dK/dV are better off side by side (FLEXATTN_BWD_KERNEL=fused or =split in the environment decides instead). */
+ * aligned, no contents kept between calls) of flexattn_bwd_scratch_bytes(p) bytes: the f32 sums of dQ, at most 1 GiB of them
+ * (unless one slice needs more, under a causal window or documents three), and 1 KB per 128 query rows.  A host without room
+ * for it calls flexattn_bwd, which needs none.  The size is 0 where flexattn_bwd is the call to make: other types, a dense
+ * bias, a window no call accepts, or sizes at which dQ and dK/dV side by side are faster (FLEXATTN_BWD_KERNEL=fused or =split
+ * in the environment decides instead). */
 size_t flexattn_bwd_scratch_bytes(const FlexAttnParams* p);
 int flexattn_bwd_fused(void* stream, const FlexAttnParams* p, void* scratch, size_t scratch_bytes);
 

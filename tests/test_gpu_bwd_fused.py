@@ -130,3 +130,22 @@ def test_which_backward_serves_a_call(B, H, Sq, Sk, D, mask_kind, score_kind, fu
     p.batch, p.heads, p.seq_q, p.seq_k, p.head_dim, p.window, p.stride = B, H, Sq, Sk, D, 256, 64
     p.mask_kind, p.score_kind = _binding.MASK_KIND_IDS[mask_kind], _binding.SCORE_KIND_IDS[score_kind]
     assert (_binding.lib.flexattn_bwd_scratch_bytes(ctypes.byref(p)) > 0) == fused
+
+
+def test_a_scratch_that_does_not_fit():
+    """... leaves the call to the separate kernels: memory for the results, but not for the sums of dQ."""
+    import flex_attention_tpu_b200 as fa
+    B, H, S, D = 8, 16, 2048, 128
+    (q, k, v, do), _ = make_qkvdo((B, H, S, D), (B, H, S, D), 8, torch.bfloat16)
+    fw = run_hot_path(fa, q, k, v, do, sm_scale=0.09, mask_kind="causal")
+    args, kw = (q, k, v, fw["o"], fw["l"], fw["m"], do), dict(sm_scale=0.09, mask_fns=fa.masks.make_causal_mask_fns(128, 128))
+    total = torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.empty_cache()
+    try:   # dq, dk, dv and delta take 194 MiB, the scratch 130
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (260 << 20)) / total)
+        got = fa.flex_attention_bwd(*args, **kw)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    torch.cuda.synchronize()
+    assert all(torch.equal(t, fw[n]) for n, t in zip(("dq", "dk", "dv"), got))
+    assert not torch.equal(fa.flex_attention_bwd(*args, **kw)[0], fw["dq"])   # with room: sums in another order

@@ -1,4 +1,4 @@
-"""What a problem keeps alive, without a GPU: a fake library in the place of the kernels."""
+"""What a problem keeps alive, and which backward it calls, without a GPU: a fake library in the place of the kernels."""
 import gc
 import weakref
 
@@ -10,11 +10,21 @@ from flex_attention_tpu_b200.flex_attention import _FlexAttentionFn
 
 
 class FakeLib:
+    fused_status = 0
+
+    def __init__(self):
+        self.calls = []
+
     def flexattn_fwd(self, stream, ref):
         return 0
 
     def flexattn_bwd(self, stream, side, ref):
+        self.calls.append("separate")
         return 0
+
+    def flexattn_bwd_fused(self, stream, ref, scratch, nbytes):
+        self.calls.append("fused")
+        return self.fused_status
 
 
 @pytest.fixture
@@ -42,3 +52,24 @@ def test_a_training_step_leaves_nothing_for_the_garbage_collector(prob):
         assert [r() is None for r in gone] == [True] * 4
     finally:
         gc.enable()
+
+
+def _backward(prob):
+    t = torch.zeros(1, 2, 8, 64, dtype=torch.bfloat16)
+    r = torch.zeros(1, 2, 8)
+    return prob.backward(t, t, t, t, t, r, r)
+
+
+def test_a_backward_whose_scratch_does_not_fit_runs_the_separate_kernels(prob, monkeypatch):
+    """A call fits where its operands and results do: those kernels take no scratch."""
+    empty = torch.empty
+    prob._bwd_scratch = 12345
+    _backward(prob)
+
+    def full(size, **kw):
+        if size == 12345:
+            raise torch.OutOfMemoryError("no room")
+        return empty(size, **kw)
+    monkeypatch.setattr(torch, "empty", full)
+    assert [tuple(t.shape) for t in _backward(prob)] == [(1, 2, 8)] + 3 * [(1, 2, 8, 64)]
+    assert B.lib.calls == ["fused", "separate"]
