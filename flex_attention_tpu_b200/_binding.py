@@ -467,9 +467,10 @@ class Problem:
             except torch.OutOfMemoryError:   # the separate kernels need none
                 pass
         if scratch is not None:   # one kernel for all three gradients, on one stream
-            check_user(lib.flexattn_bwd_fused(stream, ctypes.byref(p), scratch.data_ptr(), self._bwd_scratch),
-                       "flexattn_bwd_fused", p.user_score)
-            return delta, dq, dk, dv
+            code = lib.flexattn_bwd_fused(stream, ctypes.byref(p), scratch.data_ptr(), self._bwd_scratch)
+            if code not in (10, 13):   # those: not built for this call, and nothing launched
+                check(code, "flexattn_bwd_fused")
+                return delta, dq, dk, dv
         side = _side_stream(self.device).cuda_stream if two_streams else stream
         try:
             check_user(lib.flexattn_bwd(stream, side, ctypes.byref(p)), "flexattn_bwd", p.user_score)

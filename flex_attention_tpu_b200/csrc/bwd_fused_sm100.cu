@@ -962,12 +962,19 @@ struct Maps {
   CUtensorMap q, d_o, k, v, dk, dv, dq;
 };
 
+// grid 0: only prepares the kernel and says whether it can be launched
 template <int D, int SK, int MK>
 int launch_one(cudaStream_t st, const DevParams& d, const FusedArgs& f, const Maps& t, unsigned grid, int* af) {
   constexpr size_t smem = smem_bytes(D);
   auto kern = fused_sm100_kernel<D, SK, MK>;
+  static const bool whole_file = [kern] {  // compiled for fewer registers than its warpgroups hand round, it would wait without end
+    cudaFuncAttributes a;
+    return cudaFuncGetAttributes(&a, reinterpret_cast<const void*>(kern)) == cudaSuccess && a.numRegs >= 128;
+  }();
+  if (!whole_file) return FLEXATTN_ERR_UNSUPPORTED_BACKEND;
   static SmemAttrOnce attr_once{};  // per kernel instantiation, per device
   if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), (int)smem, &attr_once) != FLEXATTN_OK) return FLEXATTN_ERR_CUDA;
+  if (grid == 0) return FLEXATTN_OK;
   kern<<<grid, kThreads, smem, st>>>(t.q, t.d_o, t.k, t.v, t.dk, t.dv, t.dq, d, f, af);
   return cudaGetLastError() == cudaSuccess ? FLEXATTN_OK : FLEXATTN_ERR_CUDA;
 }
@@ -1070,6 +1077,10 @@ int launch_sm100_bwd_fused(cudaStream_t st, const DevParams& d, int score, int m
   if (!e) e = make_tile_map(&t.dk, d.dk, slices, d.seq_k, D);
   if (!e) e = make_tile_map(&t.dv, d.dv, slices, d.seq_k, D);
   if (!e) e = make_tile_map(&t.dq, d.dq, slices, d.seq_q, D, 32);  // a drain warp's rows
+  auto launch = [&](const FusedArgs& f, unsigned grid) {
+    return D == 128 ? launch_score<128>(st, d, score, mask, f, t, grid, af) : launch_score<64>(st, d, score, mask, f, t, grid, af);
+  };
+  if (!e) e = score == FLEXATTN_SCORE_USER ? jit_fused_ready(d.user_score, D, mask, smem_bytes(D), st) : launch(FusedArgs{}, 0);
   char* base = static_cast<char*>(scratch);
   for (int s0 = 0; s0 < slices && !e; s0 += L.launch) {
     FusedArgs f;
@@ -1091,7 +1102,7 @@ int launch_sm100_bwd_fused(cudaStream_t st, const DevParams& d, int score, int m
       void* args[] = {&t.q, &t.d_o, &t.k, &t.v, &t.dk, &t.dv, &t.dq, const_cast<DevParams*>(&d), &f, &af};
       e = jit_launch(4, false, d.user_score, D, mask, grid, 1, kThreads, smem_bytes(D), st, args);
     } else {
-      e = D == 128 ? launch_score<128>(st, d, score, mask, f, t, grid, af) : launch_score<64>(st, d, score, mask, f, t, grid, af);
+      e = launch(f, grid);
     }
     if (e || f.store_dq) continue;
     if (D == 128) finish_kernel<128><<<(unsigned)tiles, 256, 0, st>>>(d, f);

@@ -278,6 +278,9 @@ int launch_sm100_dkv_bias(cudaStream_t st, const DevParams& d, int score, int ma
 // args: the kernel's parameters as for cuLaunchKernel.  Returns a FlexAttnStatus.
 int jit_launch(int which, bool bias, int handle, int head_dim, int mask, unsigned grid_x, unsigned grid_y, unsigned threads,
                size_t smem_bytes, cudaStream_t st, void** args);
+// Compiles and loads the fused backward for a user score function where that is still to do.  FLEXATTN_ERR_JIT_COMPILE: it
+// cannot serve the call (nothing has been launched), the separate kernels may.
+int jit_fused_ready(int handle, int head_dim, int mask, size_t smem_bytes, cudaStream_t st);
 #endif  // !FLEXATTN_JIT
 
 }  // namespace flexattn

@@ -15,8 +15,10 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <set>
 #include <string>
 #include <tuple>
+#include <utility>
 #include <vector>
 
 #include "common.cuh"
@@ -125,6 +127,7 @@ struct UserScore {
   std::string score, dscore, log;
   std::map<std::tuple<int, bool, int, int>, Compiled> compiled;   // (which, dense bias, head_dim, mask)
   std::map<std::tuple<int, bool, int, int, int>, Loaded> loaded;  // (which, dense bias, head_dim, mask, device)
+  std::set<std::pair<int, int>> no_fused;  // (head_dim, mask) the fused backward cannot be compiled for: not tried again
   bool alive = true;
 };
 
@@ -138,6 +141,7 @@ UserScore* find(int handle) {
 }
 
 constexpr int kKernels = 5;  // forward (persistent), dQ, dK/dV, forward for long rows, fused backward
+constexpr int kFusedKernel = 4;
 const char* const kKernelFile[kKernels] = {"fwd_pipe_sm100.cu", "bwd_dq_sm100.cu", "bwd_dkv_sm100.cu", "fwd_pair_sm100.cu",
                                              "bwd_fused_sm100.cu"};
 const char* const kKernelName[kKernels] = {"fwd_pipe_sm100_kernel", "dq_sm100_kernel", "dkv_sm100_kernel", "fwd_pair_sm100_kernel",
@@ -212,48 +216,77 @@ int compile_locked(UserScore* u, int which, bool bias, int head_dim, int mask, c
 
 }  // namespace
 
-int jit_launch(int which, bool bias, int handle, int head_dim, int mask, unsigned grid_x, unsigned grid_y, unsigned threads,
-               size_t smem_bytes, cudaStream_t st, void** args) {
-  if (which < 0 || which >= kKernels) return FLEXATTN_ERR_UNSUPPORTED_MOD;
+namespace {
+// The kernel, compiled and loaded where it was not yet.  Caller holds g_mu.
+int load_locked(UserScore* u, int which, bool bias, int head_dim, int mask, size_t smem_bytes, CUfunction* fn) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return FLEXATTN_ERR_CUDA;
   const Driver& d = driver();
   if (!d.ok) return FLEXATTN_ERR_JIT_UNAVAILABLE;
+  Loaded& L = u->loaded[std::make_tuple(which, bias, head_dim, mask, dev)];
+  if (L.fn == nullptr) {
+    const Compiled* c = nullptr;
+    const int e = compile_locked(u, which, bias, head_dim, mask, &c);
+    if (e != FLEXATTN_OK) return e;
+    if (cudaFree(nullptr) != cudaSuccess) return FLEXATTN_ERR_CUDA;  // the runtime's context is current from here on
+    if (d.ModuleLoadData(&L.module, c->cubin.data()) != CUDA_SUCCESS) return FLEXATTN_ERR_CUDA;
+    if (d.ModuleGetFunction(&L.fn, L.module, c->lowered.c_str()) != CUDA_SUCCESS) {
+      d.ModuleUnload(L.module);
+      L = Loaded{};
+      return FLEXATTN_ERR_CUDA;
+    }
+    // The fused backward hands the registers it was launched with round among its warpgroups; compiled for fewer it would
+    // wait for them without end.
+    int regs = 0;
+    if (which == kFusedKernel && (d.FuncGetAttribute(&regs, CU_FUNC_ATTRIBUTE_NUM_REGS, L.fn) != CUDA_SUCCESS || regs < 128)) {
+      d.ModuleUnload(L.module);
+      L = Loaded{};
+      return FLEXATTN_ERR_JIT_COMPILE;
+    }
+  }
+  if (L.smem_set < smem_bytes) {
+    if (d.FuncSetAttribute(L.fn, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, (int)smem_bytes) != CUDA_SUCCESS)
+      return FLEXATTN_ERR_CUDA;
+    L.smem_set = smem_bytes;
+  }
+  *fn = L.fn;
+  return FLEXATTN_OK;
+}
+}  // namespace
+
+int jit_fused_ready(int handle, int head_dim, int mask, size_t smem_bytes, cudaStream_t st) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return FLEXATTN_ERR_CUDA;
+  std::lock_guard<std::mutex> lock(g_mu);
+  UserScore* u = find(handle);
+  if (u == nullptr) return FLEXATTN_ERR_UNSUPPORTED_MOD;
+  const auto key = std::make_pair(head_dim, mask);
+  if (u->no_fused.count(key)) return FLEXATTN_ERR_JIT_COMPILE;
+  const auto it = u->loaded.find(std::make_tuple(kFusedKernel, false, head_dim, mask, dev));
+  if (it == u->loaded.end() || it->second.fn == nullptr) {  // under capture nothing can be loaded; the others may be there
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) return FLEXATTN_ERR_CUDA;
+    if (cap != cudaStreamCaptureStatusNone) return FLEXATTN_ERR_JIT_COMPILE;
+  }
+  CUfunction fn = nullptr;
+  const int e = load_locked(u, kFusedKernel, false, head_dim, mask, smem_bytes, &fn);
+  if (e == FLEXATTN_ERR_JIT_COMPILE) u->no_fused.insert(key);
+  return e;
+}
+
+int jit_launch(int which, bool bias, int handle, int head_dim, int mask, unsigned grid_x, unsigned grid_y, unsigned threads,
+               size_t smem_bytes, cudaStream_t st, void** args) {
+  if (which < 0 || which >= kKernels) return FLEXATTN_ERR_UNSUPPORTED_MOD;
   CUfunction fn = nullptr;
   {
     std::lock_guard<std::mutex> lock(g_mu);
     UserScore* u = find(handle);
     if (u == nullptr) return FLEXATTN_ERR_UNSUPPORTED_MOD;
-    Loaded& L = u->loaded[std::make_tuple(which, bias, head_dim, mask, dev)];
-    if (L.fn == nullptr) {
-      const Compiled* c = nullptr;
-      const int e = compile_locked(u, which, bias, head_dim, mask, &c);
-      if (e != FLEXATTN_OK) return e;
-      if (cudaFree(nullptr) != cudaSuccess) return FLEXATTN_ERR_CUDA;  // the runtime's context is current from here on
-      if (d.ModuleLoadData(&L.module, c->cubin.data()) != CUDA_SUCCESS) return FLEXATTN_ERR_CUDA;
-      if (d.ModuleGetFunction(&L.fn, L.module, c->lowered.c_str()) != CUDA_SUCCESS) {
-        d.ModuleUnload(L.module);
-        L = Loaded{};
-        return FLEXATTN_ERR_CUDA;
-      }
-      // The fused backward hands the registers it was launched with round among its warpgroups; compiled for fewer it would
-      // wait for them without end.
-      int regs = 0;
-      if (which == 4 && (d.FuncGetAttribute(&regs, CU_FUNC_ATTRIBUTE_NUM_REGS, L.fn) != CUDA_SUCCESS || regs < 128)) {
-        d.ModuleUnload(L.module);
-        L = Loaded{};
-        return FLEXATTN_ERR_JIT_COMPILE;
-      }
-    }
-    if (L.smem_set < smem_bytes) {
-      if (d.FuncSetAttribute(L.fn, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, (int)smem_bytes) != CUDA_SUCCESS)
-        return FLEXATTN_ERR_CUDA;
-      L.smem_set = smem_bytes;
-    }
-    fn = L.fn;
+    const int e = load_locked(u, which, bias, head_dim, mask, smem_bytes, &fn);
+    if (e != FLEXATTN_OK) return e;
   }
-  const CUresult r = d.LaunchKernel(fn, grid_x, grid_y, 1, threads, 1, 1, (unsigned)smem_bytes,
-                                    reinterpret_cast<CUstream>(st), args, nullptr);
+  const CUresult r = driver().LaunchKernel(fn, grid_x, grid_y, 1, threads, 1, 1, (unsigned)smem_bytes,
+                                           reinterpret_cast<CUstream>(st), args, nullptr);
   return r == CUDA_SUCCESS ? FLEXATTN_OK : FLEXATTN_ERR_CUDA;
 }
 
@@ -299,10 +332,12 @@ extern "C" int flexattn_user_score_compile(int32_t handle, int which, int32_t he
   std::lock_guard<std::mutex> lock(g_mu);
   UserScore* u = find(handle);
   if (u == nullptr) return FLEXATTN_ERR_UNSUPPORTED_MOD;
-  // every form a launch may ask for: with a dense bias too (the forward for long rows takes none), and with dK/dV the fused
-  // backward, which serves in its place
+  // every form a launch may ask for: with a dense bias too (the forward for long rows takes none), and before dK/dV the fused
+  // backward, which serves in its place where it compiles
   const Compiled* c = nullptr;
-  int e = compile_locked(u, which, false, head_dim, mask_kind, &c);
-  if (e == FLEXATTN_OK && which == 2) e = compile_locked(u, 4, false, head_dim, mask_kind, &c);
+  if (which == 2 && u->no_fused.count({head_dim, mask_kind}) == 0 &&
+      compile_locked(u, kFusedKernel, false, head_dim, mask_kind, &c) == FLEXATTN_ERR_JIT_COMPILE)
+    u->no_fused.insert({head_dim, mask_kind});
+  const int e = compile_locked(u, which, false, head_dim, mask_kind, &c);
   return e != FLEXATTN_OK || which == 3 ? e : compile_locked(u, which, true, head_dim, mask_kind, &c);
 }

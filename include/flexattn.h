@@ -183,7 +183,9 @@ int flexattn_bwd(void* stream, void* side_stream, const FlexAttnParams* p);
  * (unless one slice needs more, under a causal window or documents three), and 1 KB per 128 query rows.  A host without room
  * for it calls flexattn_bwd, which needs none.  The size is 0 where flexattn_bwd is the call to make: other types, a dense
  * bias, a window no call accepts, or sizes at which dQ and dK/dV side by side are faster (FLEXATTN_BWD_KERNEL=fused or =split
- * in the environment decides instead). */
+ * in the environment decides instead).  FLEXATTN_ERR_JIT_COMPILE (a user score function this kernel cannot be compiled around,
+ * or not while the stream is captured) and FLEXATTN_ERR_UNSUPPORTED_BACKEND: nothing was launched, flexattn_bwd may serve
+ * the call. */
 size_t flexattn_bwd_scratch_bytes(const FlexAttnParams* p);
 int flexattn_bwd_fused(void* stream, const FlexAttnParams* p, void* scratch, size_t scratch_bytes);
 
@@ -242,7 +244,7 @@ int flexattn_user_score_destroy(int32_t handle);
 const char* flexattn_user_score_log(int32_t handle);
 /* Compiles (without loading or launching: needs no GPU) the kernel `which` (0 forward, 1 dQ, 2 dK/dV, 3 forward for long rows) for the
  * handle, head_dim and mask_kind, exactly as the first launch would: the form without and, but for 3, the form with a dense
- * bias.  Returns FLEXATTN_OK, or FLEXATTN_ERR_JIT_COMPILE / FLEXATTN_ERR_JIT_UNAVAILABLE.  A test and warm-up hook. */
+ * bias; with 2 the fused backward too, whose failure is not one of the call (flexattn_bwd_fused reports it).  Returns FLEXATTN_OK, or FLEXATTN_ERR_JIT_COMPILE / FLEXATTN_ERR_JIT_UNAVAILABLE.  A test and warm-up hook. */
 int flexattn_user_score_compile(int32_t handle, int which, int32_t head_dim, int32_t mask_kind);
 
 /* Clears the calling device's abort word (stream-ordered memset on `stream`), re-enabling the tensor-core

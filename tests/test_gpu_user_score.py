@@ -96,3 +96,52 @@ def test_user_score_with_a_dense_bias(mask_kind, Sq, Sk, D):
                  what=f"user score with bias {mask_kind}/D{D}")
     e = errors(dab, rdab)   # float32, but delta comes from the bf16-rounded o: the relative bound of the bias tests
     assert e["max_rel"] <= 1e-2, e
+
+
+def _call(S, spec=None):
+    """A causal call at D = 64 that the library gives to the fused backward: its arguments and the separate kernels' gradients."""
+    import flex_attention_tpu_b200 as fa
+    from flex_attention_tpu_b200._resolve import make_problem
+    (q, k, v, do), _ = make_qkvdo((2, 8, S, 64), (2, 8, S, 64), 1500 + S, torch.bfloat16)
+    sf = fa.util.make_jax_score_fn(_distance_and_head)
+    if spec is not None:
+        sf.spec = spec
+    fns = fa.masks.make_causal_mask_fns(128, 128)
+    want = run_hot_path(fa, q, k, v, do, sm_scale=0.125, mask_kind="causal", score_kind="user", user_fn=sf)
+    prob = make_problem(q, k, ab=None, segment_ids=None, causal=False, sm_scale=0.125, mask_fn=fns[0], block_mask_fn=fns[1], score_fn=sf)
+    assert prob._bwd_scratch > 0
+    args = (q, k, v, want["o"], want["l"], want["m"], do)
+    return (lambda: fa.flex_attention_bwd(*args, sm_scale=0.125, mask_fns=fns, score_fn=sf)), [want[n] for n in ("dq", "dk", "dv")], prob
+
+
+def test_user_score_through_the_fused_backward():
+    from flex_attention_tpu_b200 import _binding as B
+    backward, want, prob = _call(2048)
+    first, second = backward(), backward()
+    torch.cuda.synchronize()
+    B.raise_if_failed(prob.device)
+    assert all(torch.equal(a, b) for a, b in zip(first, second))
+    for got, ref in zip(first, want):   # the same operands in another order of summation
+        assert float((got.float() - ref.float()).norm() / ref.float().norm()) < 2e-3
+    assert not torch.equal(first[0], want[0])
+
+
+def test_a_function_the_fused_backward_cannot_be_compiled_around():
+    from test_user_score import only_the_fused_backward_fails
+    from flex_attention_tpu_b200.scores import ScoreSpec
+    backward, want, _ = _call(2050, ScoreSpec("user", expr=only_the_fused_backward_fails().decode(), dexpr="1.0f"))
+    for _ in range(2):
+        assert all(torch.equal(a, b) for a, b in zip(backward(), want))
+
+
+def test_a_captured_backward_whose_fused_kernel_is_not_loaded():
+    """Nothing can be loaded during a capture: dQ and dK/dV, which an earlier call has loaded, are recorded."""
+    from flex_attention_tpu_b200.scores import ScoreSpec
+    backward, want, _ = _call(2060, ScoreSpec("user", expr="0.75f * s - 0.01f * fabsf((float)(i - j))", dexpr="0.75f"))
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        out = backward()
+    g.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(out, want))
+    assert not torch.equal(backward()[0], want[0])   # outside: the fused kernel

@@ -26,6 +26,9 @@ class FakeLib:
         self.calls.append("fused")
         return self.fused_status
 
+    def flexattn_status_string(self, code):
+        return b"a status"
+
 
 @pytest.fixture
 def prob(monkeypatch):
@@ -73,3 +76,13 @@ def test_a_backward_whose_scratch_does_not_fit_runs_the_separate_kernels(prob, m
     monkeypatch.setattr(torch, "empty", full)
     assert [tuple(t.shape) for t in _backward(prob)] == [(1, 2, 8)] + 3 * [(1, 2, 8, 64)]
     assert B.lib.calls == ["fused", "separate"]
+
+
+def test_a_fused_backward_that_was_not_built_for_the_call(prob):
+    prob._bwd_scratch = 256
+    B.lib.fused_status = 13                 # a user score function it cannot be compiled around
+    assert len(_backward(prob)) == 4 and B.lib.calls == ["fused", "separate"]
+    B.lib.fused_status = 8
+    with pytest.raises(B.FlexAttnError):
+        _backward(prob)
+    assert B.lib.calls == ["fused", "separate", "fused"]

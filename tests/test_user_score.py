@@ -96,3 +96,21 @@ def test_the_warm_up_hook_compiles_the_dense_bias_form_as_well():
     if 12 in codes:
         pytest.skip("libnvrtc is not installed here")
     assert codes == [13, 13, 13, 0], log.decode()      # (the forward for long rows has no such form)
+
+
+def only_the_fused_backward_fails():
+    """A score function none of whose kernels but the fused backward minds that a name of it is taken."""
+    return b"s); }\n#define kAllAdded (\n__device__ __forceinline__ float user_score_unused(float s) { return (s"
+
+
+def test_the_warm_up_hook_does_without_the_fused_backward():
+    """dQ and dK/dV serve a function that kernel cannot be compiled around."""
+    from flex_attention_tpu_b200 import _binding as B
+    h = ctypes.c_int32(0)
+    assert B.lib.flexattn_user_score_create(only_the_fused_backward_fails(), b"1.0f", ctypes.byref(h)) == 0
+    codes = [B.lib.flexattn_user_score_compile(h.value, which, 64, B.MASK_NONE) for which in (1, 2, 2)]
+    log = B.lib.flexattn_user_score_log(h.value)
+    B.lib.flexattn_user_score_destroy(h.value)
+    if 12 in codes:
+        pytest.skip("libnvrtc is not installed here")
+    assert codes == [0, 0, 0], log.decode()
