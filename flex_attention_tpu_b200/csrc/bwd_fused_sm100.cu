@@ -32,7 +32,7 @@ namespace flexattn {
 namespace FLEXATTN_TU_NAMESPACE {
 
 constexpr int kThreads = 512;
-constexpr int kDrainWarp = 8, kMmaWarp = 12, kTmaWarp = 13, kTurnWarp = 14, kFlagWarp = 15;
+constexpr int kDrainWarp = 8, kMmaWarp = 12, kTmaWarp = 13, kTurnWarp = 14;  // 15: flags
 constexpr int kRegsEw = 152, kRegsDrain = 152, kRegsRest = 56;  // 2 * 152 + 152 + 56 = 4 * 128: what the launch holds
 constexpr int kItemRing = 4;
 constexpr int kFusedId = 7;  // kernel id in the status words
@@ -280,14 +280,15 @@ __global__ void __launch_bounds__(kThreads, 1)
     x.capl2 = P.cap * kLog2e;
     x.csc = (SK == FLEXATTN_SCORE_SOFTCAP) ? P.sm_scale / P.cap : 0.f;
     const long long n_doc = (long long)P.batch * P.doc_stride;
-    int T = 0, u = 0, stores = 0, fail_at = 0;
+    int T = 0, u = 0, fail_at = 0;
     bool ok = true;
-    // one 64-column panel of this warpgroup, already written, leaves through a bulk store; the panel is free on return
-    auto store_panel = [&](const CUtensorMap* tm, int col, int kt, int bh) {
+    // one 64-column panel of this warpgroup, already written, leaves through a bulk store; the panel is free on return.
+    // phase: of the panels so far
+    auto store_panel = [&](const CUtensorMap* tm, int col, int kt, int bh, uint32_t phase) {
       ptx::fence_proxy_async_smem();
       ptx::mbar_arrive_warp(&sh->bar_stage[half]);
       if ((warp & 3) == 0) {
-        ok = __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_stage[half], stores & 1));
+        ok = __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_stage[half], phase));
         if (ok && lane == 0) {
           ptx::tma_store_3d(tm, panel, col, kt * kTile, bh);
           ptx::tma_store_commit();
@@ -296,9 +297,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         __syncwarp();
       }
-      ok = ok && __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_stagefree[half], stores & 1));
+      ok = ok && __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_stagefree[half], phase));
       if (!ok) fail_at = 13;
-      ++stores;
     };
     for (int r = 0; ok; ++r) {
       ok = __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_item[r % kItemRing], (r / kItemRing) & 1));
@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int c = 0; c < 8; ++c)
           *reinterpret_cast<uint4*>(panel_row + ((c ^ (row & 7)) << 4)) =
               make_uint4(out[32 * p0 + 4 * c], out[32 * p0 + 4 * c + 1], out[32 * p0 + 4 * c + 2], out[32 * p0 + 4 * c + 3]);
-        if (ok) store_panel(half ? &tm_dv : &tm_dk, p0 * 64, kt, bh);
+        if (ok) store_panel(half ? &tm_dv : &tm_dk, p0 * 64, kt, bh, (r * kPanels + p0) & 1);
       }
     }
     if (!ok && lane == 0) give_up(abort_flag, P.status, kFusedId, fail_at);
@@ -625,8 +625,9 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int st = (T + n) & 1;
             if (T + n >= 2) ok = ok && ptx::mbar_wait_relaxed(&sh->bar_qfree[st], (((T + n) >> 1) - 1) & 1, 20);
             if (!ok) return;
-            load_tile(sQ + st * kTileBytes, &tm_q, &sh->bar_q[st], (cm.x + n) * kTile, bh, kStatBytes);
-            bulk_load(sh->stats[st], F.stats + ((size_t)slice * P.n_qt + cm.x + n) * 2 * kTile, kStatBytes, &sh->bar_q[st]);
+            const bool in = FLEXATTN_DBG_OK((long long)slice * P.n_qt + cm.x + n, (long long)F.slices * P.n_qt, kFusedId, 709);
+            load_tile(sQ + st * kTileBytes, &tm_q, &sh->bar_q[st], (cm.x + n) * kTile, bh, in ? kStatBytes : 0);
+            if (in) bulk_load(sh->stats[st], F.stats + ((size_t)slice * P.n_qt + cm.x + n) * 2 * kTile, kStatBytes, &sh->bar_q[st]);
           };
           auto load_do = [&](int n) {
             const int st = (T + n) % kDoStages;
@@ -879,8 +880,9 @@ __global__ void __launch_bounds__(256) prep_kernel(const DevParams P, const Fuse
   const long long row = (long long)blockIdx.x * kRows + threadIdx.x / kTpr;
   const long long tile = row / kTile, slice = tile / P.n_qt;
   const int qt = (int)(tile - slice * P.n_qt), i = qt * kTile + (int)(row % kTile);
-  const bool live = i < P.seq_q;
   const long long at = (F.slice0 + slice) * P.seq_q + i;
+  const bool live = i < P.seq_q && FLEXATTN_DBG_OK(at, (long long)P.batch * P.heads * P.seq_q, kFusedId, 710);
+  const bool in = FLEXATTN_DBG_OK(tile, (long long)F.slices * P.n_qt, kFusedId, 711);
   float acc = 0.f;
   if (live) {
     const uint4 a = __ldg(static_cast<const uint4*>(P.o) + at * kTpr + (threadIdx.x & (kTpr - 1)));
@@ -903,11 +905,13 @@ __global__ void __launch_bounds__(256) prep_kernel(const DevParams P, const Fuse
       const float l = P.l[at];
       if (l > 0.f) nl = ptx::kRoundLog2 - fmaf(P.m[at], kLog2e, __log2f(l));
     }
-    float* t = F.stats + tile * 2 * kTile + (row % kTile);
-    t[0] = nl;
-    t[kTile] = acc;
+    if (in) {
+      float* t = F.stats + tile * 2 * kTile + (row % kTile);
+      t[0] = nl;
+      t[kTile] = acc;
+    }
   }
-  if (blockIdx.x % (kTile / kRows) == 0) {  // the first block of a tile
+  if (blockIdx.x % (kTile / kRows) == 0 && in) {  // the first block of a tile
     const int4* cmap = P.col_map + (size_t)(P.map_rows > 1 ? (F.slice0 + slice) / P.heads : 0) * P.n_kt;
     bool seen = false;
     for (int j = threadIdx.x; j < P.n_kt; j += 256) {
@@ -922,7 +926,9 @@ __global__ void __launch_bounds__(256) prep_kernel(const DevParams P, const Fuse
     if (!seen) {
       const long long first = ((F.slice0 + slice) * P.seq_q + qt * kTile) * kTpr;
       const int n = min(kTile, P.seq_q - qt * kTile) * kTpr;
-      for (int c = threadIdx.x; c < n; c += 256) static_cast<uint4*>(P.dq)[first + c] = make_uint4(0u, 0u, 0u, 0u);
+      for (int c = threadIdx.x; c < n; c += 256)
+        if (FLEXATTN_DBG_OK(first + c, (long long)P.batch * P.heads * P.seq_q * kTpr, kFusedId, 712))
+          static_cast<uint4*>(P.dq)[first + c] = make_uint4(0u, 0u, 0u, 0u);
     }
   }
 }
@@ -932,6 +938,7 @@ __global__ void __launch_bounds__(256) prep_kernel(const DevParams P, const Fuse
 template <int D>
 __global__ void __launch_bounds__(256) finish_kernel(const DevParams P, const FusedArgs F) {
   const int tile = blockIdx.x, slice = tile / P.n_qt, qt = tile - slice * P.n_qt;
+  if (!FLEXATTN_DBG_OK(tile, (long long)F.slices * P.n_qt, kFusedId, 713)) return;
   if (F.flags[tile] == kAllAdded) return;  // no kv tile sees it: zeroed before
   const float* src = F.dq_acc + (size_t)tile * kTile * D;
 #pragma unroll
@@ -945,7 +952,7 @@ __global__ void __launch_bounds__(256) finish_kernel(const DevParams P, const Fu
       out[2 * c] = ptx::pack_bf16(v.x * P.sm_scale, v.y * P.sm_scale);
       out[2 * c + 1] = ptx::pack_bf16(v.z * P.sm_scale, v.w * P.sm_scale);
     }
-    if (i < P.seq_q) {
+    if (i < P.seq_q && FLEXATTN_DBG_OK((long long)(F.slice0 + slice) * P.seq_q + i, (long long)P.batch * P.heads * P.seq_q, kFusedId, 714)) {
       uint4* dst = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(P.dq) + ((size_t)(F.slice0 + slice) * P.seq_q + i) * D + 16 * c16);
       dst[0] = make_uint4(out[0], out[1], out[2], out[3]);
       dst[1] = make_uint4(out[4], out[5], out[6], out[7]);

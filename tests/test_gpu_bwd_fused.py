@@ -79,34 +79,46 @@ def test_fused_backward(B, H, Sq, Sk, D, mask_kind, score_kind):
     assert torch.equal(got["delta"], fw["delta"])
 
 
-@pytest.mark.parametrize("B,H,S,D,mask_kind", [
-    (16, 16, 640, 64, "none"),                        # hundreds of items a CTA walks through, dq with the last part
-    (1, 30, 4096, 128, "sliding_window_causal"),      # more slices than the ring of sums holds
-    (3, 2, 16384, 128, "document"),                   # ... with groups of two slices
-    (4, 8, 2048, 128, "causal"),
+@pytest.mark.parametrize("B,H,S,D,mask_kind,sums", [
+    (16, 16, 640, 64, "none", 256),                   # hundreds of items a CTA walks through, dq with the last part
+    (4, 70, 700, 128, "sliding_window_causal", 264),  # fewer sums than slices: a slice takes the place of one 264 before
+    (1, 16, 16384, 128, "document", 9),               # ... of one nine before, in groups of three
+    (4, 24, 1152, 128, "causal", 96),                 # the finishing kernel
+    (5, 104, 8192, 64, "causal", 260),                # ... of two launches
 ])
-def test_fused_backward_repeats_and_agrees(B, H, S, D, mask_kind):
-    """Larger problems, chosen by the library itself: the same bits every time, and the separate kernels' results."""
+def test_fused_backward_repeats_and_agrees(B, H, S, D, mask_kind, sums):
+    """Larger problems, given to the fused backward by the library itself (sums: slices its scratch holds the f32 sums of dQ of):
+    the same bits every time, and the separate kernels' results."""
     import flex_attention_tpu_b200 as fa
     from flex_attention_tpu_b200 import _binding
-    (q, k, v, do), _ = make_qkvdo((B, H, S, D), (B, H, S, D), 31, torch.bfloat16)
+    from flex_attention_tpu_b200._resolve import make_problem
+    g = torch.Generator(device="cuda").manual_seed(31)
+    q, k, v, do = (torch.randn((B, H, S, D), generator=g, device="cuda", dtype=torch.bfloat16) for _ in range(4))
     kw = dict(window=300) if mask_kind == "sliding_window_causal" else {}
     if mask_kind == "document":
         ids = workloads.draw_documents(np.random.default_rng(5), B, S, lo=100, hi=3000)[0]
-        ids[1] = np.roll(ids[1], S // 3)              # one batch row whose ids come back: compared one by one
+        ids[0] = np.roll(ids[0], S // 3)              # ids that come back: compared one by one
         kw["doc_ids"] = ids
     sm = 1.0 / np.sqrt(D)
-    fw = run_hot_path(fa, q, k, v, do, sm_scale=sm, mask_kind=mask_kind, **kw)
     mf, bf, _, seg = build_mods(fa, mask_kind, "none", **kw)
+    prob = make_problem(q, k, ab=None, segment_ids=seg, causal=False, sm_scale=sm, mask_fn=mf, block_mask_fn=bf, score_fn=None)
+    tiles = (S + 127) // 128
+    launch = sums if mask_kind in ("none", "causal") else B * H   # the statistics of a launch: 1 KB a tile, and its flag
+    assert prob._bwd_scratch == sums * tiles * 128 * D * 4 + launch * tiles * 1024 + -(-(launch * tiles + 1) * 4 // 256) * 256
+    fw = run_hot_path(fa, q, k, v, do, sm_scale=sm, mask_kind=mask_kind, **kw)
     args = (q, k, v, fw["o"], fw["l"], fw["m"], do)
-    outs = [fa.flex_attention_bwd(*args, segment_ids=seg, sm_scale=sm, mask_fns=None if mf is None else (mf, bf)) for _ in range(4)]
+    outs = [fa.flex_attention_bwd(*args, segment_ids=seg, sm_scale=sm, mask_fns=None if mf is None else (mf, bf)) for _ in range(3)]
     torch.cuda.synchronize()
     _binding.raise_if_failed(q.device)
     for r in outs[1:]:
         assert all(torch.equal(a, b) for a, b in zip(outs[0], r))
-    # dK, dV: the same operations in another order of q tiles at most; dQ: f32 sums of the same bf16 operands
+    assert not torch.equal(outs[0][0], fw["dq"])      # not those kernels themselves
+    # dK, dV: the same operations in another order of q tiles at most; dQ: f32 sums of the same bf16 operands.  Slice by slice,
+    # so that a single one that was left out cannot hide among the others.
     for n, t in zip(("dq", "dk", "dv"), outs[0]):
-        assert float((t.float() - fw[n].float()).norm() / fw[n].float().norm()) < 2e-3, n
+        for b in range(B):
+            e = (t[b].float() - fw[n][b].float()).flatten(1).norm(dim=1) / fw[n][b].float().flatten(1).norm(dim=1)
+            assert float(e.max()) < 2e-3, (n, b, int(e.argmax()))
 
 
 @pytest.mark.parametrize("B,H,Sq,Sk,D,mask_kind,score_kind,fused", [

@@ -11,6 +11,8 @@ slices:
     of two more slices (first, last) against the fp32 SIMT backend run on the slice alone (itself checked against
     the oracle at small sizes).
 
+The gradients are checked twice where a call of the whole backward runs other kernels than the two separate entry points do.
+
 Inputs are drawn on the device (seeded) because a host draw of these sizes takes longer than the kernels."""
 import numpy as np
 import pytest
@@ -18,7 +20,7 @@ import torch
 
 import workloads
 
-from helpers import check_output, oracle_hot_path, run_hot_path
+from helpers import build_mods, check_output, oracle_hot_path, run_hot_path
 
 pytestmark = pytest.mark.gpu
 
@@ -87,7 +89,7 @@ def _abs_dot_per_slice(a, b):
 
 def _need_memory(cfg):
     n = cfg["B"] * cfg["H"] * cfg["S"] * cfg["D"] * 2
-    need = 8 * n + 4 * n // 8 + (6 << 30)     # 8 bf16 tensors, the f64 chunks of the reductions, slack
+    need = 11 * n + 4 * n // 8 + (8 << 30)    # 11 bf16 tensors, the f64 chunks of the reductions, scratch, slack
     free, _ = torch.cuda.mem_get_info()
     if free < need:
         pytest.skip(f"needs {need >> 30} GiB of device memory, {free >> 30} GiB free")
@@ -104,7 +106,29 @@ def test_full_size_properties_and_sampled_slices(name):
     status = torch.zeros(4, dtype=torch.int32, device="cuda")
     r = run_hot_path(fa, q, k, v, do, sm_scale=sm, backend="tcgen05", status=status, **kw)
     assert int(status[0]) == 0, status.tolist()
+    refs = {}
+    _check(name, cfg, kw, q, k, v, do, r, sm, refs)
 
+    # ---- the same of a call of the whole backward, where that runs another kernel
+    mf, bf, sf, seg = build_mods(fa, **kw)
+    prob = fa._resolve.make_problem(q, k, ab=None, segment_ids=seg, causal=False, sm_scale=sm, mask_fn=mf, block_mask_fn=bf, score_fn=sf)
+    fused = prob._bwd_scratch > 0
+    assert fused == (not name.startswith("t_"))     # (eight slices there)
+    if fused:
+        grads = fa.flex_attention_bwd(q, k, v, r["o"], r["l"], r["m"], do, segment_ids=seg, sm_scale=sm,
+                                      mask_fns=None if mf is None else (mf, bf), score_fn=sf)
+        torch.cuda.synchronize()
+        fa._binding.raise_if_failed(q.device)
+        r.update(zip(("dq", "dk", "dv"), grads))
+        del grads
+        _check(name + " whole backward", cfg, kw, q, k, v, do, r, sm, refs)
+    del q, k, v, do, r
+    torch.cuda.empty_cache()
+
+
+def _check(name, cfg, kw, q, k, v, do, r, sm, refs):
+    """refs: the sampled slices' references, filled by the first call."""
+    fa = _fa()
     # ---- size-independent properties, per (batch, head) slice
     for n in ("o", "dq", "dk", "dv", "l", "m", "delta"):
         assert bool(torch.isfinite(r[n]).all()), n
@@ -125,7 +149,9 @@ def test_full_size_properties_and_sampled_slices(name):
         sl = lambda t: t[b:b + 1, h:h + 1]
         skw = _slice_kw(kw, b, h)
         case = f"{name} slice ({b},{h}) tcgen05 vs {against}"
-        if against == "oracle":
+        if (b, h, against) in refs:
+            ref, roundings = refs[b, h, against]
+        elif against == "oracle":
             host = [sl(t).float().cpu().numpy() for t in (q, k, v, do)]
             ref = oracle_hot_path(*host, sm_scale=sm, mask_kind=skw["mask_kind"], score_kind=skw["score_kind"],
                                   window=skw.get("window") or None, cap=skw.get("cap") or None,
@@ -135,9 +161,8 @@ def test_full_size_properties_and_sampled_slices(name):
         else:
             ref = run_hot_path(fa, sl(q), sl(k), sl(v), sl(do), sm_scale=sm, backend="simt", **skw)
             roundings = 2     # both sides stored in bf16
+        refs[b, h, against] = ref, roundings
         for n in ("o", "dq", "dk", "dv"):
             check_output(case, n, sl(r[n]), ref[n], torch.bfloat16, roundings=roundings)
         assert float((sl(r["m"]).cpu() - ref["m"].cpu()).abs().max()) <= 2e-2, case
         assert float((sl(r["l"]).cpu() / ref["l"].cpu() - 1).abs().max()) <= 2e-2, case
-    del q, k, v, do, r
-    torch.cuda.empty_cache()

@@ -49,3 +49,24 @@ def test_a_replay_after_many_other_shapes():
     g.replay()
     torch.cuda.synchronize()
     assert all(torch.equal(a, b) for a, b in zip(out, want))
+
+
+def test_a_replay_of_the_fused_backward():
+    """... whose scratch belongs to the graph: other calls in between get other memory, and find none of theirs changed."""
+    import flex_attention_tpu_b200 as fa
+    g_ = torch.Generator(device="cuda").manual_seed(43)
+    q, k, v, do = (torch.randn((16, 12, 300, 64), generator=g_, device="cuda", dtype=torch.bfloat16) for _ in range(4))
+    prob = fa._resolve.make_problem(q, k, ab=None, segment_ids=None, causal=True, sm_scale=0.125, mask_fn=None, block_mask_fn=None,
+                                    score_fn=None)
+    assert prob._bwd_scratch > 0
+    g, out = _capture(fa, q, k, v, do, causal=True)
+    want = [t.clone() for t in _step(fa, q, k, v, do, causal=True)]
+    for _ in range(3):
+        for t in out:
+            t.fill_(float("nan"))
+        other = _step(fa, do, v, k, q, causal=True)
+        g.replay()
+        again = _step(fa, do, v, k, q, causal=True)
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(out, want))
+        assert all(torch.equal(a, b) for a, b in zip(other, again))
