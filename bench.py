@@ -71,7 +71,7 @@ E2E_CHUNK_HEADS = 8   # the host-buffer pipeline moves chunks of 8 heads of one 
 
 # dram__bytes_read.sum + dram__bytes_write.sum per launch of each kernel, from the ncu captures summarised under
 # profiles/ (None where no capture of the current kernel exists).
-NCU_TRAFFIC_BYTES = {"c2": {"fwd": 276.4e6, "dq": 369.1e6, "dkv": 380.4e6},
+NCU_TRAFFIC_BYTES = {"c2": {"fwd": 276.4e6, "dq": 369.1e6, "dkv": 380.4e6, "bwd_fused": 518.1e6},
                      "t": {"fwd": 1064.7e6, "dq": 1862.1e6, "dkv": 1599.3e6}}
 
 
@@ -203,14 +203,30 @@ class HotPath:
                                             False, self.bf, self.mf, self.sf)
 
     def bwd(self, q, k, v, o, l, m, do):
-        # delta, then dQ and dK/dV (the package launches the two gradient kernels on two streams)
+        # one fused pass over the tile pairs, or dQ and dK/dV on two streams: the package chooses by the sizes
         return self.fa.flex_attention_bwd(q, k, v, o, l, m, do, segment_ids=self.seg, sm_scale=self.sm_scale,
                                           mask_fns=None if self.mf is None else (self.mf, self.bf), score_fn=self.sf)
+
+    def bwd_is_fused(self, q, k):
+        return self.fa._resolve.make_problem(q, k, ab=None, segment_ids=self.seg, causal=False, sm_scale=self.sm_scale, mask_fn=self.mf,
+                                             block_mask_fn=self.bf, score_fn=self.sf)._bwd_scratch > 0
 
     def step(self, q, k, v, do):
         o, l, m = self.fwd(q, k, v)
         dq, dk, dv = self.bwd(q, k, v, o, l, m, do)
         return o, dq, dk, dv
+
+
+def launches_per_step(w, fused):
+    """Kernels of one step: the forward, then delta, dQ and dK/dV, or the fused backward with the kernel before it and the one
+    after it (which short rows, windows and documents do without; the f32 sums of a launch take no more than 1 GiB)."""
+    if not fused:
+        return 4
+    tiles = (w["S"] + 127) // 128
+    if tiles <= 8 or w["mask"] == "document" or (w["mask"] == "sliding_window_causal" and w["window"] < w["S"] - 256):
+        return 3
+    most = max(1, (1 << 30) // (tiles * 128 * w["D"] * 4))
+    return 1 + 3 * -(-w["B"] * w["H"] // most)
 
 
 def capture_step(hp, q, k, v, do, torch):
@@ -254,7 +270,8 @@ def time_replays(g_fwd, g_bwd, steps, torch):
 def time_kernels(hp, q, k, v, do, torch, reps=20, rounds=3):
     """Device time per launch of each kernel of the path: a CUDA graph of `reps` back-to-back launches of that
     kernel alone, replayed `rounds` times between two events (first replay discarded), so that no host launch
-    latency sits between the events."""
+    latency sits between the events.  Where the step's backward is the fused one, "bwd_fused" is that call: its kernel
+    and the small ones before and after it (delta, statistics, dQ from the f32 sums)."""
     fa = hp.fa
     o, l, m = hp.fwd(q, k, v)
     delta = fa.bwd_preprocess(o, do)
@@ -266,6 +283,8 @@ def time_kernels(hp, q, k, v, do, torch, reps=20, rounds=3):
         "dkv": lambda: fa.flash_attention_bwd_dkv(k, v, q, None, hp.seg, l, m, delta, do, sm_scale=hp.sm_scale,
                                                   score_fn=hp.sf, mask_fn=hp.mf, block_mask_fn=hp.bf),
     }
+    if hp.bwd_is_fused(q, k):
+        calls["bwd_fused"] = lambda: hp.bwd(q, k, v, o, l, m, do)
     out = {}
     side = torch.cuda.Stream()
     for name, fn in calls.items():
@@ -659,22 +678,26 @@ def run_ours(args, w):
 
     if rank == 0:
         # executed-algorithmic FLOPs of each kernel: GEMMs it has to compute x kept pairs
-        kflops = {"fwd": 4.0, "dq": 6.0, "dkv": 8.0}
-        dom = max(("fwd", "dq", "dkv"), key=lambda n: kt[n])
+        kflops = {"fwd": 4.0, "dq": 6.0, "dkv": 8.0, "bwd_fused": 10.0}
+        kname = {"fwd": "forward", "dq": "dq_sm100_kernel", "dkv": "dkv_sm100_kernel", "bwd_fused": "fused_sm100_kernel"}
+        in_step = ("fwd", "bwd_fused") if "bwd_fused" in kt else ("fwd", "dq", "dkv")
+        dom = max(in_step, key=lambda n: kt[n])
         ach = kflops[dom] * w["D"] * pairs / (kt[dom] * 1e-3) / 1e12
         rows = w["B"] * w["H"] * w["S"]
         delta_bytes = 2 * rows * w["D"] * elt_bytes(w) + rows * 4
         peak_note = f"bf16_tflops (burst) of {peaks['source']} peaks"
-        roofline = {"kernel": f"{dom}_sm100_kernel", "bound": "tensor", "achieved": ach, "peak": peaks["tflops"],
+        roofline = {"kernel": kname[dom], "bound": "tensor", "achieved": ach, "peak": peaks["tflops"],
                     "unit": "TFLOP/s", "frac": ach / peaks["tflops"], "traffic": (NCU_TRAFFIC_BYTES.get(args.workload) or {}).get(dom),
                     "peak_source": peak_note, "ms_per_launch": kt[dom], "frac_of_nominal": ach / NOMINAL_TFLOPS}
         per_kernel = {n: {"ms": kt[n], "tflops": kflops[n] * w["D"] * pairs / (kt[n] * 1e-3) / 1e12,
                           "frac_of_peak": kflops[n] * w["D"] * pairs / (kt[n] * 1e-3) / 1e12 / peaks["tflops"]}
-                      for n in ("fwd", "dq", "dkv")}
+                      for n in kflops if n in kt}
         per_kernel["delta"] = {"ms": kt["delta"], "gbs": delta_bytes / (kt["delta"] * 1e-3) / 1e9,
                                "frac_of_hbm_peak": delta_bytes / (kt["delta"] * 1e-3) / 1e9 / peaks["hbm"]}
-        per_kernel["note"] = ("each kernel alone, from a graph of 20 back-to-back launches; inside a step dQ and dK/dV "
-                              "overlap on two streams, so their sum exceeds the step's backward time")
+        per_kernel["note"] = ("each kernel alone, from a graph of 20 back-to-back launches; " +
+                              ("the step runs fwd and bwd_fused (timed with the small kernels around it), dq, dkv and delta are the "
+                               "separate entry points" if "bwd_fused" in kt else
+                               "inside a step dQ and dK/dV overlap on two streams, so their sum exceeds the step's backward time"))
         tf_fwd, tf_bwd = flops_fwd / (fwd_ms * 1e-3) / 1e12, flops_bwd / (bwd_ms * 1e-3) / 1e12
         # which regime the timed region ran in, from the clocks sampled inside it
         regime = None
@@ -691,7 +714,7 @@ def run_ours(args, w):
                        "l2": "inputs (q,k,v,do) and outputs exceed the 126 MB L2; no flush needed",
                        "cuda_graph": not args.no_graph},
             "clocks": dict(clocks, regime=regime),
-            "gpu_launches": 4 * args.steps,
+            "gpu_launches": launches_per_step(w, "bwd_fused" in kt) * args.steps,
             "roofline": roofline,
             "frac_of_peak": value / world / peaks["tflops"], "peak_tflops": peaks["tflops"], "peak_source": peak_note,
             "fwd": {"ms": fwd_ms, "tflops": tf_fwd, "frac_of_peak": tf_fwd / peaks["tflops"],

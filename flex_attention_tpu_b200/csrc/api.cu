@@ -363,24 +363,27 @@ bool fused_can(const FlexAttnParams* p) {
 // Whether the fused backward serves the call.  It does 5 contractions of a tile pair and its exponentials once where dQ and dK/dV
 // do 7 and twice, but the parts of a query tile are added one after the other: a kv tile has to stay some 2.4 tiles behind the
 // one before it in its slice.  `slack`, the query tiles a CTA walks per kv tile of the slice that is in flight, says whether
-// there is room for that.  Times in us, fused / separate, on 148 SMs; slices x queries x keys.
+// there is room for that.  Times in us, fused / separate, on 148 SMs, calls one after the other on a stream (replayed from a
+// graph, where dQ starts before dK/dV, the separate ones are up to a tenth slower; the lines are drawn by the mean of both);
+// slices x queries x keys.
 // D = 64, where the exponentials weigh most:
 //   no mask     slack 2.6: 24 x 2048 127 / 159, 192 x 256 31 / 44; 1.7: 16 x 2048 128 / 111, 32 x 1024 x 8192 398 / 383;
 //               0.1: 16 x 128 x 8192 211 / 87.  Chains of few parts need less: 64 x 512 40 / 45, 48 x 512 37 / 37
-//   causal, S2  24 x 1024 43 / 43, 28 x 1000 43 / 48, 16 x 2048 78 / 79; 16 x 1536 65 / 54, 18 x 1152 52 / 41
+//   causal, S2  24 x 1024 43 / 43, 28 x 1000 43 / 48; 16 x 2048 88 / 82, 16 x 1536 65 / 54, 18 x 1152 52 / 41
 //   windows and documents, 16 slices on: 16 x 1280 25 / 30 and 33 / 36
 //   softcap and user functions (more per pair, the same chain): 16 x 2048 unmasked 131 / 148, 32 x 720 53 / 56;
 //               32 x 237 x 8081 303 / 185
 // D = 128, where its shared-memory traffic (dQ on its way out) takes most of the gain:
-//   no mask     128 x 1024 240 / 269, 12 x 8192 1159 / 1260, 160 x 512 x 64 53 / 61; 64 x 1024 147 / 130, 6 x 15360 1983 / 1897,
-//               32 x 2048 x 8192 976 / 870, 8 x 32768 15154 / 11871, 96 x 1024 x 384 107 / 95
-//   causal, S2  128 x 8192 6340 / 6970, 24 x 8192 1290 / 1357, 96 x 256 34 / 38; 16 x 16384 3453 / 3259, 9 x 16384 2100 / 1927,
-//               64 x 873 90 / 87, 64 x 1024 x 512 81 / 74
-//   windows and documents: 128 x 2048 documents 349 / 406, 32 x 4096 with 256 keys 143 / 148
+//   no mask     128 x 1024 240 / 269, 12 x 8192 1159 / 1260, 160 x 512 x 64 53 / 61, 96 x 256 38 / 40; 16 x 8192 1735 / 1661,
+//               64 x 1024 147 / 130, 6 x 15360 1983 / 1897, 32 x 2048 x 8192 976 / 870, 8 x 32768 15154 / 11871,
+//               96 x 1024 x 384 107 / 95
+//   causal, S2  128 x 8192 6371 / 7090, 24 x 8192 1290 / 1357, 96 x 256 31 / 33, 64 x 512 43 / 44; 64 x 873 90 / 86,
+//               16 x 16384 3453 / 3259, 9 x 16384 2100 / 1927, 64 x 1024 x 512 81 / 74, 192 x 12544 x 384 2217 / 1968
+//   windows and documents: 128 x 2048 documents 349 / 406, 48 x 4096 with 1024 keys 375 / 404; 16 x 2048 with 256 keys 49 / 46
 //   softcap     16 x 2048 causal 103 / 113, 40 x 512 38 / 39, 64 x 512 unmasked 57 / 63; 16 x 1536 causal 82 / 74,
 //               24 x 1024 unmasked 86 / 74, 64 x 14683 x 492 causal 1307 / 1205
 //   a window open ahead: 256 x 528 207 / 240; 128 x 4096 2154 / 2013
-//   user functions: none (16 x 2048 causal 113 / 108, unmasked 170 / 155; 64 x 4096 1099 / 1072, 1833 / 1910)
+//   user functions: none (16 x 2048 causal 112 / 109, unmasked 169 / 155, 64 x 1024 131 / 122; 64 x 4096 1075 / 1073, 1822 / 1905)
 // Either: 72 x 445 x 18173 causal 192 / 304, 64 x 256 x 8960 with 267 keys 66 / 113 (most kv tiles see no query);
 //         16 x 496 x 1206 causal 33 / 29, 24 x 264 x 4885 45 / 41
 bool fused_pays(const FlexAttnParams* p) {
@@ -400,24 +403,23 @@ bool fused_pays(const FlexAttnParams* p) {
   if (items < sms) return false;
   const double slack = bwd_fused_slack(*p, (int)sms);
   if (p->head_dim == 64) {
-    if (common_start) {
-      if (scored) return slices >= 16 && slack >= 1.1;
-      return slices >= 16 && (slack >= 2 || slices >= sms || (slack >= 1.25 && slices >= 8 * n_kt));
-    }
-    if (long_rows && !scored) return slices >= 24 || (slices >= 16 && slack >= 1.7);
-    return slices >= 16;
+    if (slices < 16) return false;
+    if (common_start && scored) return slack >= 1.1;
+    if (common_start) return slack >= 2 || slices >= sms || (slack >= 1.25 && slices >= 8 * n_kt);
+    return !long_rows || slices >= 24 || slack >= (scored ? 1.25 : 1.8);
   }
-  const bool few = slices < sms && items < 5 * sms;
   if (p->score_kind == FLEXATTN_SCORE_USER) return false;
+  const bool few = items < 5 * sms;
   if (scored) {
-    if (slices < 16 || (n_qt > 2 * n_kt && few)) return false;
-    return common_start ? slack >= 1.7 || slices >= sms : slices >= 40 || 5 * items >= 8 * sms;
+    if (slices < 16 || (n_qt > 2 * n_kt && few && slices < sms)) return false;
+    if (common_start) return slack >= 1.7 || slices >= sms;
+    return mask == FLEXATTN_MASK_SLIDING_WINDOW_CAUSAL || slices >= 40 || 5 * items >= 8 * sms;
   }
   if (mask == FLEXATTN_MASK_SLIDING_WINDOW) return slices >= sms && n_qt <= 8;
   if (slices >= sms && (slack >= 2.1 || n_qt <= 32)) return true;
   if (n_qt > n_kt && few && (common_start || long_rows)) return false;
-  if (common_start) return slices >= 12 && slack >= 2.2 && 2 * items >= 5 * sms;
-  if (slices >= (long_rows ? 96 : 64)) return true;
+  if (common_start) return (slack >= (slices >= 24 ? 2.2 : 2.4) && 2 * items >= 5 * sms) || (slices >= 96 && n_kt <= 2);
+  if (slices >= (long_rows && n_qt > 4 ? 96 : 64)) return true;
   return 2 * items >= 9 * sms && (long_rows ? slices >= 24 && slack >= 2.2 : slices >= 16);
 }
 }  // namespace

@@ -125,12 +125,13 @@ def test_fused_backward_repeats_and_agrees(B, H, S, D, mask_kind, sums):
     (8, 16, 2048, 2048, 128, "causal", "none", True), (4, 32, 8192, 8192, 128, "sliding_window_causal", "alibi", True),
     (2, 16, 16384, 16384, 128, "document", "softcap", True), (16, 12, 512, 512, 64, "none", "none", True),
     (2, 16, 4096, 4096, 64, "s2", "none", True), (1, 12, 8192, 8192, 128, "none", "none", True), (1, 192, 1, 8192, 64, "none", "none", True),
+    (1, 72, 445, 18173, 128, "causal", "alibi", True), (1, 96, 256, 256, 128, "none", "none", True),
     # one or a few query tiles against many kv tiles: every part of a query tile waits for the one before
     (1, 16, 128, 8192, 64, "none", "none", False), (1, 64, 128, 8192, 128, "none", "softcap", False),
     (1, 16, 2048, 2048, 64, "none", "none", False), (1, 16, 1280, 1280, 64, "causal", "none", False),
     # a few long rows at D = 128, short ones against shorter keys, a user function
     (1, 8, 16384, 16384, 128, "causal", "none", False), (1, 4, 32768, 32768, 128, "none", "none", False),
-    (3, 24, 1277, 394, 128, "none", "none", False), (2, 8, 1920, 1920, 128, "causal", "user", False),
+    (3, 24, 1277, 394, 128, "none", "none", False), (6, 32, 12544, 384, 128, "causal", "none", False), (2, 8, 1920, 1920, 128, "causal", "user", False),
     (1, 2, 384, 384, 128, "causal", "softcap", False),
 ])
 def test_which_backward_serves_a_call(B, H, Sq, Sk, D, mask_kind, score_kind, fused):
