@@ -435,11 +435,13 @@ class Problem:
         return dk, dv
 
     def backward(self, q, k, v, o, do, l, m, need_dq=True, need_dkv=True, want_dab=False, two_streams=None):
-        """delta, then dQ and dK/dV.  The two gradient kernels only share inputs, so dK/dV is launched on a side
-        stream: both kernels fill every SM on their own, but the tail of one then overlaps the head of the other.
-        Everything is ordered after the current stream's work and the current stream waits for both.
-        ``two_streams=False`` launches both on the current stream (the host-buffer pipeline does: there the
-        extra stream only adds synchronisation between the copy and compute streams)."""
+        """delta, dQ, dK and dV.  Where the library asks for scratch (`flexattn_bwd_scratch_bytes`) and there is room for it, one
+        kernel computes all of them in one pass over the tile pairs, on the current stream.  Otherwise, and with a dense bias,
+        dQ and dK/dV have a kernel each; they only share inputs, so dK/dV is launched on a side stream: both kernels fill
+        every SM on their own, but the tail of one then overlaps the head of the other.  Everything is ordered after the
+        current stream's work and the current stream waits for both.  ``two_streams=False`` launches those two on the current
+        stream (the host-buffer pipeline does: there the extra stream only adds synchronisation between the copy and compute
+        streams)."""
         if not (need_dq or want_dab) or not need_dkv:
             delta = self.preprocess(o, do)
             dk, dv = self.bwd_dkv(q, k, v, do, l, m, delta) if need_dkv else (None, None)

@@ -1015,9 +1015,11 @@ int launch_score(cudaStream_t st, const DevParams& d, int score, int mask, const
 // Group: what a slice keeps live, 8 bytes per element of a query row (Q, dO, f32 sum), times the group has 48 MB of the 126 MB
 // of L2.  Under a causal window the live rows are the few around the diagonal.
 // store_dq: storing dq with the last part saves the finishing kernel and its pass over the sums, but costs the CTA that
-// does it half a tile's time.  That is a gain where many kv tiles share the work (windows: [4,32,8192,128] with 256 keys 1066
-// -> 970 us; documents: [2,16,16384,128] 1547 -> 1475) and where rows are short ([16,12,512,64] 84 -> 70); under a causal mask
-// or none the one kv tile that every query tile meets last does it all, and long rows wait for it ([2,8,1920,128] 89 -> 107).
+// does it half a tile's time.  That is a gain where many kv tiles share the work (documents: [2,16,16384,128] 1510 -> 1436 us, with
+// softcap 1565 -> 1525, the backward alone replayed from a graph); under a causal mask or none the one kv tile that every query
+// tile meets last does it all, and long rows wait for it ([2,8,1920,128] causal 88 -> 99).  Short rows: [16,12,512,64] between
+// 76 and 93 either way.  Windows store it too and need no more than the ring, but would be faster with the finishing kernel
+// ([4,32,8192,128] with 256 keys 980 us, 939 with it; with ALiBi 1060 and 956).
 // Then the scratch is a ring of three groups: the one being finished, the one being started, and one between.  Without it the
 // scratch holds every slice of a launch, and there are as many launches as keep it within 1 GiB (one slice, if need be).
 struct FusedPlan {

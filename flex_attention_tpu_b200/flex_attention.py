@@ -5,7 +5,7 @@ with ``jax.custom_vjp``, ``_flash_attention_fwd`` saving ``(q, k, v, ab, segment
 ``_flash_attention_bwd`` calling the dkv and dq kernels); its flex kernels are only ever driven by hand
 (``flex_attention_dq_bwd.py:905-945``).  This module is the same glue for the flex kernels, with
 ``torch.autograd.Function`` in the place of ``jax.custom_vjp``: residuals saved by the forward are exactly the
-reference's, and the backward runs delta = rowsum(o * do), then dQ, then dK/dV.
+reference's, and the backward computes delta = rowsum(o * do), dQ and dK/dV.
 """
 from __future__ import annotations
 
@@ -37,11 +37,12 @@ class _FlexAttentionFn(torch.autograd.Function):
 
 def flex_attention_bwd(q, k, v, o, l, m, do, *, ab=None, segment_ids=None, causal: bool = False,
                        sm_scale: float = 1.0, mask_fns=None, score_fn=None, backend: str = "auto", two_streams=None):
-    """The whole backward in one call: delta = rowsum(o * do), then dQ and dK/dV (launched on two streams so
-    that the tail of one kernel overlaps the head of the other).  Residuals ``o, l, m`` as returned by
+    """The whole backward in one call: delta = rowsum(o * do), then dQ, dK and dV, by the sizes and options either in one
+    pass over the tile pairs on the current stream (which takes scratch memory for the call) or by two kernels on two
+    streams, so that the tail of one overlaps the head of the other.  Residuals ``o, l, m`` as returned by
     ``_flex_attention_impl(..., save_residuals=True)``; the counterpart of the reference's
-    ``_flash_attention_bwd`` (``jax_exp.py:276-321``).  ``two_streams=False`` keeps both kernels on the current
-    stream.  Returns ``(dq, dk, dv)``."""
+    ``_flash_attention_bwd`` (``jax_exp.py:276-321``).  ``two_streams=False`` keeps the two kernels on the
+    current stream as well.  Returns ``(dq, dk, dv)``."""
     mask_fn, block_mask_fn = mask_fns if mask_fns is not None else (None, None)
     prob = make_problem(q, k, ab=ab, segment_ids=segment_ids, causal=causal, sm_scale=sm_scale, mask_fn=mask_fn,
                         block_mask_fn=block_mask_fn, score_fn=score_fn, backend=backend)
