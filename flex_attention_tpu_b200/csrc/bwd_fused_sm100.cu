@@ -188,7 +188,11 @@ __device__ __forceinline__ void bulk_add_f32(float* dst, const void* smem_src, u
                : "memory");
 }
 
-template <int D, int SK, int MK>
+// kStore: whether dq is stored with the last part of a query tile (FusedArgs::store_dq), known when it is compiled: 18 KB of code that
+// the other form does not carry through the instruction cache ([2,16,8192,128] with 1024 keys and ALiBi 490 -> 455 us); kAsked (the
+// kernels compiled at run time, where each takes seconds): looked up.
+constexpr int kAsked = 2;
+template <int D, int SK, int MK, int kStore = kAsked>
 __global__ void __launch_bounds__(kThreads, 1)
     fused_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                        const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
@@ -496,7 +500,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           bulk_load(slots + (c & 1) * kSlotBytes, back + c * 1024, kSlotBytes, bar);
         };
         auto fetch_first = [&](const int4& turn) {
-          if ((turn.z & 3) == 2 && back == nullptr &&
+          if (kStore != 0 && (turn.z & 3) == 2 && back == nullptr &&
               FLEXATTN_DBG_OK((long long)turn.x * P.n_qt + turn.y, (long long)F.slices * P.n_qt, kFusedId, 708)) {
             back = F.dq_acc + ((size_t)(turn.x % F.ring) * P.n_qt + turn.y) * kTile * D + w * 32 * D;
             if (lane == 0) ptx::tma_store_wait_read();  // what the slots held has left
@@ -504,7 +508,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             fetch(1);
           }
         };
-        if (__all_sync(0xffffffffu, mbar_test_wait(&sh->bar_turn[T & 1], (T >> 1) & 1))) fetch_first(sh->turn[T & 1]);
+        if (kStore != 0 && __all_sync(0xffffffffu, mbar_test_wait(&sh->bar_turn[T & 1], (T >> 1) & 1))) fetch_first(sh->turn[T & 1]);
         ok = __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_dq, T & 1));
         if (!ok) { fail_at = 31; break; }
         ptx::tc_fence_after();
@@ -523,7 +527,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         fetch_first(turn);
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive(&sh->bar_turnfree[T & 1]);
-        const bool first = turn.z & 1, last = turn.z & 2;
+        const bool first = turn.z & 1, last = kStore != 0 && (turn.z & 2);
         float* tile = F.dq_acc + ((size_t)(turn.x % F.ring) * P.n_qt + turn.y) * kTile * D + w * 32 * D;
         if (!FLEXATTN_DBG_OK((long long)turn.x * P.n_qt + turn.y, (long long)F.slices * P.n_qt, kFusedId, 705)) {
         } else if (last) {
@@ -820,7 +824,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         };
         for (int qt = ia.z; qt < ia.w && ok; ++qt) {
           const int pred = nearest(qt, 1);  // its part is added before this one
-          const bool last = F.store_dq && nearest(qt, -1) < 0;
+          const bool last = kStore != 0 && (kStore == 1 || F.store_dq) && nearest(qt, -1) < 0;
           // the first part of a tile waits for the slice that had its place in the ring before
           const int prior = pred >= 0 ? ia.x : ia.x - F.ring;
           const int want = pred >= 0 ? P.n_kt - pred : kAllAdded;
@@ -873,45 +877,63 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 #ifndef FLEXATTN_JIT
 // Before it: delta = rowsum(o * do) to the caller, both row statistics to the padded tiles the loads take, flags and ticket
-// to zero.  One 16-byte chunk of o and do per thread, as in delta.cu.  A query tile that no kv tile sees gets its zeros here.
+// to zero.  Bound by HBM latency: all that a thread reads (16-byte chunks of kUnroll rows of o and do, l and m) is asked for before
+// the first sum.  [16,12,512,64] 9.0 -> 7.1 us, [8,16,2048,128] 37 -> 33; four rows were no faster, and slower where the grid is
+// small.  A query tile that no kv tile sees gets its zeros here.
 template <int D>
 __global__ void __launch_bounds__(256) prep_kernel(const DevParams P, const FusedArgs F) {
-  constexpr int kTpr = D / 8, kRows = 256 / kTpr;  // rows of a block: all of one tile
-  const long long row = (long long)blockIdx.x * kRows + threadIdx.x / kTpr;
-  const long long tile = row / kTile, slice = tile / P.n_qt;
-  const int qt = (int)(tile - slice * P.n_qt), i = qt * kTile + (int)(row % kTile);
-  const long long at = (F.slice0 + slice) * P.seq_q + i;
-  const bool live = i < P.seq_q && FLEXATTN_DBG_OK(at, (long long)P.batch * P.heads * P.seq_q, kFusedId, 710);
+  constexpr int kUnroll = 2, kTpr = D / 8, kRows = 256 / kTpr;  // kRows * kUnroll rows of a block: all of one tile
+  constexpr int kBlocksPerTile = kTile / (kRows * kUnroll);
+  const long long tile = blockIdx.x / kBlocksPerTile, slice = tile / P.n_qt;
+  const int qt = (int)(tile - slice * P.n_qt), row0 = (int)(blockIdx.x % kBlocksPerTile) * kRows * kUnroll + threadIdx.x / kTpr;
+  const int i0 = qt * kTile + row0, chunk = threadIdx.x & (kTpr - 1);
+  const long long at0 = (F.slice0 + slice) * P.seq_q + i0;
   const bool in = FLEXATTN_DBG_OK(tile, (long long)F.slices * P.n_qt, kFusedId, 711);
-  float acc = 0.f;
-  if (live) {
-    const uint4 a = __ldg(static_cast<const uint4*>(P.o) + at * kTpr + (threadIdx.x & (kTpr - 1)));
-    const uint4 b = __ldg(static_cast<const uint4*>(P.d_o) + at * kTpr + (threadIdx.x & (kTpr - 1)));
-    const __nv_bfloat162* pa = reinterpret_cast<const __nv_bfloat162*>(&a);
-    const __nv_bfloat162* pb = reinterpret_cast<const __nv_bfloat162*>(&b);
+  uint4 a[kUnroll], b[kUnroll];
+  float l[kUnroll], m[kUnroll];
+#pragma unroll
+  for (int u = 0; u < kUnroll; ++u) {
+    const bool live = i0 + u * kRows < P.seq_q && FLEXATTN_DBG_OK(at0 + u * kRows, (long long)P.batch * P.heads * P.seq_q, kFusedId, 710);
+    a[u] = b[u] = make_uint4(0u, 0u, 0u, 0u);
+    l[u] = m[u] = 0.f;
+    if (live) {
+      a[u] = __ldcs(static_cast<const uint4*>(P.o) + (at0 + u * kRows) * kTpr + chunk);
+      b[u] = __ldg(static_cast<const uint4*>(P.d_o) + (at0 + u * kRows) * kTpr + chunk);
+      if (chunk == 0) {
+        l[u] = P.l[at0 + u * kRows];
+        m[u] = P.m[at0 + u * kRows];
+      }
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kUnroll; ++u) {
+    const __nv_bfloat162* pa = reinterpret_cast<const __nv_bfloat162*>(&a[u]);
+    const __nv_bfloat162* pb = reinterpret_cast<const __nv_bfloat162*>(&b[u]);
+    float acc = 0.f;
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
       const float2 fa = __bfloat1622float2(pa[c]), fb = __bfloat1622float2(pb[c]);
       acc = fmaf(fa.x, fb.x, acc);
       acc = fmaf(fa.y, fb.y, acc);
     }
-  }
 #pragma unroll
-  for (int s = kTpr / 2; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
-  if ((threadIdx.x & (kTpr - 1)) == 0) {
-    float nl = -1.0e30f;  // rows past the end and fully masked ones: p = 0
-    if (live) {
-      P.delta[at] = acc;
-      const float l = P.l[at];
-      if (l > 0.f) nl = ptx::kRoundLog2 - fmaf(P.m[at], kLog2e, __log2f(l));
-    }
-    if (in) {
-      float* t = F.stats + tile * 2 * kTile + (row % kTile);
-      t[0] = nl;
-      t[kTile] = acc;
+    for (int s = kTpr / 2; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
+    if (chunk == 0) {
+      const long long at = at0 + u * kRows;
+      const int row = row0 + u * kRows;
+      float nl = -1.0e30f;  // rows past the end and fully masked ones: p = 0
+      if (i0 + u * kRows < P.seq_q && FLEXATTN_DBG_OK(at, (long long)P.batch * P.heads * P.seq_q, kFusedId, 710)) {
+        P.delta[at] = acc;
+        if (l[u] > 0.f) nl = ptx::kRoundLog2 - fmaf(m[u], kLog2e, __log2f(l[u]));
+      }
+      if (in) {
+        float* t = F.stats + tile * 2 * kTile + row;
+        t[0] = nl;
+        t[kTile] = acc;
+      }
     }
   }
-  if (blockIdx.x % (kTile / kRows) == 0 && in) {  // the first block of a tile
+  if (blockIdx.x % kBlocksPerTile == 0 && in) {  // the first block of a tile
     const int4* cmap = P.col_map + (size_t)(P.map_rows > 1 ? (F.slice0 + slice) / P.heads : 0) * P.n_kt;
     bool seen = false;
     for (int j = threadIdx.x; j < P.n_kt; j += 256) {
@@ -970,10 +992,10 @@ struct Maps {
 };
 
 // grid 0: only prepares the kernel and says whether it can be launched
-template <int D, int SK, int MK>
-int launch_one(cudaStream_t st, const DevParams& d, const FusedArgs& f, const Maps& t, unsigned grid, int* af) {
+template <int D, int SK, int MK, int kStore>
+int launch_form(cudaStream_t st, const DevParams& d, const FusedArgs& f, const Maps& t, unsigned grid, int* af) {
   constexpr size_t smem = smem_bytes(D);
-  auto kern = fused_sm100_kernel<D, SK, MK>;
+  auto kern = fused_sm100_kernel<D, SK, MK, kStore>;
   static const bool whole_file = [kern] {  // compiled for fewer registers than its warpgroups hand round, it would wait without end
     cudaFuncAttributes a;
     return cudaFuncGetAttributes(&a, reinterpret_cast<const void*>(kern)) == cudaSuccess && a.numRegs >= 128;
@@ -984,6 +1006,14 @@ int launch_one(cudaStream_t st, const DevParams& d, const FusedArgs& f, const Ma
   if (grid == 0) return FLEXATTN_OK;
   kern<<<grid, kThreads, smem, st>>>(t.q, t.d_o, t.k, t.v, t.dk, t.dv, t.dq, d, f, af);
   return cudaGetLastError() == cudaSuccess ? FLEXATTN_OK : FLEXATTN_ERR_CUDA;
+}
+
+template <int D, int SK, int MK>
+int launch_one(cudaStream_t st, const DevParams& d, const FusedArgs& f, const Maps& t, unsigned grid, int* af) {
+  if constexpr (MK != FLEXATTN_MASK_DOCUMENT) {  // (documents always store it: fused_plan)
+    if (!f.store_dq) return launch_form<D, SK, MK, 0>(st, d, f, t, grid, af);
+  }
+  return launch_form<D, SK, MK, 1>(st, d, f, t, grid, af);
 }
 
 template <int D, int SK>
@@ -1018,8 +1048,9 @@ int launch_score(cudaStream_t st, const DevParams& d, int score, int mask, const
 // does it half a tile's time.  That is a gain where many kv tiles share the work (documents: [2,16,16384,128] 1510 -> 1436 us, with
 // softcap 1565 -> 1525, the backward alone replayed from a graph); under a causal mask or none the one kv tile that every query
 // tile meets last does it all, and long rows wait for it ([2,8,1920,128] causal 88 -> 99).  Short rows: [16,12,512,64] between
-// 76 and 93 either way.  Windows store it too and need no more than the ring, but would be faster with the finishing kernel
-// ([4,32,8192,128] with 256 keys 980 us, 939 with it; with ALiBi 1060 and 956).
+// 76 and 93 either way.  Windows of D = 64 store it too ([2,16,4096,64] with 128 keys 74 us, 81 with the finishing kernel), and those of
+// D = 128 up to 6000 positions (us stored / finished: 16 heads a row, 3072 with 232 keys 206 / 226, 5756 74 / 75) and where the
+// ring is smaller than all slices; longer ones are finished ([4,32,8192,128] with 256 keys and ALiBi 1077 -> 957, [5,8,15744,128] 853 / 755).
 // Then the scratch is a ring of three groups: the one being finished, the one being started, and one between.  Without it the
 // scratch holds every slice of a launch, and there are as many launches as keep it within 1 GiB (one slice, if need be).
 struct FusedPlan {
@@ -1043,6 +1074,7 @@ FusedPlan fused_plan(int slices, int seq_q, int n_qt, int n_kt, int head_dim, in
   if (group > L.launch) group = L.launch;
   L.group = (int)group;
   L.ring = L.store_dq && 3 * group < slices ? (int)(3 * group) : L.launch;
+  if (windowed && head_dim == 128 && L.ring == L.launch && n_kt >= 48) L.store_dq = 0;
   auto up = [](size_t n) { return (n + 255) & ~(size_t)255; };
   L.off_stats = up((size_t)L.ring * acc);
   L.off_flags = L.off_stats + up((size_t)L.launch * n_qt * 2 * kTile * sizeof(float));
@@ -1086,10 +1118,12 @@ int launch_sm100_bwd_fused(cudaStream_t st, const DevParams& d, int score, int m
   if (!e) e = make_tile_map(&t.dk, d.dk, slices, d.seq_k, D);
   if (!e) e = make_tile_map(&t.dv, d.dv, slices, d.seq_k, D);
   if (!e) e = make_tile_map(&t.dq, d.dq, slices, d.seq_q, D, 32);  // a drain warp's rows
+  FusedArgs probe{};
+  probe.store_dq = L.store_dq;
   auto launch = [&](const FusedArgs& f, unsigned grid) {
     return D == 128 ? launch_score<128>(st, d, score, mask, f, t, grid, af) : launch_score<64>(st, d, score, mask, f, t, grid, af);
   };
-  if (!e) e = score == FLEXATTN_SCORE_USER ? jit_fused_ready(d.user_score, D, mask, smem_bytes(D), st) : launch(FusedArgs{}, 0);
+  if (!e) e = score == FLEXATTN_SCORE_USER ? jit_fused_ready(d.user_score, D, mask, smem_bytes(D), st) : launch(probe, 0);
   char* base = static_cast<char*>(scratch);
   for (int s0 = 0; s0 < slices && !e; s0 += L.launch) {
     FusedArgs f;
@@ -1103,8 +1137,8 @@ int launch_sm100_bwd_fused(cudaStream_t st, const DevParams& d, int score, int m
     f.store_dq = L.store_dq;
     const int tiles = f.slices * d.n_qt, items = f.slices * d.n_kt;
     f.ticket = f.flags + tiles;
-    if (D == 128) prep_kernel<128><<<tiles * 8u, 256, 0, st>>>(d, f);
-    else prep_kernel<64><<<tiles * 4u, 256, 0, st>>>(d, f);
+    if (D == 128) prep_kernel<128><<<tiles * 4u, 256, 0, st>>>(d, f);
+    else prep_kernel<64><<<tiles * 2u, 256, 0, st>>>(d, f);
     if (cudaGetLastError() != cudaSuccess) return FLEXATTN_ERR_CUDA;
     const unsigned grid = (unsigned)(items < sms ? items : sms);
     if (score == FLEXATTN_SCORE_USER) {
