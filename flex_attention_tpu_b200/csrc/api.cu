@@ -109,6 +109,12 @@ DevParams make_dev(const FlexAttnParams* p) {
   return d;
 }
 
+// for the kernels that have a gathered form of S2, where s2_gathers
+void gather_s2(DevParams* d) {
+  if (d->stride > d->seq_k) d->stride = d->seq_k;  // (key 0 is on every grid; a tensor map's pitch is bounded)
+  d->n_st = (s2_keys(d->seq_k, d->stride) + kTile - 1) / kTile;
+}
+
 #define FLEXATTN_REQUIRE(ptr)                                     \
   do {                                                            \
     if ((ptr) == nullptr) return FLEXATTN_ERR_NULL_POINTER;       \
@@ -253,6 +259,10 @@ int flexattn_fwd(void* stream, const FlexAttnParams* p) {
     // the environment forces one where it can run (read once per process).
     const bool pair_can = p->ab == nullptr;
     const int forced = forced_fwd_kernel();
+    if (forced == 0 && s2_gathers(*p)) {  // (few tiles a query tile: the persistent kernel)
+      gather_s2(&d);
+      return launch_sm100_fwd_pipe(st, d, p->score_kind, p->mask_kind);
+    }
     if (forced == 0 || forced == 3) {
       d.kv_splits = kv_splits(p);
       if (forced == 3 && d.kv_splits == 0 && pair_can && p->score_kind != FLEXATTN_SCORE_USER &&
@@ -400,6 +410,10 @@ bool fused_pays(const FlexAttnParams* p) {
   // many kv tiles that see no query: the fused kernel only stores their zeros
   if (!common_start && n_kt >= 3 * n_qt && slices >= 16 && slices * n_kt >= 7 * sms)
     return p->head_dim == 64 || p->score_kind != FLEXATTN_SCORE_USER;
+  // S2, gathered: the separate kernels walk every tile below the diagonal.  The fused one takes as long as its longest strided tile's
+  // row of query tiles, which they match while they fit the chip at once: slices x queries, 128 keys, stride 32: 8 x 3000 (D = 64)
+  // 58 / 79, 16 x 1500 37 / 52, 16 x 2000 (D = 128) 61 / 86, 16 x 8000 255 / 841; 4 x 5000 113 / 97, 8 x 2000 55 / 41, 16 x 1100 39 / 35
+  if (s2_gathers(*p)) return 5 * items >= 6 * sms;
   if (items < sms) return false;
   const double slack = bwd_fused_slack(*p, (int)sms);
   if (p->head_dim == 64) {
@@ -438,7 +452,8 @@ int flexattn_bwd_fused(void* stream, const FlexAttnParams* p, void* scratch, siz
   FLEXATTN_REQUIRE(p->l); FLEXATTN_REQUIRE(p->m); FLEXATTN_REQUIRE(p->delta);
   FLEXATTN_REQUIRE(p->dq); FLEXATTN_REQUIRE(p->dk); FLEXATTN_REQUIRE(p->dv); FLEXATTN_REQUIRE(scratch);
   if (!fused_can(p)) return FLEXATTN_ERR_UNSUPPORTED_BACKEND;
-  const DevParams d = make_dev(p);
+  DevParams d = make_dev(p);
+  if (s2_gathers(*p)) gather_s2(&d);
   if (scratch_bytes < bwd_fused_scratch_bytes(*p)) return FLEXATTN_ERR_WORKSPACE_TOO_SMALL;
   return launch_sm100_bwd_fused(static_cast<cudaStream_t>(stream), d, p->score_kind, p->mask_kind, scratch);
 }

@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (e >= kStages) ok = ptx::mbar_wait(&sh->bar_free[st], (uint32_t)((e / kStages - 1) & 1));
         return sRing + st * kStageBytes;
       };
-      for (ItemCursor it(P, kDqL2Budget); ok && it.valid(); it.next(), ++r) {
+      for (ItemCursor<> it(P, kDqL2Budget); ok && it.valid(); it.next(), ++r) {
         const int bh = it.bh(), first = it.rm.x, N = it.tiles();
         uint8_t* dst = acquire();
         if (!ok) break;

@@ -40,14 +40,24 @@ constexpr int kAllAdded = 0x40000000;
 constexpr uint32_t kSlotBytes = 4096;  // 32 columns of a drain warp's 32 rows; two slots per warp
 
 struct FusedArgs {
-  float* dq_acc;   // [ring][n_qt][128 * D]: element (32 w + lane, 4 c + k) of a tile at ((w * D / 4 + c) * 32 + lane) * 4 + k
+  float* dq_acc;   // [ring][n_qt][128 * D] (S2, gathered: [chains of a launch][n_qt]...): element (32 w + lane, 4 c + k) of a tile at ((w * D / 4 + c) * 32 + lane) * 4 + k
   float* stats;    // [slices][n_qt][2][128]: -(m log2e + log2 l) pre-scaled for pack_bf16_trunc, delta
-  int32_t* flags;  // [slices][n_qt]: n_kt - (kv tile added last), 0: none, kAllAdded
+  int32_t* flags;  // [slices * chains][n_qt]: n_kt - (kv tile added last), 0: none, kAllAdded
   int32_t* ticket;
   int slice0, slices;  // slices of this launch (of batch * heads)
   int group, ring;     // how many of them form a group, and how many the scratch holds
   int store_dq;        // the last part of a query tile stores dq; otherwise it is added like the others
+  int chains;          // sums per query tile: 2 for S2, gathered (window tiles, strided tiles: chain = 2 * slice + strided), else 1
+  float* s2_dkv;       // ... f32 dK (unscaled) and dV of the keys on the stride grid, from their window tile and their strided one:
+                       // [slices][keys on the grid][2: window, strided][2: dK, dV][D]
 };
+
+// Query tiles of kv tile `kt`: {first, end, first fully kept, end of those}
+template <int MK>
+__device__ __forceinline__ int4 col_entry(const DevParams& P, int b, int kt) {
+  if constexpr (MK == kMaskS2Gather) return s2_col(kt, P.seq_q, P.seq_k, P.n_qt, P.n_kt, P.window, P.stride);
+  return __ldg(&P.col_map[(size_t)(P.map_rows > 1 ? b : 0) * P.n_kt + kt]);
+}
 
 struct FusedSmem {
   uint64_t bar_k[2], bar_v[2], bar_kfree[2], bar_vfree[2], bar_q[2], bar_do[2], bar_qfree[2], bar_dofree[2];
@@ -197,7 +207,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     fused_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                        const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                        const __grid_constant__ CUtensorMap tm_dk, const __grid_constant__ CUtensorMap tm_dv,
-                       const __grid_constant__ CUtensorMap tm_dq, const DevParams P, const FusedArgs F, int* abort_flag) {
+                       const __grid_constant__ CUtensorMap tm_dq, const __grid_constant__ CUtensorMap tm_ks,
+                       const __grid_constant__ CUtensorMap tm_vs, const DevParams P, const FusedArgs F, int* abort_flag) {
   constexpr int kPanels = D / 64;
   constexpr uint32_t kTileBytes = kPanels * ptx::kPanelBytes;
   // At D = 128 shared memory holds one K, V (those of the next item wait for this one's last MMAs) and one dO, whose two
@@ -212,6 +223,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   constexpr bool kOwnDq = D == 64;  // dQ_part has columns of its own
   constexpr uint32_t kColDQ = kOwnDq ? 384 : kColDP;
   constexpr bool kDoc = MK == FLEXATTN_MASK_DOCUMENT;
+  constexpr bool kGather = MK == kMaskS2Gather;  // tm_ks, tm_vs: the keys and values on the stride grid
+  const int n_vt = kGather ? P.n_kt + P.n_st : P.n_kt;  // kv tiles of a slice: its window tiles, and behind them its strided ones
 
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sK = smem;
@@ -285,10 +298,11 @@ __global__ void __launch_bounds__(kThreads, 1)
     x.csc = (SK == FLEXATTN_SCORE_SOFTCAP) ? P.sm_scale / P.cap : 0.f;
     const long long n_doc = (long long)P.batch * P.doc_stride;
     int T = 0, u = 0, fail_at = 0;
+    uint32_t panels = 0;  // stored so far
     bool ok = true;
     // one 64-column panel of this warpgroup, already written, leaves through a bulk store; the panel is free on return.
-    // phase: of the panels so far
-    auto store_panel = [&](const CUtensorMap* tm, int col, int kt, int bh, uint32_t phase) {
+    auto store_panel = [&](const CUtensorMap* tm, int col, int kt, int bh) {
+      const uint32_t phase = panels++ & 1;
       ptx::fence_proxy_async_smem();
       ptx::mbar_arrive_warp(&sh->bar_stage[half]);
       if ((warp & 3) == 0) {
@@ -312,8 +326,10 @@ __global__ void __launch_bounds__(kThreads, 1)
       ptx::mbar_arrive_warp(&sh->bar_itemfree[r % kItemRing]);
       if (ia.x < 0) break;
       const int bh = F.slice0 + ia.x, kt = ia.y, N = ia.w - ia.z;
-      const int j = kt * kTile + row;  // this thread's key position
-      const bool row_ok = j < P.seq_k;
+      const bool strided = kGather && kt >= P.n_kt;
+      const int key = (strided ? kt - P.n_kt : kt) * kTile + row, keys = strided ? s2_keys(P.seq_k, P.stride) : P.seq_k;
+      const bool row_ok = key < keys;
+      const int j = strided ? min(key, keys) * P.stride : key;  // this thread's key position
       x.b = bh / P.heads;
       x.h = bh - x.b * P.heads;
       x.j = j;
@@ -324,7 +340,15 @@ __global__ void __launch_bounds__(kThreads, 1)
       bool doc_runs = false;
       int qlo = 0, qhi = 0, dj = -2;
       const int32_t* doc = nullptr;
-      if constexpr (!kDoc) row_query_interval<MK>(j, P.seq_q, P.window, P.stride, qlo, qhi);
+      if constexpr (kGather) {
+        row_query_interval<FLEXATTN_MASK_SLIDING_WINDOW_CAUSAL>(j, P.seq_q, P.window, 1, qlo, qhi);
+        if (strided) {
+          qlo = P.window < P.seq_q - j ? j + P.window : P.seq_q;
+          qhi = P.seq_q;
+        }
+      } else if constexpr (!kDoc) {
+        row_query_interval<MK>(j, P.seq_q, P.window, P.stride, qlo, qhi);
+      }
       if constexpr (kDoc) {
         const long long at = (long long)x.b * P.doc_stride + j;
         doc = P.doc_ids + (size_t)x.b * P.doc_stride;
@@ -343,7 +367,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         doc_runs = true;
         qlo = qhi = 0;
       }
-      const bool ragged = (kt + 1) * kTile > P.seq_k;
+      const bool ragged = ((strided ? kt - P.n_kt : kt) + 1) * kTile > keys;
       for (int n = 0; n < N && ok; ++n, ++T) {
         const int st = T & 1, qt = ia.z + n, i0 = qt * kTile + 64 * half;
         const bool partial = ragged || !(qt >= ib.x && qt < ib.y);
@@ -432,6 +456,14 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
       uint32_t out[D / 2];
       const float sc = half ? 1.f : P.sm_scale;
+      // a key on the stride grid has two sums, which meet in s2_finish_kernel: they leave as f32
+      float* s2_row = nullptr;
+      if constexpr (kGather) {
+        if (row_ok && (strided || j % P.stride == 0)) {
+          const long long at = ((long long)ia.x * s2_keys(P.seq_k, P.stride) + j / P.stride) * 4 + 2 * strided + half;
+          if (FLEXATTN_DBG_OK(at, (long long)F.slices * s2_keys(P.seq_k, P.stride) * 4, kFusedId, 715)) s2_row = F.s2_dkv + at * D;
+        }
+      }
 #pragma unroll
       for (int c0 = 0; c0 < D; c0 += 32) {
         uint32_t v[32];
@@ -443,6 +475,10 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
           for (int c = 0; c < 32; ++c) v[c] = 0u;
         }
+        if (kGather && s2_row != nullptr) {
+#pragma unroll
+          for (int c = 0; c < 32; c += 4) *reinterpret_cast<uint4*>(s2_row + c0 + c) = make_uint4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+        }
 #pragma unroll
         for (int c = 0; c < 32; c += 2)
           out[(c0 + c) >> 1] = ptx::pack_bf16(__uint_as_float(v[c]) * sc, __uint_as_float(v[c + 1]) * sc);
@@ -451,13 +487,14 @@ __global__ void __launch_bounds__(kThreads, 1)
         ptx::tc_fence_before();
         ptx::mbar_arrive_warp(&sh->bar_accfree);
       }
+      if (strided) continue;
 #pragma unroll
       for (int p0 = 0; p0 < kPanels; ++p0) {
 #pragma unroll
         for (int c = 0; c < 8; ++c)
           *reinterpret_cast<uint4*>(panel_row + ((c ^ (row & 7)) << 4)) =
               make_uint4(out[32 * p0 + 4 * c], out[32 * p0 + 4 * c + 1], out[32 * p0 + 4 * c + 2], out[32 * p0 + 4 * c + 3]);
-        if (ok) store_panel(half ? &tm_dv : &tm_dk, p0 * 64, kt, bh, (r * kPanels + p0) & 1);
+        if (ok) store_panel(half ? &tm_dv : &tm_dk, p0 * 64, kt, bh);
       }
     }
     if (!ok && lane == 0) give_up(abort_flag, P.status, kFusedId, fail_at);
@@ -501,7 +538,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         };
         auto fetch_first = [&](const int4& turn) {
           if (kStore != 0 && (turn.z & 3) == 2 && back == nullptr &&
-              FLEXATTN_DBG_OK((long long)turn.x * P.n_qt + turn.y, (long long)F.slices * P.n_qt, kFusedId, 708)) {
+              FLEXATTN_DBG_OK((long long)turn.x * P.n_qt + turn.y, (long long)F.slices * F.chains * P.n_qt, kFusedId, 708)) {
             back = F.dq_acc + ((size_t)(turn.x % F.ring) * P.n_qt + turn.y) * kTile * D + w * 32 * D;
             if (lane == 0) ptx::tma_store_wait_read();  // what the slots held has left
             fetch(0);
@@ -529,7 +566,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (lane == 0) ptx::mbar_arrive(&sh->bar_turnfree[T & 1]);
         const bool first = turn.z & 1, last = kStore != 0 && (turn.z & 2);
         float* tile = F.dq_acc + ((size_t)(turn.x % F.ring) * P.n_qt + turn.y) * kTile * D + w * 32 * D;
-        if (!FLEXATTN_DBG_OK((long long)turn.x * P.n_qt + turn.y, (long long)F.slices * P.n_qt, kFusedId, 705)) {
+        if (!FLEXATTN_DBG_OK((long long)turn.x * P.n_qt + turn.y, (long long)F.slices * F.chains * P.n_qt, kFusedId, 705)) {
         } else if (last) {
           uint32_t out[D / 2];
 #pragma unroll
@@ -602,7 +639,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
           for (int p = 0; p < kPanels; ++p) ptx::tma_load_3d(dst + p * ptx::kPanelBytes, tm, bar, p * 64, row0, bh);
         };
-        const int total = F.slices * P.n_kt;
+        const int total = F.slices * n_vt;
         int T = 0, u = 0;
         int w = atomicAdd(F.ticket, 1);
         for (int r = 0;; ++r) {
@@ -615,12 +652,14 @@ __global__ void __launch_bounds__(kThreads, 1)
             ptx::mbar_arrive(&sh->bar_item[r % kItemRing]);
             break;
           }
-          const int g = w / (F.group * P.n_kt), in_group = w - g * F.group * P.n_kt;
+          const int g = w / (F.group * n_vt), in_group = w - g * F.group * n_vt;
           const int width = min(F.group, F.slices - g * F.group);
           const int rank = in_group / width;
-          const int slice = g * F.group + in_group - rank * width, kt = P.n_kt - 1 - rank;
+          const int slice = g * F.group + in_group - rank * width, kt = n_vt - 1 - rank;
           const int bh = F.slice0 + slice, b = bh / P.heads;
-          const int4 cm = __ldg(&P.col_map[(size_t)(P.map_rows > 1 ? b : 0) * P.n_kt + kt]);
+          const int4 cm = col_entry<MK>(P, b, kt);
+          const bool strided = kGather && kt >= P.n_kt;
+          const int kv_row = (strided ? kt - P.n_kt : kt) * kTile;
           sh->item_a[r % kItemRing] = make_int4(slice, kt, cm.x, cm.y);
           sh->item_b[r % kItemRing] = make_int2(cm.z, cm.w);
           ptx::mbar_arrive(&sh->bar_item[r % kItemRing]);
@@ -646,11 +685,11 @@ __global__ void __launch_bounds__(kThreads, 1)
             // V and K of the previous item (D = 64: of the last but one) have been read
             if (u >= kKvStages) ok = ok && ptx::mbar_wait_relaxed(&sh->bar_vfree[ks], kph, 20);
             if (!ok) break;
-            load_tile(sV + ks * kTileBytes, &tm_v, &sh->bar_v[ks], kt * kTile, bh, 0);
+            load_tile(sV + ks * kTileBytes, strided ? &tm_vs : &tm_v, &sh->bar_v[ks], kv_row, bh, 0);
             load_do(0);
             if (u >= kKvStages) ok = ok && ptx::mbar_wait_relaxed(&sh->bar_kfree[ks], kph, 20);
             if (!ok) break;
-            load_tile(sK + ks * kTileBytes, &tm_k, &sh->bar_k[ks], kt * kTile, bh, 0);
+            load_tile(sK + ks * kTileBytes, strided ? &tm_ks : &tm_k, &sh->bar_k[ks], kv_row, bh, 0);
             for (int n = 1; n < N && ok; ++n) {
               if (kDoStages == 1) {  // dO(n) waits for dV(n-1), later than Q(n) for dK(n-2)
                 load_q(n);
@@ -807,14 +846,16 @@ __global__ void __launch_bounds__(kThreads, 1)
           break;
         }
         const int b = (F.slice0 + ia.x) / P.heads, kt = ia.y;
-        const int4* cmap = P.col_map + (size_t)(P.map_rows > 1 ? b : 0) * P.n_kt;
+        // (the strided tiles' parts are a sum of their own)
+        const int strided = kGather && kt >= P.n_kt, first_kt = strided ? P.n_kt : 0, end_kt = strided ? n_vt : P.n_kt;
+        const int chain = kGather ? 2 * ia.x + strided : ia.x;
         // nearest kv tile beyond this one, upwards or downwards, that sees query tile qt; -1: none
         auto nearest = [&](int qt, int step) {
-          for (int j0 = kt + step; j0 >= 0 && j0 < P.n_kt; j0 += 32 * step) {
+          for (int j0 = kt + step; j0 >= first_kt && j0 < end_kt; j0 += 32 * step) {
             const int j = j0 + step * lane;
             bool sees = false;
-            if (j >= 0 && j < P.n_kt) {
-              const int2 range = __ldg(reinterpret_cast<const int2*>(cmap + j));
+            if (j >= first_kt && j < end_kt) {
+              const int4 range = col_entry<MK>(P, b, j);
               sees = qt >= range.x && qt < range.y;
             }
             const unsigned any = __ballot_sync(0xffffffffu, sees);
@@ -826,11 +867,11 @@ __global__ void __launch_bounds__(kThreads, 1)
           const int pred = nearest(qt, 1);  // its part is added before this one
           const bool last = kStore != 0 && (kStore == 1 || F.store_dq) && nearest(qt, -1) < 0;
           // the first part of a tile waits for the slice that had its place in the ring before
-          const int prior = pred >= 0 ? ia.x : ia.x - F.ring;
-          const int want = pred >= 0 ? P.n_kt - pred : kAllAdded;
+          const int prior = pred >= 0 ? chain : chain - F.ring;
+          const int want = pred >= 0 ? n_vt - pred : kAllAdded;
           if (prior >= 0) {
             const long long at = (long long)prior * P.n_qt + qt;
-            if (FLEXATTN_DBG_OK(at, (long long)F.slices * P.n_qt, kFusedId, 706) && ld_acquire(F.flags + at) < want) {
+            if (FLEXATTN_DBG_OK(at, (long long)F.slices * F.chains * P.n_qt, kFusedId, 706) && ld_acquire(F.flags + at) < want) {
               const unsigned long long t0 = ptx::globaltimer_ns();
               int polls = 0;
               while (ok && ld_acquire(F.flags + at) < want) {
@@ -841,7 +882,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (!ok) { fail_at = 42; break; }
             asm volatile("fence.proxy.async.global;" ::: "memory");  // the parts are added through the async proxy
           }
-          publish(ia.x, qt, (pred < 0 ? 1 : 0) | (last ? 2 : 0), last ? kAllAdded : P.n_kt - kt);
+          publish(chain, qt, (pred < 0 ? 1 : 0) | (last ? 2 : 0), last ? kAllAdded : n_vt - kt);
         }
       }
       if (!ok && lane == 0) give_up(abort_flag, P.status, kFusedId, fail_at);
@@ -858,7 +899,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (lane == 0) {
           __threadfence();  // what the drain warps have added comes before the flag
           const long long at = (long long)turn.x * P.n_qt + turn.y;
-          if (FLEXATTN_DBG_OK(at, (long long)F.slices * P.n_qt, kFusedId, 707)) st_release(F.flags + at, turn.w);
+          if (FLEXATTN_DBG_OK(at, (long long)F.slices * F.chains * P.n_qt, kFusedId, 707)) st_release(F.flags + at, turn.w);
           ptx::mbar_arrive(&sh->bar_turnfree[T & 1]);
         }
         __syncwarp();
@@ -935,14 +976,15 @@ __global__ void __launch_bounds__(256) prep_kernel(const DevParams P, const Fuse
   }
   if (blockIdx.x % kBlocksPerTile == 0 && in) {  // the first block of a tile
     const int4* cmap = P.col_map + (size_t)(P.map_rows > 1 ? (F.slice0 + slice) / P.heads : 0) * P.n_kt;
-    bool seen = false;
-    for (int j = threadIdx.x; j < P.n_kt; j += 256) {
+    bool seen = F.chains > 1;  // (S2, gathered: the finishing kernel knows which sums there are)
+    for (int j = threadIdx.x; j < (F.chains > 1 ? 0 : P.n_kt); j += 256) {
       const int2 range = __ldg(reinterpret_cast<const int2*>(cmap + j));
       seen = seen || (qt >= range.x && qt < range.y);
     }
     seen = __syncthreads_or(seen);
     if (threadIdx.x == 0) {
-      F.flags[tile] = seen ? 0 : kAllAdded;
+      if (F.chains > 1) F.flags[2 * slice * P.n_qt + qt] = F.flags[(2 * slice + 1) * P.n_qt + qt] = 0;
+      else F.flags[tile] = seen ? 0 : kAllAdded;
       if (blockIdx.x == 0) *F.ticket = 0;
     }
     if (!seen) {
@@ -957,12 +999,20 @@ __global__ void __launch_bounds__(256) prep_kernel(const DevParams P, const Fuse
 
 // After it, where the last part of a query tile has been added like the others: the f32 tiles become dq, times sm_scale.  A
 // thread takes 16 columns of a row: the loads of a warp are 512 consecutive bytes, its stores whole 32-byte sectors.
-template <int D>
+// kGather: two sums per tile, or one of them.
+template <int D, bool kGather>
 __global__ void __launch_bounds__(256) finish_kernel(const DevParams P, const FusedArgs F) {
   const int tile = blockIdx.x, slice = tile / P.n_qt, qt = tile - slice * P.n_qt;
   if (!FLEXATTN_DBG_OK(tile, (long long)F.slices * P.n_qt, kFusedId, 713)) return;
-  if (F.flags[tile] == kAllAdded) return;  // no kv tile sees it: zeroed before
   const float* src = F.dq_acc + (size_t)tile * kTile * D;
+  const float* more = nullptr;
+  if constexpr (kGather) {
+    const int4 rm = s2_row(qt, P.seq_q, P.seq_k, P.window, P.stride);
+    src = F.dq_acc + ((size_t)(2 * slice + (rm.y > rm.z ? 0 : 1)) * P.n_qt + qt) * kTile * D;
+    if (rm.y > rm.z && rm.z > rm.x) more = F.dq_acc + ((size_t)(2 * slice + 1) * P.n_qt + qt) * kTile * D;
+  } else if (F.flags[tile] == kAllAdded) {
+    return;  // no kv tile sees it: zeroed before
+  }
 #pragma unroll
   for (int e = threadIdx.x; e < kTile * D / 16; e += 256) {
     const int lane = e & 31, c16 = (e >> 5) % (D / 16), w = (e >> 5) / (D / 16);
@@ -970,7 +1020,15 @@ __global__ void __launch_bounds__(256) finish_kernel(const DevParams P, const Fu
     uint32_t out[8];
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-      const float4 v = __ldcs(reinterpret_cast<const float4*>(src + ((size_t)(w * (D / 4) + 4 * c16 + c) * 32 + lane) * 4));
+      const size_t at = ((size_t)(w * (D / 4) + 4 * c16 + c) * 32 + lane) * 4;
+      float4 v = __ldcs(reinterpret_cast<const float4*>(src + at));
+      if (kGather && more != nullptr) {
+        const float4 t = __ldcs(reinterpret_cast<const float4*>(more + at));
+        v.x += t.x;
+        v.y += t.y;
+        v.z += t.z;
+        v.w += t.w;
+      }
       out[2 * c] = ptx::pack_bf16(v.x * P.sm_scale, v.y * P.sm_scale);
       out[2 * c + 1] = ptx::pack_bf16(v.z * P.sm_scale, v.w * P.sm_scale);
     }
@@ -982,13 +1040,32 @@ __global__ void __launch_bounds__(256) finish_kernel(const DevParams P, const Fu
   }
 }
 
+// ... and the keys on the stride grid get the sum of their two dK, dV.  A thread takes 8 columns.
+template <int D>
+__global__ void __launch_bounds__(256) s2_finish_kernel(const DevParams P, const FusedArgs F) {
+  constexpr int kTpr = D / 8;
+  const int n = s2_keys(P.seq_k, P.stride);
+  const long long e = (long long)blockIdx.x * 256 + threadIdx.x, key = e / (2 * kTpr);  // of all slices of the launch
+  const int which = (int)(e / kTpr) & 1, c = (int)(e % kTpr) * 8;
+  if (key >= (long long)F.slices * n) return;
+  const float* a = F.s2_dkv + (key * 4 + which) * D + c;
+  const float4 w0 = __ldcs(reinterpret_cast<const float4*>(a)), w1 = __ldcs(reinterpret_cast<const float4*>(a + 4));
+  const float4 s0 = __ldcs(reinterpret_cast<const float4*>(a + 2 * D)), s1 = __ldcs(reinterpret_cast<const float4*>(a + 2 * D + 4));
+  const float sc = which ? 1.f : P.sm_scale;
+  const uint4 out = make_uint4(ptx::pack_bf16((w0.x + s0.x) * sc, (w0.y + s0.y) * sc), ptx::pack_bf16((w0.z + s0.z) * sc, (w0.w + s0.w) * sc),
+                               ptx::pack_bf16((w1.x + s1.x) * sc, (w1.y + s1.y) * sc), ptx::pack_bf16((w1.z + s1.z) * sc, (w1.w + s1.w) * sc));
+  const long long slice = key / n, row = (F.slice0 + slice) * P.seq_k + (key - slice * n) * P.stride;
+  if (FLEXATTN_DBG_OK(row, (long long)P.batch * P.heads * P.seq_k, kFusedId, 716))
+    *reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(which ? P.dv : P.dk) + row * D + c) = out;
+}
+
 constexpr size_t smem_bytes(int D) {
   return (size_t)(D == 64 ? 8 : 5) * (D / 64) * ptx::kPanelBytes + (D == 64 ? 4 : 2) * ptx::kPanelBytes + 8 * kSlotBytes + sizeof(FusedSmem);
 }
 static_assert(smem_bytes(128) <= 232448 && smem_bytes(64) <= 232448, "more shared memory than a CTA can have");
 
 struct Maps {
-  CUtensorMap q, d_o, k, v, dk, dv, dq;
+  CUtensorMap q, d_o, k, v, dk, dv, dq, ks, vs;
 };
 
 // grid 0: only prepares the kernel and says whether it can be launched
@@ -1004,16 +1081,18 @@ int launch_form(cudaStream_t st, const DevParams& d, const FusedArgs& f, const M
   static SmemAttrOnce attr_once{};  // per kernel instantiation, per device
   if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), (int)smem, &attr_once) != FLEXATTN_OK) return FLEXATTN_ERR_CUDA;
   if (grid == 0) return FLEXATTN_OK;
-  kern<<<grid, kThreads, smem, st>>>(t.q, t.d_o, t.k, t.v, t.dk, t.dv, t.dq, d, f, af);
+  kern<<<grid, kThreads, smem, st>>>(t.q, t.d_o, t.k, t.v, t.dk, t.dv, t.dq, t.ks, t.vs, d, f, af);
   return cudaGetLastError() == cudaSuccess ? FLEXATTN_OK : FLEXATTN_ERR_CUDA;
 }
 
 template <int D, int SK, int MK>
 int launch_one(cudaStream_t st, const DevParams& d, const FusedArgs& f, const Maps& t, unsigned grid, int* af) {
-  if constexpr (MK != FLEXATTN_MASK_DOCUMENT) {  // (documents always store it: fused_plan)
-    if (!f.store_dq) return launch_form<D, SK, MK, 0>(st, d, f, t, grid, af);
+  // (documents always store it, S2, gathered, never: fused_plan)
+  if constexpr (MK != FLEXATTN_MASK_DOCUMENT) {
+    if (MK == kMaskS2Gather || !f.store_dq) return launch_form<D, SK, MK, 0>(st, d, f, t, grid, af);
   }
-  return launch_form<D, SK, MK, 1>(st, d, f, t, grid, af);
+  if constexpr (MK != kMaskS2Gather) return launch_form<D, SK, MK, 1>(st, d, f, t, grid, af);
+  return FLEXATTN_ERR_UNSUPPORTED_MOD;
 }
 
 template <int D, int SK>
@@ -1025,6 +1104,7 @@ int launch_mask(cudaStream_t st, const DevParams& d, int mask, const FusedArgs& 
     case FLEXATTN_MASK_SLIDING_WINDOW_CAUSAL:
       return launch_one<D, SK, FLEXATTN_MASK_SLIDING_WINDOW_CAUSAL>(st, d, f, t, grid, af);
     case FLEXATTN_MASK_DOCUMENT: return launch_one<D, SK, FLEXATTN_MASK_DOCUMENT>(st, d, f, t, grid, af);
+    case kMaskS2Gather: return launch_one<D, SK, kMaskS2Gather>(st, d, f, t, grid, af);
     case FLEXATTN_MASK_S2: return launch_one<D, SK, FLEXATTN_MASK_S2>(st, d, f, t, grid, af);
     default: return FLEXATTN_ERR_UNSUPPORTED_MOD;
   }
@@ -1055,14 +1135,18 @@ int launch_score(cudaStream_t st, const DevParams& d, int score, int mask, const
 // scratch holds every slice of a launch, and there are as many launches as keep it within 1 GiB (one slice, if need be).
 struct FusedPlan {
   int launch, group, ring, store_dq;  // slices of a launch, ...
-  size_t off_stats, off_flags, bytes;
+  int chains;                          // sums per query tile
+  size_t off_stats, off_flags, off_s2, bytes;
 };
-FusedPlan fused_plan(int slices, int seq_q, int n_qt, int n_kt, int head_dim, int mask, int window) {
+// s2_n: keys on the stride grid of an S2 call that is gathered, else 0
+FusedPlan fused_plan(int slices, int seq_q, int n_qt, int n_kt, int head_dim, int mask, int window, int s2_n) {
   constexpr long long kL2Budget = 48ll << 20, kLimit = 1ll << 30;
-  const long long acc = (long long)n_qt * kTile * head_dim * 4, most = kLimit / acc > 0 ? kLimit / acc : 1;
+  const int chains = s2_n > 0 ? 2 : 1;
+  const long long acc = (long long)chains * n_qt * kTile * head_dim * 4, s2 = 16ll * s2_n * head_dim;
+  const long long most = kLimit / (acc + s2) > 0 ? kLimit / (acc + s2) : 1;
   const bool windowed = mask == FLEXATTN_MASK_SLIDING_WINDOW_CAUSAL && window < seq_q - 2 * kTile;
   FusedPlan L;
-  L.store_dq = windowed || mask == FLEXATTN_MASK_DOCUMENT || n_kt <= 8;
+  L.store_dq = windowed || mask == FLEXATTN_MASK_DOCUMENT || (n_kt <= 8 && s2_n == 0);
   L.launch = slices;
   if (!L.store_dq) {
     const long long launches = (slices + most - 1) / most;
@@ -1078,7 +1162,9 @@ FusedPlan fused_plan(int slices, int seq_q, int n_qt, int n_kt, int head_dim, in
   auto up = [](size_t n) { return (n + 255) & ~(size_t)255; };
   L.off_stats = up((size_t)L.ring * acc);
   L.off_flags = L.off_stats + up((size_t)L.launch * n_qt * 2 * kTile * sizeof(float));
-  L.bytes = L.off_flags + up(((size_t)L.launch * n_qt + 1) * sizeof(int32_t));
+  L.off_s2 = L.off_flags + up(((size_t)L.launch * chains * n_qt + 1) * sizeof(int32_t));
+  L.bytes = L.off_s2 + up((size_t)L.launch * s2);
+  L.chains = chains;
   return L;
 }
 #endif  // !FLEXATTN_JIT
@@ -1089,7 +1175,7 @@ FusedPlan fused_plan(int slices, int seq_q, int n_qt, int n_kt, int head_dim, in
 namespace {
 FusedPlan plan_of(const FlexAttnParams& p) {
   return fused_plan(p.batch * p.heads, p.seq_q, (p.seq_q + kTile - 1) / kTile, (p.seq_k + kTile - 1) / kTile, p.head_dim,
-                    p.mask_kind, p.window);
+                    p.mask_kind, p.window, s2_gathers(p) ? s2_keys(p.seq_k, p.stride) : 0);
 }
 }  // namespace
 
@@ -1108,8 +1194,10 @@ int launch_sm100_bwd_fused(cudaStream_t st, const DevParams& d, int score, int m
   if (af == nullptr || sms <= 0) return FLEXATTN_ERR_CUDA;
   const int slices = d.batch * d.heads, D = d.head_dim;
   if (D != 64 && D != 128) return FLEXATTN_ERR_UNSUPPORTED_HEAD_DIM;
-  const FusedPlan L = fused_plan(slices, d.seq_q, d.n_qt, d.n_kt, D, mask, d.window);
-  if ((long long)L.launch * d.n_kt > 0x7fffffff - 1024 || (long long)L.launch * d.n_qt > 0x7fffffff / 16) return FLEXATTN_ERR_BAD_SHAPE;
+  const FusedPlan L = fused_plan(slices, d.seq_q, d.n_qt, d.n_kt, D, mask, d.window, d.n_st > 0 ? s2_keys(d.seq_k, d.stride) : 0);
+  const int n_vt = d.n_kt + d.n_st;
+  if (d.n_st > 0) mask = kMaskS2Gather;
+  if ((long long)L.launch * n_vt > 0x7fffffff - 1024 || (long long)L.launch * d.n_qt > 0x7fffffff / 16) return FLEXATTN_ERR_BAD_SHAPE;
   Maps t;
   int e = make_tile_map(&t.q, d.q, slices, d.seq_q, D);
   if (!e) e = make_tile_map(&t.d_o, d.d_o, slices, d.seq_q, D);
@@ -1118,6 +1206,12 @@ int launch_sm100_bwd_fused(cudaStream_t st, const DevParams& d, int score, int m
   if (!e) e = make_tile_map(&t.dk, d.dk, slices, d.seq_k, D);
   if (!e) e = make_tile_map(&t.dv, d.dv, slices, d.seq_k, D);
   if (!e) e = make_tile_map(&t.dq, d.dq, slices, d.seq_q, D, 32);  // a drain warp's rows
+  t.ks = t.k;
+  t.vs = t.v;
+  if (!e && d.n_st > 0) {
+    e = make_strided_map(&t.ks, d.k, slices, d.seq_k, D, d.stride);
+    if (!e) e = make_strided_map(&t.vs, d.v, slices, d.seq_k, D, d.stride);
+  }
   FusedArgs probe{};
   probe.store_dq = L.store_dq;
   auto launch = [&](const FusedArgs& f, unsigned grid) {
@@ -1133,23 +1227,34 @@ int launch_sm100_bwd_fused(cudaStream_t st, const DevParams& d, int score, int m
     f.slice0 = s0;
     f.slices = slices - s0 < L.launch ? slices - s0 : L.launch;
     f.group = L.group;
-    f.ring = L.ring;
+    f.ring = L.chains * L.ring;
+    f.chains = L.chains;
+    f.s2_dkv = reinterpret_cast<float*>(base + L.off_s2);
     f.store_dq = L.store_dq;
-    const int tiles = f.slices * d.n_qt, items = f.slices * d.n_kt;
-    f.ticket = f.flags + tiles;
+    const int tiles = f.slices * d.n_qt, items = f.slices * n_vt;
+    f.ticket = f.flags + tiles * L.chains;
     if (D == 128) prep_kernel<128><<<tiles * 4u, 256, 0, st>>>(d, f);
     else prep_kernel<64><<<tiles * 2u, 256, 0, st>>>(d, f);
     if (cudaGetLastError() != cudaSuccess) return FLEXATTN_ERR_CUDA;
     const unsigned grid = (unsigned)(items < sms ? items : sms);
     if (score == FLEXATTN_SCORE_USER) {
-      void* args[] = {&t.q, &t.d_o, &t.k, &t.v, &t.dk, &t.dv, &t.dq, const_cast<DevParams*>(&d), &f, &af};
+      void* args[] = {&t.q, &t.d_o, &t.k, &t.v, &t.dk, &t.dv, &t.dq, &t.ks, &t.vs, const_cast<DevParams*>(&d), &f, &af};
       e = jit_launch(4, false, d.user_score, D, mask, grid, 1, kThreads, smem_bytes(D), st, args);
     } else {
       e = launch(f, grid);
     }
     if (e || f.store_dq) continue;
-    if (D == 128) finish_kernel<128><<<(unsigned)tiles, 256, 0, st>>>(d, f);
-    else finish_kernel<64><<<(unsigned)tiles, 256, 0, st>>>(d, f);
+    if (d.n_st > 0) {
+      const unsigned blocks = (unsigned)(((long long)f.slices * s2_keys(d.seq_k, d.stride) * (D / 4) + 255) / 256);
+      if (D == 128) finish_kernel<128, true><<<(unsigned)tiles, 256, 0, st>>>(d, f);
+      else finish_kernel<64, true><<<(unsigned)tiles, 256, 0, st>>>(d, f);
+      if (D == 128) s2_finish_kernel<128><<<blocks, 256, 0, st>>>(d, f);
+      else s2_finish_kernel<64><<<blocks, 256, 0, st>>>(d, f);
+    } else if (D == 128) {
+      finish_kernel<128, false><<<(unsigned)tiles, 256, 0, st>>>(d, f);
+    } else {
+      finish_kernel<64, false><<<(unsigned)tiles, 256, 0, st>>>(d, f);
+    }
     if (cudaGetLastError() != cudaSuccess) return FLEXATTN_ERR_CUDA;
   }
   return e;

@@ -108,7 +108,57 @@ struct DevParams {
   float sm_scale, cap;
   int kv_splits;   // split forward: CTAs a query tile's kv tiles are dealt to (1, 2, 4 or 8)
   int user_score;  // handle of a run-time compiled score function (host side only)
+  int n_st;        // kMaskS2Gather: tiles of the keys on the stride grid; 0: the call is not gathered
 };
+
+// ---------------------------------------------------------------------------------------------
+// S2, gathered.  A query keeps its local window and, before it, the keys on the stride grid: walked as one causal range that is every
+// tile below the diagonal for 128 / stride keys in each.  The gathered form splits the kept pairs in two, both plain intervals:
+//   window tiles    the causal sliding window; tile kt holds keys 128 kt ..
+//   strided tiles   tile t holds the keys (128 t + c) * stride, c < 128, fetched as such by TMA (a tensor map whose row pitch is
+//                   `stride` rows); a query i keeps those with (128 t + c) * stride <= i - window
+// A query tile's kv tiles are numbered as ONE range [x, end): from z on they are window tiles (the number is kt), below it strided
+// ones (t = number - x).  Ranges follow from the sizes, so no map is built.  [2,16,4096,64], 512 keys, stride 64: 16.5 tiles a
+// query tile become 6.
+// ---------------------------------------------------------------------------------------------
+constexpr int kMaskS2Gather = FLEXATTN_MASK_S2 + 1;  // inside the kernels only
+__host__ __device__ inline int s2_keys(int seq_k, int stride) { return (seq_k - 1) / stride + 1; }
+__host__ __device__ inline int4 s2_row(int qt, int seq_q, int seq_k, int window, int stride) {  // {x, end, z, 0}
+  const int i0 = qt * kTile, i1 = (seq_q - i0 < kTile ? seq_q : i0 + kTile) - 1;
+  const int last = i1 < seq_k - 1 ? i1 : seq_k - 1, n = s2_keys(seq_k, stride) - 1;
+  const int w1 = last / kTile + 1;
+  int w0 = window <= i0 ? (i0 - window + 1) / kTile : 0;
+  if (window <= i0 && i0 - window + 1 > seq_k - 1) w0 = w1;
+  int strided = 0;
+  if (i1 >= window) {
+    const int k = (i1 - window) / stride;
+    strided = (k < n ? k : n) / kTile + 1;
+  }
+  return make_int4(w0 - strided, w1, w0, 0);
+}
+// Query tiles of kv tile `v` (strided ones behind the n_kt window tiles): {first, end, first fully kept, end of those}
+__host__ __device__ inline int4 s2_col(int v, int seq_q, int seq_k, int n_qt, int n_kt, int window, int stride) {
+  const int whole = seq_q / kTile;  // query tiles without rows past the end
+  int4 r = make_int4(0, 0, 0, 0);
+  if (v < n_kt) {
+    const int j0 = v * kTile, j1 = (seq_k - j0 < kTile ? seq_k : j0 + kTile) - 1;
+    if (j0 >= seq_q) return r;
+    r.x = v;
+    r.y = window < seq_q - j1 ? (j1 + window - 1) / kTile + 1 : n_qt;
+    r.z = v + 1;
+    r.w = window < kTile ? 0 : window < seq_q ? (window - kTile + j0) / kTile + 1 : n_qt;
+  } else {
+    const long long k0 = (long long)(v - n_kt) * kTile, first = k0 * stride + window, all = (k0 + kTile - 1) * stride + window;
+    if (first >= seq_q) return r;
+    r.x = (int)(first / kTile);
+    r.y = n_qt;
+    r.z = all < seq_q ? (int)((all + kTile - 1) / kTile) : n_qt;
+    r.w = n_qt;
+  }
+  if (r.w > whole) r.w = whole;
+  if (r.w < r.z) r.z = r.w = r.x;
+  return r;
+}
 
 // ---------------------------------------------------------------------------------------------
 // Compile-time mask functors.  True = keep.  di/dj are the document ids of positions i/j (only read
@@ -139,7 +189,7 @@ __device__ __forceinline__ bool mask_keep(int i, int j, int window, int stride, 
 // instructions, is taken once per 32 columns; per element it made S2 ten times slower than the dense causal mask).
 template <int MK>
 constexpr bool kMaskIsBits = MK == FLEXATTN_MASK_NONE || MK == FLEXATTN_MASK_CAUSAL || MK == FLEXATTN_MASK_SLIDING_WINDOW ||
-                             MK == FLEXATTN_MASK_SLIDING_WINDOW_CAUSAL || MK == FLEXATTN_MASK_S2;
+                             MK == FLEXATTN_MASK_SLIDING_WINDOW_CAUSAL || MK == FLEXATTN_MASK_S2 || MK == kMaskS2Gather;
 __device__ __forceinline__ uint32_t range_bits32(int lo, int hi) {  // bits [lo, hi) of a word, clipped to [0, 32)
   lo = lo > 0 ? lo : 0;
   hi = hi < 32 ? hi : 32;
@@ -246,6 +296,13 @@ __device__ __forceinline__ bool dbg_in_bounds(long long idx, long long limit, in
   ::flexattn::dbg_in_bounds((long long)(idx), (long long)(limit), P.status, (kernel_id), (site))
 
 #ifndef FLEXATTN_JIT
+// Whether an S2 call is gathered: where that leaves enough fewer tiles a query tile than every tile below the diagonal (a gathered
+// one costs up to 1.2 of a dense one: its mask is never skipped in the window, and the two-query-tile forward has no such form).
+inline bool s2_gathers(const FlexAttnParams& p) {
+  if (p.mask_kind != FLEXATTN_MASK_S2 || p.ab != nullptr || p.score_kind == FLEXATTN_SCORE_USER || p.stride < 2 || p.window <= 0) return false;
+  const double n = ((p.seq_q < p.seq_k ? p.seq_q : p.seq_k) + kTile - 1) / kTile;
+  return 1.2 * ((double)p.window / kTile + 2 + n / (2.0 * p.stride)) < 0.5 * (n + 1);
+}
 // Host-side validation of a forward call, shared by flexattn_fwd and flexattn_fwd_noalloc (api.cu).
 int validate_fwd_args(const FlexAttnParams* p, bool* tc);
 

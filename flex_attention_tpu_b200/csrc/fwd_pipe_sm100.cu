@@ -67,7 +67,8 @@ __device__ __forceinline__ float score_half(float (&x)[kHalf], int i, int j0, in
                                             ptx::BiasRows bias = ptx::BiasRows(), int klo = 0, int khi = 0, uint32_t pattern = 0u) {
   float mx[4] = {kMasked, kMasked, kMasked, kMasked};
   uint32_t keep = 0u;  // kept columns of the current group of 32 (kInterval on partial tiles)
-  const float abase = slope2 * (float)(j0 + c_base - i);
+  constexpr bool kGather = MK == kMaskS2Gather;
+  const float abase = slope2 * (float)((j0 + c_base) * (kGather ? ctx.step : 1) - i), astep = slope2 * (kGather ? (float)ctx.step : 1.f);
   if constexpr (SK == FLEXATTN_SCORE_SOFTCAP || SK == FLEXATTN_SCORE_USER) {
     // scalar form: the packed one costs registers here
 #pragma unroll
@@ -93,8 +94,8 @@ __device__ __forceinline__ float score_half(float (&x)[kHalf], int i, int j0, in
   // the score arithmetic runs two columns per instruction (packed f32x2); masking and the maximum are scalar
   // ALiBi: the bias of columns (c, c + 1) advances by a constant from pair to pair: one packed add instead of
   // rebuilding it from the column numbers
-  uint64_t b2 = ptx::pack2(abase, abase + slope2);
-  const uint64_t bstep2 = ptx::pack2(2.f * slope2, 2.f * slope2);
+  uint64_t b2 = ptx::pack2(abase, abase + astep);
+  const uint64_t bstep2 = ptx::pack2(2.f * astep, 2.f * astep);
 #pragma unroll
   for (int c = 0; c < kHalf; c += 2) {
     const uint64_t x2 = ptx::pack2(x[c], x[c + 1]);
@@ -133,7 +134,9 @@ template <int D, int SK, int MK>
 __global__ void __launch_bounds__(kThreads, 1)
     fwd_pipe_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                           const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
+                          const __grid_constant__ CUtensorMap tm_ks, const __grid_constant__ CUtensorMap tm_vs,
                           const DevParams P, int* abort_flag) {
+  constexpr bool kGather = MK == kMaskS2Gather;  // tm_ks, tm_vs: the keys and values on the stride grid
   constexpr int kPanels = D / 64;
   constexpr uint32_t kTileBytes = kPanels * ptx::kPanelBytes;
   constexpr uint32_t kTmemCols = 512;
@@ -189,7 +192,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       ptx::prefetch_tensormap(&tm_q);
       ptx::prefetch_tensormap(&tm_k);
       int T = 0, qi = 0;
-      for (ItemCursor it(P); ok; it.next(), ++qi) {
+      for (ItemCursor<kGather> it(P); ok; it.next(), ++qi) {
         it.skip_empty();
         if (!it.valid()) break;
         const int bh = it.bh(), first = it.rm.x, end = it.rm.y, N = it.tiles();
@@ -207,11 +210,12 @@ __global__ void __launch_bounds__(kThreads, 1)
             ok = ptx::mbar_wait(&sh->bar_kfree[T & 1], ((T - 2) >> 1) & 1);
             if (!ok) { fail_at = 21; break; }
           }
+          const int kt = kv_tile_at<SK>(first, end, t);
           ptx::mbar_arrive_expect_tx(&sh->bar_k[T & 1], kTileBytes);
 #pragma unroll
           for (int p = 0; p < kPanels; ++p)
-            ptx::tma_load_3d(sK + (T & 1) * kTileBytes + p * ptx::kPanelBytes, &tm_k, &sh->bar_k[T & 1], p * 64,
-                             kv_tile_at<SK>(first, end, t) * kTile, bh);
+            ptx::tma_load_3d(sK + (T & 1) * kTileBytes + p * ptx::kPanelBytes, kGather && kt < it.rm.z ? &tm_ks : &tm_k, &sh->bar_k[T & 1],
+                             p * 64, (kGather && kt < it.rm.z ? kt - first : kt) * kTile, bh);
         }
       }
       if (ok) {
@@ -235,7 +239,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       ptx::prefetch_tensormap(&tm_v);
       int T = 0;
       uint32_t wsb = 0, wph = 0;  // barrier (T-2) % 3 and phase ((T-2) / 3) & 1 of the P V this thread waits for
-      for (ItemCursor it(P); ok; it.next()) {
+      for (ItemCursor<kGather> it(P); ok; it.next()) {
         it.skip_empty();
         if (!it.valid()) break;
         const int bh = it.bh(), first = it.rm.x, end = it.rm.y, N = it.tiles();
@@ -245,11 +249,12 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (!ok) break;
             if (++wsb == kSBufs) { wsb = 0; wph ^= 1u; }
           }
+          const int kt = kv_tile_at<SK>(first, end, t);
           ptx::mbar_arrive_expect_tx(&sh->bar_v[T & 1], kTileBytes);
 #pragma unroll
           for (int p = 0; p < kPanels; ++p)
-            ptx::tma_load_3d(sV + (T & 1) * kTileBytes + p * ptx::kPanelBytes, &tm_v, &sh->bar_v[T & 1], p * 64,
-                             kv_tile_at<SK>(first, end, t) * kTile, bh);
+            ptx::tma_load_3d(sV + (T & 1) * kTileBytes + p * ptx::kPanelBytes, kGather && kt < it.rm.z ? &tm_vs : &tm_v, &sh->bar_v[T & 1],
+                             p * 64, (kGather && kt < it.rm.z ? kt - first : kt) * kTile, bh);
         }
       }
       if (!ok) give_up(abort_flag, P.status, 4, 23);
@@ -344,7 +349,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     int sb = 0;          // T % 3: score buffer of that tile
     uint32_t sph = 0;    // (T / 3) & 1: phase of its barriers
 
-    for (ItemCursor it(P); it.valid(); it.next()) {
+    for (ItemCursor<kGather> it(P); it.valid(); it.next()) {
       const int qt = it.qt(), bh = it.bh(), b = bh / P.heads, h = bh % P.heads;
       const int4 rm = it.rm;
       const int N = rm.y - rm.x;
@@ -360,7 +365,13 @@ __global__ void __launch_bounds__(kThreads, 1)
       bool doc_runs = false;
       int klo = 0, khi = P.seq_k;
       const uint32_t pattern = MK == FLEXATTN_MASK_S2 ? stride_pattern32(P.stride) : 0u;
-      if constexpr (kMaskIsBits<MK>) row_key_interval<MK>(i, P.seq_k, P.window, klo, khi);
+      int skhi = 0;  // kGather: the row keeps the strided keys [0, skhi), counted along the grid
+      if constexpr (kGather) {
+        row_key_interval<FLEXATTN_MASK_SLIDING_WINDOW_CAUSAL>(i, P.seq_k, P.window, klo, khi);
+        if (i >= P.window) skhi = min((i - P.window) / P.stride, s2_keys(P.seq_k, P.stride) - 1) + 1;
+      } else if constexpr (kMaskIsBits<MK>) {
+        row_key_interval<MK>(i, P.seq_k, P.window, klo, khi);
+      }
       if constexpr (MK == FLEXATTN_MASK_DOCUMENT) {
         doc_runs = FLEXATTN_DBG_OK(b, P.batch, 4, 107) && P.doc_sorted[b] != 0;
         if (doc_runs && i < P.seq_q && FLEXATTN_DBG_OK((long long)b * P.doc_stride + i, n_doc, 4, 108)) {
@@ -374,13 +385,18 @@ __global__ void __launch_bounds__(kThreads, 1)
       int ab_rows = kDenseBias ? min(32, max(0, P.seq_q - i_warp)) : 0;
       if (ab_rows > 0 && !FLEXATTN_DBG_OK((long long)bh * P.seq_q + i_warp + ab_rows - 1, n_rows, 4, 103)) ab_rows = 0;
       const float* ab_w = ab_rows > 0 ? P.ab + ((size_t)bh * P.seq_q + i_warp) * P.seq_k : P.ab;
-      const ScoreCtx ctx{P.sm_scale, b, h};
+      ScoreCtx ctx{P.sm_scale, b, h};
 
       for (int n = 0; n < N; ++n, ++T) {
         const uint32_t par = T & 1;
         const uint32_t colS = (uint32_t)sb * 128u;
-        const int kt = kv_tile_at<SK>(rm.x, rm.y, n), j0 = kt * kTile;
-        const bool partial = kDenseBias || !(kt >= rm.z && kt < rm.w);
+        const int kt = kv_tile_at<SK>(rm.x, rm.y, n);
+        const bool strided = kGather && kt < rm.z;
+        const int j0 = (strided ? kt - rm.x : kt) * kTile;  // first key, or its number along the stride grid
+        // (gathered: whether this warp's tile is fully kept follows from its row's interval)
+        const int lo = strided ? 0 : klo, hi = strided ? skhi : khi;
+        const bool partial = kDenseBias || (kGather ? __any_sync(0xffffffffu, lo > j0 || hi < j0 + kTile) : !(kt >= rm.z && kt < rm.w));
+        if constexpr (kGather) ctx.step = strided ? P.stride : 1;
         if (MK == FLEXATTN_MASK_DOCUMENT && partial && !doc_runs && half == 0) {
           const int j = j0 + row;
           sh->doc[par][row] = (j < P.seq_k && FLEXATTN_DBG_OK((long long)b * P.doc_stride + j, n_doc, 4, 104)) ? doc[j] : -1;
@@ -441,7 +457,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                                                               capl2, csc, di, sh->doc[par], ctx);
             } else {
               tmax = score_half<SK, MK, true>(x, i, j0, c_base, P.seq_k, P.window, P.stride, c2, slope2, capl2, csc, di,
-                                              sh->doc[par], ctx, ptx::BiasRows(), klo, khi, pattern);
+                                              sh->doc[par], ctx, ptx::BiasRows(), lo, hi, pattern);
             }
           } else if constexpr (SK != FLEXATTN_SCORE_NONE) {
             tmax = score_half<SK, MK, false>(x, i, j0, c_base, P.seq_k, P.window, P.stride, c2, slope2, capl2, csc, di,
@@ -600,7 +616,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 #ifndef FLEXATTN_JIT
 template <int D, int SK, int MK>
 int launch_one(cudaStream_t st, const DevParams& d, const CUtensorMap& tq, const CUtensorMap& tk,
-               const CUtensorMap& tv, const CUtensorMap& to, int* abort_flag) {
+               const CUtensorMap& tv, const CUtensorMap& to, const CUtensorMap& tks, const CUtensorMap& tvs, int* abort_flag) {
   constexpr size_t need = 6 * (D / 64) * ptx::kPanelBytes + sizeof(PipeSmem) + 1024 + (!kDenseBias || D == 128 ? 0 : kBiasScratch);
   // 512 TMEM columns per CTA: never let two CTAs share an SM (the second would spin in tcgen05.alloc)
   constexpr size_t smem = need > 120 * 1024 ? need : 120 * 1024;
@@ -612,32 +628,35 @@ int launch_one(cudaStream_t st, const DevParams& d, const CUtensorMap& tq, const
   const int sms = sm_count();
   if (sms <= 0) return FLEXATTN_ERR_CUDA;
   dim3 grid((unsigned)(items < sms ? items : sms));
-  kern<<<grid, kThreads, smem, st>>>(tq, tk, tv, to, d, abort_flag);
+  kern<<<grid, kThreads, smem, st>>>(tq, tk, tv, to, tks, tvs, d, abort_flag);
   return cudaGetLastError() == cudaSuccess ? FLEXATTN_OK : FLEXATTN_ERR_CUDA;
 }
 
 template <int D, int SK>
 int launch_mask(cudaStream_t st, const DevParams& d, int mask, const CUtensorMap& tq, const CUtensorMap& tk,
-                const CUtensorMap& tv, const CUtensorMap& to, int* af) {
+                const CUtensorMap& tv, const CUtensorMap& to, const CUtensorMap& tks, const CUtensorMap& tvs, int* af) {
   switch (mask) {
-    case FLEXATTN_MASK_NONE: return launch_one<D, SK, FLEXATTN_MASK_NONE>(st, d, tq, tk, tv, to, af);
-    case FLEXATTN_MASK_CAUSAL: return launch_one<D, SK, FLEXATTN_MASK_CAUSAL>(st, d, tq, tk, tv, to, af);
-    case FLEXATTN_MASK_SLIDING_WINDOW: return launch_one<D, SK, FLEXATTN_MASK_SLIDING_WINDOW>(st, d, tq, tk, tv, to, af);
+    case FLEXATTN_MASK_NONE: return launch_one<D, SK, FLEXATTN_MASK_NONE>(st, d, tq, tk, tv, to, tks, tvs, af);
+    case FLEXATTN_MASK_CAUSAL: return launch_one<D, SK, FLEXATTN_MASK_CAUSAL>(st, d, tq, tk, tv, to, tks, tvs, af);
+    case FLEXATTN_MASK_SLIDING_WINDOW: return launch_one<D, SK, FLEXATTN_MASK_SLIDING_WINDOW>(st, d, tq, tk, tv, to, tks, tvs, af);
     case FLEXATTN_MASK_SLIDING_WINDOW_CAUSAL:
-      return launch_one<D, SK, FLEXATTN_MASK_SLIDING_WINDOW_CAUSAL>(st, d, tq, tk, tv, to, af);
-    case FLEXATTN_MASK_DOCUMENT: return launch_one<D, SK, FLEXATTN_MASK_DOCUMENT>(st, d, tq, tk, tv, to, af);
-    case FLEXATTN_MASK_S2: return launch_one<D, SK, FLEXATTN_MASK_S2>(st, d, tq, tk, tv, to, af);
+      return launch_one<D, SK, FLEXATTN_MASK_SLIDING_WINDOW_CAUSAL>(st, d, tq, tk, tv, to, tks, tvs, af);
+    case FLEXATTN_MASK_DOCUMENT: return launch_one<D, SK, FLEXATTN_MASK_DOCUMENT>(st, d, tq, tk, tv, to, tks, tvs, af);
+#if !FLEXATTN_DENSE_BIAS
+    case kMaskS2Gather: return launch_one<D, SK, kMaskS2Gather>(st, d, tq, tk, tv, to, tks, tvs, af);
+#endif
+    case FLEXATTN_MASK_S2: return launch_one<D, SK, FLEXATTN_MASK_S2>(st, d, tq, tk, tv, to, tks, tvs, af);
     default: return FLEXATTN_ERR_UNSUPPORTED_MOD;
   }
 }
 
 template <int D>
 int launch_score(cudaStream_t st, const DevParams& d, int score, int mask, const CUtensorMap& tq,
-                 const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to, int* af) {
+                 const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to, const CUtensorMap& tks, const CUtensorMap& tvs, int* af) {
   switch (score) {
-    case FLEXATTN_SCORE_NONE: return launch_mask<D, FLEXATTN_SCORE_NONE>(st, d, mask, tq, tk, tv, to, af);
-    case FLEXATTN_SCORE_ALIBI: return launch_mask<D, FLEXATTN_SCORE_ALIBI>(st, d, mask, tq, tk, tv, to, af);
-    case FLEXATTN_SCORE_SOFTCAP: return launch_mask<D, FLEXATTN_SCORE_SOFTCAP>(st, d, mask, tq, tk, tv, to, af);
+    case FLEXATTN_SCORE_NONE: return launch_mask<D, FLEXATTN_SCORE_NONE>(st, d, mask, tq, tk, tv, to, tks, tvs, af);
+    case FLEXATTN_SCORE_ALIBI: return launch_mask<D, FLEXATTN_SCORE_ALIBI>(st, d, mask, tq, tk, tv, to, tks, tvs, af);
+    case FLEXATTN_SCORE_SOFTCAP: return launch_mask<D, FLEXATTN_SCORE_SOFTCAP>(st, d, mask, tq, tk, tv, to, tks, tvs, af);
     default: return FLEXATTN_ERR_UNSUPPORTED_MOD;
   }
 }
@@ -664,6 +683,13 @@ int launch_sm100_fwd_pipe(cudaStream_t st, const DevParams& d, int score, int ma
   if (e) return e;
   e = make_tile_map(&to, d.o, slices, d.seq_q, d.head_dim);
   if (e) return e;
+  CUtensorMap tks = tk, tvs = tv;
+  if (d.n_st > 0) {
+    mask = kMaskS2Gather;
+    e = make_strided_map(&tks, d.k, slices, d.seq_k, d.head_dim, d.stride);
+    if (!e) e = make_strided_map(&tvs, d.v, slices, d.seq_k, d.head_dim, d.stride);
+    if (e) return e;
+  }
   if (score == FLEXATTN_SCORE_USER) {
     // a kernel compiled at run time around the registered score function: same parameters, grid and shared memory
     const size_t need = 6 * (size_t)(d.head_dim / 64) * ptx::kPanelBytes + sizeof(PipeSmem) + 1024 +
@@ -671,12 +697,12 @@ int launch_sm100_fwd_pipe(cudaStream_t st, const DevParams& d, int score, int ma
     const long long items = (long long)d.n_qt * d.batch * d.heads;
     const int sms = sm_count();
     if (sms <= 0) return FLEXATTN_ERR_CUDA;
-    void* args[] = {&tq, &tk, &tv, &to, const_cast<DevParams*>(&d), &af};
+    void* args[] = {&tq, &tk, &tv, &to, &tks, &tvs, const_cast<DevParams*>(&d), &af};
     return jit_launch(0, kDenseBias, d.user_score, d.head_dim, mask, (unsigned)(items < sms ? items : sms), 1, kThreads,
                       need > 120 * 1024 ? need : 120 * 1024, st, args);
   }
-  if (d.head_dim == 128) return launch_score<128>(st, d, score, mask, tq, tk, tv, to, af);
-  if (d.head_dim == 64) return launch_score<64>(st, d, score, mask, tq, tk, tv, to, af);
+  if (d.head_dim == 128) return launch_score<128>(st, d, score, mask, tq, tk, tv, to, tks, tvs, af);
+  if (d.head_dim == 64) return launch_score<64>(st, d, score, mask, tq, tk, tv, to, tks, tvs, af);
   return FLEXATTN_ERR_UNSUPPORTED_HEAD_DIM;
 }
 #endif  // !FLEXATTN_JIT

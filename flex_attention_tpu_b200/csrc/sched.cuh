@@ -9,6 +9,8 @@ namespace flexattn {
 // work order of the q tiles (most kv tiles first), head index fastest.  The resulting list is dealt to the CTAs in
 // rounds that alternate direction (CTA c takes entry c of an even round and entry G-1-c of an odd one), which evens
 // out the work of a sorted list.  Tile order and mask-map row of the next item are fetched one item ahead.
+// kGather: S2, gathered (no map; later query tiles have more kv tiles).
+template <bool kGather = false>
 struct ItemCursor {
   const DevParams& P;
   int total, per_row, group, full_groups;
@@ -29,6 +31,10 @@ struct ItemCursor {
     const int r2 = r - gi * group * P.n_qt;
     const int rank = r2 / width;
     bh = b * P.heads + gi * group + (r2 - rank * width);
+    if constexpr (kGather) {
+      qt = P.n_qt - 1 - rank;
+      return s2_row(qt, P.seq_q, P.seq_k, P.window, P.stride);
+    }
     const size_t row = (size_t)(P.map_rows > 1 ? b : 0) * P.n_qt;
     qt = __ldg(&P.order[row + rank]);
     return __ldg(&P.order_rm[row + rank]);  // the row-map entry of that q tile: two independent loads

@@ -21,6 +21,7 @@ __device__ __forceinline__ int kv_tile_at(int first, int end, int n) {
 struct ScoreCtx {
   float sm_scale;
   int b, h;
+  int step = 1;  // positions from one column to the next (the strided tiles of S2, gathered)
 };
 
 // x: this thread's 128 raw scores of one tile -> log2-domain logits in place; returns their maximum.

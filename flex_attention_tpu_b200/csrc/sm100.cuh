@@ -481,6 +481,8 @@ int ensure_dynamic_smem(const void* kernel, int bytes, SmemAttrOnce* once);
 // Host side: 3-D tensor map over a [slices, rows, cols] bf16 array, box = {64 cols, box_rows rows, 1 slice},
 // 128-byte swizzle, out-of-range rows read as zero.
 int make_tile_map(CUtensorMap* out, const void* base, int slices, int rows, int cols, int box_rows = kTile);
+// ... over every step-th row of such an array (rows 0, step, 2 step ... of each slice)
+int make_strided_map(CUtensorMap* out, const void* base, int slices, int rows, int cols, int step);
 #endif  // !FLEXATTN_JIT
 
 // Kernels live in an unnamed namespace in ahead-of-time builds and in a named one when compiled at run time
