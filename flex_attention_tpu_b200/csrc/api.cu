@@ -94,6 +94,7 @@ DevParams make_dev(const FlexAttnParams* p) {
   d.col_map = reinterpret_cast<const int4*>(ws + L.off_col);
   d.order = reinterpret_cast<const int32_t*>(ws + L.off_order);
   d.order_rm = reinterpret_cast<const int4*>(ws + L.off_order_rm);
+  d.order_pair = reinterpret_cast<const int32_t*>(ws + L.off_order_pair);
   if (p->mask_kind == FLEXATTN_MASK_DOCUMENT) {
     d.run_lo = reinterpret_cast<const int32_t*>(ws + L.off_run_lo);
     d.run_hi = reinterpret_cast<const int32_t*>(ws + L.off_run_hi);
@@ -200,20 +201,34 @@ int mean_kv_tiles(const FlexAttnParams* p) {
     default: return 0;
   }
 }
-constexpr int kPairMinTiles = 12;  // measured: at 12.5 tiles the two kernels tie, at 16 the pair kernel is 5-12 % faster, at 32 15 %
-// Whether the two-query-tile kernel serves the call (rows of kPairMinTiles kv tiles given): it does a tile in 0.87 of the
-// persistent kernel's time, but in units of two query tiles that are dealt out by the hardware one CTA at a time, so it
-// needs enough of them.  Rows of equal length: whole waves of either kernel compared (8 x 8 x 1600, D = 128: 109 us against
-// 97 for the persistent kernel; 4 x 8 x 1800, D = 64: 61 against 71).  Other masks, where the longest rows make the tail:
-// four waves of pairs, three at D = 64 ([1,16,3001,128] causal, 1.3 waves: 65 us against 47; [1,16,8192,128], 3.5: 287
-// against 264; [2,16,4096,64], 3.5: 148 against 151; [1,32,8192,128], 6.9: 507 against 534).
+constexpr int kSplitMinTiles = 12;  // kv tiles a query tile sees from which its split over CTAs pays
+// Whether the two-query-tile kernel serves the call.  It takes 0.75 to 0.9 of the persistent kernel's time per tile, but in units
+// of two query tiles, and fewer of them than CTAs leave SMs idle.  Times in us, two-query-tile / persistent, on 148 SMs; slices x
+// queries, no score function.
+//   no mask (rows of equal length: whole waves of either compared; one of pairs takes 1.75 of one of query tiles)
+//       D = 128: 24 x 1024 (0.65 waves of pairs, 1.3 of query tiles) 23 / 27, 32 x 1536 (1.3, 2.6) 58 / 52, 16 x 4096 (1.7, 3.5) 126 / 147
+//   windows   p = waves of pairs: 24 x 777 0.65 15 / 12, 16 x 2048 0.86 20 / 21, 24 x 2048 1.3 31 / 29, 32 x 2048 1.7 33 / 38
+//   causal    D = 64: 16 x 3001 1.3 65 / 63, 32 x 2048 1.7 36 / 42, 64 x 2048 3.5 62 / 76; D = 128: 64 x 777 1.7 30 / 28, 32 x 2048 1.7
+//             43 / 48, 64 x 2048 3.5 76 / 102; but 96 x 1024 2.6 50 / 47 (short rows, the last of a wave stands alone)
+//   documents D = 64: 8 x 3001 0.65 33 / 30, 24 x 1536 0.97 39 / 46; D = 128: 24 x 2048 1.3 48 / 44, 32 x 2048 1.7 48 / 54,
+//             softcap 24 x 1536 0.97 46 / 53
 bool pair_pays(const FlexAttnParams* p) {
   const int sms = sm_count();
   if (sms <= 0) return true;
   const long long n_qt = (p->seq_q + FLEXATTN_TILE - 1) / FLEXATTN_TILE, slices = (long long)p->batch * p->heads;
   const long long pairs = (n_qt + 1) / 2 * slices, items = n_qt * slices;
-  if (p->mask_kind == FLEXATTN_MASK_NONE) return 1.74 * ((pairs + sms - 1) / sms) < (double)((items + sms - 1) / sms);
-  return pairs >= (p->head_dim == 128 ? 4 : 3) * (long long)sms;
+  const double waves = (double)pairs / sms;
+  if (n_qt < 2) return false;  // its second stream would have nothing to do
+  const bool scored = p->score_kind == FLEXATTN_SCORE_SOFTCAP || p->score_kind == FLEXATTN_SCORE_USER;
+  switch (p->mask_kind) {
+    case FLEXATTN_MASK_NONE:
+      return waves >= 2.5 || 1.75 * ((pairs + sms - 1) / sms) < (double)((items + sms - 1) / sms);
+    case FLEXATTN_MASK_SLIDING_WINDOW_CAUSAL: return waves >= 1.7 || (waves >= 0.8 && waves <= 1 && 4 * items >= 5ll * sms);
+    case FLEXATTN_MASK_DOCUMENT: return waves >= 1.7 || ((scored || p->head_dim == 64) && waves >= 0.85 && 2 * items >= 3ll * sms);
+    default:  // causal, S2, a window open ahead: the longest rows make the tail
+      if (p->head_dim == 64) return waves >= 1.7;
+      return 10 * items >= 34ll * sms && (waves >= 3 || waves < 2.2 || n_qt > 8);
+  }
 }
 int forced_fwd_kernel() {  // 0: choose by shape, 1: two-query-tile kernel, 2: persistent kernel, 3: split kernel
   static const int choice = [] {
@@ -226,7 +241,7 @@ int forced_fwd_kernel() {  // 0: choose by shape, 1: two-query-tile kernel, 2: p
   }();
   return choice;
 }
-// CTAs per query tile of the split kernel (fwd_split_sm100.cu); 0: another kernel.  It takes rows of kPairMinTiles kv tiles
+// CTAs per query tile of the split kernel (fwd_split_sm100.cu); 0: another kernel.  It takes rows of kSplitMinTiles kv tiles
 // where a query tile gets at least two CTAs, or where its only tile has no more than 32 rows (the other warps then skip
 // their part).  Against the persistent kernel: 64 slices x 1 row x 8191 keys 108 (two-query-tile kernel) -> 47 us, 74 x 4096
 // 39 -> 31, 256 x 6 rows x 8663 (D = 64) 146 -> 127, one causal slice of 4096 39 -> 20; with one CTA per tile and full
@@ -236,7 +251,7 @@ int kv_splits(const FlexAttnParams* p) {
   if (p->ab != nullptr || p->score_kind == FLEXATTN_SCORE_USER) return 0;
   const int sms = sm_count(), tiles = mean_kv_tiles(p);
   const long long n_qt = (p->seq_q + FLEXATTN_TILE - 1) / FLEXATTN_TILE, items = n_qt * p->batch * p->heads;
-  if (sms <= 0 || tiles < kPairMinTiles || items > 0x7fffffff / 8) return 0;
+  if (sms <= 0 || tiles < kSplitMinTiles || items > 0x7fffffff / 8) return 0;
   // as many CTAs as run at once (a second wave of clusters costs what the split gains), with four kv tiles or more each
   int c = 1;
   while (c < 8 && tiles >= 8 * c && items <= split_clusters_at_once(2 * c)) c *= 2;
@@ -252,11 +267,11 @@ int flexattn_fwd(void* stream, const FlexAttnParams* p) {
   DevParams d = make_dev(p);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (tc) {
-    // Three tensor-core forward kernels: the persistent one (fwd_pipe_sm100.cu: work items streamed through each CTA,
-    // prologue and epilogue hidden, best for short rows and for few items), the two-query-tile one (fwd_pair_sm100.cu: one row
-    // per thread, K/V shared by two tiles, best for long rows and many items) and the split one (fwd_split_sm100.cu: a
-    // cluster per query tile, best for few query tiles against many keys).  FLEXATTN_FWD_KERNEL=pair, =pipe or =split in
-    // the environment forces one where it can run (read once per process).
+    // Three tensor-core forward kernels: the two-query-tile one (fwd_pair_sm100.cu: one row per thread, K/V shared by two
+    // tiles, pairs dealt out as CTAs get on; the fastest where there are enough of them), the persistent one (fwd_pipe_sm100.cu:
+    // query tiles one by one, for fewer items, a dense bias and gathered S2) and the split one (fwd_split_sm100.cu: a cluster per
+    // query tile, best for few query tiles against many keys).  FLEXATTN_FWD_KERNEL=pair, =pipe or =split in the environment
+    // forces one where it can run (read once per process).
     const bool pair_can = p->ab == nullptr;
     const int forced = forced_fwd_kernel();
     if (forced == 0 && s2_gathers(*p)) {  // (few tiles a query tile: the persistent kernel)
@@ -270,7 +285,7 @@ int flexattn_fwd(void* stream, const FlexAttnParams* p) {
         d.kv_splits = 1;
       if (d.kv_splits > 0) return launch_sm100_fwd_split(st, d, p->score_kind, p->mask_kind);
     }
-    if (pair_can && (forced == 1 || (forced == 0 && mean_kv_tiles(p) >= kPairMinTiles && pair_pays(p))))
+    if (pair_can && (forced == 1 || (forced == 0 && pair_pays(p))))
       return launch_sm100_fwd_pair(st, d, p->score_kind, p->mask_kind);
     if (d.ab != nullptr) return launch_sm100_fwd_pipe_bias(st, d, p->score_kind, p->mask_kind);
     return launch_sm100_fwd_pipe(st, d, p->score_kind, p->mask_kind);

@@ -171,15 +171,6 @@ __device__ __forceinline__ int ld_acquire(const int32_t* p) {
 __device__ __forceinline__ void st_release(int32_t* p, int v) {
   asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
-__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {  // does not wait
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred P;\n\tmbarrier.test_wait.parity.shared::cta.b64 P, [%1], %2;\n\tselp.u32 %0, 1, 0, P;\n\t}\n"
-      : "=r"(ok)
-      : "r"(ptx::smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
 __device__ __forceinline__ void bulk_load(void* smem_dst, const void* src, uint32_t bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                    ptx::smem_u32(smem_dst)),
@@ -545,7 +536,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             fetch(1);
           }
         };
-        if (kStore != 0 && __all_sync(0xffffffffu, mbar_test_wait(&sh->bar_turn[T & 1], (T >> 1) & 1))) fetch_first(sh->turn[T & 1]);
+        if (kStore != 0 && __all_sync(0xffffffffu, ptx::mbar_test_wait(&sh->bar_turn[T & 1], (T >> 1) & 1))) fetch_first(sh->turn[T & 1]);
         ok = __all_sync(0xffffffffu, ptx::mbar_wait(&sh->bar_dq, T & 1));
         if (!ok) { fail_at = 31; break; }
         ptx::tc_fence_after();

@@ -47,7 +47,7 @@ constexpr int32_t kMapMagic = 0x464c5841;  // "FLXA"
 
 struct MapLayout {
   int n_qt, n_kt, rows, n_t;
-  size_t off_row, off_col, off_doc, off_order, off_order_rm, off_run_lo, off_run_hi, off_sorted, bytes;
+  size_t off_row, off_col, off_doc, off_order, off_order_rm, off_order_pair, off_run_lo, off_run_hi, off_sorted, bytes;
 };
 
 __host__ __device__ inline MapLayout map_layout(int batch, int seq_q, int seq_k, int mask_kind) {
@@ -70,7 +70,9 @@ __host__ __device__ inline MapLayout map_layout(int batch, int seq_q, int seq_k,
   // interval, so the kernels mask partial tiles from these two numbers instead of comparing ids per element)
   const size_t len = (size_t)(seq_q > seq_k ? seq_q : seq_k);
   const size_t runs = (mask_kind == FLEXATTN_MASK_DOCUMENT) ? sizeof(int32_t) * (size_t)batch * len : 0;
-  L.off_run_lo = (L.off_order_rm + sizeof(int4) * (size_t)L.rows * L.n_qt + 15) & ~(size_t)15;
+  // ... and the pairs of adjacent q tiles in such an order (work order of the two-query-tile forward kernel)
+  L.off_order_pair = (L.off_order_rm + sizeof(int4) * (size_t)L.rows * L.n_qt + 15) & ~(size_t)15;
+  L.off_run_lo = (L.off_order_pair + sizeof(int32_t) * (size_t)L.rows * ((L.n_qt + 1) / 2) + 15) & ~(size_t)15;
   L.off_run_hi = (L.off_run_lo + runs + 15) & ~(size_t)15;
   L.off_sorted = (L.off_run_hi + runs + 15) & ~(size_t)15;
   L.bytes = (L.off_sorted + (runs ? sizeof(int32_t) * (size_t)batch : 0) + 255) & ~(size_t)255;
@@ -98,6 +100,7 @@ struct DevParams {
   const int4* col_map;  // [rows][n_kt]
   const int32_t* order;  // [rows][n_qt]: q tiles by decreasing number of kv tiles
   const int4* order_rm;  // [rows][n_qt]: row_map entry of order[i]
+  const int32_t* order_pair;  // [rows][(n_qt + 1) / 2]: pairs of q tiles (2 p, 2 p + 1) by decreasing number of kv tiles
   const int32_t* run_lo;      // document masks: [batch][doc_stride] first position of each position's run of equal ids
   const int32_t* run_hi;      // ... one past its last position
   const int32_t* doc_sorted;  // ... [batch] 1 when the row's ids never decrease (runs are whole documents)

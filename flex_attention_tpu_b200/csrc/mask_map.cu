@@ -195,28 +195,40 @@ __global__ void mask_map_kernel(MapHeader hdr, MapHeader* __restrict__ hdr_out, 
   }
 }
 
-// Work order of the q tiles of one map row: by decreasing number of kv tiles (counting sort; ties by decreasing
-// tile index, so the result is deterministic).  One CTA per map row; hist has n_kt + 2 entries.
-__global__ void order_kernel(const int4* __restrict__ row_map, int32_t* __restrict__ order, int4* __restrict__ order_rm,
-                             int n_qt, int n_kt) {
-  extern __shared__ int hist[];
-  const int4* rm = row_map + (size_t)blockIdx.x * n_qt;
-  int32_t* ord = order + (size_t)blockIdx.x * n_qt;
-  int4* ord_rm = order_rm + (size_t)blockIdx.x * n_qt;
+// Work order of the n entries of one list: by decreasing count (at most n_kt; counting sort; ties by decreasing index, so the
+// result is deterministic).  One CTA; hist has n_kt + 2 entries.
+template <class Count>
+__device__ void sort_by_count(Count count, int32_t* ord, int n, int n_kt, int* hist) {
   for (int i = threadIdx.x; i < n_kt + 2; i += blockDim.x) hist[i] = 0;
   __syncthreads();
-  for (int t = threadIdx.x; t < n_qt; t += blockDim.x) atomicAdd(&hist[rm[t].y - rm[t].x], 1);
+  for (int t = threadIdx.x; t < n; t += blockDim.x) atomicAdd(&hist[count(t)], 1);
   __syncthreads();
   if (threadIdx.x == 0) {
     int running = 0;
-    for (int n = n_kt; n >= 0; --n) {  // exclusive offsets, largest count first
-      const int c = hist[n];
-      hist[n] = running;
-      running += c;
+    for (int c = n_kt; c >= 0; --c) {  // exclusive offsets, largest count first
+      const int k = hist[c];
+      hist[c] = running;
+      running += k;
     }
-    for (int t = n_qt - 1; t >= 0; --t) ord[hist[rm[t].y - rm[t].x]++] = t;
+    for (int t = n - 1; t >= 0; --t) ord[hist[count(t)]++] = t;
   }
   __syncthreads();
+}
+// The q tiles of one map row by their number of kv tiles (y = 0), and the pairs of adjacent q tiles by the mean of theirs (y = 1).
+__global__ void order_kernel(const int4* __restrict__ row_map, int32_t* __restrict__ order, int4* __restrict__ order_rm,
+                             int32_t* __restrict__ order_pair, int n_qt, int n_kt) {
+  extern __shared__ int hist[];
+  const int n_pairs = (n_qt + 1) / 2;
+  const int4* rm = row_map + (size_t)blockIdx.x * n_qt;
+  int32_t* ord = order + (size_t)blockIdx.x * n_qt;
+  int4* ord_rm = order_rm + (size_t)blockIdx.x * n_qt;
+  auto tiles = [&](int t) { return rm[t].y - rm[t].x; };
+  if (blockIdx.y == 1) {
+    sort_by_count([&](int p) { return (tiles(2 * p) + (2 * p + 1 < n_qt ? tiles(2 * p + 1) : 0) + 1) / 2; },
+                  order_pair + (size_t)blockIdx.x * n_pairs, n_pairs, n_kt, hist);
+    return;
+  }
+  sort_by_count(tiles, ord, n_qt, n_kt, hist);
   for (int i = threadIdx.x; i < n_qt; i += blockDim.x) ord_rm[i] = rm[ord[i]];
 }
 
@@ -250,9 +262,10 @@ cudaError_t launch_mask_map(cudaStream_t st, const FlexAttnParams& p) {
       hdr, reinterpret_cast<MapHeader*>(ws), reinterpret_cast<int4*>(ws + L.off_row), reinterpret_cast<int4*>(ws + L.off_col), docmm, L.n_t);
   const size_t hist_bytes = sizeof(int) * (size_t)(L.n_kt + 2);
   if (hist_bytes > 48 * 1024) return cudaErrorInvalidValue;  // more than 12 286 kv tiles (1.5 M keys)
-  order_kernel<<<L.rows, 256, hist_bytes, st>>>(reinterpret_cast<const int4*>(ws + L.off_row),
+  order_kernel<<<dim3(L.rows, 2), 256, hist_bytes, st>>>(reinterpret_cast<const int4*>(ws + L.off_row),
                                                  reinterpret_cast<int32_t*>(ws + L.off_order),
-                                                 reinterpret_cast<int4*>(ws + L.off_order_rm), L.n_qt, L.n_kt);
+                                                 reinterpret_cast<int4*>(ws + L.off_order_rm),
+                                                 reinterpret_cast<int32_t*>(ws + L.off_order_pair), L.n_qt, L.n_kt);
   return cudaGetLastError();
 }
 

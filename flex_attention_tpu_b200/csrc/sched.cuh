@@ -73,6 +73,43 @@ struct ItemCursor {
   }
 };
 
+// The same list of pairs of adjacent q tiles, for the two-query-tile forward kernel, which takes them one by one.
+struct PairItem {
+  int4 rm0, rm1;  // mask-map rows of q tiles 2 pair and 2 pair + 1 (which may not exist: no kv tiles)
+  int bh, pair;   // bh < 0: no more
+};
+struct PairList {
+  const DevParams& P;
+  int per_row, group, full_groups, n_pairs;
+  __device__ __forceinline__ explicit PairList(const DevParams& p) : P(p) {
+    n_pairs = (p.n_qt + 1) / 2;
+    per_row = p.heads * n_pairs;
+    const long long slice_bytes = 4ll * p.seq_k * p.head_dim;
+    // groups of equal size, or nearly: the heaviest pairs of a small last one would come last ([1,16,8192,128] causal 268 -> 224 us)
+    const int most = (int)max(1ll, min((long long)p.heads, (48ll << 20) / slice_bytes)), groups = (p.heads + most - 1) / most;
+    group = (p.heads + groups - 1) / groups;
+    full_groups = p.heads / group;
+  }
+  __device__ __forceinline__ PairItem fetch(int item) const {
+    PairItem o;
+    const int b = item / per_row, r = item - b * per_row;
+    int gi = r / (group * n_pairs), width = group;
+    if (gi >= full_groups) {
+      gi = full_groups;
+      width = P.heads - full_groups * group;
+    }
+    const int r2 = r - gi * group * n_pairs;
+    const int rank = r2 / width;
+    o.bh = b * P.heads + gi * group + (r2 - rank * width);
+    const int row = P.map_rows > 1 ? b : 0;
+    o.pair = __ldg(&P.order_pair[(size_t)row * n_pairs + rank]);
+    const int4* rm = P.row_map + (size_t)row * P.n_qt + 2 * o.pair;
+    o.rm0 = __ldg(rm);
+    o.rm1 = 2 * o.pair + 1 < P.n_qt ? __ldg(rm + 1) : make_int4(0, 0, 0, 0);
+    return o;
+  }
+};
+
 #ifndef FLEXATTN_JIT
 // Number of SMs of the current device (queried once per device); -1 on error.
 inline int sm_count() {

@@ -59,6 +59,15 @@ __device__ __forceinline__ uint32_t globaltimer_lo() {
   asm volatile("mov.u32 %0, %globaltimer_lo;" : "=r"(t));
   return t;
 }
+__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {  // does not wait
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred P;\n\tmbarrier.test_wait.parity.shared::cta.b64 P, [%1], %2;\n\tselp.u32 %0, 1, 0, P;\n\t}\n"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 // Waits for the phase with the given parity to complete.  false = gave up (time limit).  Kept short: a kernel holds some sixty
 // copies of it, and its roles run different code side by side out of one instruction cache.  (32 bits of the clock: 4.3 s.)
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
@@ -137,6 +146,28 @@ __device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.b
 // generic-proxy writes to shared memory -> visible to the async proxy (TMA store, tcgen05.mma operands)
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
+// ------------------------------------------------------------------ work distribution
+// Takes over a CTA of this grid that has not been launched yet: 16 bytes that arrive on `bar`.  After a refusal no other may be
+// asked for.
+__device__ __forceinline__ void cancel_cta(void* smem_dst, uint64_t* bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(
+                   smem_u32(smem_dst)),
+               "r"(smem_u32(bar))
+               : "memory");
+}
+// its blockIdx.x, or -1: there is none
+__device__ __forceinline__ int cancelled_cta(const void* smem_src) {
+  int x;
+  asm volatile(
+      "{\n\t.reg .b128 h;\n\t.reg .pred p;\n\tld.shared.b128 h, [%1];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\tmov.s32 %0, -1;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, h;\n\t}\n"
+      : "=r"(x)
+      : "r"(smem_u32(smem_src))
+      : "memory");
+  return x;
 }
 
 // ------------------------------------------------------------------ tensor memory
@@ -445,6 +476,17 @@ __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
+// ... and all of them learn whether `ok` held for every one
+__device__ __forceinline__ bool named_bar_all(int id, int nthreads, bool ok) {
+  uint32_t all;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %3, 0;\n\tbar.red.and.pred q, %1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}\n"
+      : "=r"(all)
+      : "r"(id), "r"(nthreads), "r"((uint32_t)ok)
+      : "memory");
+  return all != 0;
+}
+
 }  // namespace ptx
 
 // Per-device abort word (device address): set when any bounded wait gives up, checked by every tensor-core CTA
@@ -478,9 +520,9 @@ struct SmemAttrOnce {
 };
 int ensure_dynamic_smem(const void* kernel, int bytes, SmemAttrOnce* once);
 
-// Host side: 3-D tensor map over a [slices, rows, cols] bf16 array, box = {64 cols, box_rows rows, 1 slice},
-// 128-byte swizzle, out-of-range rows read as zero.
-int make_tile_map(CUtensorMap* out, const void* base, int slices, int rows, int cols, int box_rows = kTile);
+// Host side: 3-D tensor map over a [slices, rows, cols] bf16 array, box = {box_cols (64 or 32) cols, box_rows rows, 1 slice},
+// 128-byte swizzle (32 columns: 64-byte), out-of-range rows read as zero.
+int make_tile_map(CUtensorMap* out, const void* base, int slices, int rows, int cols, int box_rows = kTile, int box_cols = 64);
 // ... over every step-th row of such an array (rows 0, step, 2 step ... of each slice)
 int make_strided_map(CUtensorMap* out, const void* base, int slices, int rows, int cols, int step);
 #endif  // !FLEXATTN_JIT

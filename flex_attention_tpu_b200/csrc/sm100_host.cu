@@ -52,23 +52,23 @@ static EncodeFn encode_fn() {
   return fn;
 }
 
-static int make_map(CUtensorMap* out, const void* base, int slices, int rows, int cols, int box_rows, int step) {
+static int make_map(CUtensorMap* out, const void* base, int slices, int rows, int cols, int box_rows, int box_cols, int step) {
   EncodeFn fn = encode_fn();
   if (fn == nullptr) return FLEXATTN_ERR_CUDA;
   const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)((rows - 1) / step + 1), (cuuint64_t)slices};
   const cuuint64_t strides[2] = {(cuuint64_t)cols * 2 * (cuuint64_t)step, (cuuint64_t)cols * 2 * (cuuint64_t)rows};  // bytes, dims 1..2
-  const cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 1};
+  const cuuint32_t box[3] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows, 1};
   const cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, box_cols == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? FLEXATTN_OK : FLEXATTN_ERR_CUDA;
 }
-int make_tile_map(CUtensorMap* out, const void* base, int slices, int rows, int cols, int box_rows) {
-  return make_map(out, base, slices, rows, cols, box_rows, 1);
+int make_tile_map(CUtensorMap* out, const void* base, int slices, int rows, int cols, int box_rows, int box_cols) {
+  return make_map(out, base, slices, rows, cols, box_rows, box_cols, 1);
 }
 int make_strided_map(CUtensorMap* out, const void* base, int slices, int rows, int cols, int step) {
-  return make_map(out, base, slices, rows, cols, kTile, step);
+  return make_map(out, base, slices, rows, cols, kTile, 64, step);
 }
 
 }  // namespace flexattn
