@@ -5,15 +5,18 @@
 // kernels.  Tile skipping follows the same mask map as the tensor-core kernels.
 //
 // A CTA owns a tile of rows (queries in fwd/dq, keys in dkv) and walks the opposite side 64 positions at a time; both
-// sides sit in shared memory as f32 and every contraction is register-blocked: thread (ty, tx) of 16 x 16 computes RM rows
+// sides sit in shared memory as f32 and every contraction is register-blocked: thread (ty, tx) of NT / 16 x 16 computes RM rows
 // x 4 columns of the scores and RM rows x D / 16 columns of the outputs.  What bounds it is shared memory (RM = 4: 8
 // 16-byte reads per 64 FMAs, 53 % of the data pipe and 43 % of the FMA pipe busy at [16,16,256,64]); one warp per row with
 // the rows read from global memory, as before, was bound by those uncoalesced reads (1.3 TFLOP/s at every size).
 //   * enough 64-row tiles for every SM: RM = 4, one group of 256 threads per CTA.  [4,16,512,128] causal softcap forward +
 //     dq + dkv 849 us, 17.8 TFLOP/s.
-//   * fewer: RM = 1 (16-row tiles, four times the CTAs), and several groups of 256 threads per CTA that take every G-th
-//     step and add up their partial results at the end, because the chain of steps is what such a launch waits for.
-//     [1,4,512,64] causal forward / dq / dkv 134 / 194 / 215 us -> 28 / 38 / 49 (RM = 4 there: 65 / 93 / 122).
+//   * fewer: 16-row tiles (four times the CTAs), and several groups of threads per CTA that take every G-th step and add up
+//     their partial results at the end, because the chain of steps is what such a launch waits for.  A group is 128 threads of
+//     two rows each: with 256 of one row the reads of the opposite side (9 accesses of the data pipe per 16 FMAs, now 10 per 32)
+//     took the time, with 64 of four rows a step is too long a chain where there are few.  Forward, dq and dkv of a pass, us,
+//     256 / 128 / 64 threads: [1,4,512,64] causal 78 / 58 / 65, [3,8,208,128] 271 / 195 / 215, [1,2,2048,128] causal 736 / 517 / 550,
+//     [9,12,64,128] 105 / 93 / 136, [1,4,128,32] causal 20.8 / 20.8 / 29.
 #include "sched.cuh"
 #include "sm100.cuh"
 
@@ -23,11 +26,11 @@ namespace {
 __device__ __forceinline__ void from_f(float* p, float x) { *p = x; }
 __device__ __forceinline__ void from_f(__nv_bfloat16* p, float x) { *p = __float2bfloat16_rn(x); }
 
-constexpr int kThreadsS = 256;  // 16 x 16: thread (ty, tx) owns RM adjacent rows and every 16th of 64 columns
 constexpr int kCols = 64;       // opposite-side positions per step
 
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void group_sync(int group) { asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(kThreadsS) : "memory"); }
+template <int NT>
+__device__ __forceinline__ void group_sync(int group) { asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(NT) : "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
@@ -156,11 +159,14 @@ __device__ __forceinline__ float dsig_rt(int kind, float s, float inv_cap) {
   return kind == FLEXATTN_SCORE_SOFTCAP ? score_dsig<FLEXATTN_SCORE_SOFTCAP>(s, inv_cap) : 1.0f;
 }
 
-// Shared memory of a CTA: `row_tiles` tiles [16 RM][D + 4] of its own rows, and per group two tiles [64][D + 4] of the
-// opposite side and one of weights [16 RM][68].
-template <int D, int RM, int G>
+// Rows of a tile.
+template <int RM, int NT>
+constexpr int kRowsOf = NT / 16 * RM;
+// Shared memory of a CTA: `row_tiles` tiles [rows][D + 4] of its own rows, and per group two tiles [64][D + 4] of the
+// opposite side and one of weights [rows][68].
+template <int D, int RM, int G, int NT>
 constexpr size_t simt_smem(int row_tiles) {
-  return sizeof(float) * ((size_t)row_tiles * 16 * RM * (D + 4) + (size_t)G * (2 * kCols * (D + 4) + 16 * RM * (kCols + 4)));
+  return sizeof(float) * ((size_t)row_tiles * kRowsOf<RM, NT> * (D + 4) + (size_t)G * (2 * kCols * (D + 4) + kRowsOf<RM, NT> * (kCols + 4)));
 }
 
 // Which (slice, tile) a CTA works on: the last tiles of every slice first (under a causal mask they are the longest).
@@ -198,15 +204,15 @@ __device__ __forceinline__ void key_range(const DevParams& P, const int4& rm, in
 
 // Adds the accumulators of all groups into group 0's (true there); `work`: the group's own two tiles, no longer read.
 // Called by every thread of the CTA.
-template <int D, int RM, int G>
+template <int D, int RM, int G, int NT>
 __device__ __forceinline__ bool sum_groups(float (&acc)[RM][D / 16], float* work, int group, int tid) {
-  constexpr int kStride = 2 * kCols * (D + 4) + 16 * RM * (kCols + 4);
-  static_assert(RM * (D / 16) * kThreadsS <= 2 * kCols * (D + 4), "a group's partial results fit its two tiles");
+  constexpr int kStride = 2 * kCols * (D + 4) + kRowsOf<RM, NT> * (kCols + 4);
+  static_assert(RM * (D / 16) * NT <= 2 * kCols * (D + 4), "a group's partial results fit its two tiles");
   __syncthreads();  // earlier readers of `work` are done
 #pragma unroll
   for (int r = 0; r < RM; ++r)
 #pragma unroll
-    for (int n = 0; n < D / 16; ++n) work[(r * (D / 16) + n) * kThreadsS + tid] = acc[r][n];
+    for (int n = 0; n < D / 16; ++n) work[(r * (D / 16) + n) * NT + tid] = acc[r][n];
   __syncthreads();
   if (group > 0) return false;
 #pragma unroll
@@ -214,15 +220,15 @@ __device__ __forceinline__ bool sum_groups(float (&acc)[RM][D / 16], float* work
 #pragma unroll
     for (int r = 0; r < RM; ++r)
 #pragma unroll
-      for (int n = 0; n < D / 16; ++n) acc[r][n] += work[g * kStride + (r * (D / 16) + n) * kThreadsS + tid];
+      for (int n = 0; n < D / 16; ++n) acc[r][n] += work[g * kStride + (r * (D / 16) + n) * NT + tid];
   return true;
 }
 
-template <typename T, int D, int RM, int G>
-__global__ void __launch_bounds__(kThreadsS * G, G == 1 && D <= 64 ? 2 : 1) simt_fwd_kernel(DevParams P, int score, int mask, int n_tiles) {
-  constexpr int BM = 16 * RM, LD = D + 4, LP = kCols + 4;
+template <typename T, int D, int RM, int G, int NT>
+__global__ void __launch_bounds__(NT * G, G == 1 && D <= 64 ? 2 : 1) simt_fwd_kernel(DevParams P, int score, int mask, int n_tiles) {
+  constexpr int BM = kRowsOf<RM, NT>, LD = D + 4, LP = kCols + 4;
   extern __shared__ float4 smem_f4[];
-  const int group = G > 1 ? (int)threadIdx.x / kThreadsS : 0, tid = (int)threadIdx.x - group * kThreadsS;
+  const int group = G > 1 ? (int)threadIdx.x / NT : 0, tid = (int)threadIdx.x - group * NT;
   const int ty = tid >> 4, tx = tid & 15;
   float* sQ = reinterpret_cast<float*>(smem_f4);
   float* sK = sQ + BM * LD + group * (2 * kCols * LD + BM * LP);
@@ -251,10 +257,10 @@ __global__ void __launch_bounds__(kThreadsS * G, G == 1 && D <= 64 ? 2 : 1) simt
     for (int n = 0; n < D / 16; ++n) acc[r][n] = 0.f;
   }
   kbeg += group * kCols;  // the groups take every G-th step
-  load_rows<D>(sQ, q, i0, BM, P.seq_q, threadIdx.x, kThreadsS * G);
-  if (kbeg < kend) load_rows<D>(sK, k, kbeg, kCols, kend, tid, kThreadsS);
+  load_rows<D>(sQ, q, i0, BM, P.seq_q, threadIdx.x, NT * G);
+  if (kbeg < kend) load_rows<D>(sK, k, kbeg, kCols, kend, tid, NT);
   cp_commit();
-  if (kbeg < kend) load_rows<D>(sV, v, kbeg, kCols, kend, tid, kThreadsS);
+  if (kbeg < kend) load_rows<D>(sV, v, kbeg, kCols, kend, tid, NT);
   cp_commit();
   if constexpr (G > 1) {
     cp_wait<1>();
@@ -263,11 +269,11 @@ __global__ void __launch_bounds__(kThreadsS * G, G == 1 && D <= 64 ? 2 : 1) simt
   for (int j0 = kbeg; j0 < kend; j0 += G * kCols) {
     const bool full = j0 >= rm.z * kTile && j0 + kCols <= rm.w * kTile;  // every pair of the tile is kept
     cp_wait<1>();
-    group_sync(group);  // Q and K of this step have landed
+    group_sync<NT>(group);  // Q and K of this step have landed
     float s[RM][4];
     mm_abt<D, RM>(s, sQ, sK, ty, tx);
-    group_sync(group);  // K has been read: the next one is loaded during the softmax and P V
-    if (j0 + G * kCols < kend) load_rows<D>(sK, k, j0 + G * kCols, kCols, kend, tid, kThreadsS);
+    group_sync<NT>(group);  // K has been read: the next one is loaded during the softmax and P V
+    if (j0 + G * kCols < kend) load_rows<D>(sK, k, j0 + G * kCols, kCols, kend, tid, NT);
     cp_commit();
 #pragma unroll
     for (int r = 0; r < RM; ++r) {
@@ -301,37 +307,37 @@ __global__ void __launch_bounds__(kThreadsS * G, G == 1 && D <= 64 ? 2 : 1) simt
       for (int n = 0; n < D / 16; ++n) acc[r][n] *= alpha;
     }
     cp_wait<1>();
-    group_sync(group);  // P is in place, V has landed
+    group_sync<NT>(group);  // P is in place, V has landed
     mm_pb<D, RM>(acc, sP, sV, ty, tx);
-    group_sync(group);  // V and P have been read
-    if (j0 + G * kCols < kend) load_rows<D>(sV, v, j0 + G * kCols, kCols, kend, tid, kThreadsS);
+    group_sync<NT>(group);  // V and P have been read
+    if (j0 + G * kCols < kend) load_rows<D>(sV, v, j0 + G * kCols, kCols, kend, tid, NT);
     cp_commit();
   }
   cp_wait<0>();
   if constexpr (G > 1) {
     // merge the groups' partial softmaxes: each leaves (m, l, acc) of its threads in its own K / V tiles
     constexpr int kVals = RM * (2 + D / 16);
-    static_assert(kVals * kThreadsS <= 2 * kCols * LD, "a group's partial results fit its K and V tiles");
+    static_assert(kVals * NT <= 2 * kCols * LD, "a group's partial results fit its K and V tiles");
 #pragma unroll
     for (int r = 0; r < RM; ++r) {
-      float* w = sK + r * (2 + D / 16) * kThreadsS + tid;
+      float* w = sK + r * (2 + D / 16) * NT + tid;
       w[0] = m[r];
-      w[kThreadsS] = l[r];
+      w[NT] = l[r];
 #pragma unroll
-      for (int n = 0; n < D / 16; ++n) w[(2 + n) * kThreadsS] = acc[r][n];
+      for (int n = 0; n < D / 16; ++n) w[(2 + n) * NT] = acc[r][n];
     }
     __syncthreads();
     if (group > 0) return;
     for (int g = 1; g < G; ++g) {
       const float* w = sK + g * (2 * kCols * LD + BM * LP) + tid;
 #pragma unroll
-      for (int r = 0; r < RM; ++r, w += (2 + D / 16) * kThreadsS) {
+      for (int r = 0; r < RM; ++r, w += (2 + D / 16) * NT) {
         const float m_new = fmaxf(m[r], w[0]);
         const float a = __expf(m[r] - m_new), b = __expf(w[0] - m_new);
-        l[r] = l[r] * a + w[kThreadsS] * b;
+        l[r] = l[r] * a + w[NT] * b;
         m[r] = m_new;
 #pragma unroll
-        for (int n = 0; n < D / 16; ++n) acc[r][n] = acc[r][n] * a + w[(2 + n) * kThreadsS] * b;
+        for (int n = 0; n < D / 16; ++n) acc[r][n] = acc[r][n] * a + w[(2 + n) * NT] * b;
       }
     }
   }
@@ -345,11 +351,11 @@ __global__ void __launch_bounds__(kThreadsS * G, G == 1 && D <= 64 ? 2 : 1) simt
   }
 }
 
-template <typename T, int D, int RM, int G>
-__global__ void __launch_bounds__(kThreadsS * G, G == 1 && D <= 64 ? 2 : 1) simt_dq_kernel(DevParams P, int score, int mask, int n_tiles) {
-  constexpr int BM = 16 * RM, LD = D + 4, LP = kCols + 4;
+template <typename T, int D, int RM, int G, int NT>
+__global__ void __launch_bounds__(NT * G, G == 1 && D <= 64 ? 2 : 1) simt_dq_kernel(DevParams P, int score, int mask, int n_tiles) {
+  constexpr int BM = kRowsOf<RM, NT>, LD = D + 4, LP = kCols + 4;
   extern __shared__ float4 smem_f4[];
-  const int group = G > 1 ? (int)threadIdx.x / kThreadsS : 0, tid = (int)threadIdx.x - group * kThreadsS;
+  const int group = G > 1 ? (int)threadIdx.x / NT : 0, tid = (int)threadIdx.x - group * NT;
   const int ty = tid >> 4, tx = tid & 15;
   float* sQ = reinterpret_cast<float*>(smem_f4);
   float* sDO = sQ + BM * LD;
@@ -371,11 +377,11 @@ __global__ void __launch_bounds__(kThreadsS * G, G == 1 && D <= 64 ? 2 : 1) simt
   float m[RM], inv_l[RM], delta[RM], acc[RM][D / 16];
   int di[RM];
   const int kfirst = kbeg + group * kCols;  // the groups take every G-th step
-  load_rows<D>(sQ, q, i0, BM, P.seq_q, threadIdx.x, kThreadsS * G);
-  load_rows<D>(sDO, dO, i0, BM, P.seq_q, threadIdx.x, kThreadsS * G);
+  load_rows<D>(sQ, q, i0, BM, P.seq_q, threadIdx.x, NT * G);
+  load_rows<D>(sDO, dO, i0, BM, P.seq_q, threadIdx.x, NT * G);
   if (kfirst < kend) {
-    load_rows<D>(sK, k, kfirst, kCols, kend, tid, kThreadsS);
-    load_rows<D>(sV, v, kfirst, kCols, kend, tid, kThreadsS);
+    load_rows<D>(sK, k, kfirst, kCols, kend, tid, NT);
+    load_rows<D>(sV, v, kfirst, kCols, kend, tid, NT);
   }
   cp_commit();
 #pragma unroll
@@ -403,12 +409,12 @@ __global__ void __launch_bounds__(kThreadsS * G, G == 1 && D <= 64 ? 2 : 1) simt
   for (int j0 = kfirst; j0 < kend; j0 += G * kCols) {
     const bool full = j0 >= rm.z * kTile && j0 + kCols <= rm.w * kTile;
     cp_wait<0>();
-    group_sync(group);
+    group_sync<NT>(group);
     float s[RM][4], dp[RM][4];
     mm_abt<D, RM>(s, sQ, sK, ty, tx);
     mm_abt<D, RM>(dp, sDO, sV, ty, tx);
-    group_sync(group);  // V has been read (K is needed once more)
-    if (j0 + G * kCols < kend) load_rows<D>(sV, v, j0 + G * kCols, kCols, kend, tid, kThreadsS);
+    group_sync<NT>(group);  // V has been read (K is needed once more)
+    if (j0 + G * kCols < kend) load_rows<D>(sV, v, j0 + G * kCols, kCols, kend, tid, NT);
 #pragma unroll
     for (int r = 0; r < RM; ++r) {
       const int i = i0 + ty * RM + r;
@@ -427,15 +433,15 @@ __global__ void __launch_bounds__(kThreadsS * G, G == 1 && D <= 64 ? 2 : 1) simt
         sP[(ty * RM + r) * LP + tx + 16 * c] = ds;
       }
     }
-    group_sync(group);
+    group_sync<NT>(group);
     mm_pb<D, RM>(acc, sP, sK, ty, tx);
-    group_sync(group);
-    if (j0 + G * kCols < kend) load_rows<D>(sK, k, j0 + G * kCols, kCols, kend, tid, kThreadsS);
+    group_sync<NT>(group);
+    if (j0 + G * kCols < kend) load_rows<D>(sK, k, j0 + G * kCols, kCols, kend, tid, NT);
     cp_commit();
   }
   cp_wait<0>();
   if constexpr (G > 1) {
-    if (!sum_groups<D, RM, G>(acc, sK, group, tid)) return;
+    if (!sum_groups<D, RM, G, NT>(acc, sK, group, tid)) return;
   }
 #pragma unroll
   for (int r = 0; r < RM; ++r) {
@@ -444,11 +450,11 @@ __global__ void __launch_bounds__(kThreadsS * G, G == 1 && D <= 64 ? 2 : 1) simt
   }
 }
 
-template <typename T, int D, int RM, int G>
-__global__ void __launch_bounds__(kThreadsS * G, G == 1 && D <= 64 ? 2 : 1) simt_dkv_kernel(DevParams P, int score, int mask, int n_tiles) {
-  constexpr int BM = 16 * RM, LD = D + 4, LP = kCols + 4;
+template <typename T, int D, int RM, int G, int NT>
+__global__ void __launch_bounds__(NT * G, G == 1 && D <= 64 ? 2 : 1) simt_dkv_kernel(DevParams P, int score, int mask, int n_tiles) {
+  constexpr int BM = kRowsOf<RM, NT>, LD = D + 4, LP = kCols + 4;
   extern __shared__ float4 smem_f4[];
-  const int group = G > 1 ? (int)threadIdx.x / kThreadsS : 0, tid = (int)threadIdx.x - group * kThreadsS;
+  const int group = G > 1 ? (int)threadIdx.x / NT : 0, tid = (int)threadIdx.x - group * NT;
   const int ty = tid >> 4, tx = tid & 15;
   float* sK = reinterpret_cast<float*>(smem_f4);
   float* sV = sK + BM * LD;
@@ -482,11 +488,11 @@ __global__ void __launch_bounds__(kThreadsS * G, G == 1 && D <= 64 ? 2 : 1) simt
     for (int n = 0; n < D / 16; ++n) { acc_k[r][n] = 0.f; acc_v[r][n] = 0.f; }
   }
   qbeg += group * kCols;  // the groups take every G-th step
-  load_rows<D>(sK, k, k0, BM, P.seq_k, threadIdx.x, kThreadsS * G);
-  load_rows<D>(sV, v, k0, BM, P.seq_k, threadIdx.x, kThreadsS * G);
+  load_rows<D>(sK, k, k0, BM, P.seq_k, threadIdx.x, NT * G);
+  load_rows<D>(sV, v, k0, BM, P.seq_k, threadIdx.x, NT * G);
   if (qbeg < qend) {
-    load_rows<D>(sQ, q, qbeg, kCols, qend, tid, kThreadsS);
-    load_rows<D>(sDO, dO, qbeg, kCols, qend, tid, kThreadsS);
+    load_rows<D>(sQ, q, qbeg, kCols, qend, tid, NT);
+    load_rows<D>(sDO, dO, qbeg, kCols, qend, tid, NT);
   }
   cp_commit();
   if constexpr (G > 1) {
@@ -505,7 +511,7 @@ __global__ void __launch_bounds__(kThreadsS * G, G == 1 && D <= 64 ? 2 : 1) simt
       de[c] = i < qend ? drow[i] : 0.f;
     }
     cp_wait<0>();
-    group_sync(group);
+    group_sync<NT>(group);
     float s[RM][4], dp[RM][4];
     mm_abt<D, RM>(s, sK, sQ, ty, tx);
     mm_abt<D, RM>(dp, sV, sDO, ty, tx);
@@ -527,27 +533,27 @@ __global__ void __launch_bounds__(kThreadsS * G, G == 1 && D <= 64 ? 2 : 1) simt
         dp[r][c] = ds;
       }
     }
-    group_sync(group);
+    group_sync<NT>(group);
     mm_pb<D, RM>(acc_v, sP, sDO, ty, tx);
-    group_sync(group);  // dO and P have been read: the next dO is loaded during dS^T Q
-    if (i0 + G * kCols < qend) load_rows<D>(sDO, dO, i0 + G * kCols, kCols, qend, tid, kThreadsS);
+    group_sync<NT>(group);  // dO and P have been read: the next dO is loaded during dS^T Q
+    if (i0 + G * kCols < qend) load_rows<D>(sDO, dO, i0 + G * kCols, kCols, qend, tid, NT);
 #pragma unroll
     for (int r = 0; r < RM; ++r)
 #pragma unroll
       for (int c = 0; c < 4; ++c) sP[(ty * RM + r) * LP + tx + 16 * c] = dp[r][c];
-    group_sync(group);
+    group_sync<NT>(group);
     mm_pb<D, RM>(acc_k, sP, sQ, ty, tx);
-    group_sync(group);
-    if (i0 + G * kCols < qend) load_rows<D>(sQ, q, i0 + G * kCols, kCols, qend, tid, kThreadsS);
+    group_sync<NT>(group);
+    if (i0 + G * kCols < qend) load_rows<D>(sQ, q, i0 + G * kCols, kCols, qend, tid, NT);
     cp_commit();
   }
   cp_wait<0>();
   if constexpr (G > 1) {
-    if (!sum_groups<D, RM, G>(acc_k, sQ, group, tid)) {
-      sum_groups<D, RM, G>(acc_v, sQ, group, tid);
+    if (!sum_groups<D, RM, G, NT>(acc_k, sQ, group, tid)) {
+      sum_groups<D, RM, G, NT>(acc_v, sQ, group, tid);
       return;
     }
-    sum_groups<D, RM, G>(acc_v, sQ, group, tid);
+    sum_groups<D, RM, G, NT>(acc_v, sQ, group, tid);
   }
 #pragma unroll
   for (int r = 0; r < RM; ++r) {
@@ -565,7 +571,7 @@ using SimtKernel = void (*)(DevParams, int, int, int);
 struct SimtChoice {
   SimtKernel kernel;
   size_t smem;
-  int groups;
+  int threads;
   SmemAttrOnce* once;
 };
 cudaError_t simt_launch(cudaStream_t st, const DevParams& d, int score, int mask, int rows, const SimtChoice& big,
@@ -573,15 +579,15 @@ cudaError_t simt_launch(cudaStream_t st, const DevParams& d, int score, int mask
   const long long slices = (long long)d.batch * d.heads;
   const int sms = sm_count();
   if (sms <= 0) return cudaErrorInvalidDevice;
-  // The line: at 128 such tiles [1,8,1024,64] takes 421 us with the small form and 653 with the big one, [2,8,512,128]
-  // 437 and 423; at 512 tiles [4,16,512,128] takes 1655 and 848.
+  // The line, us of forward and backward with the small form and the big one: 128 such tiles [4,8,200,64] causal 87 (the big
+  // one would leave SMs idle), 180 [5,12,153,64] causal 121 and 98, 243 [9,3,555,32] 222 and 181, 256 [2,64,112,64] 177 and 111.
   const bool use_big = (rows + 63) / 64 * slices >= sms;
   const SimtChoice& c = use_big ? big : small;
   const int bm = use_big ? 64 : 16;
   const int n_tiles = (rows + bm - 1) / bm;
   if (n_tiles * slices > 0x7fffffffLL) return cudaErrorInvalidValue;
   if (ensure_dynamic_smem(reinterpret_cast<const void*>(c.kernel), (int)c.smem, c.once) != FLEXATTN_OK) return cudaErrorInvalidValue;
-  c.kernel<<<(unsigned)(n_tiles * slices), kThreadsS * c.groups, c.smem, st>>>(d, score, mask, n_tiles);
+  c.kernel<<<(unsigned)(n_tiles * slices), c.threads, c.smem, st>>>(d, score, mask, n_tiles);
   return cudaGetLastError();
 }
 
@@ -590,8 +596,9 @@ cudaError_t simt_launch(cudaStream_t st, const DevParams& d, int score, int mask
   do {                                                                                                             \
     constexpr int kG = DD == 128 ? 2 : 4;                                                                          \
     static SmemAttrOnce big_once{}, small_once{};                                                                  \
-    return simt_launch(st, d, score, mask, rows, SimtChoice{KERNEL<T, DD, 4, 1>, simt_smem<DD, 4, 1>(ROW_TILES), 1, &big_once}, \
-                       SimtChoice{KERNEL<T, DD, 1, kG>, simt_smem<DD, 1, kG>(ROW_TILES), kG, &small_once});        \
+    return simt_launch(st, d, score, mask, rows,                                                                   \
+                       SimtChoice{KERNEL<T, DD, 4, 1, 256>, simt_smem<DD, 4, 1, 256>(ROW_TILES), 256, &big_once},  \
+                       SimtChoice{KERNEL<T, DD, 2, kG, 128>, simt_smem<DD, 2, kG, 128>(ROW_TILES), 128 * kG, &small_once}); \
   } while (0)
 #define FLEXATTN_SIMT_DISPATCH(KERNEL, ROW_TILES)                                              \
   do {                                                                                                             \
