@@ -1113,8 +1113,12 @@ int launch_score(cudaStream_t st, const DevParams& d, int score, int mask, const
 }
 
 // How a call is cut up.
-// Group: what a slice keeps live, 8 bytes per element of a query row (Q, dO, f32 sum), times the group has 48 MB of the 126 MB
-// of L2.  Under a causal window the live rows are the few around the diagonal.
+// Group: the slices whose kv tiles are in the list side by side.  What a slice keeps live, 8 bytes per element of a query row (Q, dO,
+// f32 sum; under a causal window the few rows around the diagonal), times the group has 80 MB of the 126 MB of L2.  Few slices
+// mean many kv tiles of each in flight, which wait for one another's parts; many of them spill.  us of the backward with 48 MB,
+// as before / 72 / 80 in groups of equal size / 92 / 160: [4,32,8192,128] causal 6244 / 5848 / 5884 / 5928 / 6618,
+// [4,16,2048,128] 466 / 414 / 405 / 404 / 394, [4,16,2048,64] 297 / 243 / 241 / 243 / 236, [1,24,8192,64] 1325 / 1381 / 1327 / 1331 /
+// 1425; 24 MB: 8592, 587, 321, 1604.
 // store_dq: storing dq with the last part saves the finishing kernel and its pass over the sums, but costs the CTA that
 // does it half a tile's time.  That is a gain where many kv tiles share the work (documents: [2,16,16384,128] 1510 -> 1436 us, with
 // softcap 1565 -> 1525, the backward alone replayed from a graph); under a causal mask or none the one kv tile that every query
@@ -1122,16 +1126,18 @@ int launch_score(cudaStream_t st, const DevParams& d, int score, int mask, const
 // 76 and 93 either way.  Windows of D = 64 store it too ([2,16,4096,64] with 128 keys 74 us, 81 with the finishing kernel), and those of
 // D = 128 up to 6000 positions (us stored / finished: 16 heads a row, 3072 with 232 keys 206 / 226, 5756 74 / 75) and where the
 // ring is smaller than all slices; longer ones are finished ([4,32,8192,128] with 256 keys and ALiBi 1077 -> 957, [5,8,15744,128] 853 / 755).
-// Then the scratch is a ring of three groups: the one being finished, the one being started, and one between.  Without it the
+// Then the scratch is a ring: three groups of 48 MB, and no group has more than half of it (one is being finished while the next
+// is started).  Without it the
 // scratch holds every slice of a launch, and there are as many launches as keep it within 1 GiB (one slice, if need be).
 struct FusedPlan {
   int launch, group, ring, store_dq;  // slices of a launch, ...
+  int measure;                        // group of 48 MB: what fused_pays measures the room by, a third of the ring
   int chains;                          // sums per query tile
   size_t off_stats, off_flags, off_s2, bytes;
 };
 // s2_n: keys on the stride grid of an S2 call that is gathered, else 0
 FusedPlan fused_plan(int slices, int seq_q, int n_qt, int n_kt, int head_dim, int mask, int window, int s2_n) {
-  constexpr long long kL2Budget = 48ll << 20, kLimit = 1ll << 30;
+  constexpr long long kL2Budget = 48ll << 20, kGroupBudget = 80ll << 20, kLimit = 1ll << 30;
   const int chains = s2_n > 0 ? 2 : 1;
   const long long acc = (long long)chains * n_qt * kTile * head_dim * 4, s2 = 16ll * s2_n * head_dim;
   const long long most = kLimit / (acc + s2) > 0 ? kLimit / (acc + s2) : 1;
@@ -1147,9 +1153,14 @@ FusedPlan fused_plan(int slices, int seq_q, int n_qt, int n_kt, int head_dim, in
   if (L.store_dq && 3 * group > most) group = most / 3;
   if (group < 1) group = 1;
   if (group > L.launch) group = L.launch;
-  L.group = (int)group;
+  L.measure = (int)group;
   L.ring = L.store_dq && 3 * group < slices ? (int)(3 * group) : L.launch;
   if (windowed && head_dim == 128 && L.ring == L.launch && n_kt >= 48) L.store_dq = 0;
+  long long most_at_once = kGroupBudget / (8ll * (windowed ? window + 2 * kTile : seq_q) * head_dim);
+  if (L.ring < L.launch && most_at_once > L.ring / 2) most_at_once = L.ring / 2;
+  if (most_at_once < 1) most_at_once = 1;
+  const long long groups = (L.launch + most_at_once - 1) / most_at_once;
+  L.group = (int)((L.launch + groups - 1) / groups);
   auto up = [](size_t n) { return (n + 255) & ~(size_t)255; };
   L.off_stats = up((size_t)L.ring * acc);
   L.off_flags = L.off_stats + up((size_t)L.launch * n_qt * 2 * kTile * sizeof(float));
@@ -1172,10 +1183,11 @@ FusedPlan plan_of(const FlexAttnParams& p) {
 
 size_t bwd_fused_scratch_bytes(const FlexAttnParams& p) { return plan_of(p).bytes; }
 
-// A group of `width` slices on `sms` CTAs has sms / width kv tiles of each slice in flight (the groups of a launch taken as equal)
+// A group of `width` slices on `sms` CTAs has sms / width kv tiles of each slice in flight.  (Measured by groups of 48 MB, with which
+// the lines of fused_pays were drawn, all taken as equal.)
 double bwd_fused_slack(const FlexAttnParams& p, int sms) {
   const FusedPlan L = plan_of(p);
-  const double width = (double)L.launch / ((L.launch + L.group - 1) / L.group);
+  const double width = (double)L.launch / ((L.launch + L.measure - 1) / L.measure);
   return (p.seq_q + kTile - 1) / kTile * width / sms;
 }
 
