@@ -70,12 +70,13 @@ __host__ __device__ inline MapLayout map_layout(int batch, int seq_q, int seq_k,
   // interval, so the kernels mask partial tiles from these two numbers instead of comparing ids per element)
   const size_t len = (size_t)(seq_q > seq_k ? seq_q : seq_k);
   const size_t runs = (mask_kind == FLEXATTN_MASK_DOCUMENT) ? sizeof(int32_t) * (size_t)batch * len : 0;
-  // ... and the pairs of adjacent q tiles in such an order (work order of the two-query-tile forward kernel)
-  L.off_order_pair = (L.off_order_rm + sizeof(int4) * (size_t)L.rows * L.n_qt + 15) & ~(size_t)15;
-  L.off_run_lo = (L.off_order_pair + sizeof(int32_t) * (size_t)L.rows * ((L.n_qt + 1) / 2) + 15) & ~(size_t)15;
+  L.off_run_lo = (L.off_order_rm + sizeof(int4) * (size_t)L.rows * L.n_qt + 15) & ~(size_t)15;
   L.off_run_hi = (L.off_run_lo + runs + 15) & ~(size_t)15;
   L.off_sorted = (L.off_run_hi + runs + 15) & ~(size_t)15;
-  L.bytes = (L.off_sorted + (runs ? sizeof(int32_t) * (size_t)batch : 0) + 255) & ~(size_t)255;
+  // the pairs of adjacent q tiles in such an order as well (work order of the two-query-tile forward kernel); behind the rest,
+  // at most a 17th of it (4 bytes a pair, 68 and more a q tile of a document row)
+  L.off_order_pair = (L.off_sorted + (runs ? sizeof(int32_t) * (size_t)batch : 0) + 255) & ~(size_t)255;
+  L.bytes = (L.off_order_pair + sizeof(int32_t) * (size_t)L.rows * ((L.n_qt + 1) / 2) + 255) & ~(size_t)255;
   return L;
 }
 

@@ -18,7 +18,9 @@ namespace flexattn {
 namespace {
 
 constexpr size_t kNoAllocScratchBytes = 1u << 20;  // 1 MiB: mask maps up to e.g. S = 32768 with 32 document rows
-static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
+// ... without the order of the pairs of q tiles that lies behind a map (map_layout)
+constexpr size_t kNoAllocPairBytes = 64u << 10;
+static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes + kNoAllocPairBytes];
 
 // Device address of the array on the current device; nullptr (and *err set) if it cannot be resolved.
 void* scratch_for_current_device(cudaError_t* err) {
@@ -59,12 +61,14 @@ extern "C" int flexattn_fwd_noalloc(void* stream, const FlexAttnParams* p) {
     const int e = flexattn_fwd(stream, &local);
     return e != FLEXATTN_OK ? e : FLEXATTN_ERR_BAD_SHAPE;
   }
-  if (need > kNoAllocScratchBytes) return FLEXATTN_ERR_NOALLOC_LIMIT;
+  if (map_layout(local.batch, local.seq_q, local.seq_k, local.mask_kind).off_order_pair > kNoAllocScratchBytes ||
+      need > kNoAllocScratchBytes + kNoAllocPairBytes)
+    return FLEXATTN_ERR_NOALLOC_LIMIT;
   cudaError_t err = cudaSuccess;
   void* scratch = scratch_for_current_device(&err);
   if (scratch == nullptr) return FLEXATTN_ERR_CUDA;
   local.workspace = scratch;
-  local.workspace_bytes = kNoAllocScratchBytes;
+  local.workspace_bytes = kNoAllocScratchBytes + kNoAllocPairBytes;
   // Every check the forward makes runs BEFORE anything is enqueued: a call that is going to be refused (null or
   // misaligned pointer, unsupported backend) must not have overwritten the shared array on its way out.
   bool tc = false;
