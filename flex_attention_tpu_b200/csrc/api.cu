@@ -283,10 +283,15 @@ int flexattn_fwd(void* stream, const FlexAttnParams* p) {
       if (forced == 3 && d.kv_splits == 0 && pair_can && p->score_kind != FLEXATTN_SCORE_USER &&
           p->mask_kind != FLEXATTN_MASK_DOCUMENT)
         d.kv_splits = 1;
-      if (d.kv_splits > 0) return launch_sm100_fwd_split(st, d, p->score_kind, p->mask_kind);
+      if (d.kv_splits > 0) {
+        const int r = launch_sm100_fwd_split(st, d, p->score_kind, p->mask_kind);
+        if (r != FLEXATTN_ERR_UNSUPPORTED_BACKEND) return r;
+      }
     }
-    if (pair_can && (forced == 1 || (forced == 0 && pair_pays(p))))
-      return launch_sm100_fwd_pair(st, d, p->score_kind, p->mask_kind);
+    if (pair_can && (forced == 1 || (forced == 0 && pair_pays(p)))) {
+      const int r = launch_sm100_fwd_pair(st, d, p->score_kind, p->mask_kind);
+      if (r != FLEXATTN_ERR_UNSUPPORTED_BACKEND && r != FLEXATTN_ERR_JIT_COMPILE) return r;
+    }
     if (d.ab != nullptr) return launch_sm100_fwd_pipe_bias(st, d, p->score_kind, p->mask_kind);
     return launch_sm100_fwd_pipe(st, d, p->score_kind, p->mask_kind);
   }

@@ -908,6 +908,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 }
 
 #ifndef FLEXATTN_JIT
+static_assert(256 * kRegsEw + 128 * kRegsDrain + 128 * kRegsRest <= kThreads * kFusedLaunchRegs, "more registers than the CTA is launched with");
+
 // Before it: delta = rowsum(o * do) to the caller, both row statistics to the padded tiles the loads take, flags and ticket
 // to zero.  Bound by HBM latency: all that a thread reads (16-byte chunks of kUnroll rows of o and do, l and m) is asked for before
 // the first sum.  [16,12,512,64] 9.0 -> 7.1 us, [8,16,2048,128] 37 -> 33; four rows were no faster, and slower where the grid is
@@ -1064,10 +1066,7 @@ template <int D, int SK, int MK, int kStore>
 int launch_form(cudaStream_t st, const DevParams& d, const FusedArgs& f, const Maps& t, unsigned grid, int* af) {
   constexpr size_t smem = smem_bytes(D);
   auto kern = fused_sm100_kernel<D, SK, MK, kStore>;
-  static const bool whole_file = [kern] {  // compiled for fewer registers than its warpgroups hand round, it would wait without end
-    cudaFuncAttributes a;
-    return cudaFuncGetAttributes(&a, reinterpret_cast<const void*>(kern)) == cudaSuccess && a.numRegs >= 128;
-  }();
+  static const bool whole_file = launch_registers(reinterpret_cast<const void*>(kern)) >= kFusedLaunchRegs;
   if (!whole_file) return FLEXATTN_ERR_UNSUPPORTED_BACKEND;
   static SmemAttrOnce attr_once{};  // per kernel instantiation, per device
   if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), (int)smem, &attr_once) != FLEXATTN_OK) return FLEXATTN_ERR_CUDA;

@@ -310,6 +310,17 @@ inline bool s2_gathers(const FlexAttnParams& p) {
 // Host-side validation of a forward call, shared by flexattn_fwd and flexattn_fwd_noalloc (api.cu).
 int validate_fwd_args(const FlexAttnParams* p, bool* tc);
 
+// Registers per thread the kernels that hand them round among their warpgroups have to be launched with
+constexpr int kPairLaunchRegs = 168, kSplitLaunchRegs = 168, kFusedLaunchRegs = 128;
+
+// Bounds-checked build: whether FLEXATTN_HOST_FAULT in the environment names `what`, a fault that the host code is to see as if it
+// had happened (tests): "registers", the kernels that hand registers round were compiled for too few of them.
+#ifdef FLEXATTN_DEBUG
+bool host_fault(const char* what);
+#else
+inline bool host_fault(const char*) { return false; }
+#endif
+
 // ---------------------------------------------------------------------------------------------
 // Launchers implemented by the kernel translation units; each returns a cudaError_t.
 // ---------------------------------------------------------------------------------------------
@@ -320,8 +331,10 @@ cudaError_t launch_simt_dq(cudaStream_t st, const DevParams& d, int dtype, int s
 cudaError_t launch_simt_dkv(cudaStream_t st, const DevParams& d, int dtype, int score, int mask);
 // tensor-core (tcgen05) kernels: bf16, D in {64,128}
 int launch_sm100_fwd_pipe(cudaStream_t st, const DevParams& d, int score, int mask);  // persistent, three score tiles in flight
-int launch_sm100_fwd_pair(cudaStream_t st, const DevParams& d, int score, int mask);  // two query tiles per CTA, one row per thread
-int launch_sm100_fwd_split(cudaStream_t st, const DevParams& d, int score, int mask);  // few query tiles: a cluster each
+// Two query tiles per CTA, one row per thread; few query tiles, a cluster each.  FLEXATTN_ERR_UNSUPPORTED_BACKEND (of the first around a
+// user score function also FLEXATTN_ERR_JIT_COMPILE): this build of it cannot run, nothing was launched, the persistent one serves the call.
+int launch_sm100_fwd_pair(cudaStream_t st, const DevParams& d, int score, int mask);
+int launch_sm100_fwd_split(cudaStream_t st, const DevParams& d, int score, int mask);
 int split_clusters_at_once(int c);  // clusters of c CTAs of that kernel the device holds at a time; 0: unknown
 int launch_sm100_dq(cudaStream_t st, const DevParams& d, int score, int mask);
 int launch_sm100_dkv(cudaStream_t st, const DevParams& d, int score, int mask);

@@ -29,6 +29,7 @@ namespace FLEXATTN_TU_NAMESPACE {
 constexpr int kThreads = 384;
 constexpr int kMmaWarp = 8, kTmaWarp = 9;
 constexpr int kItemRing = 2;
+constexpr int kRegsSoftmax = 208, kRegsRest = 88;
 struct PairSmem {
   uint64_t bar_q[2], bar_qfree[2], bar_k[2], bar_v[2], bar_kfree[2], bar_vfree[2], bar_s[2], bar_p[2], bar_pv[2];
   uint64_t bar_item[kItemRing], bar_itemfree[kItemRing], bar_next;
@@ -99,7 +100,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   // phase (T >> 1) & 1), u = index of a query tile among those of a stream that have keys, c = index of a tile among a
   // stream's own (phases u & 1, c & 1).
   if (warp >= 8) {
-    ptx::setmaxnreg_dec<88>();
+    ptx::setmaxnreg_dec<kRegsRest>();
     if (warp == kTmaWarp) {
       // ---------------------------------------------------------------- TMA producer
       if (ptx::elect_one()) {
@@ -262,7 +263,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
     }
   } else {
-    ptx::setmaxnreg_inc<208>();
+    ptx::setmaxnreg_inc<kRegsSoftmax>();
     // ------------------------------------------------------------------ softmax: warpgroup s = stream s
     const int row = tid & 127;
     const int s = tid >> 7;
@@ -489,6 +490,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 }
 
 #ifndef FLEXATTN_JIT
+static_assert(256 * kRegsSoftmax + 128 * kRegsRest <= kThreads * kPairLaunchRegs, "more registers than the CTA is launched with");
 unsigned pair_grid(const DevParams& d) {  // one CTA per pair; 0: too many
   const long long pairs = (long long)((d.n_qt + 1) / 2) * d.batch * d.heads;
   return pairs > 0x7fffffff ? 0u : (unsigned)pairs;
@@ -501,6 +503,8 @@ int launch_one(cudaStream_t st, const DevParams& d, const CUtensorMap& tq, const
   // 512 TMEM columns per CTA: never let two CTAs share an SM (the second would spin in tcgen05.alloc)
   constexpr size_t smem = need > 120 * 1024 ? need : 120 * 1024;
   auto kern = fwd_pair_sm100_kernel<D, SK, MK>;
+  static const bool whole_file = launch_registers(reinterpret_cast<const void*>(kern)) >= kPairLaunchRegs;
+  if (!whole_file) return FLEXATTN_ERR_UNSUPPORTED_BACKEND;
   static SmemAttrOnce attr_once{};  // per kernel instantiation, per device
   if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), (int)smem, &attr_once) != FLEXATTN_OK) return FLEXATTN_ERR_CUDA;
   const unsigned grid = pair_grid(d);

@@ -25,6 +25,8 @@ namespace FLEXATTN_TU_NAMESPACE {
 constexpr int kThreads = 384;
 constexpr int kMmaWarp = 8, kTmaWarp = 9;
 constexpr int kMaxStages = 6;
+constexpr int kRegsSoftmax = 208, kRegsRest = 88;
+static_assert(256 * kRegsSoftmax + 128 * kRegsRest <= kThreads * kSplitLaunchRegs, "more registers than the CTA is launched with");
 
 struct SplitSmem {
   uint64_t bar_q, bar_k[kMaxStages], bar_v[kMaxStages], bar_kfree[kMaxStages], bar_vfree[kMaxStages], bar_s[2], bar_p[2], bar_pv[2];
@@ -124,7 +126,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int NT = dead ? 0 : hi - lo;
 
   if (warp >= 8) {
-    ptx::setmaxnreg_dec<88>();
+    ptx::setmaxnreg_dec<kRegsRest>();
     if (warp == kTmaWarp) {
       // ---------------------------------------------------------------- TMA producer
       if (ptx::elect_one() && NT > 0) {
@@ -206,7 +208,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     __syncwarp();
   } else {
-    ptx::setmaxnreg_inc<208>();
+    ptx::setmaxnreg_inc<kRegsSoftmax>();
     // ------------------------------------------------------------------ softmax: warpgroup s = stream s
     const int row = tid & 127;
     const int s = tid >> 7;
@@ -426,6 +428,8 @@ int launch_one(cudaStream_t st, const DevParams& d, const CUtensorMap& tq, const
                int* abort_flag) {
   constexpr size_t smem = split_smem(D);
   auto kern = fwd_split_sm100_kernel<D, SK, MK>;
+  static const bool whole_file = launch_registers(reinterpret_cast<const void*>(kern)) >= kSplitLaunchRegs;
+  if (!whole_file) return FLEXATTN_ERR_UNSUPPORTED_BACKEND;
   static SmemAttrOnce attr_once{};  // per kernel instantiation, per device
   if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), (int)smem, &attr_once) != FLEXATTN_OK) return FLEXATTN_ERR_CUDA;
   cudaLaunchAttribute attr{};

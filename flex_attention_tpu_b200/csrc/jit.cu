@@ -127,7 +127,7 @@ struct UserScore {
   std::string score, dscore, log;
   std::map<std::tuple<int, bool, int, int>, Compiled> compiled;   // (which, dense bias, head_dim, mask)
   std::map<std::tuple<int, bool, int, int, int>, Loaded> loaded;  // (which, dense bias, head_dim, mask, device)
-  std::set<std::pair<int, int>> no_fused;  // (head_dim, mask) the fused backward cannot be compiled for: not tried again
+  std::set<std::tuple<int, int, int>> without;  // (which, head_dim, mask) another kernel serves, for this one cannot be compiled: not tried again
   bool alive = true;
 };
 
@@ -140,8 +140,9 @@ UserScore* find(int handle) {
   return u->alive ? u : nullptr;
 }
 
-constexpr int kKernels = 5;  // forward (persistent), dQ, dK/dV, forward for long rows, fused backward
-constexpr int kFusedKernel = 4;
+constexpr int kKernels = 5;  // forward (persistent), dQ, dK/dV, forward (two query tiles), fused backward
+constexpr int kPairKernel = 3, kFusedKernel = 4;
+constexpr int kLaunchRegs[kKernels] = {0, 0, 0, kPairLaunchRegs, kFusedLaunchRegs};  // those that hand registers round: launch_registers
 const char* const kKernelFile[kKernels] = {"fwd_pipe_sm100.cu", "bwd_dq_sm100.cu", "bwd_dkv_sm100.cu", "fwd_pair_sm100.cu",
                                              "bwd_fused_sm100.cu"};
 const char* const kKernelName[kKernels] = {"fwd_pipe_sm100_kernel", "dq_sm100_kernel", "dkv_sm100_kernel", "fwd_pair_sm100_kernel",
@@ -217,8 +218,7 @@ int compile_locked(UserScore* u, int which, bool bias, int head_dim, int mask, c
 }  // namespace
 
 namespace {
-// The kernel, compiled and loaded where it was not yet.  Caller holds g_mu.
-int load_locked(UserScore* u, int which, bool bias, int head_dim, int mask, size_t smem_bytes, CUfunction* fn) {
+int load(UserScore* u, int which, bool bias, int head_dim, int mask, size_t smem_bytes, CUfunction* fn) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return FLEXATTN_ERR_CUDA;
   const Driver& d = driver();
@@ -235,10 +235,9 @@ int load_locked(UserScore* u, int which, bool bias, int head_dim, int mask, size
       L = Loaded{};
       return FLEXATTN_ERR_CUDA;
     }
-    // The fused backward hands the registers it was launched with round among its warpgroups; compiled for fewer it would
-    // wait for them without end.
     int regs = 0;
-    if (which == kFusedKernel && (d.FuncGetAttribute(&regs, CU_FUNC_ATTRIBUTE_NUM_REGS, L.fn) != CUDA_SUCCESS || regs < 128)) {
+    if (kLaunchRegs[which] > 0 && (host_fault("registers") || d.FuncGetAttribute(&regs, CU_FUNC_ATTRIBUTE_NUM_REGS, L.fn) != CUDA_SUCCESS ||
+                                   regs < kLaunchRegs[which])) {
       d.ModuleUnload(L.module);
       L = Loaded{};
       return FLEXATTN_ERR_JIT_COMPILE;
@@ -252,6 +251,14 @@ int load_locked(UserScore* u, int which, bool bias, int head_dim, int mask, size
   *fn = L.fn;
   return FLEXATTN_OK;
 }
+// The kernel, compiled and loaded where it was not yet.  Caller holds g_mu.
+int load_locked(UserScore* u, int which, bool bias, int head_dim, int mask, size_t smem_bytes, CUfunction* fn) {
+  const auto key = std::make_tuple(which, head_dim, mask);
+  if (u->without.count(key)) return FLEXATTN_ERR_JIT_COMPILE;
+  const int e = load(u, which, bias, head_dim, mask, smem_bytes, fn);
+  if (e == FLEXATTN_ERR_JIT_COMPILE && kLaunchRegs[which] > 0) u->without.insert(key);
+  return e;
+}
 }  // namespace
 
 int jit_fused_ready(int handle, int head_dim, int mask, size_t smem_bytes, cudaStream_t st) {
@@ -260,8 +267,6 @@ int jit_fused_ready(int handle, int head_dim, int mask, size_t smem_bytes, cudaS
   std::lock_guard<std::mutex> lock(g_mu);
   UserScore* u = find(handle);
   if (u == nullptr) return FLEXATTN_ERR_UNSUPPORTED_MOD;
-  const auto key = std::make_pair(head_dim, mask);
-  if (u->no_fused.count(key)) return FLEXATTN_ERR_JIT_COMPILE;
   const auto it = u->loaded.find(std::make_tuple(kFusedKernel, false, head_dim, mask, dev));
   if (it == u->loaded.end() || it->second.fn == nullptr) {  // under capture nothing can be loaded; the others may be there
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -269,9 +274,7 @@ int jit_fused_ready(int handle, int head_dim, int mask, size_t smem_bytes, cudaS
     if (cap != cudaStreamCaptureStatusNone) return FLEXATTN_ERR_JIT_COMPILE;
   }
   CUfunction fn = nullptr;
-  const int e = load_locked(u, kFusedKernel, false, head_dim, mask, smem_bytes, &fn);
-  if (e == FLEXATTN_ERR_JIT_COMPILE) u->no_fused.insert(key);
-  return e;
+  return load_locked(u, kFusedKernel, false, head_dim, mask, smem_bytes, &fn);
 }
 
 int jit_launch(int which, bool bias, int handle, int head_dim, int mask, unsigned grid_x, unsigned grid_y, unsigned threads,
@@ -335,9 +338,9 @@ extern "C" int flexattn_user_score_compile(int32_t handle, int which, int32_t he
   // every form a launch may ask for: with a dense bias too (the forward for long rows takes none), and before dK/dV the fused
   // backward, which serves in its place where it compiles
   const Compiled* c = nullptr;
-  if (which == 2 && u->no_fused.count({head_dim, mask_kind}) == 0 &&
+  if (which == 2 && u->without.count({kFusedKernel, head_dim, mask_kind}) == 0 &&
       compile_locked(u, kFusedKernel, false, head_dim, mask_kind, &c) == FLEXATTN_ERR_JIT_COMPILE)
-    u->no_fused.insert({head_dim, mask_kind});
+    u->without.insert({kFusedKernel, head_dim, mask_kind});
   const int e = compile_locked(u, which, false, head_dim, mask_kind, &c);
   return e != FLEXATTN_OK || which == 3 ? e : compile_locked(u, which, true, head_dim, mask_kind, &c);
 }

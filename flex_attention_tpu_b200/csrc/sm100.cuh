@@ -519,6 +519,10 @@ struct SmemAttrOnce {
   unsigned char done[kMaxDevices];
 };
 int ensure_dynamic_smem(const void* kernel, int bytes, SmemAttrOnce* once);
+// Registers a thread of `kernel` is launched with; 0: unknown.  The kernels whose warpgroups hand registers round (setmaxnreg) are
+// launched only where that covers the shares (k...LaunchRegs in common.cuh): compiled for fewer, a warpgroup would wait without end
+// for registers that nobody gives back.
+int launch_registers(const void* kernel);
 
 // Host side: 3-D tensor map over a [slices, rows, cols] bf16 array, box = {box_cols (64 or 32) cols, box_rows rows, 1 slice},
 // 128-byte swizzle (32 columns: 64-byte), out-of-range rows read as zero.

@@ -1,6 +1,8 @@
 // Host helpers of the tensor-core kernels: TMA tensor-map construction (driver entry point resolved
 // through the runtime, so libcuda is not a link-time dependency), the per-device abort word and the per-device
 // record of kernels whose dynamic shared-memory limit has been raised.
+#include <cstdlib>
+#include <cstring>
 #include <mutex>
 
 #include "sm100.cuh"
@@ -35,6 +37,21 @@ int ensure_dynamic_smem(const void* kernel, int bytes, SmemAttrOnce* once) {
   }
   return FLEXATTN_OK;
 }
+
+int launch_registers(const void* kernel) {
+  if (host_fault("registers")) return 0;
+  cudaFuncAttributes a;
+  if (cudaFuncGetAttributes(&a, kernel) == cudaSuccess) return a.numRegs;
+  cudaGetLastError();
+  return 0;
+}
+
+#ifdef FLEXATTN_DEBUG
+bool host_fault(const char* what) {
+  const char* e = getenv("FLEXATTN_HOST_FAULT");
+  return e != nullptr && strstr(e, what) != nullptr;
+}
+#endif
 
 using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                               const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
