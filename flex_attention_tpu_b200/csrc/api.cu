@@ -288,7 +288,11 @@ int flexattn_fwd(void* stream, const FlexAttnParams* p) {
         if (r != FLEXATTN_ERR_UNSUPPORTED_BACKEND) return r;
       }
     }
-    if (pair_can && (forced == 1 || (forced == 0 && pair_pays(p)))) {
+    bool pair = pair_can && (forced == 1 || (forced == 0 && pair_pays(p)));
+    if (pair_can && forced == 0 && p->score_kind == FLEXATTN_SCORE_USER)
+      pair = jit_first_or_loaded(pair ? kJitForwardPair : kJitForward, pair ? kJitForward : kJitForwardPair, p->user_score, p->head_dim,
+                                 p->mask_kind, st) == kJitForwardPair;
+    if (pair) {
       const int r = launch_sm100_fwd_pair(st, d, p->score_kind, p->mask_kind);
       if (r != FLEXATTN_ERR_UNSUPPORTED_BACKEND && r != FLEXATTN_ERR_JIT_COMPILE) return r;
     }

@@ -348,10 +348,14 @@ int launch_sm100_dq_bias(cudaStream_t st, const DevParams& d, int score, int mas
 int launch_sm100_dkv_bias(cudaStream_t st, const DevParams& d, int score, int mask);
 
 // Launch of a kernel compiled at run time around a user score function (jit.cu).  which: 0 forward, 1 dQ, 2 dK/dV, each
-// also in a form for a dense bias, 3 forward for long rows, 4 fused backward;
+// also in a form for a dense bias, 3 forward of two query tiles, 4 fused backward;
 // args: the kernel's parameters as for cuLaunchKernel.  Returns a FlexAttnStatus.
+constexpr int kJitForward = 0, kJitForwardPair = 3;
 int jit_launch(int which, bool bias, int handle, int head_dim, int mask, unsigned grid_x, unsigned grid_y, unsigned threads,
                size_t smem_bytes, cudaStream_t st, void** args);
+// Which of two kernels that can both serve a call around a user score function does: the first, but under capture, where nothing can
+// be loaded, the second if only that one is there.
+int jit_first_or_loaded(int first, int second, int handle, int head_dim, int mask, cudaStream_t st);
 // Compiles and loads the fused backward for a user score function where that is still to do.  FLEXATTN_ERR_JIT_COMPILE: it
 // cannot serve the call (nothing has been launched), the separate kernels may.
 int jit_fused_ready(int handle, int head_dim, int mask, size_t smem_bytes, cudaStream_t st);

@@ -564,7 +564,7 @@ int launch_sm100_fwd_pair(cudaStream_t st, const DevParams& d, int score, int ma
     const unsigned grid = pair_grid(d);
     if (grid == 0) return FLEXATTN_ERR_BAD_SHAPE;
     void* args[] = {&tq, &tk, &tv, &to, const_cast<DevParams*>(&d), &af};
-    return jit_launch(3, false, d.user_score, d.head_dim, mask, grid, 1, kThreads,
+    return jit_launch(kJitForwardPair, false, d.user_score, d.head_dim, mask, grid, 1, kThreads,
                       need > 120 * 1024 ? need : 120 * 1024, st, args);
   }
   if (d.head_dim == 128) return launch_score<128>(st, d, score, mask, tq, tk, tv, to, af);

@@ -698,7 +698,7 @@ int launch_sm100_fwd_pipe(cudaStream_t st, const DevParams& d, int score, int ma
     const int sms = sm_count();
     if (sms <= 0) return FLEXATTN_ERR_CUDA;
     void* args[] = {&tq, &tk, &tv, &to, &tks, &tvs, const_cast<DevParams*>(&d), &af};
-    return jit_launch(0, kDenseBias, d.user_score, d.head_dim, mask, (unsigned)(items < sms ? items : sms), 1, kThreads,
+    return jit_launch(kJitForward, kDenseBias, d.user_score, d.head_dim, mask, (unsigned)(items < sms ? items : sms), 1, kThreads,
                       need > 120 * 1024 ? need : 120 * 1024, st, args);
   }
   if (d.head_dim == 128) return launch_score<128>(st, d, score, mask, tq, tk, tv, to, tks, tvs, af);

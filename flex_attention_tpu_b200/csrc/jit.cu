@@ -141,7 +141,7 @@ UserScore* find(int handle) {
 }
 
 constexpr int kKernels = 5;  // forward (persistent), dQ, dK/dV, forward (two query tiles), fused backward
-constexpr int kPairKernel = 3, kFusedKernel = 4;
+constexpr int kPairKernel = kJitForwardPair, kFusedKernel = 4;
 constexpr int kLaunchRegs[kKernels] = {0, 0, 0, kPairLaunchRegs, kFusedLaunchRegs};  // those that hand registers round: launch_registers
 const char* const kKernelFile[kKernels] = {"fwd_pipe_sm100.cu", "bwd_dq_sm100.cu", "bwd_dkv_sm100.cu", "fwd_pair_sm100.cu",
                                              "bwd_fused_sm100.cu"};
@@ -261,18 +261,35 @@ int load_locked(UserScore* u, int which, bool bias, int head_dim, int mask, size
 }
 }  // namespace
 
+namespace {
+bool loaded_locked(const UserScore* u, int which, int head_dim, int mask, int dev) {
+  const auto it = u->loaded.find(std::make_tuple(which, false, head_dim, mask, dev));
+  return it != u->loaded.end() && it->second.fn != nullptr;
+}
+// false also where it cannot be told: the launch will say
+bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap != cudaStreamCaptureStatusNone;
+}
+}  // namespace
+
+int jit_first_or_loaded(int first, int second, int handle, int head_dim, int mask, cudaStream_t st) {
+  int dev = 0;
+  if (!capturing(st) || cudaGetDevice(&dev) != cudaSuccess) return first;
+  std::lock_guard<std::mutex> lock(g_mu);
+  const UserScore* u = find(handle);
+  if (u == nullptr || loaded_locked(u, first, head_dim, mask, dev)) return first;
+  return loaded_locked(u, second, head_dim, mask, dev) ? second : first;
+}
+
 int jit_fused_ready(int handle, int head_dim, int mask, size_t smem_bytes, cudaStream_t st) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return FLEXATTN_ERR_CUDA;
   std::lock_guard<std::mutex> lock(g_mu);
   UserScore* u = find(handle);
   if (u == nullptr) return FLEXATTN_ERR_UNSUPPORTED_MOD;
-  const auto it = u->loaded.find(std::make_tuple(kFusedKernel, false, head_dim, mask, dev));
-  if (it == u->loaded.end() || it->second.fn == nullptr) {  // under capture nothing can be loaded; the others may be there
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) return FLEXATTN_ERR_CUDA;
-    if (cap != cudaStreamCaptureStatusNone) return FLEXATTN_ERR_JIT_COMPILE;
-  }
+  // under capture nothing can be loaded; the others may be there
+  if (!loaded_locked(u, kFusedKernel, head_dim, mask, dev) && capturing(st)) return FLEXATTN_ERR_JIT_COMPILE;
   CUfunction fn = nullptr;
   return load_locked(u, kFusedKernel, false, head_dim, mask, smem_bytes, &fn);
 }

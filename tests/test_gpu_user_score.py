@@ -145,3 +145,26 @@ def test_a_captured_backward_whose_fused_kernel_is_not_loaded():
     torch.cuda.synchronize()
     assert all(torch.equal(a, b) for a, b in zip(out, want))
     assert not torch.equal(backward()[0], want[0])   # outside: the fused kernel
+
+
+@pytest.mark.parametrize("first,then", [((1, 2, 300), (8, 16, 1024)), ((8, 16, 1024), (1, 2, 300))])
+def test_a_captured_forward_whose_kernel_is_not_loaded(first, then):
+    """Which forward kernel serves a call depends on its size; under capture one that an earlier call of another size has loaded takes
+    the place of one that cannot be loaded then."""
+    import flex_attention_tpu_b200 as fa
+    B, H, S = first
+    sf = fa.util.make_jax_score_fn(lambda s, b, h, qi, ki: (0.5 + 0.125 * B) * s - 0.015 * abs(qi - ki))   # a function of this test's own
+    mf, bf, _, _ = build_mods(fa, "causal", "none")
+
+    def forward(B, H, S):
+        (q, k, v, _), _ = make_qkvdo((B, H, S, 64), (B, H, S, 64), 1600 + S, torch.bfloat16)
+        return lambda: fa._flex_attention_impl(q, k, v, None, None, True, False, 0.125, 1, 128, 128, 128, False, bf, mf, sf)
+    forward(*first)()
+    call = forward(*then)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        out = call()
+    g.replay()
+    torch.cuda.synchronize()
+    for name, got, want in zip(("o", "l", "m"), out, call()):   # outside: the kernel of this size; p rounded to bf16 in both
+        assert float((got.float() - want.float()).norm() / want.float().norm()) < 5e-3, name
