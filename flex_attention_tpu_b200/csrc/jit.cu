@@ -352,12 +352,13 @@ extern "C" int flexattn_user_score_compile(int32_t handle, int which, int32_t he
   std::lock_guard<std::mutex> lock(g_mu);
   UserScore* u = find(handle);
   if (u == nullptr) return FLEXATTN_ERR_UNSUPPORTED_MOD;
-  // every form a launch may ask for: with a dense bias too (the forward for long rows takes none), and before dK/dV the fused
-  // backward, which serves in its place where it compiles
+  // every form a launch may ask for: with a dense bias too (the two-query-tile forward takes none), and before the persistent forward
+  // the two-query-tile one, before dK/dV the fused backward, which serve in their place where they compile
   const Compiled* c = nullptr;
-  if (which == 2 && u->without.count({kFusedKernel, head_dim, mask_kind}) == 0 &&
-      compile_locked(u, kFusedKernel, false, head_dim, mask_kind, &c) == FLEXATTN_ERR_JIT_COMPILE)
-    u->without.insert({kFusedKernel, head_dim, mask_kind});
+  const int also = which == kJitForward ? kPairKernel : which == 2 ? kFusedKernel : -1;
+  if (also >= 0 && u->without.count({also, head_dim, mask_kind}) == 0 &&
+      compile_locked(u, also, false, head_dim, mask_kind, &c) == FLEXATTN_ERR_JIT_COMPILE)
+    u->without.insert({also, head_dim, mask_kind});
   const int e = compile_locked(u, which, false, head_dim, mask_kind, &c);
   return e != FLEXATTN_OK || which == 3 ? e : compile_locked(u, which, true, head_dim, mask_kind, &c);
 }

@@ -242,9 +242,10 @@ int flexattn_user_score_destroy(int32_t handle);
 /* The compiler's log of the most recent failed compilation for `handle` ("" if none).  Valid until the next call
  * that uses the handle.  Never NULL. */
 const char* flexattn_user_score_log(int32_t handle);
-/* Compiles (without loading or launching: needs no GPU) the kernel `which` (0 forward, 1 dQ, 2 dK/dV, 3 forward for long rows) for the
- * handle, head_dim and mask_kind, exactly as the first launch would: the form without and, but for 3, the form with a dense
- * bias; with 2 the fused backward too, whose failure is not one of the call (flexattn_bwd_fused reports it).  Returns FLEXATTN_OK, or FLEXATTN_ERR_JIT_COMPILE / FLEXATTN_ERR_JIT_UNAVAILABLE.  A test and warm-up hook. */
+/* Compiles (without loading or launching: needs no GPU) the kernel `which` (0 forward, 1 dQ, 2 dK/dV, 3 the forward of two query tiles
+ * alone) for the handle, head_dim and mask_kind, exactly as the first launch would: the form without and, but for 3, the form with a
+ * dense bias; with 0 both forwards, whichever the sizes of a call ask for, and with 2 the fused backward too.  A failure of the
+ * two-query-tile forward or of the fused backward beside another kernel is not one of the call: that one serves.  Returns FLEXATTN_OK, or FLEXATTN_ERR_JIT_COMPILE / FLEXATTN_ERR_JIT_UNAVAILABLE.  A test and warm-up hook. */
 int flexattn_user_score_compile(int32_t handle, int which, int32_t head_dim, int32_t mask_kind);
 
 /* Clears the calling device's abort word (stream-ordered memset on `stream`), re-enabling the tensor-core

@@ -114,3 +114,30 @@ def test_the_warm_up_hook_does_without_the_fused_backward():
     if 12 in codes:
         pytest.skip("libnvrtc is not installed here")
     assert codes == [0, 0, 0], log.decode()
+
+
+def two_query_tiles_only():
+    """A score function that only the two-query-tile forward minds: a name of its is taken."""
+    return b"s); }\n#define kRegsSoftmax (\n__device__ __forceinline__ float user_score_unused(float s) { return (s"
+
+
+def test_the_warm_up_hook_compiles_both_forward_kernels():
+    """Which of the two serves a call depends on its sizes: with the forward the hook compiles both, a second call of it or of the
+    other one alone finds them compiled, and a function only the two-query-tile one cannot be compiled around is served by the other."""
+    import time
+    from flex_attention_tpu_b200 import _binding as B
+    h, bad = ctypes.c_int32(0), ctypes.c_int32(0)
+    assert B.lib.flexattn_user_score_create(b"0.5f * s", b"0.5f", ctypes.byref(h)) == 0
+    assert B.lib.flexattn_user_score_create(two_query_tiles_only(), b"1.0f", ctypes.byref(bad)) == 0
+    codes, seconds = [], []
+    for which in (0, 3):
+        t = time.perf_counter()
+        codes.append(B.lib.flexattn_user_score_compile(h.value, which, 64, B.MASK_NONE))
+        seconds.append(time.perf_counter() - t)
+    codes += [B.lib.flexattn_user_score_compile(bad.value, which, 64, B.MASK_NONE) for which in (3, 0)]
+    for handle in (h, bad):
+        B.lib.flexattn_user_score_destroy(handle.value)
+    if 12 in codes:
+        pytest.skip("libnvrtc is not installed here")
+    assert codes == [0, 0, 13, 0]
+    assert seconds[1] < 0.05 * seconds[0], seconds   # microseconds against three compilations of seconds
