@@ -275,8 +275,10 @@ int flexattn_fwd(void* stream, const FlexAttnParams* p) {
     const bool pair_can = p->ab == nullptr;
     const int forced = forced_fwd_kernel();
     if (forced == 0 && s2_gathers(*p)) {  // (few tiles a query tile: the persistent kernel)
-      gather_s2(&d);
-      return launch_sm100_fwd_pipe(st, d, p->score_kind, p->mask_kind);
+      DevParams g = d;
+      gather_s2(&g);
+      const int r = launch_sm100_fwd_pipe(st, g, p->score_kind, p->mask_kind);
+      if (r != FLEXATTN_ERR_UNSUPPORTED_BACKEND) return r;  // (its tensor maps were refused, nothing launched: the dense form)
     }
     if (forced == 0 || forced == 3) {
       d.kv_splits = kv_splits(p);

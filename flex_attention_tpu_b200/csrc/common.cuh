@@ -314,7 +314,8 @@ int validate_fwd_args(const FlexAttnParams* p, bool* tc);
 constexpr int kPairLaunchRegs = 168, kSplitLaunchRegs = 168, kFusedLaunchRegs = 128;
 
 // Bounds-checked build: whether FLEXATTN_HOST_FAULT in the environment names `what`, a fault that the host code is to see as if it
-// had happened (tests): "registers", the kernels that hand registers round were compiled for too few of them.
+// had happened (tests): "registers", the kernels that hand registers round were compiled for too few of them; "strided_map", the encoder
+// refuses the tensor maps of gathered S2.
 #ifdef FLEXATTN_DEBUG
 bool host_fault(const char* what);
 #else

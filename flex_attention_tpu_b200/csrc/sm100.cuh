@@ -527,7 +527,9 @@ int launch_registers(const void* kernel);
 // Host side: 3-D tensor map over a [slices, rows, cols] bf16 array, box = {box_cols (64 or 32) cols, box_rows rows, 1 slice},
 // 128-byte swizzle (32 columns: 64-byte), out-of-range rows read as zero.
 int make_tile_map(CUtensorMap* out, const void* base, int slices, int rows, int cols, int box_rows = kTile, int box_cols = 64);
-// ... over every step-th row of such an array (rows 0, step, 2 step ... of each slice)
+// ... over every step-th row of such an array (rows 0, step, 2 step ... of each slice).  Where `step` does not divide `rows`, a slice's
+// pitch is no multiple of a row's: the encoder takes that (it asks for multiples of 16 bytes below 2^40), but the driver's documents
+// build a pitch up from the one below it.  FLEXATTN_ERR_UNSUPPORTED_BACKEND: it does not; the dense form of the call needs no such map.
 int make_strided_map(CUtensorMap* out, const void* base, int slices, int rows, int cols, int step);
 #endif  // !FLEXATTN_JIT
 

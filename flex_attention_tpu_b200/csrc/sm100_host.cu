@@ -85,7 +85,8 @@ int make_tile_map(CUtensorMap* out, const void* base, int slices, int rows, int 
   return make_map(out, base, slices, rows, cols, box_rows, box_cols, 1);
 }
 int make_strided_map(CUtensorMap* out, const void* base, int slices, int rows, int cols, int step) {
-  return make_map(out, base, slices, rows, cols, kTile, 64, step);
+  if (host_fault("strided_map")) return FLEXATTN_ERR_UNSUPPORTED_BACKEND;
+  return make_map(out, base, slices, rows, cols, kTile, 64, step) == FLEXATTN_OK ? FLEXATTN_OK : FLEXATTN_ERR_UNSUPPORTED_BACKEND;
 }
 
 }  // namespace flexattn

@@ -74,3 +74,16 @@ def test_a_kernel_compiled_for_too_few_registers_is_not_launched(fault, names):
     """Its warpgroups raise their registers out of what the CTA was launched with, and would wait for good: the kernels that hand none
     round serve the call, ahead-of-time compiled and around a user function."""
     _run(fault, REGISTERS.format(**names))
+
+
+STRIDED = """
+    case("s2", "none", 1, 3, 2049, 2049, 64, "{fwd}", "{bwd}", window=257, stride=16)     # 2049 rows: no multiple of the stride
+    case("s2", "softcap", 2, 8, 2048, 2048, 128, "{fwd}", "{bwd16}", window=128, stride=32)
+"""
+
+
+@pytest.mark.parametrize("fault,names", [("", dict(fwd=", 6>", bwd="dq_sm100", bwd16="fused_sm100")),   # mask kind 6: gathered
+                                         ("strided_map", dict(fwd=", 5>", bwd="dq_sm100", bwd16="dq_sm100"))])
+def test_a_refused_strided_tensor_map_leaves_s2_to_the_dense_form(fault, names):
+    """The gathered form fetches the keys on the stride grid through a tensor map of that pitch; every S2 call has a form without."""
+    _run(fault, STRIDED.format(**names))
