@@ -70,14 +70,26 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
 }
 // Waits for the phase with the given parity to complete.  false = gave up (time limit).  Kept short: a kernel holds some sixty
 // copies of it, and its roles run different code side by side out of one instruction cache.  (32 bits of the clock: 4.3 s.)
+// kPolls: polls between two looks at the clock; a kernel that is slower with the short form asks for more than one.
+template <int kPolls = 1>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   if (mbar_try_wait(bar, parity)) return true;
-  const uint32_t t0 = globaltimer_lo();
+  if constexpr (kPolls > 1) {
+    const unsigned long long t0 = globaltimer_ns();
+    for (;;) {
 #pragma unroll 1
-  do {
-    if (mbar_try_wait(bar, parity)) return true;
-  } while (globaltimer_lo() - t0 < (uint32_t)kWaitLimitNs);
-  return false;
+      for (int it = 0; it < kPolls; ++it)
+        if (mbar_try_wait(bar, parity)) return true;
+      if (globaltimer_ns() - t0 > kWaitLimitNs) return false;
+    }
+  } else {
+    const uint32_t t0 = globaltimer_lo();
+#pragma unroll 1
+    do {
+      if (mbar_try_wait(bar, parity)) return true;
+    } while (globaltimer_lo() - t0 < (uint32_t)kWaitLimitNs);
+    return false;
+  }
 }
 
 // Register reallocation between warpgroups (all four warps of a warpgroup execute it): the element-wise warpgroups
