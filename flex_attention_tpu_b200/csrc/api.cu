@@ -187,8 +187,7 @@ int flexattn_build_mask_map(void* stream, const FlexAttnParams* p) {
 }
 
 namespace {
-// kv tiles an average query tile visits, from the mask kind alone (a document mask depends on the data: 0, which
-// keeps the persistent kernel).
+// kv tiles an average query tile visits, from the mask kind alone (a document mask depends on the data: 0, never split)
 int mean_kv_tiles(const FlexAttnParams* p) {
   const int n_kt = (p->seq_k + FLEXATTN_TILE - 1) / FLEXATTN_TILE;
   const int in_window = p->window / FLEXATTN_TILE + 1;
@@ -202,34 +201,6 @@ int mean_kv_tiles(const FlexAttnParams* p) {
   }
 }
 constexpr int kSplitMinTiles = 12;  // kv tiles a query tile sees from which its split over CTAs pays
-// Whether the two-query-tile kernel serves the call.  It takes 0.75 to 0.9 of the persistent kernel's time per tile, but in units
-// of two query tiles, and fewer of them than CTAs leave SMs idle.  Times in us, two-query-tile / persistent, on 148 SMs; slices x
-// queries, no score function.
-//   no mask (rows of equal length: whole waves of either compared; one of pairs takes 1.75 of one of query tiles)
-//       D = 128: 24 x 1024 (0.65 waves of pairs, 1.3 of query tiles) 23 / 27, 32 x 1536 (1.3, 2.6) 58 / 52, 16 x 4096 (1.7, 3.5) 126 / 147
-//   windows   p = waves of pairs: 24 x 777 0.65 15 / 12, 16 x 2048 0.86 20 / 21, 24 x 2048 1.3 31 / 29, 32 x 2048 1.7 33 / 38
-//   causal    D = 64: 16 x 3001 1.3 65 / 63, 32 x 2048 1.7 36 / 42, 64 x 2048 3.5 62 / 76; D = 128: 64 x 777 1.7 30 / 28, 32 x 2048 1.7
-//             43 / 48, 64 x 2048 3.5 76 / 102; but 96 x 1024 2.6 50 / 47 (short rows, the last of a wave stands alone)
-//   documents D = 64: 8 x 3001 0.65 33 / 30, 24 x 1536 0.97 39 / 46; D = 128: 24 x 2048 1.3 48 / 44, 32 x 2048 1.7 48 / 54,
-//             softcap 24 x 1536 0.97 46 / 53
-bool pair_pays(const FlexAttnParams* p) {
-  const int sms = sm_count();
-  if (sms <= 0) return true;
-  const long long n_qt = (p->seq_q + FLEXATTN_TILE - 1) / FLEXATTN_TILE, slices = (long long)p->batch * p->heads;
-  const long long pairs = (n_qt + 1) / 2 * slices, items = n_qt * slices;
-  const double waves = (double)pairs / sms;
-  if (n_qt < 2) return false;  // its second stream would have nothing to do
-  const bool scored = p->score_kind == FLEXATTN_SCORE_SOFTCAP || p->score_kind == FLEXATTN_SCORE_USER;
-  switch (p->mask_kind) {
-    case FLEXATTN_MASK_NONE:
-      return waves >= 2.5 || 1.75 * ((pairs + sms - 1) / sms) < (double)((items + sms - 1) / sms);
-    case FLEXATTN_MASK_SLIDING_WINDOW_CAUSAL: return waves >= 1.7 || (waves >= 0.8 && waves <= 1 && 4 * items >= 5ll * sms);
-    case FLEXATTN_MASK_DOCUMENT: return waves >= 1.7 || ((scored || p->head_dim == 64) && waves >= 0.85 && 2 * items >= 3ll * sms);
-    default:  // causal, S2, a window open ahead: the longest rows make the tail
-      if (p->head_dim == 64) return waves >= 1.7;
-      return 10 * items >= 34ll * sms && (waves >= 3 || waves < 2.2 || n_qt > 8);
-  }
-}
 int forced_fwd_kernel() {  // 0: choose by shape, 1: two-query-tile kernel, 2: persistent kernel, 3: split kernel
   static const int choice = [] {
     const char* e = getenv("FLEXATTN_FWD_KERNEL");
@@ -290,7 +261,7 @@ int flexattn_fwd(void* stream, const FlexAttnParams* p) {
         if (r != FLEXATTN_ERR_UNSUPPORTED_BACKEND) return r;
       }
     }
-    bool pair = pair_can && (forced == 1 || (forced == 0 && pair_pays(p)));
+    bool pair = pair_can && (forced == 1 || (forced == 0 && fwd_pair_pays(*p, sm_count())));
     if (pair_can && forced == 0 && p->score_kind == FLEXATTN_SCORE_USER)
       pair = jit_first_or_loaded(pair ? kJitForwardPair : kJitForward, pair ? kJitForward : kJitForwardPair, p->user_score, p->head_dim,
                                  p->mask_kind, st) == kJitForwardPair;

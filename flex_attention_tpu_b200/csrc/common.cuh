@@ -336,6 +336,7 @@ int launch_sm100_fwd_pipe(cudaStream_t st, const DevParams& d, int score, int ma
 // user score function also FLEXATTN_ERR_JIT_COMPILE): this build of it cannot run, nothing was launched, the persistent one serves the call.
 int launch_sm100_fwd_pair(cudaStream_t st, const DevParams& d, int score, int mask);
 int launch_sm100_fwd_split(cudaStream_t st, const DevParams& d, int score, int mask);
+bool fwd_pair_pays(const FlexAttnParams& p, int sms);  // whether the first of them serves a call rather than the persistent one (fwd_choice.cu)
 int split_clusters_at_once(int c);  // clusters of c CTAs of that kernel the device holds at a time; 0: unknown
 int launch_sm100_dq(cudaStream_t st, const DevParams& d, int score, int mask);
 int launch_sm100_dkv(cudaStream_t st, const DevParams& d, int score, int mask);
