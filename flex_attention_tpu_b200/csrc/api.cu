@@ -5,6 +5,8 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
+
 #include <nvtx3/nvToolsExt.h>
 
 #include "common.cuh"
@@ -228,6 +230,13 @@ int kv_splits(const FlexAttnParams* p) {
   while (c < 8 && tiles >= 8 * c && items <= split_clusters_at_once(2 * c)) c *= 2;
   return c > 1 || p->seq_q <= 32 ? c : 0;
 }
+// Whether S2 that would be gathered goes to the split kernel, in its dense form: where that takes the rows of a few query tiles apart
+// so far that one of its streams has less than a quarter of the longest gathered row.  One slice of 4096, D = 64, us gathered / split: 64 keys
+// and stride 2 25.4 / 20.3, 512 and 3 21.9 / 20.4, 64 and 3 20.1 / 20.3, 512 and 4 19.2 / 20.5; 5000 (two CTAs a query tile) 64 and 2 29.4 / 35.3.
+bool split_beats_gathered_s2(const FlexAttnParams* p) {
+  const int c = kv_splits(p), n = (std::min(p->seq_q, p->seq_k) + FLEXATTN_TILE - 1) / FLEXATTN_TILE;
+  return c > 0 && (double)p->window / FLEXATTN_TILE + 2 + (double)n / p->stride > 4.0 * n / (2 * c);
+}
 }  // namespace
 
 int flexattn_fwd(void* stream, const FlexAttnParams* p) {
@@ -245,7 +254,7 @@ int flexattn_fwd(void* stream, const FlexAttnParams* p) {
     // forces one where it can run (read once per process).
     const bool pair_can = p->ab == nullptr;
     const int forced = forced_fwd_kernel();
-    if (forced == 0 && s2_gathers(*p)) {  // (few tiles a query tile: the persistent kernel)
+    if (forced == 0 && s2_gathers(*p) && !split_beats_gathered_s2(p)) {  // (few tiles a query tile: the persistent kernel)
       DevParams g = d;
       gather_s2(&g);
       const int r = launch_sm100_fwd_pipe(st, g, p->score_kind, p->mask_kind);
@@ -409,8 +418,11 @@ bool fused_pays(const FlexAttnParams* p) {
     return p->head_dim == 64 || p->score_kind != FLEXATTN_SCORE_USER;
   // S2, gathered: the separate kernels walk every tile below the diagonal.  The fused one takes as long as its longest strided tile's
   // row of query tiles, which they match while they fit the chip at once: slices x queries, 128 keys, stride 32: 8 x 3000 (D = 64)
-  // 58 / 79, 16 x 1500 37 / 52, 16 x 2000 (D = 128) 61 / 86, 16 x 8000 255 / 841; 4 x 5000 113 / 97, 8 x 2000 55 / 41, 16 x 1100 39 / 35
-  if (s2_gathers(*p)) return 5 * items >= 6 * sms;
+  // 58 / 79, 16 x 1500 37 / 52, 16 x 2000 (D = 128) 61 / 86, 16 x 8000 255 / 841; 4 x 5000 113 / 97, 8 x 2000 55 / 41, 16 x 1100 39 / 35.
+  // Every other key on the grid makes as many strided tiles as window tiles, and all of them see the last query tiles, one after the
+  // other; long rows of few slices wait alike at D = 128 (64 keys): stride 2 3 x 8192 (D = 64) 194 / 155, 8 x 3200 86 / 85, 4 x 8192 201 / 223;
+  // stride 4 at D = 128 2 x 12000 241 / 226, 3 x 8192 174 / 166, 6 x 4096 104 / 105.
+  if (s2_gathers(*p)) return 5 * items >= (p->stride == 2 || (p->head_dim == 128 && slices < 4) ? 8 : 6) * sms;
   if (items < sms) return false;
   const double slack = bwd_fused_slack(*p, (int)sms);
   if (p->head_dim == 64) {

@@ -48,3 +48,34 @@ def test_which_forward_kernel(H, Sq, Sk, D, mask_kind, score_kind, window, kerne
         call()
     names = [e.key for e in prof.key_averages() if "_sm100_kernel" in e.key]
     assert len(names) == 1 and kernel in names[0], names
+
+
+@pytest.mark.parametrize("H,S,D,window,stride,kernel,fused", [
+    # S2, gathered (", 6>"), against the split kernel's dense form and the separate backward kernels
+    (1, 4096, 64, 64, 2, "fwd_split", False),      # forward 25.4 / 20.3
+    (1, 4096, 64, 512, 3, "fwd_split", False),     # 21.9 / 20.4
+    (1, 4096, 64, 512, 4, ", 6>", False),          # 19.2 / 20.5
+    (1, 5000, 64, 64, 2, ", 6>", False),           # 29.4 / 35.3
+    (3, 8192, 64, 64, 2, ", 6>", False),           # backward 194 / 155
+    (3, 8192, 64, 64, 4, ", 6>", True),
+    (3, 8192, 128, 64, 4, ", 6>", False),          # 174 / 166
+    (4, 8192, 64, 64, 2, ", 6>", True),            # 201 / 223
+    (6, 4096, 128, 64, 4, ", 6>", True),           # 104 / 105
+])
+def test_where_s2_is_gathered(H, S, D, window, stride, kernel, fused):
+    import ctypes
+    import flex_attention_tpu_b200 as fa
+    from flex_attention_tpu_b200 import _binding
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the lines were drawn for 148 SMs")
+    q = torch.zeros(1, H, S, D, device="cuda", dtype=torch.bfloat16)
+    call = lambda: fa.flex_attention(q, q, q, mask_fns=fa.masks.make_s2_mask_fns(128, 128, window, stride))
+    call()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        call()
+        torch.cuda.synchronize()
+    names = [e.key for e in prof.key_averages() if "_sm100_kernel" in e.key]
+    assert len(names) == 1 and kernel in names[0], names
+    p = _binding.FlexAttnParams()
+    p.batch, p.heads, p.seq_q, p.seq_k, p.head_dim, p.window, p.stride, p.mask_kind = 1, H, S, S, D, window, stride, _binding.MASK_S2
+    assert (_binding.lib.flexattn_bwd_scratch_bytes(ctypes.byref(p)) > 0) == fused
