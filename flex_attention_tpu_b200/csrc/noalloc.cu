@@ -6,8 +6,8 @@
 // another allocator, so that any allocation made on their behalf would either fail or be invisible to
 // that planner.  For them the mask map lives in a fixed array inside this library's device image.
 //
-// The array is file-scope `static __device__`: every GPU that loads the library holds
-// kNoAllocScratchBytes of it until the process exits.  Host code may not use the array's name as a
+// The array is file-scope `static __device__`: every GPU that loads the library holds it
+// until the process exits.  Host code may not use the array's name as a
 // pointer (in host code it is only a handle); the device address is looked up once per device with
 // cudaGetSymbolAddress, with that device current, and handed to the kernels like any workspace.
 #include <mutex>
@@ -17,9 +17,9 @@
 namespace flexattn {
 namespace {
 
-constexpr size_t kNoAllocScratchBytes = 1u << 20;  // 1 MiB: mask maps up to e.g. S = 32768 with 32 document rows
-// ... without the order of the pairs of q tiles that lies behind a map (map_layout)
-constexpr size_t kNoAllocPairBytes = 64u << 10;
+// The limit: 1 MiB of mask map, e.g. three document rows of 32768 positions (four need 1.1 MiB).  It does not count the order of the
+// pairs of q tiles that lies behind a map (map_layout), for which there is room besides: at most a 17th of the rest.
+constexpr size_t kNoAllocScratchBytes = 1u << 20, kNoAllocPairBytes = 64u << 10;
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes + kNoAllocPairBytes];
 
 // Device address of the array on the current device; nullptr (and *err set) if it cannot be resolved.

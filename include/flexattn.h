@@ -195,17 +195,19 @@ int flexattn_bwd_fused(void* stream, const FlexAttnParams* p, void* scratch, siz
  * under a memory planner that assigned every buffer before launch, or inside a process whose allocator
  * owns the whole device.  Same inputs and outputs as flexattn_fwd (q, k, v -> o, l, m; doc_ids /
  * alibi_slopes as the mask / score kinds require); `workspace` and `workspace_bytes` are ignored.  The
- * mask map is built, on `stream`, into a fixed array of flexattn_noalloc_scratch_bytes() = 1 MiB that is
- * part of the library's device image (each GPU that loads the library carries it until the process
- * exits), then the forward kernel runs from it.  The entry point itself never calls an allocating or
+ * mask map is built, on `stream`, into a fixed array that is part of the library's device image (1 MiB and
+ * 64 KiB; each GPU that loads the library carries it until the process exits), then the forward kernel runs
+ * from it.  The entry point itself never calls an allocating or
  * freeing routine of the CUDA runtime or of any library.  What the driver does on its own when a device
  * first uses the library (loading the module, which is when the array and the kernels' code take their
  * place in device memory) happens during the first call on that device; after that call, device memory
  * does not change across calls.  Arguments are validated before anything is enqueued, so a refused call
  * leaves the array as it was.
  *
- *  - A problem whose mask map needs more than that (flexattn_workspace_bytes(p) > 1 MiB) is refused with
- *    FLEXATTN_ERR_NOALLOC_LIMIT; use flexattn_fwd with your own workspace instead.
+ *  - A problem whose mask map needs more than flexattn_noalloc_scratch_bytes() = 1 MiB is refused with
+ *    FLEXATTN_ERR_NOALLOC_LIMIT; use flexattn_fwd with your own workspace instead.  Not counted is the work order of the
+ *    pairs of query tiles that ends a map (at most a 17th of it; the 64 KiB are for that): what flexattn_workspace_bytes(p) <= 1 MiB
+ *    holds for is never refused, nor is anything that was served before maps had that part.  In between the call says.
  *  - The first call on each device resolves the array's device address (cudaGetSymbolAddress, with that
  *    device current).  Make that first call outside any stream capture.
  *  - All calls on a device share the one array, which always holds the map of the most recent call.  Calls
@@ -213,7 +215,8 @@ int flexattn_bwd_fused(void* stream, const FlexAttnParams* p, void* scratch, siz
  *    it: serialise them, e.g. by using a single stream. */
 int flexattn_fwd_noalloc(void* stream, const FlexAttnParams* p);
 
-/* Size in bytes of the fixed scratch array behind flexattn_fwd_noalloc.  No counterpart in the reference. */
+/* The largest mask map in bytes, without the order of the pairs of query tiles, that flexattn_fwd_noalloc serves.  No counterpart
+ * in the reference. */
 size_t flexattn_noalloc_scratch_bytes(void);
 
 /* Decodes the mask map in `workspace` for tests and tools: copies entry `index` of the row map

@@ -128,3 +128,34 @@ def test_noalloc_refused_call_leaves_the_array_alone():
     assert B.lib.flexattn_fwd_noalloc(stream, ctypes.byref(p)) == 0
     torch.cuda.synchronize()
     assert torch.equal(o, good)
+
+
+def test_noalloc_serves_a_map_up_to_its_limit():
+    """The longest document row whose map fits (its size counts without the order of the pairs of q tiles, so the workspace the ordinary
+    forward asks for is larger than the limit there), and the next one."""
+    from flex_attention_tpu_b200 import _binding as B
+    limit = B.lib.flexattn_noalloc_scratch_bytes()
+
+    def sizes(S):
+        p = B.FlexAttnParams()
+        p.batch, p.heads, p.seq_q, p.seq_k, p.head_dim, p.mask_kind = 1, 1, S, S, 64, B.MASK_DOCUMENT
+        total = B.lib.flexattn_workspace_bytes(ctypes.byref(p))
+        pairs = (-(-S // 128) + 1) // 2
+        return total, total - (4 * pairs + 255) // 256 * 256
+    lo, hi = 1, 1 << 20          # map sizes grow with S
+    while hi - lo > 1:
+        mid = (lo + hi) // 2
+        lo, hi = (mid, hi) if sizes(mid)[1] <= limit else (lo, mid)
+    assert sizes(lo)[0] > limit and sizes(lo)[1] <= limit < sizes(hi)[1] and hi == lo + 1
+    three, four = (B.FlexAttnParams(), B.FlexAttnParams())
+    for p, rows in ((three, 3), (four, 4)):
+        p.batch, p.heads, p.seq_q, p.seq_k, p.head_dim, p.mask_kind = rows, 1, 32768, 32768, 64, B.MASK_DOCUMENT
+    assert B.lib.flexattn_workspace_bytes(ctypes.byref(three)) <= limit < B.lib.flexattn_workspace_bytes(ctypes.byref(four))
+    g = torch.Generator(device="cuda").manual_seed(4)
+    doc = (torch.arange(hi, device="cuda", dtype=torch.int32) // 300)[None].contiguous()
+    q, k, v = (torch.randn((1, 1, hi, 64), generator=g, device="cuda", dtype=torch.bfloat16) for _ in range(3))
+    a, b = _run_both(B, *(t[:, :, :lo].contiguous() for t in (q, k, v)), mask_kind=B.MASK_DOCUMENT, doc=doc[:, :lo].contiguous())
+    assert all(torch.equal(x, y) for x, y in zip(a, b))
+    o = torch.empty_like(q); l = torch.empty(q.shape[:3], dtype=torch.float32, device="cuda"); m = torch.empty_like(l)
+    p = _params(B, None, q, k, v, o, l, m, mask_kind=B.MASK_DOCUMENT, doc=doc)
+    assert B.lib.flexattn_fwd_noalloc(ctypes.c_void_p(torch.cuda.current_stream().cuda_stream), ctypes.byref(p)) == 11
