@@ -122,7 +122,7 @@ struct DevParams {
 //   strided tiles   tile t holds the keys (128 t + c) * stride, c < 128, fetched as such by TMA (a tensor map whose row pitch is
 //                   `stride` rows); a query i keeps those with (128 t + c) * stride <= i - window
 // A query tile's kv tiles are numbered as ONE range [x, end): from z on they are window tiles (the number is kt), below it strided
-// ones (t = number - x).  Ranges follow from the sizes, so no map is built.  [2,16,4096,64], 512 keys, stride 64: 16.5 tiles a
+// ones (t = number - x).  Ranges follow from the sizes: the gathered kernels read no map.  [2,16,4096,64], 512 keys, stride 64: 16.5 tiles a
 // query tile become 6.
 // ---------------------------------------------------------------------------------------------
 constexpr int kMaskS2Gather = FLEXATTN_MASK_S2 + 1;  // inside the kernels only

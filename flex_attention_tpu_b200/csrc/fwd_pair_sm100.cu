@@ -1,4 +1,4 @@
-// Forward flex attention for long rows, two query tiles per CTA (sm_100a).
+// Forward flex attention, two query tiles at a time (sm_100a).
 //
 // Same math and interface as fwd_pipe_sm100.cu (reference: flex_attention_kernel.py:196-327).  A CTA owns two
 // adjacent 128-row query tiles of one (batch, head) and runs them as two independent online-softmax streams over the

@@ -18,15 +18,10 @@ CHILD = textwrap.dedent("""
     import flex_attention_tpu_b200 as fa
     from flex_attention_tpu_b200 import _binding as B
     from helpers import assert_close, build_mods, make_qkvdo, run_hot_path
-    from torch.profiler import ProfilerActivity, profile
+    from kernel_names import launched_kernels
     assert B.DEBUG_BUILD
 
-    def kernels(fn):
-        fn()
-        with profile(activities=[ProfilerActivity.CUDA]) as prof:
-            fn()
-            torch.cuda.synchronize()
-        return [e.name for e in prof.events() if "sm100_kernel" in e.name]
+    kernels = lambda fn: launched_kernels(fn)[1]
 
     def case(mask, score, Bn, H, Sq, Sk, D, fwd, bwd, user=None, **kw):
         (q, k, v, do), _ = make_qkvdo((Bn, H, Sq, D), (Bn, H, Sk, D), 11, torch.bfloat16)

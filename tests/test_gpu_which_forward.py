@@ -1,17 +1,16 @@
 """Which of the two forward kernels that work through a list of query tiles the library gives a call, on both sides of the lines that
-were drawn from timings with either (148 SMs)."""
-import numpy as np
+were drawn from timings with either (148 SMs), and where S2 is gathered."""
+import ctypes
+
 import pytest
 import torch
-from torch.profiler import ProfilerActivity, profile
 
-import workloads
-from helpers import build_mods
+from kernel_names import forward_kernels
 
 pytestmark = pytest.mark.gpu
 
-
-@pytest.mark.parametrize("H,Sq,Sk,D,mask_kind,score_kind,window,kernel", [
+# heads, queries, keys, head dimension, mask, score function, window, kernel
+CALLS = [
     # pairs that are half empty, in calls of three, five and seven query tiles; two-query-tile / persistent, us
     (192, 384, 384, 64, "causal", "softcap", 0, "fwd_pipe"),                   # 26.0 / 23.4
     (64, 777, 777, 64, "causal", "softcap", 0, "fwd_pipe"),                    # 33 / 30
@@ -30,27 +29,9 @@ pytestmark = pytest.mark.gpu
     (128, 777, 777, 128, "document", "none", 0, "fwd_pipe"),                   # 66 / 62
     (24, 1536, 1536, 64, "document", "none", 0, "fwd_pair"),                   # 36 / 42
     (96, 1024, 1024, 128, "document", "none", 0, "fwd_pair"),                  # 49 / 54
-])
-def test_which_forward_kernel(H, Sq, Sk, D, mask_kind, score_kind, window, kernel):
-    import flex_attention_tpu_b200 as fa
-    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
-        pytest.skip("the lines were drawn for 148 SMs")
-    B = 2 if mask_kind == "document" else 1
-    q, k = (torch.zeros(B, H // B, s, D, device="cuda", dtype=torch.bfloat16) for s in (Sq, Sk))
-    ids = workloads.draw_documents(np.random.default_rng(1), B, Sq, lo=64, hi=1500)[0] if mask_kind == "document" else None
-    mf, bf, sf, seg = build_mods(fa, mask_kind, score_kind, window=window, stride=64, cap=20.0, doc_ids=ids)
-
-    def call():
-        fa._flex_attention_impl(q, k, k, None, seg, False, False, 0.1, 1, 128, 128, 128, False, bf, mf, sf)
-        torch.cuda.synchronize()
-    call()
-    with profile(activities=[ProfilerActivity.CUDA]) as prof:
-        call()
-    names = [e.key for e in prof.key_averages() if "_sm100_kernel" in e.key]
-    assert len(names) == 1 and kernel in names[0], names
-
-
-@pytest.mark.parametrize("H,S,D,window,stride,kernel,fused", [
+]
+# heads, positions, head dimension, window, stride, forward kernel, whether the fused backward serves it
+S2_CALLS = [
     # S2, gathered (", 6>"), against the split kernel's dense form and the separate backward kernels
     (1, 4096, 64, 64, 2, "fwd_split", False),      # forward 25.4 / 20.3
     (1, 4096, 64, 512, 3, "fwd_split", False),     # 21.9 / 20.4
@@ -61,21 +42,30 @@ def test_which_forward_kernel(H, Sq, Sk, D, mask_kind, score_kind, window, kerne
     (3, 8192, 128, 64, 4, ", 6>", False),          # 174 / 166
     (4, 8192, 64, 64, 2, ", 6>", True),            # 201 / 223
     (6, 4096, 128, 64, 4, ", 6>", True),           # 104 / 105
-])
-def test_where_s2_is_gathered(H, S, D, window, stride, kernel, fused):
-    import ctypes
-    import flex_attention_tpu_b200 as fa
-    from flex_attention_tpu_b200 import _binding
+]
+
+
+@pytest.fixture(scope="module")
+def names():
     if torch.cuda.get_device_properties(0).multi_processor_count != 148:
         pytest.skip("the lines were drawn for 148 SMs")
-    q = torch.zeros(1, H, S, D, device="cuda", dtype=torch.bfloat16)
-    call = lambda: fa.flex_attention(q, q, q, mask_fns=fa.masks.make_s2_mask_fns(128, 128, window, stride))
-    call()
-    with profile(activities=[ProfilerActivity.CUDA]) as prof:
-        call()
-        torch.cuda.synchronize()
-    names = [e.key for e in prof.key_averages() if "_sm100_kernel" in e.key]
-    assert len(names) == 1 and kernel in names[0], names
+    calls = [(2 if mask == "document" else 1, H // 2 if mask == "document" else H, Sq, Sk, D, mask, score, window, 64)
+             for H, Sq, Sk, D, mask, score, window, _ in CALLS]
+    calls += [(1, H, S, S, D, "s2", "none", window, stride) for H, S, D, window, stride, _, _ in S2_CALLS]
+    return forward_kernels(calls)
+
+
+@pytest.mark.parametrize("i", range(len(CALLS)), ids=["-".join(map(str, c)) for c in CALLS])
+def test_which_forward_kernel(names, i):
+    assert len(names[i]) == 1 and CALLS[i][-1] in names[i][0], names[i]
+
+
+@pytest.mark.parametrize("i", range(len(S2_CALLS)), ids=["-".join(map(str, c)) for c in S2_CALLS])
+def test_where_s2_is_gathered(names, i):
+    from flex_attention_tpu_b200 import _binding
+    H, S, D, window, stride, kernel, fused = S2_CALLS[i]
+    got = names[len(CALLS) + i]
+    assert len(got) == 1 and kernel in got[0], got
     p = _binding.FlexAttnParams()
     p.batch, p.heads, p.seq_q, p.seq_k, p.head_dim, p.window, p.stride, p.mask_kind = 1, H, S, S, D, window, stride, _binding.MASK_S2
     assert (_binding.lib.flexattn_bwd_scratch_bytes(ctypes.byref(p)) > 0) == fused
