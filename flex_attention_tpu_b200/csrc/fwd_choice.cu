@@ -26,7 +26,9 @@ FwdCosts fwd_costs(const FlexAttnParams& p) {
   switch (p.score_kind) {
     case FLEXATTN_SCORE_NONE: return d64 ? FwdCosts{1.04f, 1.29f, 1.68f, 1.33f, 1.56f} : FwdCosts{1.09f, 1.79f, 1.87f, 1.72f, 2.04f};
     case FLEXATTN_SCORE_ALIBI: return d64 ? FwdCosts{1.15f, 1.78f, 1.83f, 1.07f, 2.38f} : FwdCosts{1.19f, 2.40f, 2.00f, 1.46f, 2.97f};
-    default: return d64 ? FwdCosts{1.53f, 1.42f, 2.90f, 1.85f, 1.77f} : FwdCosts{1.57f, 1.97f, 2.88f, 2.12f, 2.69f};  // softcap, user
+    case FLEXATTN_SCORE_SOFTCAP: return d64 ? FwdCosts{1.53f, 1.42f, 2.90f, 1.85f, 1.77f} : FwdCosts{1.57f, 1.97f, 2.88f, 2.12f, 2.69f};
+    // a user function (a distance penalty, scalar code): 96 x 512 causal, D = 64, 24.1 / 21.3, which the costs of softcap took the other way
+    default: return d64 ? FwdCosts{1.54f, 1.75f, 3.00f, 2.21f, 2.89f} : FwdCosts{1.63f, 2.32f, 3.19f, 2.40f, 3.57f};
   }
 }
 

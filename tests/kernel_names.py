@@ -18,7 +18,8 @@ out = []
 for B, H, Sq, Sk, D, mask, score, window, stride in json.loads(sys.argv[1]):
     q, k = (torch.zeros(B, H, s, D, device="cuda", dtype=torch.bfloat16) for s in (Sq, Sk))
     ids = workloads.draw_documents(np.random.default_rng(1), B, Sq, lo=64, hi=1500)[0] if mask == "document" else None
-    mf, bf, sf, seg = build_mods(fa, mask, score, window=window, stride=stride, cap=20.0, doc_ids=ids)
+    mf, bf, sf, seg = build_mods(fa, mask, score, window=window, stride=stride, cap=20.0, doc_ids=ids,
+                                 user_fn=lambda s, b, h, qi, ki: s - 0.03 * (h + 1) * abs(qi - ki))
     out.append(launched_kernels(lambda: fa._flex_attention_impl(q, k, k, None, seg, False, False, 0.1, 1, 128, 128, 128, False, bf, mf, sf))[1])
 print("NAMES", json.dumps(out))
 """

@@ -18,6 +18,8 @@ CALLS = [
     (8, 4096, 512, 128, "sliding_window_causal", "none", 256, "fwd_pipe"),     # 15.1 / 10.6, query tiles without keys
     (16, 2048, 512, 64, "sliding_window_causal", "none", 256, "fwd_pipe"),     # 13.6 / 9.9
     (16, 3001, 3001, 128, "causal", "none", 0, "fwd_pipe"),
+    (96, 512, 512, 64, "causal", "user", 0, "fwd_pipe"),                       # 24.1 / 21.3
+    (64, 2048, 2048, 64, "causal", "user", 0, "fwd_pair"),
     (32, 2048, 2048, 64, "causal", "none", 0, "fwd_pair"),                     # 36 / 42
     (24, 1024, 1024, 128, "none", "none", 0, "fwd_pair"),                      # 23 / 27
     (96, 1024, 1024, 64, "sliding_window", "none", 1000, "fwd_pair"),          # 49 / 62
