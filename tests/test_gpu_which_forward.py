@@ -9,7 +9,7 @@ from kernel_names import forward_kernels
 
 pytestmark = pytest.mark.gpu
 
-# heads, queries, keys, head dimension, mask, score function, window, kernel
+# slices (batch rows x heads where more than one; documents: two rows), queries, keys, head dimension, mask, score function, window, kernel
 CALLS = [
     # pairs that are half empty, in calls of three, five and seven query tiles; two-query-tile / persistent, us
     (192, 384, 384, 64, "causal", "softcap", 0, "fwd_pipe"),                   # 26.0 / 23.4
@@ -18,6 +18,8 @@ CALLS = [
     (8, 4096, 512, 128, "sliding_window_causal", "none", 256, "fwd_pipe"),     # 15.1 / 10.6, query tiles without keys
     (16, 2048, 512, 64, "sliding_window_causal", "none", 256, "fwd_pipe"),     # 13.6 / 9.9
     (16, 3001, 3001, 128, "causal", "none", 0, "fwd_pipe"),
+    ((3, 24), 1088, 1088, 64, "causal", "softcap", 0, "fwd_pair"),             # 52 / 74: the list begins anew with every row
+    ((1, 72), 1088, 1088, 64, "causal", "softcap", 0, "fwd_pipe"),
     (96, 512, 512, 64, "causal", "user", 0, "fwd_pipe"),                       # 24.1 / 21.3
     (64, 2048, 2048, 64, "causal", "user", 0, "fwd_pair"),
     (32, 2048, 2048, 64, "causal", "none", 0, "fwd_pair"),                     # 36 / 42
@@ -27,6 +29,8 @@ CALLS = [
     # documents
     (96, 384, 384, 64, "document", "none", 0, "fwd_pipe"),                     # 23.9 / 22.5
     (22, 2048, 2048, 64, "document", "none", 0, "fwd_pipe"),                   # 44 / 41
+    ((1, 24), 1472, 1472, 128, "document", "softcap", 0, "fwd_pipe"),          # 55 / 43
+    ((7, 2), 2985, 2985, 64, "document", "none", 0, "fwd_pair"),               # 40 / 45
     (128, 384, 384, 128, "document", "none", 0, "fwd_pipe"),                   # 29.5 / 28.3
     (128, 777, 777, 128, "document", "none", 0, "fwd_pipe"),                   # 66 / 62
     (24, 1536, 1536, 64, "document", "none", 0, "fwd_pair"),                   # 36 / 42
@@ -51,8 +55,8 @@ S2_CALLS = [
 def names():
     if torch.cuda.get_device_properties(0).multi_processor_count != 148:
         pytest.skip("the lines were drawn for 148 SMs")
-    calls = [(2 if mask == "document" else 1, H // 2 if mask == "document" else H, Sq, Sk, D, mask, score, window, 64)
-             for H, Sq, Sk, D, mask, score, window, _ in CALLS]
+    rows = lambda H, mask: H if isinstance(H, tuple) else (2, H // 2) if mask == "document" else (1, H)
+    calls = [(*rows(H, mask), Sq, Sk, D, mask, score, window, 64) for H, Sq, Sk, D, mask, score, window, _ in CALLS]
     calls += [(1, H, S, S, D, "s2", "none", window, stride) for H, S, D, window, stride, _, _ in S2_CALLS]
     return forward_kernels(calls)
 
